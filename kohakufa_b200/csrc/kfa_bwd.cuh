@@ -102,13 +102,21 @@ struct PrepParams {
 };
 
 // ---------------------------------------------------------------------------------------
-// prepare: HBM-bound; D / 8 lanes per row (rounded up to a power of two), 16-byte loads.
+// prepare: HBM-bound; D / 8 lanes per row (rounded up to a power of two), 16-byte loads. A CTA has 128 rows and
+// 256 threads; a warp has all its 16 rows' loads of O and dO in flight together. With 4 warps that went through 32
+// rows each, pass by pass, every pass waited for memory: 5.4 -> 2.3 us at 2 x 4 x 512 rows of D = 64, 9.9 -> 6.3 at
+// 16 x 4096 of D = 128 (both L2 hits), 34.8 -> 32.3 at 32 x 8192 of D = 128 (134 MB: 4.2 of the 6.4 TB/s that a copy
+// reaches); with the zero fill of the fused backward's accumulator 32.6 -> 22.4 us at 64 x 4096 of D = 64.
 // ---------------------------------------------------------------------------------------
+constexpr int PREP_THREADS = 256;
+
 template <int D, bool BF16>
-__global__ void __launch_bounds__(128) kfa_bwd_prepare_kernel(const PrepParams p) {
+__global__ void __launch_bounds__(PREP_THREADS) kfa_bwd_prepare_kernel(const PrepParams p) {
   constexpr int VECS = D / 8;                                                      // 16-byte pieces of a row
   constexpr int LPR = VECS <= 2 ? 2 : (VECS <= 4 ? 4 : (VECS <= 8 ? 8 : 16));      // lanes per row (a power of two)
   constexpr int RPW = 32 / LPR;                                                    // rows per warp pass
+  constexpr int ROWS = 128 / (PREP_THREADS / 32);                                  // rows of a warp
+  constexpr int PASSES = ROWS / RPW;
   const int tile = blockIdx.x;
   const int bh = blockIdx.y;
   const int b = bh / p.H, h = bh % p.H;
@@ -125,37 +133,44 @@ __global__ void __launch_bounds__(128) kfa_bwd_prepare_kernel(const PrepParams p
   const uint8_t* gb = reinterpret_cast<const uint8_t*>(p.dout) + 2 * (bc * p.do_sb + h * p.do_sh + q_base * p.do_ss);
   float* st = p.stats + (static_cast<long long>(bh) * p.n_q128 + tile) * 384;
   const float* lse = p.lse + (static_cast<long long>(bc) * p.H + h) * 2 * p.Sq + q_base;
+  uint4 ov[PASSES], gv[PASSES];
+#pragma unroll
+  for (int i = 0; i < PASSES; ++i) {
+    const int row = tile * 128 + warp * ROWS + i * RPW + sub;
+    ov[i] = gv[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (row < Sq && vec < VECS) {
+      ov[i] = *reinterpret_cast<const uint4*>(ob + 2 * (row * p.o_ss + vec * 8));
+      gv[i] = *reinterpret_cast<const uint4*>(gb + 2 * (row * p.do_ss + vec * 8));
+    }
+  }
+  if (threadIdx.x < 128) {
+    const int row = tile * 128 + threadIdx.x;
+    const bool valid = row < Sq;
+    // stored negated, so the consumers only add; padded rows: -m = -inf makes their P exactly 0
+    st[threadIdx.x] = valid ? -lse[row] : -INFINITY;
+    st[128 + threadIdx.x] = valid ? -lse[p.Sq + row] : 0.f;
+  }
   if (p.dq_acc != nullptr) {
     float4* acc = reinterpret_cast<float4*>(p.dq_acc + (static_cast<long long>(bh) * p.n_q128 + tile) * (128 * D));
 #pragma unroll 4
-    for (int i = threadIdx.x; i < 128 * D / 4; i += 128) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = threadIdx.x; i < 128 * D / 4; i += PREP_THREADS) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  for (int r0 = warp * 32; r0 < warp * 32 + 32; r0 += RPW) {
-    const int r_in = r0 + sub;
-    const int row = tile * 128 + r_in;
-    float acc = 0.f;
-    if (row < Sq && vec < VECS) {
-      const uint4 ov = *reinterpret_cast<const uint4*>(ob + 2 * (row * p.o_ss + vec * 8));
-      const uint4 gv = *reinterpret_cast<const uint4*>(gb + 2 * (row * p.do_ss + vec * 8));
-      const uint32_t ow[4] = {ov.x, ov.y, ov.z, ov.w};
-      const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 a = unpack16<BF16>(ow[i]);
-        const float2 g = unpack16<BF16>(gw[i]);
-        acc = fmaf(a.x, g.x, acc);
-        acc = fmaf(a.y, g.y, acc);
-      }
+  for (int i = 0; i < PASSES; ++i) {
+    const uint32_t ow[4] = {ov[i].x, ov[i].y, ov[i].z, ov[i].w};
+    const uint32_t gw[4] = {gv[i].x, gv[i].y, gv[i].z, gv[i].w};
+    float acc = 0.f;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float2 a = unpack16<BF16>(ow[x]);
+      const float2 g = unpack16<BF16>(gw[x]);
+      acc = fmaf(a.x, g.x, acc);
+      acc = fmaf(a.y, g.y, acc);
     }
 #pragma unroll
     for (int off = LPR / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (vec == 0) {
-      const bool valid = row < Sq;
-      // stored negated, so the consumers only add; padded rows: -m = -inf makes their P exactly 0
-      st[r_in] = valid ? -lse[row] : -INFINITY;
-      st[128 + r_in] = valid ? -lse[p.Sq + row] : 0.f;
-      st[256 + r_in] = valid ? -acc : 0.f;
-    }
+    const int r_in = warp * ROWS + i * RPW + sub;
+    if (vec == 0) st[256 + r_in] = (tile * 128 + r_in < Sq) ? -acc : 0.f;
   }
 }
 
