@@ -159,8 +159,8 @@ typedef struct KfaMaskTiles {
 /* mask: bytes, nonzero = visible, element (b, h, r, c) at mask[b * s[0] + h * s[1] + r * s[2] + c * s[3]]
  * with mask_batch x mask_heads x Sq x Skv elements. words: int32[mask_batch * mask_heads * Sq *
  * 4 ceil(Skv / 128)], words_t: int32[mask_batch * mask_heads * Skv * 4 ceil(Sq / 128)], both contiguous.
- * tiles (optional): int32[mask_batch * mask_heads * ceil(Sq / 128) * ceil(Skv / 128)], ZEROED by the
- * caller; the kernel sets the entries of tiles that hold a visible pair. */
+ * tiles (optional): int32[mask_batch * mask_heads * ceil(Sq / 128) * ceil(Skv / 128)], written in full:
+ * 1 for the tiles that hold a visible pair, else 0. */
 int kfa_pack_mask(const void* mask, const int64_t* mask_stride, int mask_batch, int mask_heads, int Sq,
                   int Skv, int32_t* words, int32_t* words_t, int32_t* tiles, void* stream);
 int kfa_fwd_masked(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out,

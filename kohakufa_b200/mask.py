@@ -44,7 +44,7 @@ def pack_mask_op(mask: Tensor, s_q: int, s_kv: int) -> tuple[Tensor, Tensor, Ten
     dev = mask_bytes.device
     words = torch.empty(bm, hm, s_q, words_per_row(s_kv), dtype=torch.int32, device=dev)
     words_t = torch.empty(bm, hm, s_kv, words_per_row(s_q), dtype=torch.int32, device=dev)
-    tiles = torch.zeros(bm, hm, -(-s_q // TILE), -(-s_kv // TILE), dtype=torch.int32, device=dev)
+    tiles = torch.empty(bm, hm, -(-s_q // TILE), -(-s_kv // TILE), dtype=torch.int32, device=dev)
     lib = _lib.load()
     strides = (ctypes.c_int64 * 4)(*mask_bytes.stride())
     with torch.cuda.device(dev):
