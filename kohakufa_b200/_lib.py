@@ -152,6 +152,35 @@ def load() -> ctypes.CDLL:
     return _lib
 
 
+# Entry points the host extension calls (a subset of SYMBOLS, in no particular order).
+HOST_SYMBOLS = (
+    "kfa_last_error", "kfa_fwd", "kfa_bwd", "kfa_bwd_fused", "kfa_fwd_masked", "kfa_bwd_masked", "kfa_fwd_varlen",
+    "kfa_bwd_varlen", "kfa_pack_mask",
+)  # fmt: skip
+HOST_PATH = Path(__file__).resolve().parent / "_kfa_host.so"
+_host = None
+
+
+def host():
+    """The C++ launch path (``csrc/kfa_host.cpp``), bound to the loaded library; raises if it has not been built."""
+    global _host
+    if _host is not None:
+        return _host
+    lib = load()
+    with _lock:
+        if _host is None:
+            if not HOST_PATH.exists():
+                raise KfaError(
+                    f"{HOST_PATH} is missing: build it with `python -m kohakufa_b200.build` "
+                    "(needs a C++ compiler; there is no fallback path)"
+                )
+            from kohakufa_b200 import _kfa_host
+
+            _kfa_host.bind(KfaError, {n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in HOST_SYMBOLS})
+            _host = _kfa_host
+    return _host
+
+
 def check(rc: int) -> None:
     if rc != 0:
         raise KfaError(f"libkfa error {rc}: {load().kfa_last_error().decode()}")
@@ -252,3 +281,21 @@ def selftest() -> str:
     if rc != 0:
         raise KfaError(f"kfa_selftest failed ({rc}): {load().kfa_last_error().decode()}\n{report}")
     return report
+
+
+def plain_eager(*tensors: torch.Tensor) -> bool:
+    """Whether a call on these tensors is plain eager execution: no compiler or tracer, no dispatch or function
+    mode, no ``torch.func`` transform, no forward-mode level, no tensor subclass. Only then may it pass the
+    dispatcher by; everything else sees the registered custom ops."""
+    if torch.compiler.is_compiling():
+        return False
+    for t in tensors:
+        if type(t) is not torch.Tensor:
+            return False
+    return not (
+        torch._C._len_torch_dispatch_stack()
+        or torch._C._len_torch_function_stack()
+        or torch._C._are_functorch_transforms_active()
+        or torch.autograd.forward_ad._current_level >= 0
+        or torch._C._get_tracing_state() is not None
+    )

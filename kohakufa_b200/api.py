@@ -109,7 +109,9 @@ def attention(
     if mask is not None and frame:
         raise ValueError("give a mask or causal / block_causal, not both (fold them in)")
     softmax_scale = head_dim**-0.5 if scale is None else scale
-    out = _op.attention(q, k, v, softmax_scale, frame, mask)[..., :head_dim]
+    out = _op.attention(q, k, v, softmax_scale, frame, mask)
+    if out.shape[-1] != head_dim:
+        out = out[..., :head_dim]
     return out.to(result_dtype) if out.dtype != result_dtype else out
 
 
@@ -150,4 +152,4 @@ def attention_varlen(
         block_causal=frame,
         plan=plan,
     )
-    return out[..., :head_dim]
+    return out if out.shape[-1] == head_dim else out[..., :head_dim]

@@ -1,0 +1,327 @@
+// The launch path of a call, in C++: argument checks, output and scratch allocation, tensor descriptors and the
+// libkfa call itself, for the torch ops of op.py and mask.py. In Python (a dozen ctypes structures, half a dozen
+// allocations, the dispatch of a Python custom op) a small problem's call took several times its kernels: a forward
+// of 1 x 8 heads x 64 rows 67 us, now 15; forward + backward of 2 x 4 heads x 512 rows 286 us, now 122, of which
+// about 50 are the autograd engine's own; with a boolean mask of 2048 x 2048 395 us, now 139.
+//
+// A plain CPython extension module (`_kfa_host`). It holds no state but the addresses of the libkfa entry points
+// it was given (`bind`): which library is loaded, and every policy (status word, backward mode), stays in Python.
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/Exceptions.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include "../../include/kfa.h"
+
+namespace {
+
+struct Api {
+  decltype(&kfa_last_error) last_error = nullptr;
+  decltype(&kfa_fwd) fwd = nullptr;
+  decltype(&kfa_bwd) bwd = nullptr;
+  decltype(&kfa_bwd_fused) bwd_fused = nullptr;
+  decltype(&kfa_fwd_masked) fwd_masked = nullptr;
+  decltype(&kfa_bwd_masked) bwd_masked = nullptr;
+  decltype(&kfa_fwd_varlen) fwd_varlen = nullptr;
+  decltype(&kfa_bwd_varlen) bwd_varlen = nullptr;
+  decltype(&kfa_pack_mask) pack_mask = nullptr;
+} api;
+
+PyObject* g_error = nullptr;  // kohakufa_b200._lib.KfaError
+
+struct PyError {};  // a Python exception is set
+
+const at::Tensor& tensor(PyObject* o) {
+  if (!THPVariable_Check(o)) {
+    PyErr_SetString(PyExc_TypeError, "expected a tensor");
+    throw PyError();
+  }
+  return THPVariable_Unpack(o);
+}
+double number(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw PyError();
+  return v;
+}
+int64_t integer(PyObject* o) {
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) throw PyError();
+  return v;
+}
+
+void check(int rc) {
+  if (rc == 0) return;
+  PyErr_Format(g_error ? g_error : PyExc_RuntimeError, "libkfa error %d: %s", rc, api.last_error());
+  throw PyError();
+}
+
+KfaTensor4 desc(const at::Tensor& t) {
+  TORCH_CHECK(t.dim() == 4 && t.is_cuda(), "a 4-D CUDA tensor");
+  KfaTensor4 d;
+  d.ptr = t.data_ptr();
+  for (int i = 0; i < 4; ++i) {
+    d.shape[i] = t.size(i);
+    d.stride[i] = t.stride(i);
+  }
+  return d;
+}
+// [T, H, D] packed rows as the [1, H, T, D] view the library takes
+KfaTensor4 desc_packed(const at::Tensor& t) {
+  TORCH_CHECK(t.dim() == 3 && t.is_cuda(), "a 3-D CUDA tensor");
+  KfaTensor4 d;
+  d.ptr = t.data_ptr();
+  const int64_t shape[4] = {1, t.size(1), t.size(0), t.size(2)};
+  const int64_t stride[4] = {t.size(0) * t.stride(0), t.stride(1), t.stride(0), t.stride(2)};
+  for (int i = 0; i < 4; ++i) {
+    d.shape[i] = shape[i];
+    d.stride[i] = stride[i];
+  }
+  return d;
+}
+
+int dtype_code(const at::Tensor& t) {
+  if (t.scalar_type() == at::kHalf) return KFA_F16;
+  if (t.scalar_type() == at::kBFloat16) return KFA_BF16;
+  TORCH_CHECK_TYPE(false, "libkfa: fp16 or bf16");
+}
+
+// [B, H, S, D] view of fresh [B, S, H, D] storage
+at::Tensor bshd_like(const at::Tensor& t) {
+  return at::empty({t.size(0), t.size(2), t.size(1), t.size(3)}, t.options()).transpose(1, 2);
+}
+at::Tensor floats(const at::Tensor& like, at::IntArrayRef shape) {
+  return at::empty(shape, like.options().dtype(at::kFloat));
+}
+at::Tensor stats_scratch(const at::Tensor& like, int64_t batch, int64_t heads, int64_t seq) {
+  return floats(like, {batch * heads * ((seq + 127) / 128) * 384});
+}
+void* stream_of(const at::Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+bool strides_ok(const at::Tensor& t) {
+  const int64_t n = t.dim();
+  if (t.stride(n - 1) != 1) return false;
+  for (int64_t i = 0; i + 1 < n; ++i)
+    if (t.size(i) > 1 && (t.stride(i) <= 0 || t.stride(i) % 8 != 0)) return false;
+  return true;
+}
+
+// Whether q, k, v are what the kernels take (the conditions of op.py's _check, which raises for the rest).
+bool inputs_ok(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, int64_t dims) {
+  if (q.dim() != dims || k.dim() != dims || v.dim() != dims) return false;
+  if ((q.scalar_type() != at::kHalf && q.scalar_type() != at::kBFloat16) || k.scalar_type() != q.scalar_type() ||
+      v.scalar_type() != q.scalar_type())
+    return false;
+  if (!q.is_cuda() || k.device() != q.device() || v.device() != q.device()) return false;
+  if (q.layout() != at::kStrided || k.layout() != at::kStrided || v.layout() != at::kStrided) return false;
+  const int64_t d = q.size(-1), heads = q.size(1), kv_heads = k.size(1);
+  if (d < 16 || d > 128 || d % 16 || k.size(-1) != d) return false;
+  if (k.sizes() != v.sizes() || (dims == 4 && k.size(0) != q.size(0))) return false;
+  if (q.numel() == 0 || k.numel() == 0 || kv_heads == 0 || heads % kv_heads) return false;
+  return strides_ok(q) && strides_ok(k) && strides_ok(v);
+}
+
+KfaMaskWords mask_words(const at::Tensor& w) {
+  TORCH_CHECK(w.dim() == 4 && w.scalar_type() == at::kInt && w.stride(3) == 1, "packed mask words");
+  return {w.data_ptr<int32_t>(), w.size(0) > 1 ? w.stride(0) : 0, w.size(1) > 1 ? w.stride(1) : 0, w.stride(2)};
+}
+KfaMaskTiles mask_tiles(const at::Tensor& t) {
+  TORCH_CHECK(t.dim() == 4 && t.scalar_type() == at::kInt && t.is_contiguous(), "mask tile table");
+  return {t.data_ptr<int32_t>(), t.size(0) > 1 ? t.stride(0) : 0, t.size(1) > 1 ? t.stride(1) : 0};
+}
+
+template <typename... T>
+PyObject* pack(T&&... ts) {
+  PyObject* items[] = {THPVariable_Wrap(std::move(ts))...};
+  PyObject* tuple = PyTuple_New(sizeof...(ts));
+  for (size_t i = 0; i < sizeof...(ts); ++i) PyTuple_SET_ITEM(tuple, i, items[i]);
+  return tuple;
+}
+
+void need(Py_ssize_t got, Py_ssize_t want) {
+  if (got != want) {
+    PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", want, got);
+    throw PyError();
+  }
+}
+
+using Args = PyObject* const*;
+
+// inputs_ok(q, k, v) -> bool
+PyObject* py_inputs_ok(Args a, Py_ssize_t n) {
+  need(n, 3);
+  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]);
+  return PyBool_FromLong(inputs_ok(q, k, v, q.dim() == 3 ? 3 : 4));
+}
+
+// forward(q, k, v, scale, block, status) -> out, lse
+PyObject* py_forward(Args a, Py_ssize_t n) {
+  need(n, 6);
+  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]);
+  const c10::cuda::CUDAGuard guard(q.device());
+  at::Tensor out = bshd_like(q);
+  at::Tensor lse = floats(q, {q.size(0), q.size(1), 2, q.size(2)});
+  const KfaTensor4 dq = desc(q), dk = desc(k), dv = desc(v), dout = desc(out);
+  check(api.fwd(&dq, &dk, &dv, &dout, lse.data_ptr<float>(), static_cast<float>(number(a[3])),
+                static_cast<int>(integer(a[4])), dtype_code(q), tensor(a[5]).data_ptr<int32_t>(), stream_of(q)));
+  return pack(out, lse);
+}
+
+// backward(q, k, v, out, dout, lse, scale, block, status, fused) -> dq, dk, dv
+PyObject* py_backward(Args a, Py_ssize_t n) {
+  need(n, 10);
+  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]), &o = tensor(a[3]), &g = tensor(a[4]), &lse = tensor(a[5]);
+  const float scale = static_cast<float>(number(a[6]));
+  const int block = static_cast<int>(integer(a[7]));
+  int* status = tensor(a[8]).data_ptr<int32_t>();
+  const bool fused = PyObject_IsTrue(a[9]) == 1;
+  const c10::cuda::CUDAGuard guard(q.device());
+  at::Tensor dq = bshd_like(q), dk = bshd_like(k), dv = bshd_like(v);
+  at::Tensor stats = stats_scratch(q, q.size(0), q.size(1), q.size(2));
+  const KfaTensor4 d[8] = {desc(q), desc(k), desc(v), desc(o), desc(g), desc(dq), desc(dk), desc(dv)};
+  if (fused) {
+    at::Tensor acc = floats(q, {q.size(0) * q.size(1) * ((q.size(2) + 127) / 128) * 128 * q.size(3)});
+    check(api.bwd_fused(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), acc.data_ptr<float>(),
+                        d + 5, d + 6, d + 7, scale, block, dtype_code(q), status, stream_of(q)));
+  } else {
+    check(api.bwd(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), d + 5, d + 6, d + 7, scale,
+                  block, dtype_code(q), status, stream_of(q)));
+  }
+  return pack(dq, dk, dv);
+}
+
+// forward_masked(q, k, v, words, tiles, scale, status) -> out, lse
+PyObject* py_forward_masked(Args a, Py_ssize_t n) {
+  need(n, 7);
+  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]);
+  const c10::cuda::CUDAGuard guard(q.device());
+  at::Tensor out = bshd_like(q);
+  at::Tensor lse = floats(q, {q.size(0), q.size(1), 2, q.size(2)});
+  const KfaTensor4 dq = desc(q), dk = desc(k), dv = desc(v), dout = desc(out);
+  const KfaMaskWords w = mask_words(tensor(a[3]));
+  const KfaMaskTiles t = mask_tiles(tensor(a[4]));
+  check(api.fwd_masked(&dq, &dk, &dv, &dout, lse.data_ptr<float>(), &w, &t, static_cast<float>(number(a[5])), dtype_code(q),
+                       tensor(a[6]).data_ptr<int32_t>(), stream_of(q)));
+  return pack(out, lse);
+}
+
+// backward_masked(q, k, v, out, dout, lse, words, words_t, tiles, scale, status) -> dq, dk, dv
+PyObject* py_backward_masked(Args a, Py_ssize_t n) {
+  need(n, 11);
+  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]), &o = tensor(a[3]), &g = tensor(a[4]), &lse = tensor(a[5]);
+  const c10::cuda::CUDAGuard guard(q.device());
+  at::Tensor dq = bshd_like(q), dk = bshd_like(k), dv = bshd_like(v);
+  at::Tensor stats = stats_scratch(q, q.size(0), q.size(1), q.size(2));
+  const KfaTensor4 d[8] = {desc(q), desc(k), desc(v), desc(o), desc(g), desc(dq), desc(dk), desc(dv)};
+  const KfaMaskWords w = mask_words(tensor(a[6])), wt = mask_words(tensor(a[7]));
+  const KfaMaskTiles t = mask_tiles(tensor(a[8]));
+  check(api.bwd_masked(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), d + 5, d + 6, d + 7, &w,
+                       &wt, &t, static_cast<float>(number(a[9])), dtype_code(q), tensor(a[10]).data_ptr<int32_t>(),
+                       stream_of(q)));
+  return pack(dq, dk, dv);
+}
+
+// forward_varlen(q, k, v, cu_q, cu_k, max_q, max_k, scale, block, status) -> out, lse
+PyObject* py_forward_varlen(Args a, Py_ssize_t n) {
+  need(n, 10);
+  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]), &cu_q = tensor(a[3]), &cu_k = tensor(a[4]);
+  const c10::cuda::CUDAGuard guard(q.device());
+  // zero-filled: rows no CTA writes (a sequence with queries but no keys, rows outside cu_seqlens) read as "no
+  // visible key": output 0, statistics 0
+  at::Tensor out = at::zeros_like(q);
+  at::Tensor lse = at::zeros({1, q.size(1), 2, q.size(0)}, q.options().dtype(at::kFloat));
+  const KfaTensor4 dq = desc_packed(q), dk = desc_packed(k), dv = desc_packed(v), dout = desc_packed(out);
+  check(api.fwd_varlen(&dq, &dk, &dv, &dout, lse.data_ptr<float>(), cu_q.data_ptr<int32_t>(), cu_k.data_ptr<int32_t>(),
+                       static_cast<int>(cu_q.numel() - 1), static_cast<int>(integer(a[5])), static_cast<int>(integer(a[6])),
+                       static_cast<float>(number(a[7])), static_cast<int>(integer(a[8])), dtype_code(q),
+                       tensor(a[9]).data_ptr<int32_t>(), stream_of(q)));
+  return pack(out, lse);
+}
+
+// backward_varlen(q, k, v, out, dout, lse, cu_q, cu_k, max_q, max_k, scale, block, status) -> dq, dk, dv
+PyObject* py_backward_varlen(Args a, Py_ssize_t n) {
+  need(n, 13);
+  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]), &o = tensor(a[3]), &g = tensor(a[4]), &lse = tensor(a[5]),
+                   &cu_q = tensor(a[6]), &cu_k = tensor(a[7]);
+  const int64_t n_seqs = cu_q.numel() - 1, max_q = integer(a[8]), max_k = integer(a[9]);
+  const c10::cuda::CUDAGuard guard(q.device());
+  at::Tensor dq = at::zeros_like(q), dk = at::zeros_like(k), dv = at::zeros_like(v);  // unwritten rows: zero gradient
+  at::Tensor stats = stats_scratch(q, n_seqs, q.size(1), max_q);
+  const KfaTensor4 d[8] = {desc_packed(q), desc_packed(k), desc_packed(v),  desc_packed(o),
+                           desc_packed(g), desc_packed(dq), desc_packed(dk), desc_packed(dv)};
+  check(api.bwd_varlen(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), d + 5, d + 6, d + 7,
+                       cu_q.data_ptr<int32_t>(), cu_k.data_ptr<int32_t>(), static_cast<int>(n_seqs), static_cast<int>(max_q),
+                       static_cast<int>(max_k), static_cast<float>(number(a[10])), static_cast<int>(integer(a[11])),
+                       dtype_code(q), tensor(a[12]).data_ptr<int32_t>(), stream_of(q)));
+  return pack(dq, dk, dv);
+}
+
+// pack_mask(mask [Bm, Hm, Sq, Skv] bool or bytes, any strides, s_q, s_kv) -> words, words_t, tiles
+PyObject* py_pack_mask(Args a, Py_ssize_t n) {
+  need(n, 3);
+  const at::Tensor& m = tensor(a[0]);
+  const int64_t s_q = integer(a[1]), s_kv = integer(a[2]);
+  TORCH_CHECK(m.dim() == 4 && m.is_cuda() && m.element_size() == 1, "a 4-D mask of bytes on the GPU");
+  const c10::cuda::CUDAGuard guard(m.device());
+  const int64_t bm = m.size(0), hm = m.size(1), tq = (s_q + 127) / 128, tk = (s_kv + 127) / 128;
+  const auto ints = m.options().dtype(at::kInt);
+  at::Tensor words = at::empty({bm, hm, s_q, 4 * tk}, ints);
+  at::Tensor words_t = at::empty({bm, hm, s_kv, 4 * tq}, ints);
+  at::Tensor tiles = at::empty({bm, hm, tq, tk}, ints);
+  const int64_t strides[4] = {m.stride(0), m.stride(1), m.stride(2), m.stride(3)};
+  check(api.pack_mask(m.data_ptr(), strides, static_cast<int>(bm), static_cast<int>(hm), static_cast<int>(s_q),
+                      static_cast<int>(s_kv), words.data_ptr<int32_t>(), words_t.data_ptr<int32_t>(),
+                      tiles.data_ptr<int32_t>(), stream_of(m)));
+  return pack(words, words_t, tiles);
+}
+
+// bind(KfaError, {entry point: address})
+PyObject* py_bind(Args a, Py_ssize_t n) {
+  need(n, 2);
+  auto take = [&](const char* name, auto& slot) {
+    PyObject* v = PyDict_GetItemString(a[1], name);
+    if (!v) {
+      PyErr_Format(PyExc_KeyError, "%s", name);
+      throw PyError();
+    }
+    slot = reinterpret_cast<std::remove_reference_t<decltype(slot)>>(static_cast<uintptr_t>(integer(v)));
+  };
+  take("kfa_last_error", api.last_error);
+  take("kfa_fwd", api.fwd);
+  take("kfa_bwd", api.bwd);
+  take("kfa_bwd_fused", api.bwd_fused);
+  take("kfa_fwd_masked", api.fwd_masked);
+  take("kfa_bwd_masked", api.bwd_masked);
+  take("kfa_fwd_varlen", api.fwd_varlen);
+  take("kfa_bwd_varlen", api.bwd_varlen);
+  take("kfa_pack_mask", api.pack_mask);
+  Py_INCREF(a[0]);
+  Py_XDECREF(g_error);
+  g_error = a[0];
+  Py_RETURN_NONE;
+}
+
+// C++ exceptions end here: torch's become the Python exceptions they stand for.
+template <PyObject* (*F)(Args, Py_ssize_t)>
+PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  try {
+    return F(args, n);
+  } catch (const PyError&) {
+    return nullptr;
+  }
+  END_HANDLE_TH_ERRORS
+}
+
+#define KFA_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(entry<py_##name>)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {
+    KFA_METHOD(bind),           KFA_METHOD(inputs_ok),       KFA_METHOD(forward),        KFA_METHOD(backward),
+    KFA_METHOD(forward_masked), KFA_METHOD(backward_masked), KFA_METHOD(forward_varlen), KFA_METHOD(backward_varlen),
+    KFA_METHOD(pack_mask),      {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_kfa_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__kfa_host(void) { return PyModule_Create(&module_def); }

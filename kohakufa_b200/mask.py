@@ -9,8 +9,6 @@ instead of a Triton kernel. In place of the reference's tile classes and host-bu
 the tile holds a visible pair; the kernels list the tiles they visit from it and skip the rest.
 """
 
-import ctypes
-
 import torch
 from torch import Tensor
 
@@ -39,21 +37,7 @@ def words_per_row(n: int) -> int:
 @torch.library.custom_op("kohakufa_b200::pack_mask", mutates_args=(), device_types="cuda")
 def pack_mask_op(mask: Tensor, s_q: int, s_kv: int) -> tuple[Tensor, Tensor, Tensor]:
     """words, words_t, tiles of a ``[Bm, Hm, Sq, Skv]`` bool mask (True = visible), any strides."""
-    mask_bytes = mask.view(torch.uint8)
-    bm, hm = mask_bytes.shape[:2]
-    dev = mask_bytes.device
-    words = torch.empty(bm, hm, s_q, words_per_row(s_kv), dtype=torch.int32, device=dev)
-    words_t = torch.empty(bm, hm, s_kv, words_per_row(s_q), dtype=torch.int32, device=dev)
-    tiles = torch.empty(bm, hm, -(-s_q // TILE), -(-s_kv // TILE), dtype=torch.int32, device=dev)
-    lib = _lib.load()
-    strides = (ctypes.c_int64 * 4)(*mask_bytes.stride())
-    with torch.cuda.device(dev):
-        rc = lib.kfa_pack_mask(
-            mask_bytes.data_ptr(), strides, bm, hm, s_q, s_kv, words.data_ptr(), words_t.data_ptr(),
-            tiles.data_ptr(), _lib.stream_ptr(dev),
-        )  # fmt: skip
-    _lib.check(rc)
-    return words, words_t, tiles
+    return _lib.host().pack_mask(mask, s_q, s_kv)
 
 
 @pack_mask_op.register_fake
@@ -73,7 +57,8 @@ class PackedMask:
         if not dense.is_cuda:
             raise ValueError("mask: a CUDA tensor (there is no CPU path)")
         self.shape = (batch, heads, s_q, s_kv)
-        self.words, self.words_t, self.tiles = pack_mask_op(dense, s_q, s_kv)
+        pack = _lib.host().pack_mask if _lib.plain_eager(dense) else pack_mask_op
+        self.words, self.words_t, self.tiles = pack(dense, s_q, s_kv)
 
 
 def pack_mask(mask: Tensor, batch: int, heads: int, s_q: int, s_kv: int) -> PackedMask:
@@ -81,23 +66,3 @@ def pack_mask(mask: Tensor, batch: int, heads: int, s_q: int, s_kv: int) -> Pack
     as ``attention(..., mask=packed)``."""
     return PackedMask(mask, batch, heads, s_q, s_kv)
 
-
-def mask_words(words: Tensor, batch: int, heads: int) -> "_lib.KfaMaskWords":
-    """The library's descriptor of ``words [Bm, Hm, rows, row_words]`` (size-1 dimensions broadcast)."""
-    assert words.dtype == torch.int32 and words.dim() == 4 and words.stride(3) == 1
-    d = _lib.KfaMaskWords()
-    d.words = words.data_ptr()
-    d.stride_batch = words.stride(0) if words.shape[0] > 1 else 0
-    d.stride_head = words.stride(1) if words.shape[1] > 1 else 0
-    d.stride_row = words.stride(2)
-    return d
-
-
-def mask_tiles(tiles: Tensor) -> "_lib.KfaMaskTiles":
-    """The library's descriptor of the tile table ``[Bm, Hm, ceil(Sq / 128), ceil(Skv / 128)]``."""
-    assert tiles.dtype == torch.int32 and tiles.dim() == 4 and tiles.is_contiguous()
-    d = _lib.KfaMaskTiles()
-    d.any = tiles.data_ptr()
-    d.stride_batch = tiles.stride(0) if tiles.shape[0] > 1 else 0
-    d.stride_head = tiles.stride(1) if tiles.shape[1] > 1 else 0
-    return d

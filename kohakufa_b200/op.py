@@ -10,22 +10,27 @@ Mirrors the operator boundary of the reference (KohakuFA ``src/kohakufa/sm100/op
 
 The ops live in their own namespace (``kohakufa_b200::sm100_forward`` / ``_backward``; the
 reference registers ``kohakufa::sm100_*``), so both packages can be imported side by side.
-Their bodies call ``libkfa.so`` through ctypes on the current stream: no host synchronisation,
-every buffer from the caching allocator, so ``torch.compile`` keeps them in the graph and CUDA
-graph capture works (after one eager call on the device, which creates the status word).
+Their bodies call ``libkfa.so`` through the C++ launch path (``csrc/kfa_host.cpp``) on the current stream: no host
+synchronisation, every buffer from the caching allocator, so ``torch.compile`` keeps them in the graph and
+CUDA graph capture works (after one eager call on the device, which creates the status word).
+
+``attention`` and ``attention_varlen`` enter that launch path directly when nothing but plain eager execution
+is going on (``_lib.plain_eager``), through a ``torch.autograd.Function`` of their own where gradients are needed: the
+dispatch of a Python custom op costs more than a small problem's kernels. Under ``torch.compile``,
+dispatch or function modes, ``torch.func`` transforms, forward-mode differentiation, tracing or with tensor
+subclasses, and in a backward that is itself recorded, the custom ops run as they always have.
 
 Extra memory: forward statistics (row max and log2 sum, fp32 [B, H, 2, Sq]); backward
 (m, log2 l, delta) per query row (fp32, padded to 128 rows) while it runs.
 """
 
-import ctypes
+import os
 
 import torch
 from torch import Tensor
+from torch.autograd import Function
 
 from kohakufa_b200 import _lib
-
-import os
 
 KERNEL_DIMS = tuple(range(16, 129, 16))  # head dims the kernels are built for (the reference's multiples of 16: api.py:18-29); the API zero-pads up to one
 FUSED_DIMS = (64, 128)  # ... and those the fused backward is built for
@@ -112,6 +117,11 @@ def _check(q: Tensor, k: Tensor, v: Tensor) -> None:
             raise ValueError("attention: inputs need a contiguous last dim and 16-byte strides")
 
 
+def _records(q: Tensor, k: Tensor, v: Tensor) -> bool:
+    """Whether autograd records this call."""
+    return torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
+
+
 def _bshd_like(t: Tensor) -> Tensor:
     batch, heads, seq, dim = t.shape
     return t.new_empty(batch, seq, heads, dim).transpose(1, 2)
@@ -119,25 +129,7 @@ def _bshd_like(t: Tensor) -> Tensor:
 
 @torch.library.custom_op("kohakufa_b200::sm100_forward", mutates_args=(), device_types="cuda")
 def attention_fwd_op(q: Tensor, k: Tensor, v: Tensor, scale: float, block: int) -> tuple[Tensor, Tensor]:
-    lib = _lib.load()
-    batch, heads, seq_q, _ = q.shape
-    out = _bshd_like(q)
-    lse = q.new_empty(batch, heads, 2, seq_q, dtype=torch.float32)
-    with torch.cuda.device(q.device):
-        rc = lib.kfa_fwd(
-            ctypes.byref(_lib.tensor4(q)),
-            ctypes.byref(_lib.tensor4(k)),
-            ctypes.byref(_lib.tensor4(v)),
-            ctypes.byref(_lib.tensor4(out)),
-            lse.data_ptr(),
-            float(scale),
-            int(block),
-            _lib.dtype_code(q.dtype),
-            _lib.status_word(q.device).data_ptr(),
-            _lib.stream_ptr(q.device),
-        )
-    _lib.check(rc)
-    return out, lse
+    return _lib.host().forward(q, k, v, scale, block, _lib.status_word(q.device))
 
 
 @attention_fwd_op.register_fake
@@ -152,28 +144,8 @@ def _(q, k, v, scale, block):
 def attention_bwd_op(
     q: Tensor, k: Tensor, v: Tensor, out: Tensor, dout: Tensor, lse: Tensor, scale: float, block: int
 ) -> tuple[Tensor, Tensor, Tensor]:
-    lib = _lib.load()
-    batch, heads, seq_q, dim = q.shape
-    dq, dk, dv = _bshd_like(q), _bshd_like(k), _bshd_like(v)
-    stats = q.new_empty(lib.kfa_bwd_stats_bytes(batch, heads, seq_q) // 4, dtype=torch.float32)
-    tensors = [ctypes.byref(_lib.tensor4(t)) for t in (q, k, v, out, dout, dq, dk, dv)]
-    tail = (
-        float(scale),
-        int(block),
-        _lib.dtype_code(q.dtype),
-        _lib.status_word(q.device).data_ptr(),
-        _lib.stream_ptr(q.device),
-    )
-    with torch.cuda.device(q.device):
-        if not use_fused_backward(dim, batch * heads):
-            rc = lib.kfa_bwd(*tensors[:5], lse.data_ptr(), stats.data_ptr(), *tensors[5:], *tail)
-        else:
-            dq_acc = q.new_empty(lib.kfa_bwd_dq_acc_bytes(batch, heads, seq_q, dim) // 4, dtype=torch.float32)
-            rc = lib.kfa_bwd_fused(
-                *tensors[:5], lse.data_ptr(), stats.data_ptr(), dq_acc.data_ptr(), *tensors[5:], *tail
-            )
-    _lib.check(rc)
-    return dq, dk, dv
+    fused = use_fused_backward(q.shape[-1], q.shape[0] * q.shape[1])
+    return _lib.host().backward(q, k, v, out, dout, lse, scale, block, _lib.status_word(q.device), fused)
 
 
 @attention_bwd_op.register_fake
@@ -201,6 +173,29 @@ def _backward(ctx, dout, dlse):
 attention_fwd_op.register_autograd(_backward, setup_context=_setup_context)
 
 
+class _Attention(Function):
+    """``attention_fwd_op`` with its gradient, for plain eager calls."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, scale, block):
+        out, lse = _lib.host().forward(q, k, v, scale, block, _lib.status_word(q.device))
+        ctx.save_for_backward(q, k, v, out, lse)
+        ctx.scale, ctx.block = scale, block
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        q, k, v, out, lse = ctx.saved_tensors
+        if not _strides_ok(dout):
+            dout = dout.contiguous()
+        if torch.is_grad_enabled() or not _lib.plain_eager(q, k, v, out, dout, lse):
+            grads = attention_bwd_op(q, k, v, out, dout, lse, ctx.scale, ctx.block)
+        else:
+            fused = use_fused_backward(q.shape[-1], q.shape[0] * q.shape[1])
+            grads = _lib.host().backward(q, k, v, out, dout, lse, ctx.scale, ctx.block, _lib.status_word(q.device), fused)
+        return *grads, None, None
+
+
 # --------------------------------------------------------------------------------------
 # Boolean masks: ops of their own (the reference passes optional word tensors to its one op pair,
 # op.py:58-121); the packed words are saved for the backward.
@@ -211,25 +206,7 @@ attention_fwd_op.register_autograd(_backward, setup_context=_setup_context)
 def masked_fwd_op(
     q: Tensor, k: Tensor, v: Tensor, words: Tensor, words_t: Tensor, tiles: Tensor, scale: float
 ) -> tuple[Tensor, Tensor]:
-    from kohakufa_b200.mask import mask_tiles, mask_words
-
-    lib = _lib.load()
-    batch, heads, seq_q, _ = q.shape
-    out = _bshd_like(q)
-    lse = q.new_empty(batch, heads, 2, seq_q, dtype=torch.float32)
-    with torch.cuda.device(q.device):
-        rc = lib.kfa_fwd_masked(
-            *(ctypes.byref(_lib.tensor4(t)) for t in (q, k, v, out)),
-            lse.data_ptr(),
-            ctypes.byref(mask_words(words, batch, heads)),
-            ctypes.byref(mask_tiles(tiles)),
-            float(scale),
-            _lib.dtype_code(q.dtype),
-            _lib.status_word(q.device).data_ptr(),
-            _lib.stream_ptr(q.device),
-        )
-    _lib.check(rc)
-    return out, lse
+    return _lib.host().forward_masked(q, k, v, words, tiles, scale, _lib.status_word(q.device))
 
 
 @masked_fwd_op.register_fake
@@ -243,28 +220,7 @@ def masked_bwd_op(
     q: Tensor, k: Tensor, v: Tensor, out: Tensor, dout: Tensor, lse: Tensor, words: Tensor, words_t: Tensor,
     tiles: Tensor, scale: float,
 ) -> tuple[Tensor, Tensor, Tensor]:  # fmt: skip
-    from kohakufa_b200.mask import mask_tiles, mask_words
-
-    lib = _lib.load()
-    batch, heads, seq_q, _ = q.shape
-    dq, dk, dv = _bshd_like(q), _bshd_like(k), _bshd_like(v)
-    stats = q.new_empty(lib.kfa_bwd_stats_bytes(batch, heads, seq_q) // 4, dtype=torch.float32)
-    with torch.cuda.device(q.device):
-        rc = lib.kfa_bwd_masked(
-            *(ctypes.byref(_lib.tensor4(t)) for t in (q, k, v, out, dout)),
-            lse.data_ptr(),
-            stats.data_ptr(),
-            *(ctypes.byref(_lib.tensor4(t)) for t in (dq, dk, dv)),
-            ctypes.byref(mask_words(words, batch, heads)),
-            ctypes.byref(mask_words(words_t, batch, heads)),
-            ctypes.byref(mask_tiles(tiles)),
-            float(scale),
-            _lib.dtype_code(q.dtype),
-            _lib.status_word(q.device).data_ptr(),
-            _lib.stream_ptr(q.device),
-        )
-    _lib.check(rc)
-    return dq, dk, dv
+    return _lib.host().backward_masked(q, k, v, out, dout, lse, words, words_t, tiles, scale, _lib.status_word(q.device))
 
 
 @masked_bwd_op.register_fake
@@ -291,6 +247,30 @@ def _masked_backward(ctx, dout, dlse):
 masked_fwd_op.register_autograd(_masked_backward, setup_context=_masked_setup)
 
 
+class _MaskedAttention(Function):
+    """``masked_fwd_op`` with its gradient, for plain eager calls."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, words, words_t, tiles, scale):
+        out, lse = _lib.host().forward_masked(q, k, v, words, tiles, scale, _lib.status_word(q.device))
+        ctx.save_for_backward(q, k, v, out, lse, words, words_t, tiles)
+        ctx.scale = scale
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        saved = ctx.saved_tensors
+        q, k, v, out, lse, words, words_t, tiles = saved
+        if not _strides_ok(dout):
+            dout = dout.contiguous()
+        args = (q, k, v, out, dout, lse, words, words_t, tiles, ctx.scale)
+        if torch.is_grad_enabled() or not _lib.plain_eager(dout, *saved):
+            grads = masked_bwd_op(*args)
+        else:
+            grads = _lib.host().backward_masked(*args, _lib.status_word(q.device))
+        return *grads, None, None, None, None
+
+
 def attention(
     q: Tensor,
     k: Tensor,
@@ -305,7 +285,9 @@ def attention(
     (reference: op.py:146-175)."""
     from kohakufa_b200.mask import PackedMask
 
-    _check(q, k, v)
+    direct = _lib.plain_eager(q, k, v) and _lib.host().inputs_ok(q, k, v)  # (the conditions of _check, in C++)
+    if not direct:
+        _check(q, k, v)
     if scale is None:
         scale = q.shape[-1] ** -0.5
     if mask is not None:
@@ -315,10 +297,17 @@ def attention(
         packed = mask if isinstance(mask, PackedMask) else PackedMask(mask, *shape)
         if packed.shape != shape:
             raise ValueError(f"packed mask for {packed.shape}, inputs are {shape}")
-        out, _ = masked_fwd_op(q, k, v, packed.words, packed.words_t, packed.tiles, float(scale))
-        return out
-    out, _ = attention_fwd_op(q, k, v, float(scale), int(block_causal))
-    return out
+        words = (packed.words, packed.words_t, packed.tiles)
+        if not direct or not _lib.plain_eager(*words):
+            return masked_fwd_op(q, k, v, *words, float(scale))[0]
+        if _records(q, k, v):
+            return _MaskedAttention.apply(q, k, v, *words, float(scale))
+        return _lib.host().forward_masked(q, k, v, packed.words, packed.tiles, float(scale), _lib.status_word(q.device))[0]
+    if not direct:
+        return attention_fwd_op(q, k, v, float(scale), int(block_causal))[0]
+    if _records(q, k, v):
+        return _Attention.apply(q, k, v, float(scale), int(block_causal))
+    return _lib.host().forward(q, k, v, float(scale), int(block_causal), _lib.status_word(q.device))[0]
 
 
 # --------------------------------------------------------------------------------------
@@ -338,29 +327,8 @@ def varlen_fwd_op(
     q: Tensor, k: Tensor, v: Tensor, cu_seqlens_q: Tensor, cu_seqlens_k: Tensor, max_q: int, max_k: int,
     scale: float, block: int,
 ) -> tuple[Tensor, Tensor]:  # fmt: skip
-    lib = _lib.load()
-    total_q, heads, _ = q.shape
-    # zero-filled: rows no CTA writes (a sequence with queries but no keys, rows outside cu_seqlens) read
-    # as "no visible key": output 0, statistics 0
-    out = torch.zeros_like(q)
-    lse = q.new_zeros(1, heads, 2, total_q, dtype=torch.float32)
-    with torch.cuda.device(q.device):
-        rc = lib.kfa_fwd_varlen(
-            *(ctypes.byref(_lib.tensor4(_as4(t))) for t in (q, k, v, out)),
-            lse.data_ptr(),
-            cu_seqlens_q.data_ptr(),
-            cu_seqlens_k.data_ptr(),
-            cu_seqlens_q.numel() - 1,
-            max_q,
-            max_k,
-            float(scale),
-            int(block),
-            _lib.dtype_code(q.dtype),
-            _lib.status_word(q.device).data_ptr(),
-            _lib.stream_ptr(q.device),
-        )
-    _lib.check(rc)
-    return out, lse
+    word = _lib.status_word(q.device)
+    return _lib.host().forward_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, max_q, max_k, scale, block, word)
 
 
 @varlen_fwd_op.register_fake
@@ -373,29 +341,10 @@ def varlen_bwd_op(
     q: Tensor, k: Tensor, v: Tensor, out: Tensor, dout: Tensor, lse: Tensor, cu_seqlens_q: Tensor,
     cu_seqlens_k: Tensor, max_q: int, max_k: int, scale: float, block: int,
 ) -> tuple[Tensor, Tensor, Tensor]:  # fmt: skip
-    lib = _lib.load()
-    n_seqs = cu_seqlens_q.numel() - 1
-    dq, dk, dv = torch.zeros_like(q), torch.zeros_like(k), torch.zeros_like(v)  # unwritten rows: zero gradient
-    stats = q.new_empty(lib.kfa_bwd_stats_bytes(n_seqs, q.shape[1], max_q) // 4, dtype=torch.float32)
-    with torch.cuda.device(q.device):
-        rc = lib.kfa_bwd_varlen(
-            *(ctypes.byref(_lib.tensor4(_as4(t))) for t in (q, k, v, out, dout)),
-            lse.data_ptr(),
-            stats.data_ptr(),
-            *(ctypes.byref(_lib.tensor4(_as4(t))) for t in (dq, dk, dv)),
-            cu_seqlens_q.data_ptr(),
-            cu_seqlens_k.data_ptr(),
-            n_seqs,
-            max_q,
-            max_k,
-            float(scale),
-            int(block),
-            _lib.dtype_code(q.dtype),
-            _lib.status_word(q.device).data_ptr(),
-            _lib.stream_ptr(q.device),
-        )
-    _lib.check(rc)
-    return dq, dk, dv
+    word = _lib.status_word(q.device)
+    return _lib.host().backward_varlen(
+        q, k, v, out, dout, lse, cu_seqlens_q, cu_seqlens_k, max_q, max_k, scale, block, word
+    )
 
 
 @varlen_bwd_op.register_fake
@@ -419,6 +368,28 @@ def _varlen_backward(ctx, dout, dlse):
 
 
 varlen_fwd_op.register_autograd(_varlen_backward, setup_context=_varlen_setup)
+
+
+class _VarlenAttention(Function):
+    """``varlen_fwd_op`` with its gradient, for plain eager calls."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, cu_q, cu_k, max_q, max_k, scale, block):
+        out, lse = _lib.host().forward_varlen(q, k, v, cu_q, cu_k, max_q, max_k, scale, block, _lib.status_word(q.device))
+        ctx.save_for_backward(q, k, v, out, lse, cu_q, cu_k)
+        ctx.plan = (max_q, max_k, scale, block)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        saved = ctx.saved_tensors
+        q, k, v, out, lse, cu_q, cu_k = saved
+        args = (q, k, v, out, dout.contiguous(), lse, cu_q, cu_k, *ctx.plan)
+        if torch.is_grad_enabled() or not _lib.plain_eager(dout, *saved):
+            grads = varlen_bwd_op(*args)
+        else:
+            grads = _lib.host().backward_varlen(*args, _lib.status_word(q.device))
+        return *grads, None, None, None, None, None, None
 
 
 def varlen_plan(
@@ -455,7 +426,9 @@ def attention_varlen(
     ``plan`` from ``varlen_plan`` (built here if None). Reference: op.py:264-289."""
     if q.dim() != 3 or k.dim() != 3 or v.dim() != 3:
         raise ValueError("attention_varlen: q, k, v must be [T, H, D]")
-    _check(*(_as4(t) for t in (q, k, v)))
+    direct = _lib.plain_eager(q, k, v, cu_seqlens_q, cu_seqlens_k) and _lib.host().inputs_ok(q, k, v)
+    if not direct:
+        _check(*(_as4(t) for t in (q, k, v)))
     if scale is None:
         scale = q.shape[-1] ** -0.5
     cu_seqlens_q, cu_seqlens_k = cu_seqlens_q.int(), cu_seqlens_k.int()
@@ -464,5 +437,9 @@ def attention_varlen(
     n_seqs, max_q, max_k = plan
     if cu_seqlens_q.numel() != n_seqs + 1 or cu_seqlens_k.numel() != n_seqs + 1:
         raise ValueError(f"attention_varlen: the plan is for {n_seqs} sequences")
-    out, _ = varlen_fwd_op(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_q), int(max_k), float(scale), int(block_causal))
-    return out
+    args = (q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_q), int(max_k), float(scale), int(block_causal))
+    if not direct:
+        return varlen_fwd_op(*args)[0]
+    if _records(q, k, v):
+        return _VarlenAttention.apply(*args)
+    return _lib.host().forward_varlen(*args, _lib.status_word(q.device))[0]

@@ -1,0 +1,119 @@
+"""The direct launch path of plain eager calls: taken only there, and equal to the custom ops."""
+
+import pytest
+import torch
+
+from kohakufa_b200 import _lib, attention, attention_varlen, pack_mask, set_backward, varlen_plan
+from kohakufa_b200 import op
+
+
+def test_plain_eager_is_plain():
+    t = torch.ones(2)
+    assert _lib.plain_eager(t, t)
+    assert not _lib.plain_eager(t, torch.nn.Parameter(t))
+
+    class Sub(torch.Tensor):
+        pass
+
+    assert not _lib.plain_eager(t.as_subclass(Sub))
+    seen = []
+
+    class Mode(torch.utils._python_dispatch.TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    class FunctionMode(torch.overrides.TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    with Mode():
+        assert not _lib.plain_eager(t)
+    with FunctionMode():
+        assert not _lib.plain_eager(t)
+    with torch.autograd.forward_ad.dual_level():
+        assert not _lib.plain_eager(t)
+    torch.func.vmap(lambda x: (seen.append(_lib.plain_eager(x)), x)[1])(t)
+    torch.func.grad(lambda x: (seen.append(_lib.plain_eager(x)), x.sum())[1])(t)
+    torch.jit.trace(lambda x: (seen.append(_lib.plain_eager(x)), x + 1)[1], t, check_trace=False)
+    assert seen == [False, False, False]
+    assert _lib.plain_eager(t)
+
+
+def inputs(dim=128, seq=200, heads=4, kv_heads=2, packed=False):
+    gen = torch.Generator().manual_seed(dim + seq)
+    shape = (seq, heads, dim) if packed else (2, seq, heads, dim)
+    kv_shape = (seq, kv_heads, dim) if packed else (2, seq, kv_heads, dim)
+    ts = [torch.randn(s, generator=gen).bfloat16().cuda() for s in (shape, kv_shape, kv_shape, shape)]
+    if not packed:
+        ts = [t.transpose(1, 2) for t in ts]
+    return [t.requires_grad_() for t in ts[:3]], ts[3]
+
+
+def both_ways(call, qkv, dout, monkeypatch):
+    """(out, dq, dk, dv) of the direct path and of the custom ops."""
+    results = []
+    for direct in (True, False):
+        with monkeypatch.context() as m:
+            if not direct:
+                m.setattr(_lib, "plain_eager", lambda *ts: False)
+            out = call(*qkv)
+            assert ("sm100" in type(out.grad_fn).__name__) == (not direct)
+            results.append([out.detach(), *torch.autograd.grad(out, qkv, dout)])
+            with torch.no_grad():
+                assert torch.equal(call(*qkv), out)
+    return results
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["plain", "mask", "varlen"])
+def test_direct_path_equals_the_ops(kind, monkeypatch):
+    (q, k, v), dout = inputs(packed=kind == "varlen")
+    if kind == "mask":
+        mask = (torch.rand(200, 200, generator=torch.Generator().manual_seed(1)) < 0.4).cuda()
+        call = lambda q, k, v: attention(q, k, v, mask=mask)  # noqa: E731
+    elif kind == "varlen":
+        cu = torch.tensor([0, 70, 200], dtype=torch.int32, device="cuda")
+        plan = varlen_plan(cu, cu)
+        call = lambda q, k, v: attention_varlen(q, k, v, cu, cu, causal=True, plan=plan)  # noqa: E731
+    else:
+        call = lambda q, k, v: attention(q, k, v, causal=True)  # noqa: E731
+    direct, ops = both_ways(call, (q, k, v), dout, monkeypatch)
+    for a, b in zip(direct, ops):
+        assert a.dtype == b.dtype and a.shape == b.shape and a.stride() == b.stride()
+        assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
+def test_direct_path_and_autograd_features():
+    (q, k, v), dout = inputs()
+    out = attention(q, k, v)
+    want = torch.autograd.grad(out, (q, k, v), dout)
+    with torch.autograd.graph.save_on_cpu():  # saved tensors leave the GPU and come back with other strides
+        out = attention(q, k, v)
+    for a, b in zip(torch.autograd.grad(out, (q, k, v), dout), want):
+        assert torch.equal(a, b)
+    out = attention(q, k, v)  # an expanded gradient has strides of 0
+    grads = torch.autograd.grad(out.sum(), (q, k, v))
+    ones = torch.autograd.grad(attention(q, k, v), (q, k, v), torch.ones_like(out))
+    assert all(torch.equal(a, b) for a, b in zip(grads, ones))
+    (dq,) = torch.autograd.grad(attention(q, k, v), (q,), dout, create_graph=True)
+    with pytest.raises(RuntimeError):  # there is no second derivative
+        torch.autograd.grad(dq.sum(), (q,))
+    out = attention(q, k, v)
+    with torch.no_grad():
+        q.mul_(1.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.backward(dout)
+
+
+@pytest.mark.gpu
+def test_direct_path_refuses_what_the_ops_refuse():
+    (q, k, v), _ = inputs()
+    for bad, error in (((q.float(), k, v), TypeError), ((q, k[:, :1], v), ValueError), ((q[:, :3], k, v), ValueError),
+                       ((q.mT, k.mT, v.mT), ValueError), ((q.cpu(), k.cpu(), v.cpu()), ValueError)):  # fmt: skip
+        with pytest.raises(error):
+            op.attention(*bad)
+    packed = pack_mask(torch.ones(100, 200, dtype=torch.bool, device="cuda"), 2, 4, 100, 200)
+    with pytest.raises(ValueError):
+        op.attention(q, k, v, mask=packed)
+    set_backward("auto")
