@@ -446,7 +446,7 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t bar0 = smem_u32(bars);
   auto bar = [&](int i) { return bar0 + 8u * i; };
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
 #ifdef KFA_TRACE
   const bool trace_on = (blockIdx.x == 0) && (lane == 0);
 #endif
@@ -839,7 +839,7 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const uint32_t bar0 = smem_u32(bars);
   auto bar = [&](int i) { return bar0 + 8u * i; };
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
 
   int bh, t;
   decode_tile(blockIdx.x, p.B * p.H, p.n_q128, bh, t);

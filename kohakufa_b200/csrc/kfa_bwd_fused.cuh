@@ -15,9 +15,9 @@
 //                     accumulator in global memory (thread <-> query row)
 //   warp 12           MMA issue (converged, one elected lane issues)
 //   warp 13 / 14      TMA producers: K, V, then the Q ring / the dO ring
-// dS^T is written once, to shared memory (128-byte swizzled [key][query] boxes): the dK MMA reads it
-// as a K-major A operand, the dQ MMA reads the same bytes as an MN-major (transposed) A operand
-// (bwd.py:614-618). P^T goes to tensor memory over the S^T columns it came from (A operand of dV).
+// dS^T is written to shared memory (128-byte swizzled [key][query] boxes): the dQ MMA reads it as an MN-major
+// (transposed) A operand, the dK MMA the same bytes as a K-major one (bwd.py:614-618), or, at D = 64, a copy in tensor
+// memory. P^T goes to tensor memory over the S^T columns it came from (A operand of dV).
 //
 // Tensor memory (512 columns): S^T 128 | dP^T 128 | dV D | dK D | dQ D. At D = 128 that is 640, so dQ_i
 // shares the dP^T columns (bwd.py:46-51): dQ(i) is issued once both warpgroups have read dP^T(i), and
@@ -74,6 +74,12 @@ struct FusedCfg {
   static constexpr uint32_t TM_S = 0, TM_DP = 128, TM_DV = 256, TM_DK = 256 + D;
   static constexpr uint32_t TM_DQ = (D == 128) ? TM_DP : 256 + 2 * D;
   static constexpr bool DQ_ALIASES_DP = (D == 128);
+  // The 64 columns left at D = 64 hold a second copy of dS^T, the A operand of dK. Shared memory is what the step is
+  // short of there: of its 3400 clk, 2600 moved operands, dS^T and dQ at 128 B / clk when dQ and dK both read dS^T from it;
+  // this takes 256 off. With dP^T(s+1) issued before dQ(s): 488 -> 465 us (64 x 4096, frames of 256), 243 -> 229 us
+  // (16 x 4100 dense). Four compute warpgroups instead of two changed nothing (467) and cost 4 % on two-step problems.
+  static constexpr bool DS_IN_TMEM = (D == 64);
+  static constexpr uint32_t TM_DS = 448;
 };
 static_assert(FusedCfg<128>::SMEM_BYTES <= 232448 && FusedCfg<64>::SMEM_BYTES <= 232448, "shared memory");
 
@@ -90,10 +96,10 @@ __host__ __device__ constexpr uint32_t make_idesc_amn(bool bf16, int m, int n) {
 // dS^T = (dP^T - delta) * P of the same elements, rounded once to 16 bits, unscaled, written to the
 // 128-byte swizzled [key][64 queries] box of this warpgroup: element order as above, so word
 // (key row, query pair 8j + 2(lane % 4)) lands in 16-byte chunk j ^ (row % 8) of its row.
-// nd: -delta of this thread's first column, in shared memory.
+// nd: -delta of this thread's first column, in shared memory. dk: the packed words, in the same element order.
 template <bool BF16>
 __device__ __forceinline__ void ds_frag_to_smem(const float2* dp, const float2* pr, const float* nd_s, uint32_t s_row0,
-                                                int lane) {
+                                                int lane, uint32_t* dk) {
   const uint32_t sw = static_cast<uint32_t>(lane >> 2);  // row % 8 of every row this thread owns
   const uint32_t word = static_cast<uint32_t>(lane & 3) * 4u;
 #pragma unroll
@@ -104,7 +110,7 @@ __device__ __forceinline__ void ds_frag_to_smem(const float2* dp, const float2* 
     for (int e = 0; e < 4; ++e) {  // e = 2 * half + sel: row offset 16 * half + 8 * sel
       const int idx = 16 * (e >> 1) + 2 * j + (e & 1);
       const float2 d = __fmul2_rn(__fadd2_rn(dp[idx], nd), pr[idx]);
-      const uint32_t w = pack16<BF16>(d.x, d.y);
+      const uint32_t w = dk[idx] = pack16<BF16>(d.x, d.y);
       const uint32_t addr = s_row0 + static_cast<uint32_t>(16 * (e >> 1) + 8 * (e & 1)) * 128u + col;
       asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(w) : "memory");
     }
@@ -194,7 +200,7 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const uint32_t bar0 = smem_u32(bars);
   auto bar = [&](int i) { return bar0 + 8u * i; };
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
 
   // tile decode (groups of heads, tile-major inside); under a causal mask the first key tiles see the most queries and come first
   int bh, kt;  // bh over batch x K / V heads
@@ -389,28 +395,33 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           issue_kmajor_n128<D>(lead, tST, k_lo, sdesc_lo(sQ + ((s + 1) % NQ) * TB, 16), IDESC_S);
           umma_commit_lead(lead, bar(B_S));
         }
-        // dS^T(s) is in shared memory and dP^T(s) has been read: dQ_s = dS K (into columns of its own, or
-        // over dP^T), dK += dS^T Q_s
-        ok = mbar_wait_warp(bar(B_DS), s & 1, ctl, 39);
-        if (!ok) break;
-        if (!Cfg::DQ_ALIASES_DP && s > 0) {  // the previous dQ tile must have left its columns
-          ok = mbar_wait_warp(bar(B_DQFREE), (s - 1) & 1, ctl, 40);
-          if (!ok) break;
-        }
-        tc_fence_after();
-        issue_smemA_mnmajor_bmn<D>(lead, tDQ, ds_mn_lo, k_mn_lo, IDESC_DQ);
-        umma_commit_lead(lead, bar(B_DQ));
-        issue_smemA_kmajor_bmn<D>(lead, tDK, ds_k_lo, sdesc_lo(q_s, TILE_BYTES_64), IDESC_ACC, s > 0);
-        umma_commit_lead(lead, bar(B_QFREE + s % NQ));
-        umma_commit_lead(lead, bar(B_DSFREE));
-        if (more) {
+        // dS^T(s) is stored and dP^T(s) has been read: dP^T(s+1), dQ_s = dS K, dK += dS^T Q_s. With dQ in columns of its
+        // own dP^T(s+1) goes first: behind the two other products it was what the next dS waited for (the step was
+        // the loop dS -> dQ, dK, dP^T -> dS). Over the dP^T columns dQ has to come first.
+        auto issue_dP_next = [&]() {
           ok = mbar_wait_warp(bar(B_DOREADY + (s + 1) % NDO), ((s + 1) / NDO) & 1, ctl, 41);
           if (ok && Cfg::DQ_ALIASES_DP) ok = mbar_wait_warp(bar(B_DQFREE), s & 1, ctl, 42);
-          if (!ok) break;
+          if (!ok) return;
           tc_fence_after();
           issue_kmajor_n128<D>(lead, tDP, v_lo, sdesc_lo(sDO + ((s + 1) % NDO) * TB, 16), IDESC_S);
           umma_commit_lead(lead, bar(B_DP));
-        }
+        };
+        ok = mbar_wait_warp(bar(B_DS), s & 1, ctl, 39);
+        if (!ok) break;
+        if (!Cfg::DQ_ALIASES_DP && more) issue_dP_next();
+        if (ok && !Cfg::DQ_ALIASES_DP && s > 0)  // the previous dQ tile must have left its columns
+          ok = mbar_wait_warp(bar(B_DQFREE), (s - 1) & 1, ctl, 40);
+        if (!ok) break;
+        tc_fence_after();
+        issue_smemA_mnmajor_bmn<D>(lead, tDQ, ds_mn_lo, k_mn_lo, IDESC_DQ);
+        umma_commit_lead(lead, bar(B_DQ));
+        if constexpr (Cfg::DS_IN_TMEM)
+          issue_tmemA_k128_packed<D>(lead, tDK, tmem + Cfg::TM_DS, sdesc_lo(q_s, TILE_BYTES_64), IDESC_ACC, s > 0);
+        else
+          issue_smemA_kmajor_bmn<D>(lead, tDK, ds_k_lo, sdesc_lo(q_s, TILE_BYTES_64), IDESC_ACC, s > 0);
+        umma_commit_lead(lead, bar(B_QFREE + s % NQ));
+        umma_commit_lead(lead, bar(B_DSFREE));
+        if (Cfg::DQ_ALIASES_DP && more) issue_dP_next();
       }
       if (ok) umma_commit_lead(lead, bar(B_ACC));
       umma_commit_lead(lead, bar(B_DRAIN));
@@ -494,6 +505,7 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t tS = tmem + Cfg::TM_S + 64 * hq + lane_base;
     const uint32_t tDP = tmem + Cfg::TM_DP + 64 * hq + lane_base;
+    const uint32_t tDS = tmem + Cfg::TM_DS + 32 * hq + lane_base;  // (DS_IN_TMEM)
     constexpr uint32_t HALF = 16u << 16;  // the warp's second 16 lanes
     // In the compute phases a thread works on 4 key rows x 16 query columns (see p_frag):
     // first query that sees each of its keys; padded keys see nothing
@@ -562,11 +574,9 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if constexpr (D != 128) mbar_arrive(bar(B_PLO));
       mbar_arrive(bar(B_P));
       mbar_arrive(bar(B_MLFREE + (s & 1)));
-      if (!__all_sync(0xffffffffu, dp_probe && dsfree_probe && dl_probe)) {
-        ok = mbar_wait_warp(bar(B_DP), s & 1, ctl, 45);
-        if (ok && s > 0) ok = mbar_wait_warp(bar(B_DSFREE), (s - 1) & 1, ctl, 46);
-        if (ok) ok = mbar_wait_warp(bar(B_DLREADY), s & 1, ctl, 30);
-      }
+      ok = mbar_wait_warp_probed(dp_probe, bar(B_DP), s & 1, ctl, 45);
+      if (ok && s > 0) ok = mbar_wait_warp_probed(dsfree_probe, bar(B_DSFREE), (s - 1) & 1, ctl, 46);
+      if (ok) ok = mbar_wait_warp_probed(dl_probe, bar(B_DLREADY), s & 1, ctl, 30);
       if (!ok) break;
       tc_fence_after();
       {
@@ -574,7 +584,13 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tmem_ld_16x256b_x8(tDP, reinterpret_cast<uint32_t*>(dp));
         tmem_ld_16x256b_x8(tDP + HALF, reinterpret_cast<uint32_t*>(dp + 16));
         tmem_wait_ld();
-        ds_frag_to_smem<BF16>(dp, pr, dl_smem + 64 * hq + col0, s_row0, lane);
+        uint32_t dk[32];
+        ds_frag_to_smem<BF16>(dp, pr, dl_smem + 64 * hq + col0, s_row0, lane, dk);
+        if constexpr (Cfg::DS_IN_TMEM) {
+          tmem_st_16x128b_x8(tDS, dk);
+          tmem_st_16x128b_x8(tDS + HALF, dk + 16);
+          tmem_wait_st();
+        }
       }
       fence_async_smem();  // the MMAs read dS^T through the async proxy
       tc_fence_before();
