@@ -156,6 +156,18 @@ typedef struct KfaMaskTiles {
   int64_t stride_batch, stride_head;
 } KfaMaskTiles;
 
+/* As kfa_fwd and as kfa_bwd (dq_acc null) or kfa_bwd_fused (dq_acc given; head dims 56, 64, 120, 128), for head dims
+ * that are multiples of 8: tensors of an odd multiple are computed by the kernels of the next multiple of 16, whose
+ * last 8 columns read as zeros and are not written, instead of being copied into wider ones. dq_acc is sized for that
+ * wider head dim (kfa_bwd_dq_acc_bytes).
+ * The results are those of the reference's zero padding (api.py:18-29). */
+int kfa_fwd_narrow(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out, float* lse,
+                   float scale, int block, int dtype, int* dev_status, void* stream);
+int kfa_bwd_narrow(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out,
+                   const KfaTensor4* dout, const float* lse, float* stats, float* dq_acc, const KfaTensor4* dq,
+                   const KfaTensor4* dk, const KfaTensor4* dv, float scale, int block, int dtype, int* dev_status,
+                   void* stream);
+
 /* mask: bytes, nonzero = visible, element (b, h, r, c) at mask[b * s[0] + h * s[1] + r * s[2] + c * s[3]]
  * with mask_batch x mask_heads x Sq x Skv elements. words: int32[mask_batch * mask_heads * Sq *
  * 4 ceil(Skv / 128)], words_t: int32[mask_batch * mask_heads * Skv * 4 ceil(Sq / 128)], both contiguous.

@@ -48,6 +48,8 @@ SYMBOLS = (
     "kfa_copy_rows",
     "kfa_scores",
     "kfa_selftest",
+    "kfa_fwd_narrow",
+    "kfa_bwd_narrow",
 )
 
 
@@ -125,6 +127,8 @@ def load() -> ctypes.CDLL:
         lib.kfa_bwd_fused_main.argtypes = [T, T, T, T, fp, fp, T, T, ctypes.c_float, ctypes.c_int, ctypes.c_int, ip, vp]
         lib.kfa_bwd_dq_convert.argtypes = [fp, T, ctypes.c_float, ctypes.c_int, ip, vp]
         lib.kfa_bwd_fused.argtypes = [T, T, T, T, T, fp, fp, fp, T, T, T, ctypes.c_float, ctypes.c_int, ctypes.c_int, ip, vp]
+        lib.kfa_fwd_narrow.argtypes = lib.kfa_fwd.argtypes
+        lib.kfa_bwd_narrow.argtypes = lib.kfa_bwd_fused.argtypes
         lib.kfa_bwd_static_scratch.argtypes = [T, T, T, T, T, fp, T, T, T, ctypes.c_float, ctypes.c_int, ctypes.c_int, ip, vp]
         A = ctypes.POINTER(KfaAcc32)
         i64, f32, i32 = ctypes.c_int64, ctypes.c_float, ctypes.c_int
@@ -155,7 +159,7 @@ def load() -> ctypes.CDLL:
 # Entry points the host extension calls (a subset of SYMBOLS, in no particular order).
 HOST_SYMBOLS = (
     "kfa_last_error", "kfa_fwd", "kfa_bwd", "kfa_bwd_fused", "kfa_fwd_masked", "kfa_bwd_masked", "kfa_fwd_varlen",
-    "kfa_bwd_varlen", "kfa_pack_mask",
+    "kfa_bwd_varlen", "kfa_pack_mask", "kfa_fwd_narrow", "kfa_bwd_narrow",
 )  # fmt: skip
 HOST_PATH = Path(__file__).resolve().parent / "_kfa_host.so"
 _host = None

@@ -105,10 +105,14 @@ def attention(
     result_dtype, head_dim = q.dtype, q.shape[-1]
     if center_keys:
         k = _remove_key_mean(k, compute_dtype)
-    q, k, v = _fit_head_dim(*(t.to(compute_dtype) for t in (q, k, v)))
+    q, k, v = (t.to(compute_dtype) for t in (q, k, v))
+    softmax_scale = head_dim**-0.5 if scale is None else scale
+    if mask is None and _op.narrow(q, k, v):
+        out = _op.attention_narrow(q, k, v, softmax_scale, frame)
+        return out.to(result_dtype) if out.dtype != result_dtype else out
+    q, k, v = _fit_head_dim(q, k, v)
     if mask is not None and frame:
         raise ValueError("give a mask or causal / block_causal, not both (fold them in)")
-    softmax_scale = head_dim**-0.5 if scale is None else scale
     out = _op.attention(q, k, v, softmax_scale, frame, mask)
     if out.shape[-1] != head_dim:
         out = out[..., :head_dim]

@@ -66,9 +66,12 @@ int check_tensor(const KfaTensor4* t, const char* name) {
   return KFA_OK;
 }
 
+// The head dim whose kernels compute tensors of D columns.
+int kernel_dim(int64_t D) { return static_cast<int>((D + 15) / 16 * 16); }
+
 // 4-D tiled map over a [B, H, S, D] view: dims (D, S, H, B), box (C, 128, 1, 1) with C the chunk width of the
-// head dim (64, 32 or 16 columns) and the swizzle that spans the box's row (128, 64 or 32 bytes);
-// out-of-range rows read as zeros.
+// kernels' head dim (64, 32 or 16 columns) and the swizzle that spans the box's row (128, 64 or 32 bytes);
+// out-of-range rows (and columns D .. of a narrow tensor's last chunk) read as zeros.
 int make_map(const KfaTensor4* t, int dtype, CUtensorMap* map, const char* name) {
   EncodeFn enc = encode_fn();
   if (!enc) return fail(KFA_ERR_CUDA, "cuTensorMapEncodeTiled not available from the driver");
@@ -80,7 +83,7 @@ int make_map(const KfaTensor4* t, int dtype, CUtensorMap* map, const char* name)
     return static_cast<cuuint64_t>(s) * 2;
   };
   cuuint64_t strides[3] = {st(2), st(1), st(0)};
-  const int chunk = kfa::chunk_cols(static_cast<int>(D));
+  const int chunk = kfa::chunk_cols(kernel_dim(D));
   cuuint32_t box[4] = {static_cast<cuuint32_t>(chunk), 128, 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUtensorMapSwizzle swizzle =
@@ -92,12 +95,19 @@ int make_map(const KfaTensor4* t, int dtype, CUtensorMap* map, const char* name)
   return KFA_OK;
 }
 
-int check_qkv(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, int dtype, int block) {
+// narrow: odd multiples of 8 are taken as well
+int check_dim(int64_t D, bool narrow) {
+  if (narrow && D >= 8 && D <= 128 && D % 8 == 0) return KFA_OK;
+  if (D < 16 || D > 128 || D % 16) return fail(KFA_ERR_ARG, "head_dim %lld: a multiple of 16 up to 128", (long long)D);
+  return KFA_OK;
+}
+
+int check_qkv(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, int dtype, int block, bool narrow = false) {
   int rc;
   if ((rc = check_tensor(q, "q")) || (rc = check_tensor(k, "k")) || (rc = check_tensor(v, "v"))) return rc;
   if (dtype != KFA_F16 && dtype != KFA_BF16) return fail(KFA_ERR_ARG, "dtype %d: KFA_F16 or KFA_BF16", dtype);
   const int64_t D = q->shape[3];
-  if (D < 16 || D > 128 || D % 16) return fail(KFA_ERR_ARG, "head_dim %lld: a multiple of 16 up to 128", (long long)D);
+  if ((rc = check_dim(D, narrow))) return rc;
   for (int i = 0; i < 4; ++i)
     if (k->shape[i] != v->shape[i]) return fail(KFA_ERR_ARG, "k and v shapes differ");
   if (k->shape[0] != q->shape[0] || k->shape[3] != D) return fail(KFA_ERR_ARG, "k / v batch or head_dim differ from q");
@@ -243,6 +253,7 @@ struct Extra {
   const KfaMaskWords* mw = nullptr;   // words along query rows
   const KfaMaskWords* mwt = nullptr;  // words along key rows
   const KfaMaskTiles* mt = nullptr;   // which 128 x 128 tiles hold a visible pair (optional)
+  bool narrow = false;                // head dims that are odd multiples of 8, too
 };
 
 int check_tiles(const KfaMaskTiles* t) {
@@ -282,6 +293,7 @@ void fill_bwd_params(kfa::BwdParams& p, const KfaTensor4* q, const KfaTensor4* k
   p.group = p.H / p.Hkv;
   p.Sq = static_cast<int>(q->shape[2]);
   p.Skv = static_cast<int>(k->shape[2]);
+  p.cols = static_cast<int>(q->shape[3]);
   p.P = block;
   p.c = scale * LOG2E;
   p.scale = scale;
@@ -329,7 +341,7 @@ int fwd_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, cons
              const Extra& ex, float scale, int block, int dtype, int* dev_status, void* stream) {
   const Varlen* vl = ex.vl;
   int rc;
-  if ((rc = check_qkv(q, k, v, dtype, block)) || (rc = check_like(out, q, "out")) || (rc = check_varlen(vl, q, k)) ||
+  if ((rc = check_qkv(q, k, v, dtype, block, ex.narrow)) || (rc = check_like(out, q, "out")) || (rc = check_varlen(vl, q, k)) ||
       (rc = check_mask(ex.mw, k->shape[2], "mask words")))
     return rc;
   if (ex.mw && (block != 0 || vl)) return fail(KFA_ERR_ARG, "a boolean mask excludes block-causal and packed batches");
@@ -348,6 +360,7 @@ int fwd_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, cons
   p.H = static_cast<int>(q->shape[1]);
   p.Sq = static_cast<int>(q->shape[2]);
   p.Skv = static_cast<int>(k->shape[2]);
+  p.cols = static_cast<int>(q->shape[3]);
   p.P = block;
   p.c = scale * LOG2E;
   p.n_q_tiles = (p.Sq + 255) / 256;
@@ -374,17 +387,17 @@ int fwd_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, cons
     }
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  KFA_DISPATCH(q->shape[3], dtype, (launch_fwd<KD, KB>(mq, mk, mv, p, s)));
+  KFA_DISPATCH(kernel_dim(q->shape[3]), dtype, (launch_fwd<KD, KB>(mq, mk, mv, p, s)));
 }
 
 int prepare_impl(const KfaTensor4* out, const KfaTensor4* dout, const float* lse, float* stats, const Varlen* vl,
-                 int dtype, void* stream, float* dq_acc = nullptr) {
+                 int dtype, void* stream, float* dq_acc = nullptr, bool narrow = false) {
   int rc;
   if ((rc = check_tensor(out, "out")) || (rc = check_like(dout, out, "dout"))) return rc;
   if (!lse || !stats) return fail(KFA_ERR_ARG, "lse / stats: null pointer");
   if (dtype != KFA_F16 && dtype != KFA_BF16) return fail(KFA_ERR_ARG, "dtype %d", dtype);
-  const int64_t D = out->shape[3];
-  if (D < 16 || D > 128 || D % 16) return fail(KFA_ERR_ARG, "head_dim %lld: a multiple of 16 up to 128", (long long)D);
+  if ((rc = check_dim(out->shape[3], narrow))) return rc;
+  const int D = kernel_dim(out->shape[3]);
   if (dq_acc && D != 64 && D != 128) return fail(KFA_ERR_ARG, "fused backward: head_dim %lld: 64 or 128", (long long)D);
   kfa::PrepParams p;
   std::memset(&p, 0, sizeof(p));
@@ -403,6 +416,7 @@ int prepare_impl(const KfaTensor4* out, const KfaTensor4* dout, const float* lse
   p.H = static_cast<int>(out->shape[1]);
   p.Sq = static_cast<int>(out->shape[2]);
   p.n_q128 = (p.Sq + 127) / 128;
+  p.cols = static_cast<int>(out->shape[3]);
   if (vl) {
     p.B = vl->n_seqs;
     p.n_q128 = (vl->max_q + 127) / 128;
@@ -417,7 +431,7 @@ int dkdv_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, con
               const float* stats, const KfaTensor4* dk, const KfaTensor4* dv, const Extra& ex, float scale, int block,
               int dtype, int* dev_status, void* stream) {
   int rc;
-  if ((rc = check_qkv(q, k, v, dtype, block)) || (rc = check_like(dout, q, "dout")) ||
+  if ((rc = check_qkv(q, k, v, dtype, block, ex.narrow)) || (rc = check_like(dout, q, "dout")) ||
       (rc = check_like(dk, k, "dk")) || (rc = check_like(dv, v, "dv")) || (rc = check_varlen(ex.vl, q, k)) ||
       (rc = check_mask(ex.mwt, q->shape[2], "transposed mask words")))
     return rc;
@@ -439,13 +453,13 @@ int dkdv_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, con
   p.dv_sh = dv->stride[1];
   p.dv_ss = dv->stride[2];
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  KFA_DISPATCH(q->shape[3], dtype, (launch_dkdv<KD, KB>(mq, mk, mv, mdo, p, s)));
+  KFA_DISPATCH(kernel_dim(q->shape[3]), dtype, (launch_dkdv<KD, KB>(mq, mk, mv, mdo, p, s)));
 }
 
 int dq_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* dout, const float* stats,
             const KfaTensor4* dq, const Extra& ex, float scale, int block, int dtype, int* dev_status, void* stream) {
   int rc;
-  if ((rc = check_qkv(q, k, v, dtype, block)) || (rc = check_like(dout, q, "dout")) ||
+  if ((rc = check_qkv(q, k, v, dtype, block, ex.narrow)) || (rc = check_like(dout, q, "dout")) ||
       (rc = check_like(dq, q, "dq")) || (rc = check_varlen(ex.vl, q, k)) ||
       (rc = check_mask(ex.mw, k->shape[2], "mask words")))
     return rc;
@@ -463,7 +477,7 @@ int dq_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const
   p.dq_sh = dq->stride[1];
   p.dq_ss = dq->stride[2];
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  KFA_DISPATCH(q->shape[3], dtype, (launch_dq<KD, KB>(mq, mk, mv, mdo, p, s)));
+  KFA_DISPATCH(kernel_dim(q->shape[3]), dtype, (launch_dq<KD, KB>(mq, mk, mv, mdo, p, s)));
 }
 
 
@@ -486,17 +500,18 @@ int launch_dq_convert(const float* dq_acc, const KfaTensor4* dq, float scale, co
   const int H = static_cast<int>(dq->shape[1]), Sq = static_cast<int>(dq->shape[2]);
   auto conv = kfa::kfa_bwd_dq_convert_kernel<D, BF16>;
   conv<<<dim3((Sq + 127) / 128, static_cast<unsigned>(dq->shape[0] * H)), 256, 0, s>>>(
-      dq_acc, dq->ptr, dq->stride[0], dq->stride[1], dq->stride[2], H, Sq, scale, status);
+      dq_acc, dq->ptr, dq->stride[0], dq->stride[1], dq->stride[2], H, Sq, static_cast<int>(dq->shape[3]), scale, status);
   KFA_CUDA(cudaGetLastError());
   return KFA_OK;
 }
 
-int convert_impl(const float* dq_acc, const KfaTensor4* dq, float scale, int dtype, const int* dev_status, void* stream) {
+int convert_impl(const float* dq_acc, const KfaTensor4* dq, float scale, int dtype, const int* dev_status, void* stream,
+                 bool narrow = false) {
   int rc;
   if ((rc = check_tensor(dq, "dq"))) return rc;
   if (!dq_acc || !dev_status) return fail(KFA_ERR_ARG, "dq_acc / dev_status: null pointer");
   if (dtype != KFA_F16 && dtype != KFA_BF16) return fail(KFA_ERR_ARG, "dtype %d", dtype);
-  const int64_t D = dq->shape[3];
+  const int64_t D = narrow ? kernel_dim(dq->shape[3]) : dq->shape[3];
   if (D != 64 && D != 128) return fail(KFA_ERR_ARG, "head_dim %lld: 64 or 128", (long long)D);
   if (dq->shape[0] * dq->shape[1] > 65535) return fail(KFA_ERR_ARG, "B * H > 65535");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -505,9 +520,9 @@ int convert_impl(const float* dq_acc, const KfaTensor4* dq, float scale, int dty
 
 int fused_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* dout,
                const float* stats, float* dq_acc, const KfaTensor4* dk, const KfaTensor4* dv, float scale, int block,
-               int dtype, int* dev_status, void* stream) {
+               int dtype, int* dev_status, void* stream, bool narrow = false) {
   int rc;
-  if ((rc = check_qkv(q, k, v, dtype, block)) || (rc = check_like(dout, q, "dout")) || (rc = check_like(dk, k, "dk")) ||
+  if ((rc = check_qkv(q, k, v, dtype, block, narrow)) || (rc = check_like(dout, q, "dout")) || (rc = check_like(dk, k, "dk")) ||
       (rc = check_like(dv, v, "dv")))
     return rc;
   if (!stats || !dq_acc || !dev_status) return fail(KFA_ERR_ARG, "stats / dq_acc / dev_status: null pointer");
@@ -527,7 +542,7 @@ int fused_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, co
   p.dv_sh = dv->stride[1];
   p.dv_ss = dv->stride[2];
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  KFA_DISPATCH_FUSED(q->shape[3], dtype, (launch_fused<KD, KB>(mq, mk, mv, mdo, p, dq_acc, s)));
+  KFA_DISPATCH_FUSED(kernel_dim(q->shape[3]), dtype, (launch_fused<KD, KB>(mq, mk, mv, mdo, p, dq_acc, s)));
 }
 
 }  // namespace
@@ -621,6 +636,30 @@ int kfa_bwd(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const
   if ((rc = kfa_bwd_prepare(out, dout, lse, stats, dtype, stream))) return rc;
   if ((rc = kfa_bwd_dkdv(q, k, v, dout, stats, dk, dv, scale, block, dtype, dev_status, stream))) return rc;
   return kfa_bwd_dq(q, k, v, dout, stats, dq, scale, block, dtype, dev_status, stream);
+}
+
+int kfa_fwd_narrow(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out, float* lse,
+                   float scale, int block, int dtype, int* dev_status, void* stream) {
+  Extra ex;
+  ex.narrow = true;
+  return fwd_impl(q, k, v, out, lse, ex, scale, block, dtype, dev_status, stream);
+}
+
+int kfa_bwd_narrow(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out,
+                   const KfaTensor4* dout, const float* lse, float* stats, float* dq_acc, const KfaTensor4* dq,
+                   const KfaTensor4* dk, const KfaTensor4* dv, float scale, int block, int dtype, int* dev_status,
+                   void* stream) {
+  Extra ex;
+  ex.narrow = true;
+  int rc;
+  if ((rc = check_like(out, q, "out")) || (rc = check_like(dq, q, "dq"))) return rc;
+  if ((rc = prepare_impl(out, dout, lse, stats, nullptr, dtype, stream, dq_acc, true))) return rc;
+  if (dq_acc) {
+    if ((rc = fused_impl(q, k, v, dout, stats, dq_acc, dk, dv, scale, block, dtype, dev_status, stream, true))) return rc;
+    return convert_impl(dq_acc, dq, scale, dtype, dev_status, stream, true);
+  }
+  if ((rc = dkdv_impl(q, k, v, dout, stats, dk, dv, ex, scale, block, dtype, dev_status, stream))) return rc;
+  return dq_impl(q, k, v, dout, stats, dq, ex, scale, block, dtype, dev_status, stream);
 }
 
 #ifdef KFA_TRACE

@@ -48,6 +48,7 @@ struct BwdParams {
   long long dv_sb, dv_sh, dv_ss;
   const float* stats;  // [B*H, n_q128, 3, 128]: -m, -log2 l, -delta
   int B, H, Sq, Skv;
+  int cols;        // columns the 16-bit tensors hold: D, or D - 8 (the last 8 read as zeros and are not written)
   int Hkv, group;  // K / V heads; query heads per K / V head (H = Hkv * group)
   int P;
   float c;      // scale * log2(e)
@@ -95,6 +96,7 @@ struct PrepParams {
   const float* lse;  // [B, H, 2, Sq]
   float* stats;      // [B*H, n_q128, 3, 128]
   int B, H, Sq, n_q128;
+  int cols;         // see BwdParams
   const int* cu_q;  // packed variable-length batches: see BwdParams
   // Fused backward only (else nullptr): the fp32 dQ accumulator, whole 128-row tiles of D floats per
   // (batch, head); every CTA zero-fills the tile of its rows.
@@ -138,7 +140,7 @@ __global__ void __launch_bounds__(PREP_THREADS) kfa_bwd_prepare_kernel(const Pre
   for (int i = 0; i < PASSES; ++i) {
     const int row = tile * 128 + warp * ROWS + i * RPW + sub;
     ov[i] = gv[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (row < Sq && vec < VECS) {
+    if (row < Sq && vec * 8 < p.cols) {
       ov[i] = *reinterpret_cast<const uint4*>(ob + 2 * (row * p.o_ss + vec * 8));
       gv[i] = *reinterpret_cast<const uint4*>(gb + 2 * (row * p.do_ss + vec * 8));
     }
@@ -286,9 +288,9 @@ __device__ __forceinline__ void store_acc_row_f32(uint32_t taddr, int col0, int 
   }
 }
 
-// Writes a row of an fp32 accumulator (TMEM columns [col0, col0 + ncols)) times mul as 16-bit.
+// Writes a row of an fp32 accumulator (TMEM columns [col0, col0 + ncols), those below cols) times mul as 16-bit.
 template <bool BF16, int W = 32>
-__device__ __forceinline__ void store_acc_row(uint32_t taddr, int col0, int ncols, float mul, uint8_t* grow,
+__device__ __forceinline__ void store_acc_row(uint32_t taddr, int col0, int ncols, int cols, float mul, uint8_t* grow,
                                               bool valid) {
   for (int cc = col0; cc < col0 + ncols; cc += W) {
     float o[W];
@@ -297,6 +299,7 @@ __device__ __forceinline__ void store_acc_row(uint32_t taddr, int col0, int ncol
     if (valid) {
 #pragma unroll
       for (int i = 0; i < W; i += 8) {
+        if (cc + i >= cols) break;
         uint4 w;
         w.x = pack16<BF16>(o[i] * mul, o[i + 1] * mul);
         w.y = pack16<BF16>(o[i + 2] * mul, o[i + 3] * mul);
@@ -764,7 +767,7 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                static_cast<long long>(key) * D;
     if (n_steps == 0) {
       if (valid && p.acc_mode == 0)
-        for (int cc = 0; cc < D; cc += 8) *reinterpret_cast<uint4*>(grow + 2 * cc) = make_uint4(0, 0, 0, 0);
+        for (int cc = 0; cc < p.cols; cc += 8) *reinterpret_cast<uint4*>(grow + 2 * cc) = make_uint4(0, 0, 0, 0);
       if (valid && p.acc_mode == 1)
         for (int cc = 0; cc < D; cc += 4) *reinterpret_cast<float4*>(grow32 + cc) = make_float4(0.f, 0.f, 0.f, 0.f);
     } else {
@@ -773,7 +776,7 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tc_fence_after();
         const uint32_t tacc = tmem + (hq ? Cfg::TM_ACC1 : Cfg::TM_ACC0) + lane_base;
         if (p.acc_mode == 0)
-          store_acc_row<BF16, col_step(D)>(tacc, 0, D, hq ? p.scale : 1.0f, grow, valid);
+          store_acc_row<BF16, col_step(D)>(tacc, 0, D, p.cols, hq ? p.scale : 1.0f, grow, valid);
         else
           store_acc_row_f32<col_step(D)>(tacc, 0, D, hq ? p.scale : 1.0f, grow32, valid, p.acc_mode == 2);
       }
@@ -785,8 +788,8 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   if (*s_abort) {  // gave up (or an earlier kernel did): the rows of this CTA read as NaN
     const int r1 = min(kv0 + 128, Skv);
     if (p.acc_mode == 0) {
-      fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dk) + 2 * (bc * p.dk_sb + hk * p.dk_sh), p.dk_ss, k_base + kv0, k_base + r1, D);
-      fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dv) + 2 * (bc * p.dv_sb + hk * p.dv_sh), p.dv_ss, k_base + kv0, k_base + r1, D);
+      fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dk) + 2 * (bc * p.dk_sb + hk * p.dk_sh), p.dk_ss, k_base + kv0, k_base + r1, p.cols);
+      fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dv) + 2 * (bc * p.dv_sb + hk * p.dv_sh), p.dv_ss, k_base + kv0, k_base + r1, p.cols);
     } else if (r1 > kv0) {
       const long long bhl = static_cast<long long>(b) * p.Hkv + hk;
       fill_nan32(p.dk32 + bhl * p.dk32_sh + static_cast<long long>(kv0) * D, static_cast<long long>(r1 - kv0) * D);
@@ -1110,7 +1113,7 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       if (p.acc_mode == 0) {
         uint8_t* grow = reinterpret_cast<uint8_t*>(p.dq) +
                         2 * (bc * p.dq_sb + h * p.dq_sh + static_cast<long long>(q_base + row) * p.dq_ss);
-        store_acc_row<BF16, W>(tmem + Cfg::TM_ACC0 + lane_base, c0, nc, p.scale, grow, row < Sq);
+        store_acc_row<BF16, W>(tmem + Cfg::TM_ACC0 + lane_base, c0, nc, p.cols, p.scale, grow, row < Sq);
       } else {
         float* grow32 = p.dq32 + (static_cast<long long>(b) * p.H + h) * p.dq32_sh + static_cast<long long>(row) * D;
         store_acc_row_f32<W>(tmem + Cfg::TM_ACC0 + lane_base, c0, nc, p.scale, grow32, row < Sq, p.acc_mode == 2);
@@ -1123,7 +1126,7 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   if (*s_abort) {  // gave up (or an earlier kernel did): the rows of this CTA read as NaN
     const int r1 = min(row0 + 128, Sq);
     if (p.acc_mode == 0)
-      fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dq) + 2 * (bc * p.dq_sb + h * p.dq_sh), p.dq_ss, q_base + row0, q_base + r1, D);
+      fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dq) + 2 * (bc * p.dq_sb + h * p.dq_sh), p.dq_ss, q_base + row0, q_base + r1, p.cols);
     else if (r1 > row0)
       fill_nan32(p.dq32 + (static_cast<long long>(b) * p.H + h) * p.dq32_sh + static_cast<long long>(row0) * D,
                  static_cast<long long>(r1 - row0) * D);

@@ -606,13 +606,13 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       grow = reinterpret_cast<uint8_t*>(p.dk) + 2 * (b * p.dk_sb + hk * p.dk_sh + static_cast<long long>(key) * p.dk_ss);
     if (n_steps == 0) {
       if (valid)
-        for (int cc = 0; cc < D; cc += 8) *reinterpret_cast<uint4*>(grow + 2 * cc) = make_uint4(0, 0, 0, 0);
+        for (int cc = 0; cc < p.cols; cc += 8) *reinterpret_cast<uint4*>(grow + 2 * cc) = make_uint4(0, 0, 0, 0);
     } else {
       ok = mbar_wait_warp(bar(B_ACC), 0, ctl, 47) && ok;
       if (ok) {
         tc_fence_after();
         const uint32_t tacc = tmem + (hq ? Cfg::TM_DK : Cfg::TM_DV) + lane_base;
-        store_acc_row<BF16>(tacc, 0, D, hq ? p.scale : 1.0f, grow, valid);
+        store_acc_row<BF16>(tacc, 0, D, p.cols, hq ? p.scale : 1.0f, grow, valid);
       }
     }
   }
@@ -621,8 +621,8 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __syncthreads();
   if (*s_abort) {  // gave up (or an earlier kernel did): dK, dV rows of this CTA read as NaN (dQ: see the convert kernel)
     const int r1 = min(kv0 + 128, Skv);
-    fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dk) + 2 * (b * p.dk_sb + hk * p.dk_sh), p.dk_ss, kv0, r1, D);
-    fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dv) + 2 * (b * p.dv_sb + hk * p.dv_sh), p.dv_ss, kv0, r1, D);
+    fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dk) + 2 * (b * p.dk_sb + hk * p.dk_sh), p.dk_ss, kv0, r1, p.cols);
+    fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dv) + 2 * (b * p.dv_sb + hk * p.dv_sh), p.dv_ss, kv0, r1, p.cols);
   }
   if (warp == 0) {
     tc_fence_after();
@@ -635,7 +635,7 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 template <int D, bool BF16>
 __global__ void __launch_bounds__(256) kfa_bwd_dq_convert_kernel(const float* __restrict__ dq_acc, void* dq,
                                                                  long long dq_sb, long long dq_sh, long long dq_ss,
-                                                                 int H, int Sq, float scale, const int* status) {
+                                                                 int H, int Sq, int cols, float scale, const int* status) {
   const int tile = blockIdx.x, bh = blockIdx.y;
   const int b = bh / H, h = bh % H;
   const int r_in = threadIdx.x & 127, half = threadIdx.x >> 7;
@@ -644,13 +644,16 @@ __global__ void __launch_bounds__(256) kfa_bwd_dq_convert_kernel(const float* __
   const float* src = dq_acc + static_cast<long long>(bh) * dq_acc_head_floats(Sq, D) +
                      static_cast<long long>(tile) * (128 * D) + r_in * 4;
   uint8_t* drow = reinterpret_cast<uint8_t*>(dq) + 2 * (b * dq_sb + h * dq_sh + static_cast<long long>(row) * dq_ss);
+  const int c_end = min((half + 1) * (D / 16), cols / 8);  // in pieces of 8 columns
   if (*status != 0) {  // a kernel before this one gave up: the accumulator is incomplete
-    for (int c8 = half * (D / 16); c8 < (half + 1) * (D / 16); ++c8)
+    for (int c8 = half * (D / 16); c8 < c_end; ++c8)
       *reinterpret_cast<uint4*>(drow + 16 * c8) = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
     return;
   }
 #pragma unroll
-  for (int c8 = half * (D / 16); c8 < (half + 1) * (D / 16); ++c8) {
+  for (int x = 0; x < D / 16; ++x) {
+    const int c8 = half * (D / 16) + x;
+    if (c8 >= c_end) break;
     const float4 a = *reinterpret_cast<const float4*>(src + (2 * c8) * 512);
     const float4 c = *reinterpret_cast<const float4*>(src + (2 * c8 + 1) * 512);
     uint4 w;

@@ -89,6 +89,7 @@ int kfa_cp_fwd_step(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* 
   p.H = static_cast<int>(q->shape[1]);
   p.Sq = static_cast<int>(q->shape[2]);
   p.Skv = static_cast<int>(k->shape[2]);
+  p.cols = static_cast<int>(q->shape[3]);
   p.P = block;
   p.c = scale * LOG2E;
   p.n_q_tiles = (p.Sq + 255) / 256;

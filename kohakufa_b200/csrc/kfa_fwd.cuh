@@ -40,6 +40,7 @@ struct FwdParams {
   long long o_sb, o_sh, o_ss;
   float* lse;  // [B, H, 2, Sq]: plane 0 = m, plane 1 = log2(l)
   int B, H, Sq, Skv;
+  int cols;  // columns the 16-bit tensors hold: D, or D - 8 (the last 8 read as zeros and are not written)
   int P;    // 0 dense; P > 0: key c visible to query r iff c / P <= r / P
   float c;  // scale * log2(e)
   int n_q_tiles;
@@ -675,6 +676,7 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           if (valid) {
 #pragma unroll
             for (int i = 0; i < W; i += 8) {
+              if (cc + i >= p.cols) break;
               uint4 w;
               w.x = pack16<BF16>(o[i] * inv, o[i + 1] * inv);
               w.y = pack16<BF16>(o[i + 2] * inv, o[i + 3] * inv);
@@ -702,7 +704,7 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     const int r1 = min(row0 + 256, Sq);
     const long long bhl = static_cast<long long>(b) * p.H + h;
     if (p.mode == 0) {
-      fill_rows_nan16(reinterpret_cast<uint8_t*>(p.o) + 2 * (bc * p.o_sb + h * p.o_sh), p.o_ss, q_base + row0, q_base + r1, D);
+      fill_rows_nan16(reinterpret_cast<uint8_t*>(p.o) + 2 * (bc * p.o_sb + h * p.o_sh), p.o_ss, q_base + row0, q_base + r1, p.cols);
       float* lse = p.lse + (static_cast<long long>(bc) * p.H + h) * 2 * p.Sq + q_base;
       fill_nan32(lse + row0, r1 - row0);
       fill_nan32(lse + p.Sq + row0, r1 - row0);

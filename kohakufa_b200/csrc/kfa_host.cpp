@@ -27,6 +27,8 @@ struct Api {
   decltype(&kfa_fwd_varlen) fwd_varlen = nullptr;
   decltype(&kfa_bwd_varlen) bwd_varlen = nullptr;
   decltype(&kfa_pack_mask) pack_mask = nullptr;
+  decltype(&kfa_fwd_narrow) fwd_narrow = nullptr;
+  decltype(&kfa_bwd_narrow) bwd_narrow = nullptr;
 } api;
 
 PyObject* g_error = nullptr;  // kohakufa_b200._lib.KfaError
@@ -108,7 +110,8 @@ bool strides_ok(const at::Tensor& t) {
 }
 
 // Whether q, k, v are what the kernels take (the conditions of op.py's _check, which raises for the rest).
-bool inputs_ok(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, int64_t dims) {
+// step: the head dims taken are its multiples.
+bool inputs_ok(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, int64_t dims, int64_t step) {
   if (q.dim() != dims || k.dim() != dims || v.dim() != dims) return false;
   if ((q.scalar_type() != at::kHalf && q.scalar_type() != at::kBFloat16) || k.scalar_type() != q.scalar_type() ||
       v.scalar_type() != q.scalar_type())
@@ -116,7 +119,7 @@ bool inputs_ok(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, in
   if (!q.is_cuda() || k.device() != q.device() || v.device() != q.device()) return false;
   if (q.layout() != at::kStrided || k.layout() != at::kStrided || v.layout() != at::kStrided) return false;
   const int64_t d = q.size(-1), heads = q.size(1), kv_heads = k.size(1);
-  if (d < 16 || d > 128 || d % 16 || k.size(-1) != d) return false;
+  if (d < step || d > 128 || d % step || k.size(-1) != d) return false;
   if (k.sizes() != v.sizes() || (dims == 4 && k.size(0) != q.size(0))) return false;
   if (q.numel() == 0 || k.numel() == 0 || kv_heads == 0 || heads % kv_heads) return false;
   return strides_ok(q) && strides_ok(k) && strides_ok(v);
@@ -148,11 +151,17 @@ void need(Py_ssize_t got, Py_ssize_t want) {
 
 using Args = PyObject* const*;
 
-// inputs_ok(q, k, v) -> bool
+// inputs_ok(q, k, v) -> bool: head dims that are multiples of 16
 PyObject* py_inputs_ok(Args a, Py_ssize_t n) {
   need(n, 3);
   const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]);
-  return PyBool_FromLong(inputs_ok(q, k, v, q.dim() == 3 ? 3 : 4));
+  return PyBool_FromLong(inputs_ok(q, k, v, q.dim() == 3 ? 3 : 4, 16));
+}
+
+// narrow_ok(q, k, v) -> bool: [B, H, S, D] and head dims that are multiples of 8
+PyObject* py_narrow_ok(Args a, Py_ssize_t n) {
+  need(n, 3);
+  return PyBool_FromLong(inputs_ok(tensor(a[0]), tensor(a[1]), tensor(a[2]), 4, 8));
 }
 
 // forward(q, k, v, scale, block, status) -> out, lse
@@ -163,8 +172,9 @@ PyObject* py_forward(Args a, Py_ssize_t n) {
   at::Tensor out = bshd_like(q);
   at::Tensor lse = floats(q, {q.size(0), q.size(1), 2, q.size(2)});
   const KfaTensor4 dq = desc(q), dk = desc(k), dv = desc(v), dout = desc(out);
-  check(api.fwd(&dq, &dk, &dv, &dout, lse.data_ptr<float>(), static_cast<float>(number(a[3])),
-                static_cast<int>(integer(a[4])), dtype_code(q), tensor(a[5]).data_ptr<int32_t>(), stream_of(q)));
+  const auto call = q.size(3) % 16 ? api.fwd_narrow : api.fwd;
+  check(call(&dq, &dk, &dv, &dout, lse.data_ptr<float>(), static_cast<float>(number(a[3])), static_cast<int>(integer(a[4])),
+             dtype_code(q), tensor(a[5]).data_ptr<int32_t>(), stream_of(q)));
   return pack(out, lse);
 }
 
@@ -181,9 +191,12 @@ PyObject* py_backward(Args a, Py_ssize_t n) {
   at::Tensor stats = stats_scratch(q, q.size(0), q.size(1), q.size(2));
   const KfaTensor4 d[8] = {desc(q), desc(k), desc(v), desc(o), desc(g), desc(dq), desc(dk), desc(dv)};
   if (fused) {
-    at::Tensor acc = floats(q, {q.size(0) * q.size(1) * ((q.size(2) + 127) / 128) * 128 * q.size(3)});
-    check(api.bwd_fused(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), acc.data_ptr<float>(),
+    at::Tensor acc = floats(q, {q.size(0) * q.size(1) * ((q.size(2) + 127) / 128) * 128 * ((q.size(3) + 15) / 16 * 16)});
+    check((q.size(3) % 16 ? api.bwd_narrow : api.bwd_fused)(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), acc.data_ptr<float>(),
                         d + 5, d + 6, d + 7, scale, block, dtype_code(q), status, stream_of(q)));
+  } else if (q.size(3) % 16) {
+    check(api.bwd_narrow(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), nullptr, d + 5, d + 6,
+                         d + 7, scale, block, dtype_code(q), status, stream_of(q)));
   } else {
     check(api.bwd(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), d + 5, d + 6, d + 7, scale,
                   block, dtype_code(q), status, stream_of(q)));
@@ -296,6 +309,8 @@ PyObject* py_bind(Args a, Py_ssize_t n) {
   take("kfa_fwd_varlen", api.fwd_varlen);
   take("kfa_bwd_varlen", api.bwd_varlen);
   take("kfa_pack_mask", api.pack_mask);
+  take("kfa_fwd_narrow", api.fwd_narrow);
+  take("kfa_bwd_narrow", api.bwd_narrow);
   Py_INCREF(a[0]);
   Py_XDECREF(g_error);
   g_error = a[0];
@@ -316,7 +331,7 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 #define KFA_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(entry<py_##name>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
-    KFA_METHOD(bind),           KFA_METHOD(inputs_ok),       KFA_METHOD(forward),        KFA_METHOD(backward),
+    KFA_METHOD(bind),           KFA_METHOD(inputs_ok),       KFA_METHOD(narrow_ok), KFA_METHOD(forward),        KFA_METHOD(backward),
     KFA_METHOD(forward_masked), KFA_METHOD(backward_masked), KFA_METHOD(forward_varlen), KFA_METHOD(backward_varlen),
     KFA_METHOD(pack_mask),      {nullptr, nullptr, 0, nullptr},
 };

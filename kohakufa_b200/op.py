@@ -122,6 +122,21 @@ def _records(q: Tensor, k: Tensor, v: Tensor) -> bool:
     return torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
 
 
+def narrow(q: Tensor, k: Tensor, v: Tensor) -> bool:
+    """Whether ``attention_narrow`` takes these ``[B, H, S, D]`` inputs as they are: plain eager execution and a head
+    dim that is an odd multiple of 8, whose columns up to the next multiple of 16 the kernels read as zeros
+    (copying q, k, v, dout and the results to and from wider tensors costs more than a small problem's kernels:
+    forward + backward of 4 x 8 heads x 4096 queries x 77 keys at head dim 40 takes 128 us, 233 with the copies)."""
+    return q.shape[-1] % 16 == 8 and _lib.plain_eager(q, k, v) and _lib.host().narrow_ok(q, k, v)
+
+
+def attention_narrow(q: Tensor, k: Tensor, v: Tensor, scale: float, block_causal: int) -> Tensor:
+    """``attention`` for inputs that ``narrow`` accepts."""
+    if _records(q, k, v):
+        return _Attention.apply(q, k, v, float(scale), int(block_causal))
+    return _lib.host().forward(q, k, v, float(scale), int(block_causal), _lib.status_word(q.device))[0]
+
+
 def _bshd_like(t: Tensor) -> Tensor:
     batch, heads, seq, dim = t.shape
     return t.new_empty(batch, seq, heads, dim).transpose(1, 2)
@@ -144,7 +159,7 @@ def _(q, k, v, scale, block):
 def attention_bwd_op(
     q: Tensor, k: Tensor, v: Tensor, out: Tensor, dout: Tensor, lse: Tensor, scale: float, block: int
 ) -> tuple[Tensor, Tensor, Tensor]:
-    fused = use_fused_backward(q.shape[-1], q.shape[0] * q.shape[1])
+    fused = use_fused_backward(kernel_dim_for(q.shape[-1]), q.shape[0] * q.shape[1])
     return _lib.host().backward(q, k, v, out, dout, lse, scale, block, _lib.status_word(q.device), fused)
 
 
@@ -191,7 +206,7 @@ class _Attention(Function):
         if torch.is_grad_enabled() or not _lib.plain_eager(q, k, v, out, dout, lse):
             grads = attention_bwd_op(q, k, v, out, dout, lse, ctx.scale, ctx.block)
         else:
-            fused = use_fused_backward(q.shape[-1], q.shape[0] * q.shape[1])
+            fused = use_fused_backward(kernel_dim_for(q.shape[-1]), q.shape[0] * q.shape[1])
             grads = _lib.host().backward(q, k, v, out, dout, lse, ctx.scale, ctx.block, _lib.status_word(q.device), fused)
         return *grads, None, None
 
