@@ -168,6 +168,16 @@ int kfa_bwd_narrow(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v
                    const KfaTensor4* dk, const KfaTensor4* dv, float scale, int block, int dtype, int* dev_status,
                    void* stream);
 
+/* As kfa_bwd (and its narrow form), with the steps of every key tile shared out to several CTAs where the key tiles
+ * alone leave most of the GPU idle (cross attention to a short sequence). The CTAs leave fp32 parts of dK and dV in `parts`
+ * (16-byte aligned scratch of kfa_bwd_parts_bytes), which are then summed in a fixed order: results repeat bit for bit.
+ * kfa_bwd_parts_bytes is 0 where this would not help; kfa_bwd_parts refuses such problems. */
+int64_t kfa_bwd_parts_bytes(const KfaTensor4* q, const KfaTensor4* k);
+int kfa_bwd_parts(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out,
+                  const KfaTensor4* dout, const float* lse, float* stats, float* parts, const KfaTensor4* dq,
+                  const KfaTensor4* dk, const KfaTensor4* dv, float scale, int block, int dtype, int* dev_status,
+                  void* stream);
+
 /* mask: bytes, nonzero = visible, element (b, h, r, c) at mask[b * s[0] + h * s[1] + r * s[2] + c * s[3]]
  * with mask_batch x mask_heads x Sq x Skv elements. words: int32[mask_batch * mask_heads * Sq *
  * 4 ceil(Skv / 128)], words_t: int32[mask_batch * mask_heads * Skv * 4 ceil(Sq / 128)], both contiguous.

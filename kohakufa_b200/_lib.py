@@ -50,6 +50,8 @@ SYMBOLS = (
     "kfa_selftest",
     "kfa_fwd_narrow",
     "kfa_bwd_narrow",
+    "kfa_bwd_parts_bytes",
+    "kfa_bwd_parts",
 )
 
 
@@ -129,6 +131,9 @@ def load() -> ctypes.CDLL:
         lib.kfa_bwd_fused.argtypes = [T, T, T, T, T, fp, fp, fp, T, T, T, ctypes.c_float, ctypes.c_int, ctypes.c_int, ip, vp]
         lib.kfa_fwd_narrow.argtypes = lib.kfa_fwd.argtypes
         lib.kfa_bwd_narrow.argtypes = lib.kfa_bwd_fused.argtypes
+        lib.kfa_bwd_parts.argtypes = lib.kfa_bwd_fused.argtypes
+        lib.kfa_bwd_parts_bytes.restype = ctypes.c_int64
+        lib.kfa_bwd_parts_bytes.argtypes = [T, T]
         lib.kfa_bwd_static_scratch.argtypes = [T, T, T, T, T, fp, T, T, T, ctypes.c_float, ctypes.c_int, ctypes.c_int, ip, vp]
         A = ctypes.POINTER(KfaAcc32)
         i64, f32, i32 = ctypes.c_int64, ctypes.c_float, ctypes.c_int
@@ -148,7 +153,7 @@ def load() -> ctypes.CDLL:
         lib.kfa_scores.argtypes = [T, T, fp, i32, ip, vp]
         lib.kfa_selftest.argtypes = [ctypes.c_char_p, ctypes.c_int]
         for name in SYMBOLS:
-            if name not in ("kfa_abi_version", "kfa_last_error", "kfa_bwd_stats_bytes", "kfa_bwd_dq_acc_bytes"):
+            if name not in ("kfa_abi_version", "kfa_last_error", "kfa_bwd_stats_bytes", "kfa_bwd_dq_acc_bytes", "kfa_bwd_parts_bytes"):
                 getattr(lib, name).restype = ctypes.c_int
         if lib.kfa_abi_version() != ABI_VERSION:
             raise KfaError(f"libkfa ABI {lib.kfa_abi_version()} != expected {ABI_VERSION}: rebuild")
@@ -160,6 +165,7 @@ def load() -> ctypes.CDLL:
 HOST_SYMBOLS = (
     "kfa_last_error", "kfa_fwd", "kfa_bwd", "kfa_bwd_fused", "kfa_fwd_masked", "kfa_bwd_masked", "kfa_fwd_varlen",
     "kfa_bwd_varlen", "kfa_pack_mask", "kfa_fwd_narrow", "kfa_bwd_narrow",
+    "kfa_bwd_parts_bytes", "kfa_bwd_parts",
 )  # fmt: skip
 HOST_PATH = Path(__file__).resolve().parent / "_kfa_host.so"
 _host = None

@@ -4,6 +4,7 @@
 // already set" flags.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -169,7 +170,7 @@ int launch_dkdv_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMa
   constexpr int smem = MASKW ? kfa::BwdCfg<D>::KV_SMEM_BYTES_LIST : kfa::BwdCfg<D>::KV_SMEM_BYTES;
   int rc = set_smem(kern, smem);
   if (rc) return rc;
-  const long long grid = static_cast<long long>(p.B) * p.Hkv * p.n_k128;
+  const long long grid = static_cast<long long>(p.B) * p.Hkv * p.n_k128 * (p.n_split > 1 ? p.n_split : 1);
   if (grid > 0x7fffffffll) return fail(KFA_ERR_ARG, "too many tiles");
   kern<<<static_cast<unsigned>(grid), kfa::BWD_THREADS, smem, s>>>(mq, mk, mv, mdo, p);
   KFA_CUDA(cudaGetLastError());
@@ -254,6 +255,8 @@ struct Extra {
   const KfaMaskWords* mwt = nullptr;  // words along key rows
   const KfaMaskTiles* mt = nullptr;   // which 128 x 128 tiles hold a visible pair (optional)
   bool narrow = false;                // head dims that are odd multiples of 8, too
+  int n_split = 1;                    // dK / dV: CTAs that share a key tile's steps, and where they leave their parts
+  float* parts = nullptr;
 };
 
 int check_tiles(const KfaMaskTiles* t) {
@@ -453,7 +456,60 @@ int dkdv_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, con
   p.dv_sh = dv->stride[1];
   p.dv_ss = dv->stride[2];
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (ex.n_split > 1) {
+    const long long floats = k->shape[0] * k->shape[1] * k->shape[2] * kernel_dim(k->shape[3]);
+    p.n_split = ex.n_split;
+    p.split_stride = 2 * floats;  // a part: dK, then dV
+    p.acc_mode = 1;
+    p.dk32 = ex.parts;
+    p.dv32 = ex.parts + floats;
+    p.dk32_sh = p.dv32_sh = k->shape[2] * kernel_dim(k->shape[3]);
+  }
   KFA_DISPATCH(kernel_dim(q->shape[3]), dtype, (launch_dkdv<KD, KB>(mq, mk, mv, mdo, p, s)));
+}
+
+template <int D, bool BF16>
+int launch_sum_splits(const kfa::SumParams& p, int bh, cudaStream_t s) {
+  const dim3 grid(static_cast<unsigned>((static_cast<long long>(p.rows) * (D / 8) + 255) / 256), bh, 2);
+  kfa::kfa_bwd_sum_splits_kernel<D, BF16><<<grid, 256, 0, s>>>(p);
+  KFA_CUDA(cudaGetLastError());
+  return KFA_OK;
+}
+
+// How many CTAs share the steps of a key tile in the dK / dV kernel, 1 = a CTA runs them all. Only for attention to a much
+// shorter sequence (8 or more query tiles per key tile: key tiles are then both few and long), where the key tiles fill
+// less than half of the GPU: as many as it has SMs for, with at least 4 steps (of about 1.4 us) each, which pay for the
+// CTA's set-up and the sum of the parts. The order of the sums depends on this number, and so on batch and heads, which
+// is why self attention, whose dK and dV do not depend on what else is in the batch, is left alone.
+// (148 SMs: what this library is built for.)
+int bwd_splits(const KfaTensor4* q, const KfaTensor4* k) {
+  const int64_t n_k = (k->shape[2] + 127) / 128, n_q = (q->shape[2] + 127) / 128;
+  const int64_t tiles = k->shape[0] * k->shape[1] * n_k;
+  const int64_t steps = (q->shape[1] / k->shape[1]) * n_q;
+  if (n_q < 8 * n_k || 2 * tiles > 148) return 1;
+  const int64_t n = std::min<int64_t>(148 / tiles, steps / 4);
+  return n < 2 ? 1 : static_cast<int>(n);
+}
+
+int sum_splits_impl(const KfaTensor4* dk, const KfaTensor4* dv, const Extra& ex, int dtype, void* stream) {
+  kfa::SumParams p;
+  const int64_t rows = dk->shape[2], bh = dk->shape[0] * dk->shape[1];
+  const long long floats = bh * rows * kernel_dim(dk->shape[3]);
+  const KfaTensor4* t[2] = {dk, dv};
+  for (int i = 0; i < 2; ++i) {
+    p.part[i] = ex.parts + i * floats;
+    p.out[i] = t[i]->ptr;
+    p.sb[i] = t[i]->stride[0];
+    p.sh[i] = t[i]->stride[1];
+    p.ss[i] = t[i]->stride[2];
+  }
+  p.stride = 2 * floats;
+  p.n = ex.n_split;
+  p.H = static_cast<int>(dk->shape[1]);
+  p.rows = static_cast<int>(rows);
+  p.cols = static_cast<int>(dk->shape[3]);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  KFA_DISPATCH(kernel_dim(dk->shape[3]), dtype, (launch_sum_splits<KD, KB>(p, static_cast<int>(bh), s)));
 }
 
 int dq_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* dout, const float* stats,
@@ -659,6 +715,30 @@ int kfa_bwd_narrow(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v
     return convert_impl(dq_acc, dq, scale, dtype, dev_status, stream, true);
   }
   if ((rc = dkdv_impl(q, k, v, dout, stats, dk, dv, ex, scale, block, dtype, dev_status, stream))) return rc;
+  return dq_impl(q, k, v, dout, stats, dq, ex, scale, block, dtype, dev_status, stream);
+}
+
+int64_t kfa_bwd_parts_bytes(const KfaTensor4* q, const KfaTensor4* k) {
+  if (!q || !k || k->shape[0] < 1 || k->shape[1] < 1) return 0;
+  const int n = bwd_splits(q, k);
+  return n < 2 ? 0 : static_cast<int64_t>(n) * 8 * k->shape[0] * k->shape[1] * k->shape[2] * kernel_dim(k->shape[3]);
+}
+
+int kfa_bwd_parts(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out,
+                  const KfaTensor4* dout, const float* lse, float* stats, float* parts, const KfaTensor4* dq,
+                  const KfaTensor4* dk, const KfaTensor4* dv, float scale, int block, int dtype, int* dev_status,
+                  void* stream) {
+  int rc;
+  if ((rc = check_qkv(q, k, v, dtype, block, true)) || (rc = check_like(out, q, "out"))) return rc;
+  Extra ex;
+  ex.narrow = true;
+  ex.n_split = bwd_splits(q, k);
+  ex.parts = parts;
+  if (ex.n_split < 2) return fail(KFA_ERR_ARG, "kfa_bwd_parts: not a problem whose steps are shared out (kfa_bwd_parts_bytes is 0)");
+  if (!parts || reinterpret_cast<uintptr_t>(parts) % 16) return fail(KFA_ERR_ARG, "parts: null or not 16-byte aligned");
+  if ((rc = prepare_impl(out, dout, lse, stats, nullptr, dtype, stream, nullptr, true))) return rc;
+  if ((rc = dkdv_impl(q, k, v, dout, stats, dk, dv, ex, scale, block, dtype, dev_status, stream))) return rc;
+  if ((rc = sum_splits_impl(dk, dv, ex, dtype, stream))) return rc;
   return dq_impl(q, k, v, dout, stats, dq, ex, scale, block, dtype, dev_status, stream);
 }
 

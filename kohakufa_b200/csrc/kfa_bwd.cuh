@@ -65,6 +65,10 @@ struct BwdParams {
   long long dk32_sh;
   float* dv32;
   long long dv32_sh;
+  // dK / dV kernel, n_split > 1 (with acc_mode 1): the steps of a key tile are shared out to n_split CTAs, each of
+  // which leaves its part of the sums in accumulators split_stride floats further on.
+  int n_split;
+  long long split_stride;
   // Packed variable-length batches (cu_q != nullptr): tensors [1, H, T, D], sequence b (of B) owns query
   // rows cu_q[b] .. cu_q[b + 1] and key rows cu_k[b] .. cu_k[b + 1]. Sq, Skv are then the tensors' row
   // counts and n_q128 / n_k128 the tile counts of the longest sequence (they size the grid and the
@@ -415,6 +419,10 @@ __device__ __forceinline__ void ds_cols_by_key(const float2* dp, const float2* p
 
 // ---------------------------------------------------------------------------------------
 // dK / dV
+// With few key tiles (cross attention to a short text: one) the grid of key tiles leaves most SMs idle for as many
+// steps as there are query tiles: the steps are then shared out (BwdParams::n_split, rule in bwd_splits of kfa_api.cu) and
+// kfa_bwd_sum_splits_kernel adds up the parts, in a fixed order. 32 heads x 4096 queries x 77 keys, D = 48: 48.6 us ->
+// 18.5, and 4.5 for the sum.
 // ---------------------------------------------------------------------------------------
 template <int D, bool BF16, bool MASKW>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
@@ -456,7 +464,10 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   // tile decode (groups of heads, tile-major inside); when causal the first key tiles see the most queries and come first
   int bh, kt;  // bh over batch x K / V heads
-  decode_tile(blockIdx.x, p.B * p.Hkv, p.n_k128, bh, kt);
+  const int split = (!MASKW && p.n_split > 1) ? blockIdx.x % p.n_split : 0;
+  decode_tile((!MASKW && p.n_split > 1) ? blockIdx.x / p.n_split : blockIdx.x, p.B * p.Hkv, p.n_k128, bh, kt);
+  float* dk32 = p.dk32 + split * p.split_stride;
+  float* dv32 = p.dv32 + split * p.split_stride;
   const int b = bh / p.Hkv, hk = bh % p.Hkv;
   const int kv0 = kt * 128;  // relative to the sequence's first key
   int Sq = p.Sq, Skv = p.Skv, q_base = 0, k_base = 0, bc = b;  // bc: batch coordinate in the tensors
@@ -472,6 +483,12 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // steps: for every query head of this K / V head's group, the query tiles that see these keys
   const int n_per = max((Sq + 127) / 128 - first_i, 0);
   int n_steps = n_per * p.group;
+  int s_first = 0;  // this CTA's first step
+  if (!MASKW && p.n_split > 1) {
+    const int per = (n_steps + p.n_split - 1) / p.n_split;
+    s_first = min(split * per, n_steps);
+    n_steps = min(per, n_steps - s_first);
+  }
   const bool ragged_keys = kv0 + 128 > Skv;
   const int i_full = (p.P > 0 && !ragged_keys) ? first_full_tile(kv0, p.P) : 0;  // query tiles before it are masked steps
   // boolean masks with a tile table: the (query head, query tile) steps this CTA runs, in shared memory
@@ -520,8 +537,8 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t tmem = *s_tmem;
   if (use_list) n_steps = static_cast<int>(s_tmem[2]);
   // step s -> query tile and query head
-  auto tile_of = [&](int s) { return use_list ? static_cast<int>(s_list[s] & 0xffffu) : first_i + s % n_per; };
-  auto head_of = [&](int s) { return hk * p.group + (use_list ? static_cast<int>(s_list[s] >> 16) : s / n_per); };
+  auto tile_of = [&](int s) { return use_list ? static_cast<int>(s_list[s] & 0xffffu) : first_i + (s_first + s) % n_per; };
+  auto head_of = [&](int s) { return hk * p.group + (use_list ? static_cast<int>(s_list[s] >> 16) : (s_first + s) / n_per); };
   const Ctl ctl{s_abort, p.status};
   const bool dead = (*s_abort != 0);
 
@@ -671,6 +688,10 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (n_steps > 0) mask_fetch(0);
     }
     StepWalk walk;
+    if (!MASKW && n_steps > 0) {
+      walk.rel = s_first % n_per;
+      walk.g = s_first / n_per;
+    }
     for (int s = 0; s < n_steps; ++s, walk.next(n_per)) {
       uint2 wcur[4];
       if constexpr (MASKW) {
@@ -762,8 +783,8 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       grow = reinterpret_cast<uint8_t*>(p.dk) + 2 * (bc * p.dk_sb + hk * p.dk_sh + grow_row * p.dk_ss);
     float* grow32 = nullptr;
     if (p.acc_mode != 0)
-      grow32 = (hq == 0 ? p.dv32 + (static_cast<long long>(b) * p.Hkv + hk) * p.dv32_sh
-                        : p.dk32 + (static_cast<long long>(b) * p.Hkv + hk) * p.dk32_sh) +
+      grow32 = (hq == 0 ? dv32 + (static_cast<long long>(b) * p.Hkv + hk) * p.dv32_sh
+                        : dk32 + (static_cast<long long>(b) * p.Hkv + hk) * p.dk32_sh) +
                static_cast<long long>(key) * D;
     if (n_steps == 0) {
       if (valid && p.acc_mode == 0)
@@ -792,14 +813,48 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dv) + 2 * (bc * p.dv_sb + hk * p.dv_sh), p.dv_ss, k_base + kv0, k_base + r1, p.cols);
     } else if (r1 > kv0) {
       const long long bhl = static_cast<long long>(b) * p.Hkv + hk;
-      fill_nan32(p.dk32 + bhl * p.dk32_sh + static_cast<long long>(kv0) * D, static_cast<long long>(r1 - kv0) * D);
-      fill_nan32(p.dv32 + bhl * p.dv32_sh + static_cast<long long>(kv0) * D, static_cast<long long>(r1 - kv0) * D);
+      fill_nan32(dk32 + bhl * p.dk32_sh + static_cast<long long>(kv0) * D, static_cast<long long>(r1 - kv0) * D);
+      fill_nan32(dv32 + bhl * p.dv32_sh + static_cast<long long>(kv0) * D, static_cast<long long>(r1 - kv0) * D);
     }
   }
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem, Cfg::TMEM_COLS);
   }
+}
+
+// dK and dV = 16 bits of the parts' sums: thread <-> 8 columns of a row of dK (blockIdx.z 0) or dV (1). Bound by its
+// launch: the parts are a few MB, just written.
+struct SumParams {
+  const float* part[2];  // parts at part[i] + n * stride, rows of D floats, row r of (b, h) at (b * H + h) * rows * D + r * D
+  void* out[2];
+  long long sb[2], sh[2], ss[2];
+  long long stride;
+  int n, H, rows, cols;
+};
+template <int D, bool BF16>
+__global__ void __launch_bounds__(256) kfa_bwd_sum_splits_kernel(const SumParams p) {
+  constexpr int VECS = D / 8;
+  const int which = blockIdx.z, bh = blockIdx.y;
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  const int row = i / VECS, c = (i % VECS) * 8;
+  if (row >= p.rows || c >= p.cols) return;
+  const float* src = p.part[which] + (static_cast<long long>(bh) * p.rows + row) * D + c;
+  float acc[8];
+#pragma unroll
+  for (int x = 0; x < 8; ++x) acc[x] = 0.f;
+  for (int n = 0; n < p.n; ++n, src += p.stride) {
+    const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+    acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
+    acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
+  }
+  uint4 w;
+  w.x = pack16<BF16>(acc[0], acc[1]);
+  w.y = pack16<BF16>(acc[2], acc[3]);
+  w.z = pack16<BF16>(acc[4], acc[5]);
+  w.w = pack16<BF16>(acc[6], acc[7]);
+  const long long at = (bh / p.H) * p.sb[which] + (bh % p.H) * p.sh[which] + static_cast<long long>(row) * p.ss[which] + c;
+  *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out[which]) + 2 * at) = w;
 }
 
 // ---------------------------------------------------------------------------------------

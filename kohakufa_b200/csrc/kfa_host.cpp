@@ -29,6 +29,8 @@ struct Api {
   decltype(&kfa_pack_mask) pack_mask = nullptr;
   decltype(&kfa_fwd_narrow) fwd_narrow = nullptr;
   decltype(&kfa_bwd_narrow) bwd_narrow = nullptr;
+  decltype(&kfa_bwd_parts_bytes) bwd_parts_bytes = nullptr;
+  decltype(&kfa_bwd_parts) bwd_parts = nullptr;
 } api;
 
 PyObject* g_error = nullptr;  // kohakufa_b200._lib.KfaError
@@ -179,18 +181,24 @@ PyObject* py_forward(Args a, Py_ssize_t n) {
 }
 
 // backward(q, k, v, out, dout, lse, scale, block, status, fused) -> dq, dk, dv
+// fused: 1 the fused kernels, 0 the split ones, 2 the fused ones unless the split ones can share out their steps
 PyObject* py_backward(Args a, Py_ssize_t n) {
   need(n, 10);
   const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]), &o = tensor(a[3]), &g = tensor(a[4]), &lse = tensor(a[5]);
   const float scale = static_cast<float>(number(a[6]));
   const int block = static_cast<int>(integer(a[7]));
   int* status = tensor(a[8]).data_ptr<int32_t>();
-  const bool fused = PyObject_IsTrue(a[9]) == 1;
+  const int64_t fused = integer(a[9]);
   const c10::cuda::CUDAGuard guard(q.device());
   at::Tensor dq = bshd_like(q), dk = bshd_like(k), dv = bshd_like(v);
   at::Tensor stats = stats_scratch(q, q.size(0), q.size(1), q.size(2));
   const KfaTensor4 d[8] = {desc(q), desc(k), desc(v), desc(o), desc(g), desc(dq), desc(dk), desc(dv)};
-  if (fused) {
+  const int64_t parts_bytes = (fused == 1) ? 0 : api.bwd_parts_bytes(d, d + 1);
+  if (parts_bytes > 0) {
+    at::Tensor parts = floats(q, {parts_bytes / 4});
+    check(api.bwd_parts(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), parts.data_ptr<float>(),
+                        d + 5, d + 6, d + 7, scale, block, dtype_code(q), status, stream_of(q)));
+  } else if (fused) {
     at::Tensor acc = floats(q, {q.size(0) * q.size(1) * ((q.size(2) + 127) / 128) * 128 * ((q.size(3) + 15) / 16 * 16)});
     check((q.size(3) % 16 ? api.bwd_narrow : api.bwd_fused)(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), acc.data_ptr<float>(),
                         d + 5, d + 6, d + 7, scale, block, dtype_code(q), status, stream_of(q)));
@@ -311,6 +319,8 @@ PyObject* py_bind(Args a, Py_ssize_t n) {
   take("kfa_pack_mask", api.pack_mask);
   take("kfa_fwd_narrow", api.fwd_narrow);
   take("kfa_bwd_narrow", api.bwd_narrow);
+  take("kfa_bwd_parts_bytes", api.bwd_parts_bytes);
+  take("kfa_bwd_parts", api.bwd_parts);
   Py_INCREF(a[0]);
   Py_XDECREF(g_error);
   g_error = a[0];

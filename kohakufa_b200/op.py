@@ -90,6 +90,14 @@ def use_fused_backward(dim: int, batch_heads: int) -> bool:
     return _backward_mode == "fused" or FUSED_IS_FASTER[dim]
 
 
+def _backward_route(q: Tensor) -> int:
+    """What the library is asked for: 1 the fused kernels, 0 the split ones, 2 ("auto") the fused ones unless few
+    key tiles leave the GPU idle and the split dK / dV kernel can share out its steps (``kfa_bwd_parts``)."""
+    if not use_fused_backward(kernel_dim_for(q.shape[-1]), q.shape[0] * q.shape[1]):
+        return 0
+    return 1 if _backward_mode == "fused" else 2
+
+
 def _strides_ok(t: Tensor) -> bool:
     if t.stride(-1) != 1:  # (the base address is checked by the library: 16-byte aligned)
         return False
@@ -159,7 +167,7 @@ def _(q, k, v, scale, block):
 def attention_bwd_op(
     q: Tensor, k: Tensor, v: Tensor, out: Tensor, dout: Tensor, lse: Tensor, scale: float, block: int
 ) -> tuple[Tensor, Tensor, Tensor]:
-    fused = use_fused_backward(kernel_dim_for(q.shape[-1]), q.shape[0] * q.shape[1])
+    fused = _backward_route(q)
     return _lib.host().backward(q, k, v, out, dout, lse, scale, block, _lib.status_word(q.device), fused)
 
 
@@ -206,7 +214,7 @@ class _Attention(Function):
         if torch.is_grad_enabled() or not _lib.plain_eager(q, k, v, out, dout, lse):
             grads = attention_bwd_op(q, k, v, out, dout, lse, ctx.scale, ctx.block)
         else:
-            fused = use_fused_backward(kernel_dim_for(q.shape[-1]), q.shape[0] * q.shape[1])
+            fused = _backward_route(q)
             grads = _lib.host().backward(q, k, v, out, dout, lse, ctx.scale, ctx.block, _lib.status_word(q.device), fused)
         return *grads, None, None
 

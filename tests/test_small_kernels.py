@@ -66,3 +66,37 @@ def test_backward_statistics(dim, seq):
     error = (rows[:, :, 2, :seq].double() + products.sum(-1)).abs()
     assert bool((error <= dim * 2.0**-24 * products.abs().sum(-1)).all())
     assert bool((rows[:, :, 0, seq:] == -torch.inf).all()) and not bool(rows[:, :, 1:, seq:].any())
+
+
+@pytest.mark.parametrize("dim,dtype", [(40, torch.float16), (64, torch.float16), (128, torch.bfloat16)])
+@pytest.mark.parametrize("s_q,s_kv,heads,kv_heads,block", [(4096, 77, 4, 4, 0), (1025, 128, 4, 2, 0), (2000, 129, 2, 1, 0), (2100, 200, 2, 2, 1), (3100, 300, 2, 1, 100)])
+def test_shared_out_steps(dim, dtype, s_q, s_kv, heads, kv_heads, block):
+    """Few key tiles: several CTAs share a tile's steps and their fp32 parts are summed. dQ is the split kernels' own;
+    dK, dV differ from theirs by the order of fp32 sums, then one rounding to 16 bits (a unit in the last place: 2^-10,
+    2^-7 of a value), and repeat bit for bit."""
+    gen = torch.Generator().manual_seed(s_q + s_kv)
+
+    def one(seq, h):
+        return torch.randn(1, seq, h, dim, generator=gen).to(dtype).cuda().transpose(1, 2)
+
+    q, k, v, dout = one(s_q, heads), one(s_kv, kv_heads), one(s_kv, kv_heads), one(s_q, heads)
+    lib, host, word = _lib.load(), _lib.host(), _lib.status_word(q.device)
+    ref = lambda t: ctypes.byref(_lib.tensor4(t))  # noqa: E731
+    assert lib.kfa_bwd_parts_bytes(ref(q), ref(k)) > 0
+    out, lse = host.forward(q, k, v, dim**-0.5, block, word)
+    got = host.backward(q, k, v, out, dout, lse, dim**-0.5, block, word, 0)
+    again = host.backward(q, k, v, out, dout, lse, dim**-0.5, block, word, 2)
+    assert all(torch.equal(a, b) for a, b in zip(got, again))
+    like = lambda t: torch.empty_like(t.transpose(1, 2).contiguous()).transpose(1, 2)  # noqa: E731
+    want = [like(t) for t in (q, k, v)]
+    stats = torch.empty(lib.kfa_bwd_stats_bytes(1, heads, s_q) // 4, device="cuda")
+    _lib.check(lib.kfa_bwd_narrow(*(ref(t) for t in (q, k, v, out, dout)), lse.data_ptr(), stats.data_ptr(), None,
+                                  *(ref(t) for t in want), dim**-0.5, block, _lib.dtype_code(dtype), word.data_ptr(),
+                                  _lib.stream_ptr(q.device)))  # fmt: skip
+    assert _lib.device_status() == 0 and torch.equal(got[0], want[0])
+    ulp = 2.0**-10 if dtype == torch.float16 else 2.0**-7
+    for a, b in zip(got[1:], want[1:]):
+        a, b = a.double(), b.double()
+        # the fp32 sums: at most the count of summed products (queries x heads of the group) times 2^-24 of the largest sum
+        noise = s_q * (heads // kv_heads) * 2.0**-24 * float(b.abs().max())
+        assert bool(((a - b).abs() <= ulp * b.abs() + noise + 2.0**-24).all())
