@@ -178,6 +178,11 @@ int kfa_bwd_parts(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v,
                   const KfaTensor4* dk, const KfaTensor4* dv, float scale, int block, int dtype, int* dev_status,
                   void* stream);
 
+/* Zeros in the rows that kfa_fwd_varlen (n_tensors 1: t = {out}, with its statistics lse) or kfa_bwd_varlen (n_tensors 3:
+ * t = {dq, dk, dv}; lse null) do not write for these sequences, for outputs that were not zero-filled beforehand. */
+int kfa_varlen_zero_rows(const KfaTensor4* t, int n_tensors, const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int n_seqs,
+                         int max_q, int max_k, float* lse, void* stream);
+
 /* mask: bytes, nonzero = visible, element (b, h, r, c) at mask[b * s[0] + h * s[1] + r * s[2] + c * s[3]]
  * with mask_batch x mask_heads x Sq x Skv elements. words: int32[mask_batch * mask_heads * Sq *
  * 4 ceil(Skv / 128)], words_t: int32[mask_batch * mask_heads * Skv * 4 ceil(Sq / 128)], both contiguous.

@@ -52,6 +52,7 @@ SYMBOLS = (
     "kfa_bwd_narrow",
     "kfa_bwd_parts_bytes",
     "kfa_bwd_parts",
+    "kfa_varlen_zero_rows",
 )
 
 
@@ -132,6 +133,7 @@ def load() -> ctypes.CDLL:
         lib.kfa_fwd_narrow.argtypes = lib.kfa_fwd.argtypes
         lib.kfa_bwd_narrow.argtypes = lib.kfa_bwd_fused.argtypes
         lib.kfa_bwd_parts.argtypes = lib.kfa_bwd_fused.argtypes
+        lib.kfa_varlen_zero_rows.argtypes = [T, ctypes.c_int, ip, ip, ctypes.c_int, ctypes.c_int, ctypes.c_int, fp, vp]
         lib.kfa_bwd_parts_bytes.restype = ctypes.c_int64
         lib.kfa_bwd_parts_bytes.argtypes = [T, T]
         lib.kfa_bwd_static_scratch.argtypes = [T, T, T, T, T, fp, T, T, T, ctypes.c_float, ctypes.c_int, ctypes.c_int, ip, vp]
@@ -165,7 +167,7 @@ def load() -> ctypes.CDLL:
 HOST_SYMBOLS = (
     "kfa_last_error", "kfa_fwd", "kfa_bwd", "kfa_bwd_fused", "kfa_fwd_masked", "kfa_bwd_masked", "kfa_fwd_varlen",
     "kfa_bwd_varlen", "kfa_pack_mask", "kfa_fwd_narrow", "kfa_bwd_narrow",
-    "kfa_bwd_parts_bytes", "kfa_bwd_parts",
+    "kfa_bwd_parts_bytes", "kfa_bwd_parts", "kfa_varlen_zero_rows",
 )  # fmt: skip
 HOST_PATH = Path(__file__).resolve().parent / "_kfa_host.so"
 _host = None

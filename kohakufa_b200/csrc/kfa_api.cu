@@ -135,6 +135,11 @@ int set_smem(K kernel, int bytes) {
 
 constexpr float LOG2E = 1.4426950408889634f;
 
+// Tiles that a packed batch of n_seqs sequences, n_max tiles the longest, in `rows` rows has at most.
+long long packed_tiles(int n_seqs, int n_max, int rows, int tile) {
+  return std::min(static_cast<long long>(n_seqs) * n_max, static_cast<long long>(rows) / tile + n_seqs);
+}
+
 template <int D, bool BF16, bool MASKW>
 int launch_fwd_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const kfa::FwdParams& p,
                  cudaStream_t s) {
@@ -142,7 +147,7 @@ int launch_fwd_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap
   constexpr int smem = MASKW ? kfa::FwdCfg<D>::SMEM_BYTES_LIST : kfa::FwdCfg<D>::SMEM_BYTES;
   int rc = set_smem(kern, smem);
   if (rc) return rc;
-  const long long grid = static_cast<long long>(p.B) * p.H * p.n_q_tiles;
+  const long long grid = p.compact ? packed_tiles(p.B, p.n_q_tiles, p.Sq, 256) * p.H : static_cast<long long>(p.B) * p.H * p.n_q_tiles;
   if (grid > 0x7fffffffll) return fail(KFA_ERR_ARG, "too many tiles");
   kern<<<static_cast<unsigned>(grid), kfa::FWD_THREADS, smem, s>>>(mq, mk, mv, p);
   KFA_CUDA(cudaGetLastError());
@@ -170,7 +175,8 @@ int launch_dkdv_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMa
   constexpr int smem = MASKW ? kfa::BwdCfg<D>::KV_SMEM_BYTES_LIST : kfa::BwdCfg<D>::KV_SMEM_BYTES;
   int rc = set_smem(kern, smem);
   if (rc) return rc;
-  const long long grid = static_cast<long long>(p.B) * p.Hkv * p.n_k128 * (p.n_split > 1 ? p.n_split : 1);
+  const long long grid = p.compact ? packed_tiles(p.B, p.n_k128, p.Skv, 128) * p.Hkv
+                                   : static_cast<long long>(p.B) * p.Hkv * p.n_k128 * (p.n_split > 1 ? p.n_split : 1);
   if (grid > 0x7fffffffll) return fail(KFA_ERR_ARG, "too many tiles");
   kern<<<static_cast<unsigned>(grid), kfa::BWD_THREADS, smem, s>>>(mq, mk, mv, mdo, p);
   KFA_CUDA(cudaGetLastError());
@@ -190,7 +196,7 @@ int launch_dq_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap&
   constexpr int smem = MASKW ? kfa::BwdCfg<D>::Q_SMEM_BYTES_LIST : kfa::BwdCfg<D>::Q_SMEM_BYTES;
   int rc = set_smem(kern, smem);
   if (rc) return rc;
-  const long long grid = static_cast<long long>(p.B) * p.H * p.n_q128;
+  const long long grid = p.compact ? packed_tiles(p.B, p.n_q128, p.Sq, 128) * p.H : static_cast<long long>(p.B) * p.H * p.n_q128;
   if (grid > 0x7fffffffll) return fail(KFA_ERR_ARG, "too many tiles");
   kern<<<static_cast<unsigned>(grid), kfa::BWD_THREADS, smem, s>>>(mq, mk, mv, mdo, p);
   KFA_CUDA(cudaGetLastError());
@@ -338,6 +344,7 @@ void apply_extra(kfa::BwdParams& p, const Extra& ex) {
   p.stats_sh = static_cast<long long>(p.n_q128) * 384;
   p.cu_q = vl->cu_q;
   p.cu_k = vl->cu_k;
+  p.compact = vl->n_seqs <= kfa::VARLEN_COMPACT;
 }
 
 int fwd_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out, float* lse,
@@ -374,6 +381,7 @@ int fwd_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, cons
     p.n_q_tiles = (vl->max_q + 255) / 256;
     p.cu_q = vl->cu_q;
     p.cu_k = vl->cu_k;
+    p.compact = vl->n_seqs <= kfa::VARLEN_COMPACT;
   }
   if (ex.mw) {
     p.mw = ex.mw->words;
@@ -740,6 +748,37 @@ int kfa_bwd_parts(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v,
   if ((rc = dkdv_impl(q, k, v, dout, stats, dk, dv, ex, scale, block, dtype, dev_status, stream))) return rc;
   if ((rc = sum_splits_impl(dk, dv, ex, dtype, stream))) return rc;
   return dq_impl(q, k, v, dout, stats, dq, ex, scale, block, dtype, dev_status, stream);
+}
+
+int kfa_varlen_zero_rows(const KfaTensor4* t, int n_tensors, const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int n_seqs,
+                         int max_q, int max_k, float* lse, void* stream) {
+  if (!t || (n_tensors != 1 && n_tensors != 3) || !cu_seqlens_q || !cu_seqlens_k || n_seqs < 1 || max_q < 1 || max_k < 1)
+    return fail(KFA_ERR_ARG, "kfa_varlen_zero_rows: bad arguments");
+  kfa::ZeroRowsParams p;
+  std::memset(&p, 0, sizeof(p));
+  int64_t most = 0;
+  for (int i = 0; i < n_tensors; ++i) {
+    int rc = check_tensor(t + i, "output");
+    if (rc) return rc;
+    if (t[i].shape[0] != 1 || t[i].shape[3] % 8 || t[i].shape[3] != t[0].shape[3])
+      return fail(KFA_ERR_ARG, "kfa_varlen_zero_rows: packed [1, H, T, D] tensors of one head dim, a multiple of 8");
+    p.out[i] = t[i].ptr;
+    p.sh[i] = t[i].stride[1];
+    p.ss[i] = t[i].stride[2];
+    p.heads[i] = static_cast<int>(t[i].shape[1]);
+    p.rows[i] = static_cast<int>(t[i].shape[2]);
+    // the forward's tiles are 256 query rows, the dQ kernel's 128; a sequence without keys has no query tiles
+    p.covered[i] = i > 0 ? (max_k + 127) / 128 * 128 : (n_tensors == 1 ? (max_q + 255) / 256 * 256 : (max_q + 127) / 128 * 128);
+    p.cu[i] = i > 0 ? cu_seqlens_k : cu_seqlens_q;
+    p.cu_need[i] = i > 0 ? nullptr : cu_seqlens_k;
+    most = std::max(most, t[i].shape[2]);
+  }
+  p.lse = lse;
+  p.cols = static_cast<int>(t[0].shape[3]);
+  p.n_seqs = n_seqs;
+  kfa::kfa_zero_rows_kernel<<<dim3(static_cast<unsigned>((most + 255) / 256), n_tensors), 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  KFA_CUDA(cudaGetLastError());
+  return KFA_OK;
 }
 
 #ifdef KFA_TRACE

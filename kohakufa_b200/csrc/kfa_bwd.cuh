@@ -75,6 +75,7 @@ struct BwdParams {
   // statistics, whose tiles are numbered from each sequence's first row).
   const int* cu_q;
   const int* cu_k;
+  int compact;  // the grid numbers the tiles of a packed batch without gaps (decode_packed)
   // Boolean mask (kernels instantiated with MASKW), bit set = visible. mw: 32 keys per word along query
   // rows (row r of (b, h) at mw + b * mw_sb + h * mw_sh + r * mw_row), read by the dQ kernel; mwt: 32
   // queries per word along key rows, read by the dK / dV kernel. Strides of 0 broadcast; four words per
@@ -463,12 +464,19 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #endif
 
   // tile decode (groups of heads, tile-major inside); when causal the first key tiles see the most queries and come first
-  int bh, kt;  // bh over batch x K / V heads
+  int b, hk, kt;
   const int split = (!MASKW && p.n_split > 1) ? blockIdx.x % p.n_split : 0;
-  decode_tile((!MASKW && p.n_split > 1) ? blockIdx.x / p.n_split : blockIdx.x, p.B * p.Hkv, p.n_k128, bh, kt);
+  if (!MASKW && p.compact) {
+    int n_tiles;
+    if (!decode_packed<128>(blockIdx.x, p.cu_k, p.B, p.Hkv, p.n_k128, b, hk, kt, n_tiles)) return;
+  } else {
+    int bh;  // over batch x K / V heads
+    decode_tile((!MASKW && p.n_split > 1) ? blockIdx.x / p.n_split : blockIdx.x, p.B * p.Hkv, p.n_k128, bh, kt);
+    b = bh / p.Hkv;
+    hk = bh % p.Hkv;
+  }
   float* dk32 = p.dk32 + split * p.split_stride;
   float* dv32 = p.dv32 + split * p.split_stride;
-  const int b = bh / p.Hkv, hk = bh % p.Hkv;
   const int kv0 = kt * 128;  // relative to the sequence's first key
   int Sq = p.Sq, Skv = p.Skv, q_base = 0, k_base = 0, bc = b;  // bc: batch coordinate in the tensors
   if (p.cu_q != nullptr) {
@@ -857,6 +865,41 @@ __global__ void __launch_bounds__(256) kfa_bwd_sum_splits_kernel(const SumParams
   *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out[which]) + 2 * at) = w;
 }
 
+// Packed batches: zeros in the rows of up to three outputs that no CTA of the main kernels writes (rows outside every
+// sequence, of a sequence with queries but no keys, or past the longest length the plan states), instead of filling the
+// whole outputs beforehand: those were five passes over memory a step. One thread per row; usually no row is left over
+// and the kernel is its launch and a binary search.
+struct ZeroRowsParams {
+  void* out[3];
+  long long sh[3], ss[3];
+  int heads[3], rows[3], covered[3];  // covered: rows of a sequence the tiles reach
+  const int* cu[3];
+  const int* cu_need[3];  // if given: sequences that are empty here are not computed at all
+  float* lse;             // of out[0]: two planes per head (forward), or nullptr
+  int cols, n_seqs;
+};
+__global__ void __launch_bounds__(256) kfa_zero_rows_kernel(const ZeroRowsParams p) {
+  const int which = blockIdx.y;
+  const int row = blockIdx.x * 256 + threadIdx.x;
+  if (row >= p.rows[which]) return;
+  const int* cu = p.cu[which];
+  const int* need = p.cu_need[which];
+  int lo = 0, hi = p.n_seqs;  // the last sequence that starts at or before this row
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) / 2;
+    if (cu[mid] <= row) lo = mid;
+    else hi = mid;
+  }
+  const int first = cu[lo], end = min(cu[lo + 1], first + p.covered[which]);
+  if (row >= first && row < end && (need == nullptr || need[lo + 1] > need[lo])) return;
+  for (int h = 0; h < p.heads[which]; ++h) {
+    uint8_t* dst = reinterpret_cast<uint8_t*>(p.out[which]) + 2 * (h * p.sh[which] + static_cast<long long>(row) * p.ss[which]);
+    for (int c = 0; c < p.cols; c += 8) *reinterpret_cast<uint4*>(dst + 2 * c) = make_uint4(0u, 0u, 0u, 0u);
+    if (p.lse != nullptr && which == 0)
+      p.lse[2ll * h * p.rows[0] + row] = p.lse[(2ll * h + 1) * p.rows[0] + row] = 0.f;
+  }
+}
+
 // ---------------------------------------------------------------------------------------
 // dQ
 // ---------------------------------------------------------------------------------------
@@ -899,10 +942,17 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
 
-  int bh, t;
-  decode_tile(blockIdx.x, p.B * p.H, p.n_q128, bh, t);
-  const int qt = (p.P > 0) ? (p.n_q128 - 1 - t) : t;
-  const int b = bh / p.H, h = bh % p.H;
+  int b, h, t, n_q128 = p.n_q128;
+  if (!MASKW && p.compact) {
+    if (!decode_packed<128>(blockIdx.x, p.cu_q, p.B, p.H, p.n_q128, b, h, t, n_q128)) return;
+  } else {
+    int bh;
+    decode_tile(blockIdx.x, p.B * p.H, p.n_q128, bh, t);
+    b = bh / p.H;
+    h = bh % p.H;
+  }
+  const int bh = b * p.H + h;
+  const int qt = (p.P > 0) ? (n_q128 - 1 - t) : t;
   const int row0 = qt * 128;  // relative to the sequence's first row
   int Sq = p.Sq, Skv = p.Skv, q_base = 0, k_base = 0, bc = b;  // bc: batch coordinate in the tensors
   if (p.cu_q != nullptr) {

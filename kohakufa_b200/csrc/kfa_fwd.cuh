@@ -59,6 +59,7 @@ struct FwdParams {
   // the tiles of the longest sequence; CTAs past the end of a shorter one return at once.
   const int* cu_q;
   const int* cu_k;
+  int compact;  // the grid numbers the tiles of a packed batch without gaps (decode_packed)
   // Boolean mask (kernels instantiated with MASKW): 32 keys per word, bit set = visible; the words of
   // query row r of (b, h) start at mw + b * mw_sb + h * mw_sh + r * mw_row (a stride of 0 broadcasts),
   // four words per 128-key tile, zero bits for keys past Skv.
@@ -154,6 +155,40 @@ __device__ __forceinline__ void decode_tile(int idx, int n_bh, int n_tiles, int&
   bh = g * G + (r - t * gs);
 }
 
+// The same for a packed batch of up to VARLEN_COMPACT sequences, numbered without the tiles that shorter sequences do not
+// have: sequence after sequence, inside one as above. A CTA of the rectangular numbering (sequences x tiles of the
+// longest) that finds its sequence too short costs about 1 us of an SM, because it needs all of its shared memory to
+// start: with lengths spread evenly that was half of the CTAs. Every warp scans the lengths for itself (32 at a time).
+// Returns false past the last tile. n_max: tiles of the longest sequence; n_tiles: of sequence b.
+constexpr int VARLEN_COMPACT = 256;
+template <int TILE>
+__device__ __forceinline__ bool decode_packed(int idx, const int* cu, int n_seqs, int H, int n_max, int& b, int& h, int& t,
+                                              int& n_tiles) {
+  const int lane = threadIdx.x & 31;
+  int before = 0;  // tiles of the sequences before this group of 32, over all heads
+  for (int b0 = 0; b0 < n_seqs; b0 += 32) {
+    int n = 0;
+    if (b0 + lane < n_seqs) n = min((max(cu[b0 + lane + 1] - cu[b0 + lane], 0) + TILE - 1) / TILE, n_max);
+    int end = n * H;  // inclusive sum over the lanes
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, end, off);
+      if (lane >= off) end += up;
+    }
+    const unsigned past = __ballot_sync(0xffffffffu, before + end > idx);
+    if (past != 0u) {
+      const int f = __ffs(past) - 1;
+      n_tiles = __shfl_sync(0xffffffffu, n, f);
+      const int first = before + __shfl_sync(0xffffffffu, end, f) - n_tiles * H;
+      b = b0 + f;
+      decode_tile(idx - first, H, n_tiles, h, t);
+      return true;
+    }
+    before += __shfl_sync(0xffffffffu, end, 31);
+  }
+  return false;
+}
+
 // Walk over the steps of a key-major CTA without a division per step: query tile (relative to the first
 // one that sees the keys) and query head of the K / V head's group.
 struct StepWalk {
@@ -209,11 +244,16 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #endif
 
   // ---- tile decode (groups of heads, tile-major inside), heaviest query tile first when causal ----
-  int bh, t;
-  decode_tile(blockIdx.x, p.B * p.H, p.n_q_tiles, bh, t);
-  const int q_tile = (p.P > 0) ? (p.n_q_tiles - 1 - t) : t;
-  const int b = bh / p.H;
-  const int h = bh % p.H;
+  int b, h, t, n_q_tiles = p.n_q_tiles;
+  if (p.compact) {
+    if (!decode_packed<256>(blockIdx.x, p.cu_q, p.B, p.H, p.n_q_tiles, b, h, t, n_q_tiles)) return;
+  } else {
+    int bh;
+    decode_tile(blockIdx.x, p.B * p.H, p.n_q_tiles, bh, t);
+    b = bh / p.H;
+    h = bh % p.H;
+  }
+  const int q_tile = (p.P > 0) ? (n_q_tiles - 1 - t) : t;
   const int row0 = q_tile * 256;  // relative to the sequence's first row
   int Sq = p.Sq, Skv = p.Skv, q_base = 0, k_base = 0, bc = b;  // bc: batch coordinate in the tensors
   if (p.cu_q != nullptr) {

@@ -31,6 +31,7 @@ struct Api {
   decltype(&kfa_bwd_narrow) bwd_narrow = nullptr;
   decltype(&kfa_bwd_parts_bytes) bwd_parts_bytes = nullptr;
   decltype(&kfa_bwd_parts) bwd_parts = nullptr;
+  decltype(&kfa_varlen_zero_rows) varlen_zero_rows = nullptr;
 } api;
 
 PyObject* g_error = nullptr;  // kohakufa_b200._lib.KfaError
@@ -160,10 +161,13 @@ PyObject* py_inputs_ok(Args a, Py_ssize_t n) {
   return PyBool_FromLong(inputs_ok(q, k, v, q.dim() == 3 ? 3 : 4, 16));
 }
 
-// narrow_ok(q, k, v) -> bool: [B, H, S, D] and head dims that are multiples of 8
+// narrow_ok(q, k, v) -> bool: [B, H, S, D], head dims that are multiples of 8, 16-byte aligned
 PyObject* py_narrow_ok(Args a, Py_ssize_t n) {
   need(n, 3);
-  return PyBool_FromLong(inputs_ok(tensor(a[0]), tensor(a[1]), tensor(a[2]), 4, 8));
+  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]);
+  // (a tensor that does not start on 16 bytes is copied when it is widened)
+  auto aligned = [](const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; };
+  return PyBool_FromLong(inputs_ok(q, k, v, 4, 8) && aligned(q) && aligned(k) && aligned(v));
 }
 
 // forward(q, k, v, scale, block, status) -> out, lse
@@ -248,15 +252,17 @@ PyObject* py_forward_varlen(Args a, Py_ssize_t n) {
   need(n, 10);
   const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]), &cu_q = tensor(a[3]), &cu_k = tensor(a[4]);
   const c10::cuda::CUDAGuard guard(q.device());
-  // zero-filled: rows no CTA writes (a sequence with queries but no keys, rows outside cu_seqlens) read as "no
-  // visible key": output 0, statistics 0
-  at::Tensor out = at::zeros_like(q);
-  at::Tensor lse = at::zeros({1, q.size(1), 2, q.size(0)}, q.options().dtype(at::kFloat));
+  at::Tensor out = at::empty_like(q);
+  at::Tensor lse = floats(q, {1, q.size(1), 2, q.size(0)});
   const KfaTensor4 dq = desc_packed(q), dk = desc_packed(k), dv = desc_packed(v), dout = desc_packed(out);
   check(api.fwd_varlen(&dq, &dk, &dv, &dout, lse.data_ptr<float>(), cu_q.data_ptr<int32_t>(), cu_k.data_ptr<int32_t>(),
                        static_cast<int>(cu_q.numel() - 1), static_cast<int>(integer(a[5])), static_cast<int>(integer(a[6])),
                        static_cast<float>(number(a[7])), static_cast<int>(integer(a[8])), dtype_code(q),
                        tensor(a[9]).data_ptr<int32_t>(), stream_of(q)));
+  // rows no CTA writes (a sequence with queries but no keys, rows outside cu_seqlens) read as "no visible key":
+  // output 0, statistics 0
+  check(api.varlen_zero_rows(&dout, 1, cu_q.data_ptr<int32_t>(), cu_k.data_ptr<int32_t>(), static_cast<int>(cu_q.numel() - 1),
+                             static_cast<int>(integer(a[5])), static_cast<int>(integer(a[6])), lse.data_ptr<float>(), stream_of(q)));
   return pack(out, lse);
 }
 
@@ -267,7 +273,7 @@ PyObject* py_backward_varlen(Args a, Py_ssize_t n) {
                    &cu_q = tensor(a[6]), &cu_k = tensor(a[7]);
   const int64_t n_seqs = cu_q.numel() - 1, max_q = integer(a[8]), max_k = integer(a[9]);
   const c10::cuda::CUDAGuard guard(q.device());
-  at::Tensor dq = at::zeros_like(q), dk = at::zeros_like(k), dv = at::zeros_like(v);  // unwritten rows: zero gradient
+  at::Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);
   at::Tensor stats = stats_scratch(q, n_seqs, q.size(1), max_q);
   const KfaTensor4 d[8] = {desc_packed(q), desc_packed(k), desc_packed(v),  desc_packed(o),
                            desc_packed(g), desc_packed(dq), desc_packed(dk), desc_packed(dv)};
@@ -275,6 +281,8 @@ PyObject* py_backward_varlen(Args a, Py_ssize_t n) {
                        cu_q.data_ptr<int32_t>(), cu_k.data_ptr<int32_t>(), static_cast<int>(n_seqs), static_cast<int>(max_q),
                        static_cast<int>(max_k), static_cast<float>(number(a[10])), static_cast<int>(integer(a[11])),
                        dtype_code(q), tensor(a[12]).data_ptr<int32_t>(), stream_of(q)));
+  check(api.varlen_zero_rows(d + 5, 3, cu_q.data_ptr<int32_t>(), cu_k.data_ptr<int32_t>(), static_cast<int>(n_seqs),
+                             static_cast<int>(max_q), static_cast<int>(max_k), nullptr, stream_of(q)));  // the other rows: zero
   return pack(dq, dk, dv);
 }
 
@@ -321,6 +329,7 @@ PyObject* py_bind(Args a, Py_ssize_t n) {
   take("kfa_bwd_narrow", api.bwd_narrow);
   take("kfa_bwd_parts_bytes", api.bwd_parts_bytes);
   take("kfa_bwd_parts", api.bwd_parts);
+  take("kfa_varlen_zero_rows", api.varlen_zero_rows);
   Py_INCREF(a[0]);
   Py_XDECREF(g_error);
   g_error = a[0];

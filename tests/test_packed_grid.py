@@ -1,0 +1,66 @@
+"""Packed batches: the numbering of tiles without gaps, the rectangular one, and the rows no sequence owns."""
+
+import pytest
+import torch
+
+from kohakufa_b200 import _lib, attention_varlen, op, varlen_plan
+
+pytestmark = pytest.mark.gpu
+
+
+def run(q, k, v, dout, cu, plan, **kw):
+    qkv = [t.detach().requires_grad_() for t in (q, k, v)]
+    out = attention_varlen(*qkv, cu, cu, plan=plan, **kw)
+    grads = torch.autograd.grad(out, qkv, dout)
+    assert _lib.device_status() == 0
+    return [out.detach(), *grads]
+
+
+def packed(lengths, heads, kv_heads, dim, extra=0):
+    gen = torch.Generator().manual_seed(len(lengths))
+    total = sum(lengths) + extra
+    ts = [torch.randn(total, h, dim, generator=gen).bfloat16().cuda() for h in (heads, kv_heads, kv_heads, heads)]
+    return *ts, torch.tensor([0, *lengths]).cumsum(0).int().cuda()
+
+
+@pytest.mark.parametrize("n_seqs,longest", [(1, 1), (31, 300), (33, 700), (256, 90), (257, 90), (300, 400)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_batch_equals_its_halves(n_seqs, longest, causal):
+    """A sequence's results do not depend on the batch it is in, so a batch equals its two halves bit for bit, also
+    where the batch is numbered in the rectangular way (more than 256 sequences) and the halves without gaps."""
+    gen = torch.Generator().manual_seed(longest)
+    lengths = torch.randint(0, longest + 1, (n_seqs,), generator=gen).tolist()
+    lengths[n_seqs // 2] = longest
+    q, k, v, dout, cu = packed(lengths, 4, 2, 64)
+    whole = run(q, k, v, dout, cu, varlen_plan(cu, cu), causal=causal)
+    cut = (n_seqs + 1) // 2
+    parts = []
+    for a, b in ((0, cut), (cut, n_seqs)):
+        if a == b or sum(lengths[a:b]) == 0:
+            continue
+        rows = slice(int(cu[a]), int(cu[b]))
+        sub = (cu[a : b + 1] - cu[a]).contiguous()
+        parts.append(run(q[rows], k[rows], v[rows], dout[rows], sub, varlen_plan(sub, sub), causal=causal))
+    for i, w in enumerate(whole):
+        assert torch.equal(w, torch.cat([p[i] for p in parts]))
+
+
+@pytest.mark.parametrize("n_seqs", [3, 300])
+def test_rows_outside_the_sequences_are_zero(n_seqs):
+    """Freed memory full of NaN is what fresh outputs come from; rows before, after and between the computed ones
+    still read as zero, and so do the statistics."""
+    lengths = [200, 300, 129] + [2] * (n_seqs - 3)
+    q, k, v, dout, cu = packed(lengths, 2, 2, 64, extra=40)
+    cu = cu + 7
+    total = q.shape[0]
+    junk = [torch.full((total, 2, 64), float("nan"), dtype=q.dtype, device="cuda") for _ in range(8)]
+    lse = [torch.full((1, 2, 2, total), float("nan"), device="cuda") for _ in range(2)]
+    del junk, lse
+    out, dq, dk, dv = run(q, k, v, dout, cu, varlen_plan(cu, cu), causal=True)
+    rows = torch.arange(total, device="cuda")
+    inside = (rows >= cu[0]) & (rows < cu[-1])
+    for t in (out, dq, dk, dv):
+        assert bool(torch.isfinite(t).all()) and not bool(t[~inside].any())
+        assert float(t[inside].abs().flatten(1).sum(-1).gt(0).float().mean()) > 0.9
+    direct = op.varlen_fwd_op(q, k, v, cu, cu, 300, 300, 64**-0.5, 1)
+    assert torch.equal(direct[0], out) and not bool(direct[1][..., ~inside].any())
