@@ -70,6 +70,12 @@ def test_narrow_leaves_other_inputs_alone():
     flat = torch.randn(2, 64, 4 * 40 + 4).half().cuda()[..., :160].unflatten(-1, (4, 40)).transpose(1, 2)
     assert not op.narrow(flat, k, v)  # rows that do not start on 16 bytes
     assert attention(flat, k, v).shape == flat.shape
+    shifted = torch.randn(2 * 64 * 4 * 40 + 4).half().cuda()[4:].view(2, 64, 4, 40).transpose(1, 2)  # starts on 8 bytes
+    assert not op.narrow(q, shifted, v) and not op.narrow(shifted, k, v)
+    assert attention(q, shifted, v).shape == q.shape
+    want = torch.autograd.grad(attention(q, k, v), (q, k, v), shifted.contiguous())
+    for a, b in zip(torch.autograd.grad(attention(q, k, v), (q, k, v), shifted), want):
+        assert float((a - b).float().norm()) <= 1e-3 * float(b.float().norm())
     for bad in (lambda: op.attention(q, k, v), lambda: attention(q, k[:, :3], v[:, :3])):
         with pytest.raises(ValueError):
             bad()
