@@ -297,8 +297,9 @@ def selftest() -> str:
 
 def plain_eager(*tensors: torch.Tensor) -> bool:
     """Whether a call on these tensors is plain eager execution: no compiler or tracer, no dispatch or function
-    mode, no ``torch.func`` transform, no forward-mode level, no tensor subclass. Only then may it pass the
-    dispatcher by; everything else sees the registered custom ops."""
+    mode, no ``torch.func`` transform, no forward-mode level, no tensor subclass and no tensor that only the
+    dispatcher can resolve (batched gradients, negative views, zero tensors). Only then may it pass the dispatcher by;
+    everything else sees the registered custom ops."""
     if torch.compiler.is_compiling():
         return False
     for t in tensors:
@@ -310,4 +311,5 @@ def plain_eager(*tensors: torch.Tensor) -> bool:
         or torch._C._are_functorch_transforms_active()
         or torch.autograd.forward_ad._current_level >= 0
         or torch._C._get_tracing_state() is not None
+        or not host().plain(*tensors)
     )

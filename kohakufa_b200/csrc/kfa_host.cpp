@@ -154,6 +154,19 @@ void need(Py_ssize_t got, Py_ssize_t want) {
 
 using Args = PyObject* const*;
 
+// plain(*tensors) -> bool: whether what each tensor's address points to is its value. Batched tensors (gradients of
+// `is_grads_batched`), pending negations and zero tensors are torch.Tensor too, but only the dispatcher resolves them.
+PyObject* py_plain(Args a, Py_ssize_t n) {
+  using c10::DispatchKey;
+  static const uint64_t plain =
+      c10::DispatchKeySet({DispatchKey::CPU, DispatchKey::CUDA, DispatchKey::ADInplaceOrView, DispatchKey::AutogradCPU,
+                           DispatchKey::AutogradCUDA, DispatchKey::AutocastCPU, DispatchKey::AutocastCUDA})
+          .raw_repr();
+  for (Py_ssize_t i = 0; i < n; ++i)
+    if (tensor(a[i]).key_set().raw_repr() & ~plain) Py_RETURN_FALSE;
+  Py_RETURN_TRUE;
+}
+
 // inputs_ok(q, k, v) -> bool: head dims that are multiples of 16
 PyObject* py_inputs_ok(Args a, Py_ssize_t n) {
   need(n, 3);
@@ -350,7 +363,7 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 #define KFA_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(entry<py_##name>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
-    KFA_METHOD(bind),           KFA_METHOD(inputs_ok),       KFA_METHOD(narrow_ok), KFA_METHOD(forward),        KFA_METHOD(backward),
+    KFA_METHOD(bind),           KFA_METHOD(plain),           KFA_METHOD(inputs_ok),      KFA_METHOD(narrow_ok), KFA_METHOD(forward), KFA_METHOD(backward),
     KFA_METHOD(forward_masked), KFA_METHOD(backward_masked), KFA_METHOD(forward_varlen), KFA_METHOD(backward_varlen),
     KFA_METHOD(pack_mask),      {nullptr, nullptr, 0, nullptr},
 };

@@ -39,6 +39,27 @@ def test_plain_eager_is_plain():
     assert _lib.plain_eager(t)
 
 
+def test_plain_eager_leaves_to_the_dispatcher_what_it_resolves():
+    t = torch.ones(3, 2)
+    assert not _lib.plain_eager(torch._neg_view(t)) and not _lib.plain_eager(t, torch._efficientzerotensor(2))
+    seen = []
+
+    class Double(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x):
+            return 2 * x
+
+        @staticmethod
+        def backward(ctx, g):
+            seen.append(_lib.plain_eager(g))
+            return 2 * g
+
+    x = torch.ones(2, requires_grad=True)
+    torch.autograd.grad(Double.apply(x), x, t, is_grads_batched=True)
+    assert seen == [False]
+    assert _lib.plain_eager(t, x)
+
+
 def inputs(dim=128, seq=200, heads=4, kv_heads=2, packed=False):
     gen = torch.Generator().manual_seed(dim + seq)
     shape = (seq, heads, dim) if packed else (2, seq, heads, dim)
@@ -104,6 +125,33 @@ def test_direct_path_and_autograd_features():
         q.mul_(1.0)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         out.backward(dout)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["plain", "mask", "varlen"])
+def test_batched_gradients(kind):
+    """``is_grads_batched`` gives the rows of one call per gradient (the split kernels repeat bit for bit)."""
+    (q, k, v), dout = inputs(packed=kind == "varlen")
+    if kind == "varlen":
+        cu = torch.tensor([0, 70, 200], dtype=torch.int32, device="cuda")
+        out = attention_varlen(q, k, v, cu, cu)
+    else:
+        out = attention(q, k, v, mask=torch.ones(200, 200, dtype=torch.bool, device="cuda") if kind == "mask" else None)
+    douts = torch.stack([dout, -dout, 2 * dout])
+    got = torch.autograd.grad(out, (q, k, v), douts, is_grads_batched=True, retain_graph=True)
+    for i, g in enumerate(douts):
+        for a, b in zip(got, torch.autograd.grad(out, (q, k, v), g, retain_graph=True)):
+            assert torch.equal(a[i], b)
+
+
+@pytest.mark.gpu
+def test_negative_views():
+    (q, k, v), dout = inputs()
+    with torch.no_grad():
+        assert torch.equal(attention(torch._neg_view(q), k, v), attention(-q, k, v))
+    out = attention(q, k, v)
+    got = torch.autograd.grad(out, (q, k, v), torch._neg_view(dout), retain_graph=True)
+    assert all(torch.equal(a, b) for a, b in zip(got, torch.autograd.grad(out, (q, k, v), -dout)))
 
 
 @pytest.mark.gpu
