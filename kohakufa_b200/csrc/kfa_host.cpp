@@ -174,13 +174,14 @@ PyObject* py_inputs_ok(Args a, Py_ssize_t n) {
   return PyBool_FromLong(inputs_ok(q, k, v, q.dim() == 3 ? 3 : 4, 16));
 }
 
+bool aligned16(const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+
 // narrow_ok(q, k, v) -> bool: [B, H, S, D], head dims that are multiples of 8, 16-byte aligned
 PyObject* py_narrow_ok(Args a, Py_ssize_t n) {
   need(n, 3);
   const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]);
   // (a tensor that does not start on 16 bytes is copied when it is widened)
-  auto aligned = [](const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; };
-  return PyBool_FromLong(inputs_ok(q, k, v, 4, 8) && aligned(q) && aligned(k) && aligned(v));
+  return PyBool_FromLong(inputs_ok(q, k, v, 4, 8) && aligned16(q) && aligned16(k) && aligned16(v));
 }
 
 // forward(q, k, v, scale, block, status) -> out, lse
@@ -201,12 +202,14 @@ PyObject* py_forward(Args a, Py_ssize_t n) {
 // fused: 1 the fused kernels, 0 the split ones, 2 the fused ones unless the split ones can share out their steps
 PyObject* py_backward(Args a, Py_ssize_t n) {
   need(n, 10);
-  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]), &o = tensor(a[3]), &g = tensor(a[4]), &lse = tensor(a[5]);
+  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]), &o = tensor(a[3]), &lse = tensor(a[5]);
+  at::Tensor g = tensor(a[4]);
   const float scale = static_cast<float>(number(a[6]));
   const int block = static_cast<int>(integer(a[7]));
   int* status = tensor(a[8]).data_ptr<int32_t>();
   const int64_t fused = integer(a[9]);
   const c10::cuda::CUDAGuard guard(q.device());
+  if (q.size(3) % 16 && !aligned16(g)) g = g.clone();  // (widening copied it)
   at::Tensor dq = bshd_like(q), dk = bshd_like(k), dv = bshd_like(v);
   at::Tensor stats = stats_scratch(q, q.size(0), q.size(1), q.size(2));
   const KfaTensor4 d[8] = {desc(q), desc(k), desc(v), desc(o), desc(g), desc(dq), desc(dk), desc(dv)};

@@ -211,8 +211,6 @@ class _Attention(Function):
         q, k, v, out, lse = ctx.saved_tensors
         if not _strides_ok(dout):
             dout = dout.contiguous()
-        elif q.shape[-1] % 16 and dout.data_ptr() % 16:  # (widening would have copied it)
-            dout = dout.clone()
         if torch.is_grad_enabled() or not _lib.plain_eager(q, k, v, out, dout, lse):
             grads = attention_bwd_op(q, k, v, out, dout, lse, ctx.scale, ctx.block)
         else:

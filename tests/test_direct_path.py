@@ -128,10 +128,10 @@ def test_direct_path_and_autograd_features():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("kind", ["plain", "mask", "varlen"])
-def test_batched_gradients(kind):
+@pytest.mark.parametrize("kind,dim", [("plain", 128), ("plain", 48), ("plain", 40), ("mask", 128), ("varlen", 128)])
+def test_batched_gradients(kind, dim):
     """``is_grads_batched`` gives the rows of one call per gradient (the split kernels repeat bit for bit)."""
-    (q, k, v), dout = inputs(packed=kind == "varlen")
+    (q, k, v), dout = inputs(dim, packed=kind == "varlen")
     if kind == "varlen":
         cu = torch.tensor([0, 70, 200], dtype=torch.int32, device="cuda")
         out = attention_varlen(q, k, v, cu, cu)
