@@ -13,6 +13,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <string>
+
 #include "../../include/kfa.h"
 
 namespace {
@@ -56,11 +58,23 @@ int64_t integer(PyObject* o) {
   return v;
 }
 
+struct KfaFailure {  // becomes a KfaError once the GIL is held again
+  int rc;
+  std::string message;
+};
+
 void check(int rc) {
-  if (rc == 0) return;
-  PyErr_Format(g_error ? g_error : PyExc_RuntimeError, "libkfa error %d: %s", rc, api.last_error());
-  throw PyError();
+  if (rc != 0) throw KfaFailure{rc, api.last_error()};  // (the message is this thread's)
 }
+
+// Allocations and launches run without the GIL: an allocation may have to wait for the device, a launch for room in the
+// stream's queue, and what they wait for may need another Python thread.
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  NoGil() = default;
+  NoGil(const NoGil&) = delete;
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
 
 KfaTensor4 desc(const at::Tensor& t) {
   TORCH_CHECK(t.dim() == 4 && t.is_cuda(), "a 4-D CUDA tensor");
@@ -187,14 +201,19 @@ PyObject* py_narrow_ok(Args a, Py_ssize_t n) {
 // forward(q, k, v, scale, block, status) -> out, lse
 PyObject* py_forward(Args a, Py_ssize_t n) {
   need(n, 6);
-  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]);
-  const c10::cuda::CUDAGuard guard(q.device());
-  at::Tensor out = bshd_like(q);
-  at::Tensor lse = floats(q, {q.size(0), q.size(1), 2, q.size(2)});
-  const KfaTensor4 dq = desc(q), dk = desc(k), dv = desc(v), dout = desc(out);
-  const auto call = q.size(3) % 16 ? api.fwd_narrow : api.fwd;
-  check(call(&dq, &dk, &dv, &dout, lse.data_ptr<float>(), static_cast<float>(number(a[3])), static_cast<int>(integer(a[4])),
-             dtype_code(q), tensor(a[5]).data_ptr<int32_t>(), stream_of(q)));
+  const at::Tensor q = tensor(a[0]), k = tensor(a[1]), v = tensor(a[2]), status = tensor(a[5]);
+  const float scale = static_cast<float>(number(a[3]));
+  const int block = static_cast<int>(integer(a[4]));
+  at::Tensor out, lse;
+  {
+    const NoGil released;
+    const c10::cuda::CUDAGuard guard(q.device());
+    out = bshd_like(q);
+    lse = floats(q, {q.size(0), q.size(1), 2, q.size(2)});
+    const KfaTensor4 dq = desc(q), dk = desc(k), dv = desc(v), dout = desc(out);
+    const auto call = q.size(3) % 16 ? api.fwd_narrow : api.fwd;
+    check(call(&dq, &dk, &dv, &dout, lse.data_ptr<float>(), scale, block, dtype_code(q), status.data_ptr<int32_t>(), stream_of(q)));
+  }
   return pack(out, lse);
 }
 
@@ -202,32 +221,38 @@ PyObject* py_forward(Args a, Py_ssize_t n) {
 // fused: 1 the fused kernels, 0 the split ones, 2 the fused ones unless the split ones can share out their steps
 PyObject* py_backward(Args a, Py_ssize_t n) {
   need(n, 10);
-  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]), &o = tensor(a[3]), &lse = tensor(a[5]);
+  const at::Tensor q = tensor(a[0]), k = tensor(a[1]), v = tensor(a[2]), o = tensor(a[3]), lse = tensor(a[5]), status = tensor(a[8]);
   at::Tensor g = tensor(a[4]);
   const float scale = static_cast<float>(number(a[6]));
   const int block = static_cast<int>(integer(a[7]));
-  int* status = tensor(a[8]).data_ptr<int32_t>();
   const int64_t fused = integer(a[9]);
-  const c10::cuda::CUDAGuard guard(q.device());
-  if (q.size(3) % 16 && !aligned16(g)) g = g.clone();  // (widening copied it)
-  at::Tensor dq = bshd_like(q), dk = bshd_like(k), dv = bshd_like(v);
-  at::Tensor stats = stats_scratch(q, q.size(0), q.size(1), q.size(2));
-  const KfaTensor4 d[8] = {desc(q), desc(k), desc(v), desc(o), desc(g), desc(dq), desc(dk), desc(dv)};
-  const int64_t parts_bytes = (fused == 1) ? 0 : api.bwd_parts_bytes(d, d + 1);
-  if (parts_bytes > 0) {
-    at::Tensor parts = floats(q, {parts_bytes / 4});
-    check(api.bwd_parts(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), parts.data_ptr<float>(),
-                        d + 5, d + 6, d + 7, scale, block, dtype_code(q), status, stream_of(q)));
-  } else if (fused) {
-    at::Tensor acc = floats(q, {q.size(0) * q.size(1) * ((q.size(2) + 127) / 128) * 128 * ((q.size(3) + 15) / 16 * 16)});
-    check((q.size(3) % 16 ? api.bwd_narrow : api.bwd_fused)(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), acc.data_ptr<float>(),
-                        d + 5, d + 6, d + 7, scale, block, dtype_code(q), status, stream_of(q)));
-  } else if (q.size(3) % 16) {
-    check(api.bwd_narrow(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), nullptr, d + 5, d + 6,
-                         d + 7, scale, block, dtype_code(q), status, stream_of(q)));
-  } else {
-    check(api.bwd(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), d + 5, d + 6, d + 7, scale,
-                  block, dtype_code(q), status, stream_of(q)));
+  at::Tensor dq, dk, dv;
+  {
+    const NoGil released;
+    const c10::cuda::CUDAGuard guard(q.device());
+    if (q.size(3) % 16 && !aligned16(g)) g = g.clone();  // (widening copied it)
+    dq = bshd_like(q);
+    dk = bshd_like(k);
+    dv = bshd_like(v);
+    at::Tensor stats = stats_scratch(q, q.size(0), q.size(1), q.size(2));
+    const KfaTensor4 d[8] = {desc(q), desc(k), desc(v), desc(o), desc(g), desc(dq), desc(dk), desc(dv)};
+    float *l = lse.data_ptr<float>(), *st = stats.data_ptr<float>();
+    int* word = status.data_ptr<int32_t>();
+    const int64_t parts_bytes = (fused == 1) ? 0 : api.bwd_parts_bytes(d, d + 1);
+    if (parts_bytes > 0) {
+      at::Tensor parts = floats(q, {parts_bytes / 4});
+      check(api.bwd_parts(d, d + 1, d + 2, d + 3, d + 4, l, st, parts.data_ptr<float>(), d + 5, d + 6, d + 7, scale, block,
+                          dtype_code(q), word, stream_of(q)));
+    } else if (fused) {
+      at::Tensor acc = floats(q, {q.size(0) * q.size(1) * ((q.size(2) + 127) / 128) * 128 * ((q.size(3) + 15) / 16 * 16)});
+      check((q.size(3) % 16 ? api.bwd_narrow : api.bwd_fused)(d, d + 1, d + 2, d + 3, d + 4, l, st, acc.data_ptr<float>(), d + 5,
+                                                              d + 6, d + 7, scale, block, dtype_code(q), word, stream_of(q)));
+    } else if (q.size(3) % 16) {
+      check(api.bwd_narrow(d, d + 1, d + 2, d + 3, d + 4, l, st, nullptr, d + 5, d + 6, d + 7, scale, block, dtype_code(q), word,
+                           stream_of(q)));
+    } else {
+      check(api.bwd(d, d + 1, d + 2, d + 3, d + 4, l, st, d + 5, d + 6, d + 7, scale, block, dtype_code(q), word, stream_of(q)));
+    }
   }
   return pack(dq, dk, dv);
 }
@@ -235,89 +260,120 @@ PyObject* py_backward(Args a, Py_ssize_t n) {
 // forward_masked(q, k, v, words, tiles, scale, status) -> out, lse
 PyObject* py_forward_masked(Args a, Py_ssize_t n) {
   need(n, 7);
-  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]);
-  const c10::cuda::CUDAGuard guard(q.device());
-  at::Tensor out = bshd_like(q);
-  at::Tensor lse = floats(q, {q.size(0), q.size(1), 2, q.size(2)});
-  const KfaTensor4 dq = desc(q), dk = desc(k), dv = desc(v), dout = desc(out);
-  const KfaMaskWords w = mask_words(tensor(a[3]));
-  const KfaMaskTiles t = mask_tiles(tensor(a[4]));
-  check(api.fwd_masked(&dq, &dk, &dv, &dout, lse.data_ptr<float>(), &w, &t, static_cast<float>(number(a[5])), dtype_code(q),
-                       tensor(a[6]).data_ptr<int32_t>(), stream_of(q)));
+  const at::Tensor q = tensor(a[0]), k = tensor(a[1]), v = tensor(a[2]), words = tensor(a[3]), tiles = tensor(a[4]),
+                   status = tensor(a[6]);
+  const float scale = static_cast<float>(number(a[5]));
+  at::Tensor out, lse;
+  {
+    const NoGil released;
+    const c10::cuda::CUDAGuard guard(q.device());
+    out = bshd_like(q);
+    lse = floats(q, {q.size(0), q.size(1), 2, q.size(2)});
+    const KfaTensor4 dq = desc(q), dk = desc(k), dv = desc(v), dout = desc(out);
+    const KfaMaskWords w = mask_words(words);
+    const KfaMaskTiles t = mask_tiles(tiles);
+    check(api.fwd_masked(&dq, &dk, &dv, &dout, lse.data_ptr<float>(), &w, &t, scale, dtype_code(q), status.data_ptr<int32_t>(),
+                         stream_of(q)));
+  }
   return pack(out, lse);
 }
 
 // backward_masked(q, k, v, out, dout, lse, words, words_t, tiles, scale, status) -> dq, dk, dv
 PyObject* py_backward_masked(Args a, Py_ssize_t n) {
   need(n, 11);
-  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]), &o = tensor(a[3]), &g = tensor(a[4]), &lse = tensor(a[5]);
-  const c10::cuda::CUDAGuard guard(q.device());
-  at::Tensor dq = bshd_like(q), dk = bshd_like(k), dv = bshd_like(v);
-  at::Tensor stats = stats_scratch(q, q.size(0), q.size(1), q.size(2));
-  const KfaTensor4 d[8] = {desc(q), desc(k), desc(v), desc(o), desc(g), desc(dq), desc(dk), desc(dv)};
-  const KfaMaskWords w = mask_words(tensor(a[6])), wt = mask_words(tensor(a[7]));
-  const KfaMaskTiles t = mask_tiles(tensor(a[8]));
-  check(api.bwd_masked(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), d + 5, d + 6, d + 7, &w,
-                       &wt, &t, static_cast<float>(number(a[9])), dtype_code(q), tensor(a[10]).data_ptr<int32_t>(),
-                       stream_of(q)));
+  const at::Tensor q = tensor(a[0]), k = tensor(a[1]), v = tensor(a[2]), o = tensor(a[3]), g = tensor(a[4]), lse = tensor(a[5]),
+                   words = tensor(a[6]), words_t = tensor(a[7]), tiles = tensor(a[8]), status = tensor(a[10]);
+  const float scale = static_cast<float>(number(a[9]));
+  at::Tensor dq, dk, dv;
+  {
+    const NoGil released;
+    const c10::cuda::CUDAGuard guard(q.device());
+    dq = bshd_like(q);
+    dk = bshd_like(k);
+    dv = bshd_like(v);
+    at::Tensor stats = stats_scratch(q, q.size(0), q.size(1), q.size(2));
+    const KfaTensor4 d[8] = {desc(q), desc(k), desc(v), desc(o), desc(g), desc(dq), desc(dk), desc(dv)};
+    const KfaMaskWords w = mask_words(words), wt = mask_words(words_t);
+    const KfaMaskTiles t = mask_tiles(tiles);
+    check(api.bwd_masked(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), d + 5, d + 6, d + 7, &w,
+                         &wt, &t, scale, dtype_code(q), status.data_ptr<int32_t>(), stream_of(q)));
+  }
   return pack(dq, dk, dv);
 }
 
 // forward_varlen(q, k, v, cu_q, cu_k, max_q, max_k, scale, block, status) -> out, lse
 PyObject* py_forward_varlen(Args a, Py_ssize_t n) {
   need(n, 10);
-  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]), &cu_q = tensor(a[3]), &cu_k = tensor(a[4]);
-  const c10::cuda::CUDAGuard guard(q.device());
-  at::Tensor out = at::empty_like(q);
-  at::Tensor lse = floats(q, {1, q.size(1), 2, q.size(0)});
-  const KfaTensor4 dq = desc_packed(q), dk = desc_packed(k), dv = desc_packed(v), dout = desc_packed(out);
-  check(api.fwd_varlen(&dq, &dk, &dv, &dout, lse.data_ptr<float>(), cu_q.data_ptr<int32_t>(), cu_k.data_ptr<int32_t>(),
-                       static_cast<int>(cu_q.numel() - 1), static_cast<int>(integer(a[5])), static_cast<int>(integer(a[6])),
-                       static_cast<float>(number(a[7])), static_cast<int>(integer(a[8])), dtype_code(q),
-                       tensor(a[9]).data_ptr<int32_t>(), stream_of(q)));
-  // rows no CTA writes (a sequence with queries but no keys, rows outside cu_seqlens) read as "no visible key":
-  // output 0, statistics 0
-  check(api.varlen_zero_rows(&dout, 1, cu_q.data_ptr<int32_t>(), cu_k.data_ptr<int32_t>(), static_cast<int>(cu_q.numel() - 1),
-                             static_cast<int>(integer(a[5])), static_cast<int>(integer(a[6])), lse.data_ptr<float>(), stream_of(q)));
+  const at::Tensor q = tensor(a[0]), k = tensor(a[1]), v = tensor(a[2]), cu_q = tensor(a[3]), cu_k = tensor(a[4]),
+                   status = tensor(a[9]);
+  const int max_q = static_cast<int>(integer(a[5])), max_k = static_cast<int>(integer(a[6]));
+  const float scale = static_cast<float>(number(a[7]));
+  const int block = static_cast<int>(integer(a[8]));
+  at::Tensor out, lse;
+  {
+    const NoGil released;
+    const c10::cuda::CUDAGuard guard(q.device());
+    const int32_t *cq = cu_q.data_ptr<int32_t>(), *ck = cu_k.data_ptr<int32_t>();
+    const int n_seqs = static_cast<int>(cu_q.numel() - 1);
+    out = at::empty_like(q);
+    lse = floats(q, {1, q.size(1), 2, q.size(0)});
+    const KfaTensor4 dq = desc_packed(q), dk = desc_packed(k), dv = desc_packed(v), dout = desc_packed(out);
+    check(api.fwd_varlen(&dq, &dk, &dv, &dout, lse.data_ptr<float>(), cq, ck, n_seqs, max_q, max_k, scale, block, dtype_code(q),
+                         status.data_ptr<int32_t>(), stream_of(q)));
+    // rows no CTA writes (a sequence with queries but no keys, rows outside cu_seqlens) read as "no visible key":
+    // output 0, statistics 0
+    check(api.varlen_zero_rows(&dout, 1, cq, ck, n_seqs, max_q, max_k, lse.data_ptr<float>(), stream_of(q)));
+  }
   return pack(out, lse);
 }
 
 // backward_varlen(q, k, v, out, dout, lse, cu_q, cu_k, max_q, max_k, scale, block, status) -> dq, dk, dv
 PyObject* py_backward_varlen(Args a, Py_ssize_t n) {
   need(n, 13);
-  const at::Tensor &q = tensor(a[0]), &k = tensor(a[1]), &v = tensor(a[2]), &o = tensor(a[3]), &g = tensor(a[4]), &lse = tensor(a[5]),
-                   &cu_q = tensor(a[6]), &cu_k = tensor(a[7]);
-  const int64_t n_seqs = cu_q.numel() - 1, max_q = integer(a[8]), max_k = integer(a[9]);
-  const c10::cuda::CUDAGuard guard(q.device());
-  at::Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);
-  at::Tensor stats = stats_scratch(q, n_seqs, q.size(1), max_q);
-  const KfaTensor4 d[8] = {desc_packed(q), desc_packed(k), desc_packed(v),  desc_packed(o),
-                           desc_packed(g), desc_packed(dq), desc_packed(dk), desc_packed(dv)};
-  check(api.bwd_varlen(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), d + 5, d + 6, d + 7,
-                       cu_q.data_ptr<int32_t>(), cu_k.data_ptr<int32_t>(), static_cast<int>(n_seqs), static_cast<int>(max_q),
-                       static_cast<int>(max_k), static_cast<float>(number(a[10])), static_cast<int>(integer(a[11])),
-                       dtype_code(q), tensor(a[12]).data_ptr<int32_t>(), stream_of(q)));
-  check(api.varlen_zero_rows(d + 5, 3, cu_q.data_ptr<int32_t>(), cu_k.data_ptr<int32_t>(), static_cast<int>(n_seqs),
-                             static_cast<int>(max_q), static_cast<int>(max_k), nullptr, stream_of(q)));  // the other rows: zero
+  const at::Tensor q = tensor(a[0]), k = tensor(a[1]), v = tensor(a[2]), o = tensor(a[3]), g = tensor(a[4]), lse = tensor(a[5]),
+                   cu_q = tensor(a[6]), cu_k = tensor(a[7]), status = tensor(a[12]);
+  const int max_q = static_cast<int>(integer(a[8])), max_k = static_cast<int>(integer(a[9]));
+  const float scale = static_cast<float>(number(a[10]));
+  const int block = static_cast<int>(integer(a[11]));
+  at::Tensor dq, dk, dv;
+  {
+    const NoGil released;
+    const c10::cuda::CUDAGuard guard(q.device());
+    const int32_t *cq = cu_q.data_ptr<int32_t>(), *ck = cu_k.data_ptr<int32_t>();
+    const int n_seqs = static_cast<int>(cu_q.numel() - 1);
+    dq = at::empty_like(q);
+    dk = at::empty_like(k);
+    dv = at::empty_like(v);
+    at::Tensor stats = stats_scratch(q, n_seqs, q.size(1), max_q);
+    const KfaTensor4 d[8] = {desc_packed(q), desc_packed(k), desc_packed(v),  desc_packed(o),
+                             desc_packed(g), desc_packed(dq), desc_packed(dk), desc_packed(dv)};
+    check(api.bwd_varlen(d, d + 1, d + 2, d + 3, d + 4, lse.data_ptr<float>(), stats.data_ptr<float>(), d + 5, d + 6, d + 7, cq,
+                         ck, n_seqs, max_q, max_k, scale, block, dtype_code(q), status.data_ptr<int32_t>(), stream_of(q)));
+    check(api.varlen_zero_rows(d + 5, 3, cq, ck, n_seqs, max_q, max_k, nullptr, stream_of(q)));  // the other rows: zero
+  }
   return pack(dq, dk, dv);
 }
 
 // pack_mask(mask [Bm, Hm, Sq, Skv] bool or bytes, any strides, s_q, s_kv) -> words, words_t, tiles
 PyObject* py_pack_mask(Args a, Py_ssize_t n) {
   need(n, 3);
-  const at::Tensor& m = tensor(a[0]);
+  const at::Tensor m = tensor(a[0]);
   const int64_t s_q = integer(a[1]), s_kv = integer(a[2]);
-  TORCH_CHECK(m.dim() == 4 && m.is_cuda() && m.element_size() == 1, "a 4-D mask of bytes on the GPU");
-  const c10::cuda::CUDAGuard guard(m.device());
-  const int64_t bm = m.size(0), hm = m.size(1), tq = (s_q + 127) / 128, tk = (s_kv + 127) / 128;
-  const auto ints = m.options().dtype(at::kInt);
-  at::Tensor words = at::empty({bm, hm, s_q, 4 * tk}, ints);
-  at::Tensor words_t = at::empty({bm, hm, s_kv, 4 * tq}, ints);
-  at::Tensor tiles = at::empty({bm, hm, tq, tk}, ints);
-  const int64_t strides[4] = {m.stride(0), m.stride(1), m.stride(2), m.stride(3)};
-  check(api.pack_mask(m.data_ptr(), strides, static_cast<int>(bm), static_cast<int>(hm), static_cast<int>(s_q),
-                      static_cast<int>(s_kv), words.data_ptr<int32_t>(), words_t.data_ptr<int32_t>(),
-                      tiles.data_ptr<int32_t>(), stream_of(m)));
+  at::Tensor words, words_t, tiles;
+  {
+    const NoGil released;
+    TORCH_CHECK(m.dim() == 4 && m.is_cuda() && m.element_size() == 1, "a 4-D mask of bytes on the GPU");
+    const c10::cuda::CUDAGuard guard(m.device());
+    const int64_t bm = m.size(0), hm = m.size(1), tq = (s_q + 127) / 128, tk = (s_kv + 127) / 128;
+    const auto ints = m.options().dtype(at::kInt);
+    words = at::empty({bm, hm, s_q, 4 * tk}, ints);
+    words_t = at::empty({bm, hm, s_kv, 4 * tq}, ints);
+    tiles = at::empty({bm, hm, tq, tk}, ints);
+    const int64_t strides[4] = {m.stride(0), m.stride(1), m.stride(2), m.stride(3)};
+    check(api.pack_mask(m.data_ptr(), strides, static_cast<int>(bm), static_cast<int>(hm), static_cast<int>(s_q),
+                        static_cast<int>(s_kv), words.data_ptr<int32_t>(), words_t.data_ptr<int32_t>(),
+                        tiles.data_ptr<int32_t>(), stream_of(m)));
+  }
   return pack(words, words_t, tiles);
 }
 
@@ -359,6 +415,9 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
   try {
     return F(args, n);
   } catch (const PyError&) {
+    return nullptr;
+  } catch (const KfaFailure& e) {
+    PyErr_Format(g_error ? g_error : PyExc_RuntimeError, "libkfa error %d: %s", e.rc, e.message.c_str());
     return nullptr;
   }
   END_HANDLE_TH_ERRORS

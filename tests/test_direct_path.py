@@ -1,5 +1,8 @@
 """The direct launch path of plain eager calls: taken only there, and equal to the custom ops."""
 
+import threading
+import time
+
 import pytest
 import torch
 
@@ -152,6 +155,32 @@ def test_negative_views():
     out = attention(q, k, v)
     got = torch.autograd.grad(out, (q, k, v), torch._neg_view(dout), retain_graph=True)
     assert all(torch.equal(a, b) for a, b in zip(got, torch.autograd.grad(out, (q, k, v), -dout)))
+
+
+@pytest.mark.gpu
+def test_other_threads_run_while_launches_wait():
+    """With the stream busy and its queue full a launch waits for the device; Python's other threads do not."""
+    q, k, v = (torch.randn(1, 1, 64, 64, device="cuda").half() for _ in range(3))
+    attention(q, k, v)
+    ticks, done = [], threading.Event()
+
+    def tick():
+        while not done.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(0.002)
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    torch.cuda._sleep(int(1.2e9))  # more than half a second at any clock of the GPU
+    start = time.perf_counter()
+    for _ in range(2500):  # the queue holds about 1000 launches
+        attention(q, k, v)
+    waited = time.perf_counter() - start
+    torch.cuda.synchronize()
+    done.set()
+    thread.join()
+    assert waited > 0.4
+    assert max(b - a for a, b in zip(ticks, ticks[1:])) < 0.2
 
 
 @pytest.mark.gpu
