@@ -13,6 +13,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <initializer_list>
 #include <string>
 
 #include "../../include/kfa.h"
@@ -98,6 +99,17 @@ KfaTensor4 desc_packed(const at::Tensor& t) {
     d.stride[i] = stride[i];
   }
   return d;
+}
+
+// The kernels read these as they lie in memory: an address of another device is a fault, other strides wrong offsets.
+void check_lengths(const at::Tensor& cu_q, const at::Tensor& cu_k, const at::Tensor& q) {
+  for (const at::Tensor* cu : {&cu_q, &cu_k})
+    TORCH_CHECK_VALUE(cu->device() == q.device() && cu->scalar_type() == at::kInt && cu->is_contiguous() && cu->numel() >= 2,
+                      "attention_varlen: cu_seqlens: contiguous int32 offsets on the device of q");
+  TORCH_CHECK_VALUE(cu_q.numel() == cu_k.numel(), "attention_varlen: cu_seqlens of different lengths");
+}
+void check_device(std::initializer_list<const at::Tensor*> others, const at::Tensor& q) {
+  for (const at::Tensor* t : others) TORCH_CHECK_VALUE(t->device() == q.device(), "attention: tensors on different devices");
 }
 
 int dtype_code(const at::Tensor& t) {
@@ -207,6 +219,7 @@ PyObject* py_forward(Args a, Py_ssize_t n) {
   at::Tensor out, lse;
   {
     const NoGil released;
+    check_device({&k, &v, &status}, q);
     const c10::cuda::CUDAGuard guard(q.device());
     out = bshd_like(q);
     lse = floats(q, {q.size(0), q.size(1), 2, q.size(2)});
@@ -229,6 +242,7 @@ PyObject* py_backward(Args a, Py_ssize_t n) {
   at::Tensor dq, dk, dv;
   {
     const NoGil released;
+    check_device({&k, &v, &o, &g, &lse, &status}, q);
     const c10::cuda::CUDAGuard guard(q.device());
     if (q.size(3) % 16 && !aligned16(g)) g = g.clone();  // (widening copied it)
     dq = bshd_like(q);
@@ -266,6 +280,7 @@ PyObject* py_forward_masked(Args a, Py_ssize_t n) {
   at::Tensor out, lse;
   {
     const NoGil released;
+    check_device({&k, &v, &words, &tiles, &status}, q);
     const c10::cuda::CUDAGuard guard(q.device());
     out = bshd_like(q);
     lse = floats(q, {q.size(0), q.size(1), 2, q.size(2)});
@@ -287,6 +302,7 @@ PyObject* py_backward_masked(Args a, Py_ssize_t n) {
   at::Tensor dq, dk, dv;
   {
     const NoGil released;
+    check_device({&k, &v, &o, &g, &lse, &words, &words_t, &tiles, &status}, q);
     const c10::cuda::CUDAGuard guard(q.device());
     dq = bshd_like(q);
     dk = bshd_like(k);
@@ -312,6 +328,8 @@ PyObject* py_forward_varlen(Args a, Py_ssize_t n) {
   at::Tensor out, lse;
   {
     const NoGil released;
+    check_device({&k, &v, &status}, q);
+    check_lengths(cu_q, cu_k, q);
     const c10::cuda::CUDAGuard guard(q.device());
     const int32_t *cq = cu_q.data_ptr<int32_t>(), *ck = cu_k.data_ptr<int32_t>();
     const int n_seqs = static_cast<int>(cu_q.numel() - 1);
@@ -338,6 +356,8 @@ PyObject* py_backward_varlen(Args a, Py_ssize_t n) {
   at::Tensor dq, dk, dv;
   {
     const NoGil released;
+    check_device({&k, &v, &o, &g, &lse, &status}, q);
+    check_lengths(cu_q, cu_k, q);
     const c10::cuda::CUDAGuard guard(q.device());
     const int32_t *cq = cu_q.data_ptr<int32_t>(), *ck = cu_k.data_ptr<int32_t>();
     const int n_seqs = static_cast<int>(cu_q.numel() - 1);

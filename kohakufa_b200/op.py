@@ -454,7 +454,7 @@ def attention_varlen(
         _check(*(_as4(t) for t in (q, k, v)))
     if scale is None:
         scale = q.shape[-1] ** -0.5
-    cu_seqlens_q, cu_seqlens_k = cu_seqlens_q.int(), cu_seqlens_k.int()
+    cu_seqlens_q, cu_seqlens_k = cu_seqlens_q.int().contiguous(), cu_seqlens_k.int().contiguous()
     if plan is None:
         plan = varlen_plan(cu_seqlens_q, cu_seqlens_k, q.shape[1], k.shape[1], block_causal)
     n_seqs, max_q, max_k = plan

@@ -63,6 +63,22 @@ def test_plain_eager_leaves_to_the_dispatcher_what_it_resolves():
     assert _lib.plain_eager(t, x)
 
 
+def test_sequence_offsets_are_refused_before_a_launch():
+    """The kernels read the offsets where they lie: int32, contiguous, on the device of q, as many for q as for k."""
+    host, t = _lib.host(), torch.zeros(4, 1, 16, dtype=torch.float16)
+    lse, word = torch.zeros(1, 1, 2, 4), torch.zeros(1, dtype=torch.int32)
+    cu = torch.tensor([0, 4], dtype=torch.int32)
+    strided = torch.tensor([[0, 9], [4, 9]], dtype=torch.int32)[:, 0]
+    for bad in (strided, cu.long(), cu.to("meta"), cu[:1], torch.tensor([0, 2, 4], dtype=torch.int32)):
+        for pair in ((bad, cu), (cu, bad)):
+            with pytest.raises(ValueError, match="cu_seqlens"):
+                host.forward_varlen(t, t, t, *pair, 4, 4, 1.0, 0, word)
+            with pytest.raises(ValueError, match="cu_seqlens"):
+                host.backward_varlen(t, t, t, t, t, lse, *pair, 4, 4, 1.0, 0, word)
+    with pytest.raises(ValueError, match="different devices"):
+        host.forward_varlen(t, t.to("meta"), t, cu, cu, 4, 4, 1.0, 0, word)
+
+
 def inputs(dim=128, seq=200, heads=4, kv_heads=2, packed=False):
     gen = torch.Generator().manual_seed(dim + seq)
     shape = (seq, heads, dim) if packed else (2, seq, heads, dim)
@@ -155,6 +171,18 @@ def test_negative_views():
     out = attention(q, k, v)
     got = torch.autograd.grad(out, (q, k, v), torch._neg_view(dout), retain_graph=True)
     assert all(torch.equal(a, b) for a, b in zip(got, torch.autograd.grad(out, (q, k, v), -dout)))
+
+
+@pytest.mark.gpu
+def test_sequence_offsets_of_a_table():
+    """A column of a 2-D table is taken (as if it were contiguous); offsets in host memory are refused."""
+    (q, k, v), _ = inputs(packed=True)
+    table = torch.tensor([[0, 5], [70, 6], [200, 7]], dtype=torch.int32, device="cuda")
+    cu = table[:, 0].contiguous()
+    with torch.no_grad():
+        assert torch.equal(attention_varlen(q, k, v, table[:, 0], table[:, 0]), attention_varlen(q, k, v, cu, cu))
+        with pytest.raises(ValueError, match="cu_seqlens"):
+            attention_varlen(q, k, v, cu.cpu(), cu.cpu())
 
 
 @pytest.mark.gpu
