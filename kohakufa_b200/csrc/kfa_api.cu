@@ -491,6 +491,8 @@ int launch_sum_splits(const kfa::SumParams& p, int bh, cudaStream_t s) {
 // is why self attention, whose dK and dV do not depend on what else is in the batch, is left alone.
 // (148 SMs: what this library is built for.)
 int bwd_splits(const KfaTensor4* q, const KfaTensor4* k) {
+  for (int i = 0; i < 4; ++i)
+    if (q->shape[i] < 1 || k->shape[i] < 1) return 1;  // (kfa_bwd_parts_bytes is asked before anything is checked)
   const int64_t n_k = (k->shape[2] + 127) / 128, n_q = (q->shape[2] + 127) / 128;
   const int64_t tiles = k->shape[0] * k->shape[1] * n_k;
   const int64_t steps = (q->shape[1] / k->shape[1]) * n_q;
@@ -727,7 +729,7 @@ int kfa_bwd_narrow(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v
 }
 
 int64_t kfa_bwd_parts_bytes(const KfaTensor4* q, const KfaTensor4* k) {
-  if (!q || !k || k->shape[0] < 1 || k->shape[1] < 1) return 0;
+  if (!q || !k) return 0;
   const int n = bwd_splits(q, k);
   return n < 2 ? 0 : static_cast<int64_t>(n) * 8 * k->shape[0] * k->shape[1] * k->shape[2] * kernel_dim(k->shape[3]);
 }

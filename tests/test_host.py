@@ -52,6 +52,21 @@ def test_library_rejects_bad_arguments_without_a_gpu():
     assert rc == -1 and b"stride" in lib.kfa_last_error()
 
 
+def test_parts_bytes_of_empty_tensors():
+    lib = _lib.load()
+    q, k = _lib.KfaTensor4(), _lib.KfaTensor4()
+    shapes = ((1, 2, 4096, 64), (1, 2, 77, 64))
+    for empty in range(8):
+        for t, shape in zip((q, k), shapes):
+            t.shape[:] = shape
+        (q if empty < 4 else k).shape[empty % 4] = 0
+        assert lib.kfa_bwd_parts_bytes(ctypes.byref(q), ctypes.byref(k)) == 0
+    for t, shape in zip((q, k), shapes):
+        t.shape[:] = shape
+    assert lib.kfa_bwd_parts_bytes(ctypes.byref(q), ctypes.byref(k)) == 8 * 8 * 2 * 77 * 64  # 8 parts of dK and dV
+    assert lib.kfa_bwd_parts_bytes(None, ctypes.byref(k)) == 0
+
+
 def test_causal_and_block_causal_are_exclusive():
     q, k, v = qkv()
     with pytest.raises(ValueError, match="causal is block_causal=1"):
