@@ -778,7 +778,8 @@ int kfa_varlen_zero_rows(const KfaTensor4* t, int n_tensors, const int32_t* cu_s
   p.lse = lse;
   p.cols = static_cast<int>(t[0].shape[3]);
   p.n_seqs = n_seqs;
-  kfa::kfa_zero_rows_kernel<<<dim3(static_cast<unsigned>((most + 255) / 256), n_tensors), 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  const dim3 grid(static_cast<unsigned>((most + kfa::ZERO_ROWS - 1) / kfa::ZERO_ROWS), n_tensors);
+  kfa::kfa_zero_rows_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
   KFA_CUDA(cudaGetLastError());
   return KFA_OK;
 }

@@ -1,5 +1,7 @@
 """Packed batches: the numbering of tiles without gaps, the rectangular one, and the rows no sequence owns."""
 
+import ctypes
+
 import pytest
 import torch
 
@@ -64,3 +66,21 @@ def test_rows_outside_the_sequences_are_zero(n_seqs):
         assert float(t[inside].abs().flatten(1).sum(-1).gt(0).float().mean()) > 0.9
     direct = op.varlen_fwd_op(q, k, v, cu, cu, 300, 300, 64**-0.5, 1)
     assert torch.equal(direct[0], out) and not bool(direct[1][..., ~inside].any())
+
+
+@pytest.mark.parametrize("heads,dim", [(1, 16), (3, 48), (5, 128)])
+@pytest.mark.parametrize("first,tail", [(0, 1), (1, 63), (64, 64), (30, 300)])
+def test_left_over_rows_of_any_width(heads, dim, first, tail):
+    """Rows of 16 to 640 columns (a warp stores 256 at a time), left over in pieces that begin and end inside a CTA's 64;
+    a tensor of padded rows keeps its padding."""
+    lib, total = _lib.load(), first + 70 + tail
+    cu = torch.tensor([first, first + 70], dtype=torch.int32, device="cuda")
+    wide = torch.full((total, heads, dim + 8), 3.0, dtype=torch.bfloat16, device="cuda")
+    out = wide[..., :dim]
+    lse = torch.full((1, heads, 2, total), 3.0, device="cuda")
+    _lib.check(lib.kfa_varlen_zero_rows(ctypes.byref(_lib.tensor4(op._as4(out))), 1, cu.data_ptr(), cu.data_ptr(), 1, 70, 70,
+                                        lse.data_ptr(), _lib.stream_ptr(out.device)))  # fmt: skip
+    left = torch.ones(total, dtype=torch.bool, device="cuda")
+    left[first : first + 70] = False
+    assert not bool(out[left].any()) and not bool(lse[..., left].any())
+    assert bool((out[~left] == 3).all()) and bool((lse[..., ~left] == 3).all()) and bool((wide[..., dim:] == 3).all())
