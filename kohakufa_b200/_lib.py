@@ -186,6 +186,12 @@ def host():
                     f"{HOST_PATH} is missing: build it with `python -m kohakufa_b200.build` "
                     "(needs a C++ compiler; there is no fallback path)"
                 )
+            from kohakufa_b200.build import host_fits
+
+            if not host_fits(HOST_PATH):
+                raise KfaError(
+                    f"{HOST_PATH} was built for another torch or Python: rebuild it with `python -m kohakufa_b200.build`"
+                )
             from kohakufa_b200 import _kfa_host
 
             _kfa_host.bind(KfaError, {n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in HOST_SYMBOLS})

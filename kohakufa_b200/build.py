@@ -58,8 +58,20 @@ def nvcc_path() -> str:
     return found
 
 
+def host_stamp() -> bytes:
+    """The torch and the Python a host extension is built for: it is compiled against their C++ headers, whose inlined
+    accessors fit no other. The stamp is a string in the extension."""
+    import torch
+
+    return f"_kfa_host for torch {torch.__version__} {torch.version.git_version}, {sysconfig.get_config_var('SOABI')}".encode()
+
+
+def host_fits(lib: Path) -> bool:
+    return host_stamp() in lib.read_bytes()
+
+
 def stale(lib: Path = LIB) -> bool:
-    if not lib.exists():
+    if not lib.exists() or (lib == HOST and not host_fits(lib)):
         return True
     built = lib.stat().st_mtime
     return any(p.stat().st_mtime > built for p in (HOST_SOURCES if lib == HOST else SOURCES + HEADERS))
@@ -86,6 +98,7 @@ def _compile_host() -> None:
     include = [sysconfig.get_paths()["include"], root / "include", root / "include/torch/csrc/api/include", cuda / "include"]
     abi = int(torch.compiled_with_cxx11_abi())
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-DNDEBUG", f"-D_GLIBCXX_USE_CXX11_ABI={abi}"]
+    cmd.append(f'-DKFA_HOST_STAMP="{host_stamp().decode()}"')
     cmd += [f"-I{d}" for d in include] + ["-o", str(HOST), str(HOST_SOURCES[0]), f"-L{root / 'lib'}"]
     cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
     _run(cmd, "build_host.log", False)

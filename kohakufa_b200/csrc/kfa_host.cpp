@@ -4,8 +4,10 @@
 // of 1 x 8 heads x 64 rows 67 us, now 15; forward + backward of 2 x 4 heads x 512 rows 286 us, now 122, of which
 // about 50 are the autograd engine's own; with a boolean mask of 2048 x 2048 395 us, now 139.
 //
-// A plain CPython extension module (`_kfa_host`). It holds no state but the addresses of the libkfa entry points
-// it was given (`bind`): which library is loaded, and every policy (status word, backward mode), stays in Python.
+// A plain CPython extension module (`_kfa_host`), for the torch and the Python it was built with only: the build leaves
+// their names in it, and _lib.host() does not load it under others. It holds no state but the addresses of the libkfa
+// entry points it was given (`bind`): which library is loaded, and every policy (status word, backward mode), stays in
+// Python.
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Exceptions.h>
 
@@ -453,4 +455,8 @@ PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_kfa_host", nullptr, -1, metho
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__kfa_host(void) { return PyModule_Create(&module_def); }
+PyMODINIT_FUNC PyInit__kfa_host(void) {
+  PyObject* m = PyModule_Create(&module_def);
+  if (m && PyModule_AddStringConstant(m, "built_for", KFA_HOST_STAMP) < 0) Py_CLEAR(m);
+  return m;
+}

@@ -10,7 +10,7 @@ import pytest
 import torch
 
 import kohakufa_b200
-from kohakufa_b200 import _lib, api, op
+from kohakufa_b200 import _lib, api, build, op
 
 ROOT = Path(__file__).resolve().parent.parent
 
@@ -50,6 +50,19 @@ def test_library_rejects_bad_arguments_without_a_gpu():
     t.stride[2] = 60
     rc = lib.kfa_fwd(ctypes.byref(t), ctypes.byref(t), ctypes.byref(t), ctypes.byref(t), 64, 1.0, 0, 0, 64, None)
     assert rc == -1 and b"stride" in lib.kfa_last_error()
+
+
+def test_host_extension_of_another_torch_is_not_loaded(tmp_path, monkeypatch):
+    other = tmp_path / "_kfa_host.so"
+    stamp = build.host_stamp()
+    other.write_bytes(build.HOST.read_bytes().replace(stamp, stamp.replace(b"torch ", b"torch 0.")[: len(stamp)]))
+    assert build.host_fits(build.HOST) and _lib.host().built_for.encode() == stamp
+    monkeypatch.setattr(_lib, "_host", None)
+    monkeypatch.setattr(_lib, "HOST_PATH", other)
+    with pytest.raises(_lib.KfaError, match="another torch"):
+        _lib.host()
+    monkeypatch.setattr(build, "HOST", other)
+    assert build.stale(other)
 
 
 def test_parts_bytes_of_empty_tensors():
