@@ -163,7 +163,7 @@ int launch_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& 
 template <int D, bool BF16>
 int launch_prepare(const kfa::PrepParams& p, cudaStream_t s) {
   dim3 grid(p.n_q128, p.B * p.H);
-  kfa::kfa_bwd_prepare_kernel<D, BF16><<<grid, kfa::PREP_THREADS, 0, s>>>(p);
+  kfa::kfa_bwd_prepare_kernel<D, BF16><<<grid, kfa::PrepCfg<D>::THREADS, 0, s>>>(p);
   KFA_CUDA(cudaGetLastError());
   return KFA_OK;
 }

@@ -109,21 +109,33 @@ struct PrepParams {
 };
 
 // ---------------------------------------------------------------------------------------
-// prepare: HBM-bound; D / 8 lanes per row (rounded up to a power of two), 16-byte loads. A CTA has 128 rows and
-// 256 threads; a warp has all its 16 rows' loads of O and dO in flight together. With 4 warps that went through 32
-// rows each, pass by pass, every pass waited for memory: 5.4 -> 2.3 us at 2 x 4 x 512 rows of D = 64, 9.9 -> 6.3 at
-// 16 x 4096 of D = 128 (both L2 hits), 34.8 -> 32.3 at 32 x 8192 of D = 128 (134 MB: 4.2 of the 6.4 TB/s that a copy
-// reaches); with the zero fill of the fused backward's accumulator 32.6 -> 22.4 us at 64 x 4096 of D = 64.
+// prepare: HBM-bound; D / 8 lanes per row (rounded up to a power of two), 16-byte loads. A CTA has 128 rows. A lane has up
+// to four rows' pieces of O and dO in flight together; with the 64 registers that takes an SM holds 1024 threads: 256-thread
+// CTAs, whose warps go through their rows twice above D = 64, and 128-thread ones at D <= 32, where four pieces (two at D = 16)
+// are all the rows of a lane. In us, bf16: four warps that go through 32 rows each and wait in every pass / all rows of
+// 256 threads at once (128 registers at D = 128: two CTAs an SM, which load and reduce in lock-step; half as many tiles an
+// SM at D = 16) / now:
+//   2 x 4 x 512 rows, D = 64       5.1 / 2.2 / 2.2
+//   1 x 16 x 4096 rows, D = 128    9.1 / 6.3 / 5.4
+//   4 x 32 x 8192 rows, D = 128    101 / 111 / 91 (537 MB: 5.9 of the 6.4 TB/s that a copy reaches)
+//                       D = 96      93 / 100 / 75,   D = 80   88 / 99 / 69,   D = 16   19.4 / 22.2 / 17.2
+// With the zero fill of the fused backward's accumulator, 64 x 4096 of D = 64: 32.6 / 22.4 / 22.4.
 // ---------------------------------------------------------------------------------------
-constexpr int PREP_THREADS = 256;
+template <int D>
+struct PrepCfg {
+  static constexpr int VECS = D / 8;                                                  // 16-byte pieces of a row
+  static constexpr int LPR = VECS <= 2 ? 2 : (VECS <= 4 ? 4 : (VECS <= 8 ? 8 : 16));  // lanes per row (a power of two)
+  static constexpr int THREADS = D <= 32 ? 128 : 256;
+  static constexpr int RPW = 32 / LPR;                                                // rows per warp pass
+  static constexpr int ROWS = 128 / (THREADS / 32);                                   // rows of a warp
+  static constexpr int PASSES = ROWS / RPW < 4 ? ROWS / RPW : 4;                      // ... in flight together
+  static constexpr int MIN_CTAS = (D == 48 || D == 64) ? 0 : 1024 / THREADS;          // (there the compiler's own choice is 4)
+};
 
 template <int D, bool BF16>
-__global__ void __launch_bounds__(PREP_THREADS) kfa_bwd_prepare_kernel(const PrepParams p) {
-  constexpr int VECS = D / 8;                                                      // 16-byte pieces of a row
-  constexpr int LPR = VECS <= 2 ? 2 : (VECS <= 4 ? 4 : (VECS <= 8 ? 8 : 16));      // lanes per row (a power of two)
-  constexpr int RPW = 32 / LPR;                                                    // rows per warp pass
-  constexpr int ROWS = 128 / (PREP_THREADS / 32);                                  // rows of a warp
-  constexpr int PASSES = ROWS / RPW;
+__global__ void __launch_bounds__(PrepCfg<D>::THREADS, PrepCfg<D>::MIN_CTAS) kfa_bwd_prepare_kernel(const PrepParams p) {
+  using Cfg = PrepCfg<D>;
+  constexpr int LPR = Cfg::LPR, RPW = Cfg::RPW, PASSES = Cfg::PASSES;
   const int tile = blockIdx.x;
   const int bh = blockIdx.y;
   const int b = bh / p.H, h = bh % p.H;
@@ -140,44 +152,49 @@ __global__ void __launch_bounds__(PREP_THREADS) kfa_bwd_prepare_kernel(const Pre
   const uint8_t* gb = reinterpret_cast<const uint8_t*>(p.dout) + 2 * (bc * p.do_sb + h * p.do_sh + q_base * p.do_ss);
   float* st = p.stats + (static_cast<long long>(bh) * p.n_q128 + tile) * 384;
   const float* lse = p.lse + (static_cast<long long>(bc) * p.H + h) * 2 * p.Sq + q_base;
-  uint4 ov[PASSES], gv[PASSES];
 #pragma unroll
-  for (int i = 0; i < PASSES; ++i) {
-    const int row = tile * 128 + warp * ROWS + i * RPW + sub;
-    ov[i] = gv[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (row < Sq && vec * 8 < p.cols) {
-      ov[i] = *reinterpret_cast<const uint4*>(ob + 2 * (row * p.o_ss + vec * 8));
-      gv[i] = *reinterpret_cast<const uint4*>(gb + 2 * (row * p.do_ss + vec * 8));
+  for (int r0 = 0; r0 < Cfg::ROWS; r0 += PASSES * RPW) {
+    uint4 ov[PASSES], gv[PASSES];
+#pragma unroll
+    for (int i = 0; i < PASSES; ++i) {
+      const int row = tile * 128 + warp * Cfg::ROWS + r0 + i * RPW + sub;
+      ov[i] = gv[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (row < Sq && vec * 8 < p.cols) {
+        ov[i] = *reinterpret_cast<const uint4*>(ob + 2 * (row * p.o_ss + vec * 8));
+        gv[i] = *reinterpret_cast<const uint4*>(gb + 2 * (row * p.do_ss + vec * 8));
+      }
     }
-  }
-  if (threadIdx.x < 128) {
-    const int row = tile * 128 + threadIdx.x;
-    const bool valid = row < Sq;
-    // stored negated, so the consumers only add; padded rows: -m = -inf makes their P exactly 0
-    st[threadIdx.x] = valid ? -lse[row] : -INFINITY;
-    st[128 + threadIdx.x] = valid ? -lse[p.Sq + row] : 0.f;
-  }
-  if (p.dq_acc != nullptr) {
-    float4* acc = reinterpret_cast<float4*>(p.dq_acc + (static_cast<long long>(bh) * p.n_q128 + tile) * (128 * D));
+    if (r0 == 0) {  // while the first rows are on their way
+      if (threadIdx.x < 128) {
+        const int row = tile * 128 + threadIdx.x;
+        const bool valid = row < Sq;
+        // stored negated, so the consumers only add; padded rows: -m = -inf makes their P exactly 0
+        st[threadIdx.x] = valid ? -lse[row] : -INFINITY;
+        st[128 + threadIdx.x] = valid ? -lse[p.Sq + row] : 0.f;
+      }
+      if (p.dq_acc != nullptr) {
+        float4* acc = reinterpret_cast<float4*>(p.dq_acc + (static_cast<long long>(bh) * p.n_q128 + tile) * (128 * D));
 #pragma unroll 4
-    for (int i = threadIdx.x; i < 128 * D / 4; i += PREP_THREADS) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-#pragma unroll
-  for (int i = 0; i < PASSES; ++i) {
-    const uint32_t ow[4] = {ov[i].x, ov[i].y, ov[i].z, ov[i].w};
-    const uint32_t gw[4] = {gv[i].x, gv[i].y, gv[i].z, gv[i].w};
-    float acc = 0.f;
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      const float2 a = unpack16<BF16>(ow[x]);
-      const float2 g = unpack16<BF16>(gw[x]);
-      acc = fmaf(a.x, g.x, acc);
-      acc = fmaf(a.y, g.y, acc);
+        for (int i = threadIdx.x; i < 128 * D / 4; i += Cfg::THREADS) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
     }
 #pragma unroll
-    for (int off = LPR / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    const int r_in = warp * ROWS + i * RPW + sub;
-    if (vec == 0) st[256 + r_in] = (tile * 128 + r_in < Sq) ? -acc : 0.f;
+    for (int i = 0; i < PASSES; ++i) {
+      const uint32_t ow[4] = {ov[i].x, ov[i].y, ov[i].z, ov[i].w};
+      const uint32_t gw[4] = {gv[i].x, gv[i].y, gv[i].z, gv[i].w};
+      float acc = 0.f;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const float2 a = unpack16<BF16>(ow[x]);
+        const float2 g = unpack16<BF16>(gw[x]);
+        acc = fmaf(a.x, g.x, acc);
+        acc = fmaf(a.y, g.y, acc);
+      }
+#pragma unroll
+      for (int off = LPR / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+      const int r_in = warp * Cfg::ROWS + r0 + i * RPW + sub;
+      if (vec == 0) st[256 + r_in] = (tile * 128 + r_in < Sq) ? -acc : 0.f;
+    }
   }
 }
 

@@ -40,8 +40,8 @@ def test_pack_mask_edges(s_q, s_kv, layout):
     assert torch.equal(tiles != 0, want)
 
 
-@pytest.mark.parametrize("dim", [16, 48, 64, 80, 128])
-@pytest.mark.parametrize("seq", [1, 15, 17, 127, 128, 130])
+@pytest.mark.parametrize("dim", [16, 32, 48, 64, 80, 112, 128])
+@pytest.mark.parametrize("seq", [1, 15, 17, 65, 127, 128, 130])
 def test_backward_statistics(dim, seq):
     """(-m, -log2 l, -delta) per row, padded rows (-inf, 0, 0). delta is a sum of ``dim`` fp32 products: its
     error is at most dim * 2^-24 of the sum of the products' magnitudes in either order of summation."""
