@@ -140,6 +140,20 @@ long long packed_tiles(int n_seqs, int n_max, int rows, int tile) {
   return std::min(static_cast<long long>(n_seqs) * n_max, static_cast<long long>(rows) / tile + n_seqs);
 }
 
+// Whether the grid of a packed batch numbers the tiles that exist (decode_packed) or, as a rectangle, every sequence's up
+// to the tiles of the longest. A CTA of the rectangle that finds its sequence too short costs about 1 us of an SM, because
+// it needs all of its shared memory to start; a CTA of the other numbering first scans the lengths, 32 at a time, one
+// load's latency each. `scans`: how many of those an empty CTA costs as much as (measured: 8 in the forward, 6 in the
+// backward); how many tiles exist is estimated, the last tile of a sequence as half there. Rectangle -> numbering of the
+// tiles that exist, D = 64, 8 heads, causal, forward + backward, lengths spread evenly up to the longest, in us: 32 x 512 106
+// -> 98, 64 x 512 195 -> 183, 96 x 512 296 -> 282, 128 x 512 401 -> 398, 192 x 512 621 -> 649, 128 x 2048 1899 -> 1854, 128 x
+// 128 129 -> 139; 64 of 512 each 320 -> 326. One of 4096 rows among n of up to 64: n = 256 1689 -> 622, 1000 6234 -> 2626.
+bool number_compactly(int n_seqs, int n_max, int rows, int tile, int scans) {
+  const long long all = static_cast<long long>(n_seqs) * n_max;
+  const long long exist = std::min(all, static_cast<long long>(rows) / tile + (n_seqs + 1) / 2);
+  return scans * (all - exist) >= exist * ((n_seqs + 31) / 32);
+}
+
 template <int D, bool BF16, bool MASKW>
 int launch_fwd_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const kfa::FwdParams& p,
                  cudaStream_t s) {
@@ -344,7 +358,6 @@ void apply_extra(kfa::BwdParams& p, const Extra& ex) {
   p.stats_sh = static_cast<long long>(p.n_q128) * 384;
   p.cu_q = vl->cu_q;
   p.cu_k = vl->cu_k;
-  p.compact = vl->n_seqs <= kfa::VARLEN_COMPACT;
 }
 
 int fwd_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out, float* lse,
@@ -381,7 +394,7 @@ int fwd_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, cons
     p.n_q_tiles = (vl->max_q + 255) / 256;
     p.cu_q = vl->cu_q;
     p.cu_k = vl->cu_k;
-    p.compact = vl->n_seqs <= kfa::VARLEN_COMPACT;
+    p.compact = number_compactly(p.B, p.n_q_tiles, p.Sq, 256, 8);
   }
   if (ex.mw) {
     p.mw = ex.mw->words;
@@ -455,6 +468,7 @@ int dkdv_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, con
   kfa::BwdParams p;
   fill_bwd_params(p, q, k, stats, scale, block, dev_status);
   apply_extra(p, ex);
+  p.compact = ex.vl && number_compactly(p.B, p.n_k128, p.Skv, 128, 6);
   p.dk = dk->ptr;
   p.dk_sb = dk->stride[0];
   p.dk_sh = dk->stride[1];
@@ -538,6 +552,7 @@ int dq_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const
   kfa::BwdParams p;
   fill_bwd_params(p, q, k, stats, scale, block, dev_status);
   apply_extra(p, ex);
+  p.compact = ex.vl && number_compactly(p.B, p.n_q128, p.Sq, 128, 6);
   p.dq = dq->ptr;
   p.dq_sb = dq->stride[0];
   p.dq_sh = dq->stride[1];

@@ -55,8 +55,9 @@ struct FwdParams {
   long long ml_sh, ml_plane;
   // Packed variable-length batches (cu_q != nullptr): the tensors are [1, H, T, D]; sequence b (of B)
   // owns query rows cu_q[b] .. cu_q[b + 1] and key rows cu_k[b] .. cu_k[b + 1] and is its own attention
-  // problem. Sq is then the tensors' row count T (it sizes the statistics planes) and n_q_tiles counts
-  // the tiles of the longest sequence; CTAs past the end of a shorter one return at once.
+  // problem. Sq is then the tensors' row count T (it sizes the statistics planes) and n_q_tiles counts the tiles of the
+  // longest sequence. The grid is a rectangle (sequences x n_q_tiles x heads), whose CTAs past the end of a shorter
+  // sequence return at once, or numbers the tiles that exist (compact).
   const int* cu_q;
   const int* cu_k;
   int compact;  // the grid numbers the tiles of a packed batch without gaps (decode_packed)
@@ -155,12 +156,9 @@ __device__ __forceinline__ void decode_tile(int idx, int n_bh, int n_tiles, int&
   bh = g * G + (r - t * gs);
 }
 
-// The same for a packed batch of up to VARLEN_COMPACT sequences, numbered without the tiles that shorter sequences do not
-// have: sequence after sequence, inside one as above. A CTA of the rectangular numbering (sequences x tiles of the
-// longest) that finds its sequence too short costs about 1 us of an SM, because it needs all of its shared memory to
-// start: with lengths spread evenly that was half of the CTAs. Every warp scans the lengths for itself (32 at a time).
+// The same for a packed batch numbered without the tiles that shorter sequences do not have (rule: number_compactly in
+// kfa_api.cu): sequence after sequence, inside one as above. Every warp scans the lengths for itself (32 at a time).
 // Returns false past the last tile. n_max: tiles of the longest sequence; n_tiles: of sequence b.
-constexpr int VARLEN_COMPACT = 256;
 template <int TILE>
 __device__ __forceinline__ bool decode_packed(int idx, const int* cu, int n_seqs, int H, int n_max, int& b, int& h, int& t,
                                               int& n_tiles) {

@@ -28,11 +28,26 @@ def packed(lengths, heads, kv_heads, dim, extra=0):
 @pytest.mark.parametrize("n_seqs,longest", [(1, 1), (31, 300), (33, 700), (256, 90), (257, 90), (300, 400)])
 @pytest.mark.parametrize("causal", [True, False])
 def test_batch_equals_its_halves(n_seqs, longest, causal):
-    """A sequence's results do not depend on the batch it is in, so a batch equals its two halves bit for bit, also
-    where the batch is numbered in the rectangular way (more than 256 sequences) and the halves without gaps."""
+    """A sequence's results do not depend on the batch it is in, so a batch equals its two halves bit for bit."""
     gen = torch.Generator().manual_seed(longest)
     lengths = torch.randint(0, longest + 1, (n_seqs,), generator=gen).tolist()
     lengths[n_seqs // 2] = longest
+    check_halves(lengths, causal)
+
+
+@pytest.mark.parametrize("n_seqs,others", [(40, 130), (600, 40)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_one_long_sequence(n_seqs, others, causal):
+    """Most of the rectangle's tiles do not exist: numbered without gaps (40 sequences: two scans of 32 lengths, 600:
+    nineteen); the half of the 600 that the long one is not in has one tile a sequence and is a rectangle."""
+    gen = torch.Generator().manual_seed(n_seqs)
+    lengths = torch.randint(1, others + 1, (n_seqs,), generator=gen).tolist()
+    lengths[-2] = 2900
+    check_halves(lengths, causal)
+
+
+def check_halves(lengths, causal):
+    n_seqs = len(lengths)
     q, k, v, dout, cu = packed(lengths, 4, 2, 64)
     whole = run(q, k, v, dout, cu, varlen_plan(cu, cu), causal=causal)
     cut = (n_seqs + 1) // 2
