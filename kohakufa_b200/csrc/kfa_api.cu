@@ -154,14 +154,14 @@ bool number_compactly(int n_seqs, int n_max, int rows, int tile, int scans) {
   return scans * (all - exist) >= exist * ((n_seqs + 31) / 32);
 }
 
-template <int D, bool BF16, bool MASKW>
+template <int D, bool BF16, bool MASKW, bool COMPACT>
 int launch_fwd_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const kfa::FwdParams& p,
                  cudaStream_t s) {
-  auto kern = kfa::kfa_fwd_kernel<D, BF16, MASKW>;
+  auto kern = kfa::kfa_fwd_kernel<D, BF16, MASKW, COMPACT>;
   constexpr int smem = MASKW ? kfa::FwdCfg<D>::SMEM_BYTES_LIST : kfa::FwdCfg<D>::SMEM_BYTES;
   int rc = set_smem(kern, smem);
   if (rc) return rc;
-  const long long grid = p.compact ? packed_tiles(p.B, p.n_q_tiles, p.Sq, 256) * p.H : static_cast<long long>(p.B) * p.H * p.n_q_tiles;
+  const long long grid = COMPACT ? packed_tiles(p.B, p.n_q_tiles, p.Sq, 256) * p.H : static_cast<long long>(p.B) * p.H * p.n_q_tiles;
   if (grid > 0x7fffffffll) return fail(KFA_ERR_ARG, "too many tiles");
   kern<<<static_cast<unsigned>(grid), kfa::FWD_THREADS, smem, s>>>(mq, mk, mv, p);
   KFA_CUDA(cudaGetLastError());
@@ -171,7 +171,9 @@ int launch_fwd_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap
 template <int D, bool BF16>
 int launch_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const kfa::FwdParams& p,
                cudaStream_t s) {
-  return p.mw ? launch_fwd_t<D, BF16, true>(mq, mk, mv, p, s) : launch_fwd_t<D, BF16, false>(mq, mk, mv, p, s);
+  if (p.mw) return launch_fwd_t<D, BF16, true, false>(mq, mk, mv, p, s);
+  if (p.cu_q && number_compactly(p.B, p.n_q_tiles, p.Sq, 256, 8)) return launch_fwd_t<D, BF16, false, true>(mq, mk, mv, p, s);
+  return launch_fwd_t<D, BF16, false, false>(mq, mk, mv, p, s);
 }
 
 template <int D, bool BF16>
@@ -394,7 +396,6 @@ int fwd_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, cons
     p.n_q_tiles = (vl->max_q + 255) / 256;
     p.cu_q = vl->cu_q;
     p.cu_k = vl->cu_k;
-    p.compact = number_compactly(p.B, p.n_q_tiles, p.Sq, 256, 8);
   }
   if (ex.mw) {
     p.mw = ex.mw->words;
