@@ -182,8 +182,9 @@ void need(Py_ssize_t got, Py_ssize_t want) {
 
 using Args = PyObject* const*;
 
-// plain(*tensors) -> bool: whether what each tensor's address points to is its value. Batched tensors (gradients of
-// `is_grads_batched`), pending negations and zero tensors are torch.Tensor too, but only the dispatcher resolves them.
+// plain(*tensors) -> bool: whether each is a torch.Tensor (no subclass) and what its address points to is its value. Batched
+// tensors (gradients of `is_grads_batched`), pending negations and zero tensors are torch.Tensor too, but only the
+// dispatcher resolves them.
 PyObject* py_plain(Args a, Py_ssize_t n) {
   using c10::DispatchKey;
   static const uint64_t plain =
@@ -191,7 +192,9 @@ PyObject* py_plain(Args a, Py_ssize_t n) {
                            DispatchKey::AutogradCUDA, DispatchKey::AutocastCPU, DispatchKey::AutocastCUDA})
           .raw_repr();
   for (Py_ssize_t i = 0; i < n; ++i)
-    if (tensor(a[i]).key_set().raw_repr() & ~plain) Py_RETURN_FALSE;
+    if (Py_TYPE(a[i]) != reinterpret_cast<PyTypeObject*>(THPVariableClass) ||
+        (THPVariable_Unpack(a[i]).key_set().raw_repr() & ~plain))
+      Py_RETURN_FALSE;
   Py_RETURN_TRUE;
 }
 
