@@ -171,7 +171,10 @@ int kfa_bwd_narrow(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v
 /* As kfa_bwd (and its narrow form), with the steps of every key tile shared out to several CTAs where the key tiles
  * alone leave most of the GPU idle (cross attention to a short sequence). The CTAs leave fp32 parts of dK and dV in `parts`
  * (16-byte aligned scratch of kfa_bwd_parts_bytes), which are then summed in a fixed order: results repeat bit for bit.
- * kfa_bwd_parts_bytes is 0 where this would not help; kfa_bwd_parts refuses such problems. */
+ * kfa_bwd_parts_bytes is 0 where this would not help; kfa_bwd_parts refuses such problems. kfa_bwd_parts_count: how many
+ * CTAs share a key tile (1: none), with against_fused only where that is also faster than kfa_bwd_fused. Both look at
+ * nothing but the shapes. */
+int kfa_bwd_parts_count(const KfaTensor4* q, const KfaTensor4* k, int against_fused);
 int64_t kfa_bwd_parts_bytes(const KfaTensor4* q, const KfaTensor4* k);
 int kfa_bwd_parts(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out,
                   const KfaTensor4* dout, const float* lse, float* stats, float* parts, const KfaTensor4* dq,

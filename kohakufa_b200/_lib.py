@@ -51,6 +51,7 @@ SYMBOLS = (
     "kfa_fwd_narrow",
     "kfa_bwd_narrow",
     "kfa_bwd_parts_bytes",
+    "kfa_bwd_parts_count",
     "kfa_bwd_parts",
     "kfa_varlen_zero_rows",
 )
@@ -136,6 +137,7 @@ def load() -> ctypes.CDLL:
         lib.kfa_varlen_zero_rows.argtypes = [T, ctypes.c_int, ip, ip, ctypes.c_int, ctypes.c_int, ctypes.c_int, fp, vp]
         lib.kfa_bwd_parts_bytes.restype = ctypes.c_int64
         lib.kfa_bwd_parts_bytes.argtypes = [T, T]
+        lib.kfa_bwd_parts_count.argtypes = [T, T, ctypes.c_int]
         lib.kfa_bwd_static_scratch.argtypes = [T, T, T, T, T, fp, T, T, T, ctypes.c_float, ctypes.c_int, ctypes.c_int, ip, vp]
         A = ctypes.POINTER(KfaAcc32)
         i64, f32, i32 = ctypes.c_int64, ctypes.c_float, ctypes.c_int
@@ -167,7 +169,7 @@ def load() -> ctypes.CDLL:
 HOST_SYMBOLS = (
     "kfa_last_error", "kfa_fwd", "kfa_bwd", "kfa_bwd_fused", "kfa_fwd_masked", "kfa_bwd_masked", "kfa_fwd_varlen",
     "kfa_bwd_varlen", "kfa_pack_mask", "kfa_fwd_narrow", "kfa_bwd_narrow",
-    "kfa_bwd_parts_bytes", "kfa_bwd_parts", "kfa_varlen_zero_rows",
+    "kfa_bwd_parts_bytes", "kfa_bwd_parts_count", "kfa_bwd_parts", "kfa_varlen_zero_rows",
 )  # fmt: skip
 HOST_PATH = Path(__file__).resolve().parent / "_kfa_host.so"
 _host = None

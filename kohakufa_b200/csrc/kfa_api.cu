@@ -504,8 +504,15 @@ int launch_sum_splits(const kfa::SumParams& p, int bh, cudaStream_t s) {
 // less than half of the GPU: as many as it has SMs for, with at least 4 steps (of about 1.4 us) each, which pay for the
 // CTA's set-up and the sum of the parts. The order of the sums depends on this number, and so on batch and heads, which
 // is why self attention, whose dK and dV do not depend on what else is in the batch, is left alone.
+// against_fused: 1 also where the fused kernel takes no longer. It does five products for seven, so the dQ kernel's CTAs
+// (set-up and epilogue about two steps, spread over the GPU; nearly for nothing if they are one wave) have to take less than
+// the steps that a CTA is spared. Whole backward at D = 64, fused and shared out, in us (queries x keys, heads): 1024 x 77:
+// 8 heads 25 and 23, 20 heads 27 and 29, 74 heads 33 and 41; 2048 x 77: 37 heads 45 and 41, 49 heads 51 and 55; 4096 x 77:
+// 8 heads 64 and 29, 40 heads 86 and 81, 49 heads 96 and 99, 74 heads 114 and 141; 16384 x 77: 40 heads 321 and 290, 50 heads
+// 348 and 366; 4096 x 512: 16 heads 68 and 70, 64 query and 16 K / V heads 245 and 229; 8192 x 1024, 8 heads: 113 and 107.
+// (The line is on the faster side of all 100 shapes measured.)
 // (148 SMs: what this library is built for.)
-int bwd_splits(const KfaTensor4* q, const KfaTensor4* k) {
+int bwd_splits(const KfaTensor4* q, const KfaTensor4* k, bool against_fused = false) {
   for (int i = 0; i < 4; ++i)
     if (q->shape[i] < 1 || k->shape[i] < 1) return 1;  // (kfa_bwd_parts_bytes is asked before anything is checked)
   const int64_t n_k = (k->shape[2] + 127) / 128, n_q = (q->shape[2] + 127) / 128;
@@ -513,7 +520,10 @@ int bwd_splits(const KfaTensor4* q, const KfaTensor4* k) {
   const int64_t steps = (q->shape[1] / k->shape[1]) * n_q;
   if (n_q < 8 * n_k || 2 * tiles > 148) return 1;
   const int64_t n = std::min<int64_t>(148 / tiles, steps / 4);
-  return n < 2 ? 1 : static_cast<int>(n);
+  if (n < 2) return 1;
+  const int64_t query_tiles = q->shape[0] * q->shape[1] * n_q, spared = steps - (steps + n - 1) / n;
+  if (against_fused && query_tiles > 148 && 240 * spared < query_tiles * (2 + n_k) + 1000) return 1;
+  return static_cast<int>(n);
 }
 
 int sum_splits_impl(const KfaTensor4* dk, const KfaTensor4* dv, const Extra& ex, int dtype, void* stream) {
@@ -742,6 +752,10 @@ int kfa_bwd_narrow(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v
   }
   if ((rc = dkdv_impl(q, k, v, dout, stats, dk, dv, ex, scale, block, dtype, dev_status, stream))) return rc;
   return dq_impl(q, k, v, dout, stats, dq, ex, scale, block, dtype, dev_status, stream);
+}
+
+int kfa_bwd_parts_count(const KfaTensor4* q, const KfaTensor4* k, int against_fused) {
+  return q && k ? bwd_splits(q, k, against_fused != 0) : 1;
 }
 
 int64_t kfa_bwd_parts_bytes(const KfaTensor4* q, const KfaTensor4* k) {

@@ -35,6 +35,7 @@ struct Api {
   decltype(&kfa_fwd_narrow) fwd_narrow = nullptr;
   decltype(&kfa_bwd_narrow) bwd_narrow = nullptr;
   decltype(&kfa_bwd_parts_bytes) bwd_parts_bytes = nullptr;
+  decltype(&kfa_bwd_parts_count) bwd_parts_count = nullptr;
   decltype(&kfa_bwd_parts) bwd_parts = nullptr;
   decltype(&kfa_varlen_zero_rows) varlen_zero_rows = nullptr;
 } api;
@@ -236,7 +237,8 @@ PyObject* py_forward(Args a, Py_ssize_t n) {
 }
 
 // backward(q, k, v, out, dout, lse, scale, block, status, fused) -> dq, dk, dv
-// fused: 1 the fused kernels, 0 the split ones, 2 the fused ones unless the split ones can share out their steps
+// fused: 1 the fused kernels; 0 the split ones, which share out their steps where that helps (kfa_bwd_parts); 2 ("auto" at
+// the head dims of the fused ones) those, unless the split ones share out their steps and are faster for it
 PyObject* py_backward(Args a, Py_ssize_t n) {
   need(n, 10);
   const at::Tensor q = tensor(a[0]), k = tensor(a[1]), v = tensor(a[2]), o = tensor(a[3]), lse = tensor(a[5]), status = tensor(a[8]);
@@ -257,9 +259,8 @@ PyObject* py_backward(Args a, Py_ssize_t n) {
     const KfaTensor4 d[8] = {desc(q), desc(k), desc(v), desc(o), desc(g), desc(dq), desc(dk), desc(dv)};
     float *l = lse.data_ptr<float>(), *st = stats.data_ptr<float>();
     int* word = status.data_ptr<int32_t>();
-    const int64_t parts_bytes = (fused == 1) ? 0 : api.bwd_parts_bytes(d, d + 1);
-    if (parts_bytes > 0) {
-      at::Tensor parts = floats(q, {parts_bytes / 4});
+    if (fused != 1 && api.bwd_parts_count(d, d + 1, fused == 2) > 1) {
+      at::Tensor parts = floats(q, {api.bwd_parts_bytes(d, d + 1) / 4});
       check(api.bwd_parts(d, d + 1, d + 2, d + 3, d + 4, l, st, parts.data_ptr<float>(), d + 5, d + 6, d + 7, scale, block,
                           dtype_code(q), word, stream_of(q)));
     } else if (fused) {
@@ -425,6 +426,7 @@ PyObject* py_bind(Args a, Py_ssize_t n) {
   take("kfa_fwd_narrow", api.fwd_narrow);
   take("kfa_bwd_narrow", api.bwd_narrow);
   take("kfa_bwd_parts_bytes", api.bwd_parts_bytes);
+  take("kfa_bwd_parts_count", api.bwd_parts_count);
   take("kfa_bwd_parts", api.bwd_parts);
   take("kfa_varlen_zero_rows", api.varlen_zero_rows);
   Py_INCREF(a[0]);

@@ -82,7 +82,8 @@ def is_deterministic() -> bool:
 
 
 def use_fused_backward(dim: int, batch_heads: int) -> bool:
-    """Whether the fused kernel runs for this head dim under the current mode."""
+    """Whether the fused kernel is there for this head dim and the current mode prefers it to the split ones (that it runs
+    then is up to the lengths in "auto" mode: ``_backward_route``)."""
     if _backward_mode == "split" or batch_heads > 65535:
         return False
     if dim not in FUSED_DIMS:
@@ -91,8 +92,8 @@ def use_fused_backward(dim: int, batch_heads: int) -> bool:
 
 
 def _backward_route(q: Tensor) -> int:
-    """What the library is asked for: 1 the fused kernels, 0 the split ones, 2 ("auto") the fused ones unless few
-    key tiles leave the GPU idle and the split dK / dV kernel can share out its steps (``kfa_bwd_parts``)."""
+    """What the launch path is asked for: 1 the fused kernels, 0 the split ones, which share out their steps where few key
+    tiles leave the GPU idle (``kfa_bwd_parts``), 2 ("auto") the fused ones unless that is faster."""
     if not use_fused_backward(kernel_dim_for(q.shape[-1]), q.shape[0] * q.shape[1]):
         return 0
     return 1 if _backward_mode == "fused" else 2

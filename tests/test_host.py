@@ -80,6 +80,23 @@ def test_parts_bytes_of_empty_tensors():
     assert lib.kfa_bwd_parts_bytes(None, ctypes.byref(k)) == 0
 
 
+def test_shared_out_steps_against_the_fused_kernel():
+    """The line of the measurements beside the rule: many query tiles for few steps stay with the fused kernel."""
+    lib = _lib.load()
+
+    def count(heads, kv_heads, s_q, s_kv, against_fused):
+        q, k = _lib.KfaTensor4(), _lib.KfaTensor4()
+        q.shape[:], k.shape[:] = (1, heads, s_q, 64), (1, kv_heads, s_kv, 64)
+        return lib.kfa_bwd_parts_count(ctypes.byref(q), ctypes.byref(k), against_fused)
+
+    for heads, kv_heads, s_q, s_kv, n in ((8, 8, 1024, 77, 2), (8, 8, 4096, 77, 8), (37, 37, 4096, 77, 4), (32, 8, 8192, 1024, 2)):
+        assert count(heads, kv_heads, s_q, s_kv, 0) == count(heads, kv_heads, s_q, s_kv, 1) == n
+    for heads, kv_heads, s_q, s_kv in ((74, 74, 1024, 77), (74, 74, 4096, 77), (60, 60, 2048, 77), (16, 16, 4096, 512)):
+        assert count(heads, kv_heads, s_q, s_kv, 0) == 2 and count(heads, kv_heads, s_q, s_kv, 1) == 1
+    for heads, kv_heads, s_q, s_kv in ((75, 75, 4096, 77), (8, 8, 896, 77), (8, 8, 4096, 4096)):
+        assert count(heads, kv_heads, s_q, s_kv, 0) == 1
+
+
 def test_causal_and_block_causal_are_exclusive():
     q, k, v = qkv()
     with pytest.raises(ValueError, match="causal is block_causal=1"):
