@@ -237,8 +237,9 @@ PyObject* py_forward(Args a, Py_ssize_t n) {
 }
 
 // backward(q, k, v, out, dout, lse, scale, block, status, fused) -> dq, dk, dv
-// fused: 1 the fused kernels; 0 the split ones, which share out their steps where that helps (kfa_bwd_parts); 2 ("auto" at
-// the head dims of the fused ones) those, unless the split ones share out their steps and are faster for it
+// fused: 1 the fused kernels; 3 the split ones, one CTA per tile; 0 the split ones, which share out their steps where that
+// helps (kfa_bwd_parts); 2 ("auto" at the head dims of the fused ones) those, unless the split ones share out their steps
+// and are faster for it
 PyObject* py_backward(Args a, Py_ssize_t n) {
   need(n, 10);
   const at::Tensor q = tensor(a[0]), k = tensor(a[1]), v = tensor(a[2]), o = tensor(a[3]), lse = tensor(a[5]), status = tensor(a[8]);
@@ -259,11 +260,11 @@ PyObject* py_backward(Args a, Py_ssize_t n) {
     const KfaTensor4 d[8] = {desc(q), desc(k), desc(v), desc(o), desc(g), desc(dq), desc(dk), desc(dv)};
     float *l = lse.data_ptr<float>(), *st = stats.data_ptr<float>();
     int* word = status.data_ptr<int32_t>();
-    if (fused != 1 && api.bwd_parts_count(d, d + 1, fused == 2) > 1) {
+    if ((fused == 0 || fused == 2) && api.bwd_parts_count(d, d + 1, fused == 2) > 1) {
       at::Tensor parts = floats(q, {api.bwd_parts_bytes(d, d + 1) / 4});
       check(api.bwd_parts(d, d + 1, d + 2, d + 3, d + 4, l, st, parts.data_ptr<float>(), d + 5, d + 6, d + 7, scale, block,
                           dtype_code(q), word, stream_of(q)));
-    } else if (fused) {
+    } else if (fused == 1 || fused == 2) {
       at::Tensor acc = floats(q, {q.size(0) * q.size(1) * ((q.size(2) + 127) / 128) * 128 * ((q.size(3) + 15) / 16 * 16)});
       check((q.size(3) % 16 ? api.bwd_narrow : api.bwd_fused)(d, d + 1, d + 2, d + 3, d + 4, l, st, acc.data_ptr<float>(), d + 5,
                                                               d + 6, d + 7, scale, block, dtype_code(q), word, stream_of(q)));

@@ -72,8 +72,10 @@ def get_backward() -> str:
 
 
 def set_deterministic(flag: bool) -> None:
-    """``True``: every later backward uses the split kernels, whose gradients repeat bit for bit;
-    ``False``: back to ``"auto"``. (``KFA_DETERMINISTIC=1`` in the environment does the same.)"""
+    """``True``: every later backward uses the split kernels, one CTA per tile, whose gradients repeat bit for bit and do not
+    depend on what else is in the batch; ``False``: back to ``"auto"``. (``KFA_DETERMINISTIC=1`` in the environment does the
+    same.) In ``"auto"`` mode the last bits of dK and dV of attention to a much shorter sequence depend on the number of
+    batch entries and heads: it decides how many CTAs share out a key tile's steps."""
     set_backward("split" if flag else "auto")
 
 
@@ -92,8 +94,11 @@ def use_fused_backward(dim: int, batch_heads: int) -> bool:
 
 
 def _backward_route(q: Tensor) -> int:
-    """What the launch path is asked for: 1 the fused kernels, 0 the split ones, which share out their steps where few key
-    tiles leave the GPU idle (``kfa_bwd_parts``), 2 ("auto") the fused ones unless that is faster."""
+    """What the launch path is asked for: 3 the split kernels, one CTA per tile, 1 the fused ones, and in "auto" mode 0 the
+    split ones, which share out their steps where few key tiles leave the GPU idle (``kfa_bwd_parts``), or 2 the fused ones
+    unless that is faster."""
+    if _backward_mode == "split":
+        return 3
     if not use_fused_backward(kernel_dim_for(q.shape[-1]), q.shape[0] * q.shape[1]):
         return 0
     return 1 if _backward_mode == "fused" else 2

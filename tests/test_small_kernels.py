@@ -6,7 +6,7 @@ import ctypes
 import pytest
 import torch
 
-from kohakufa_b200 import _lib, op
+from kohakufa_b200 import _lib, attention, op, set_backward
 from kohakufa_b200.mask import pack_mask_op
 
 pytestmark = pytest.mark.gpu
@@ -100,3 +100,22 @@ def test_shared_out_steps(dim, dtype, s_q, s_kv, heads, kv_heads, block):
         # the fp32 sums: at most the count of summed products (queries x heads of the group) times 2^-24 of the largest sum
         noise = s_q * (heads // kv_heads) * 2.0**-24 * float(b.abs().max())
         assert bool(((a - b).abs() <= ulp * b.abs() + noise + 2.0**-24).all())
+
+
+@pytest.mark.parametrize("dim", [64, 80])
+def test_split_mode_does_not_depend_on_the_batch(dim):
+    """In "split" mode a batch entry's gradients are the bits of that entry alone, also where queries outnumber keys so far
+    that "auto" shares out a key tile's steps by the number of tiles in the batch."""
+    gen = torch.Generator().manual_seed(dim)
+    q, k, v, dout = (torch.randn(3, s, 2, dim, generator=gen).half().cuda().transpose(1, 2) for s in (2100, 77, 77, 2100))
+
+    def grads(rows):
+        qkv = [t[rows].detach().requires_grad_() for t in (q, k, v)]
+        return torch.autograd.grad(attention(*qkv), qkv, dout[rows])
+
+    try:
+        set_backward("split")
+        whole, alone = grads(slice(0, 3)), grads(slice(1, 2))
+    finally:
+        set_backward("auto")
+    assert all(torch.equal(a[1:2], b) for a, b in zip(whole, alone))
