@@ -181,6 +181,14 @@ int kfa_bwd_parts(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v,
                   const KfaTensor4* dk, const KfaTensor4* dv, float scale, int block, int dtype, int* dev_status,
                   void* stream);
 
+/* kfa_bwd_parts with n_parts CTAs a key tile (2 .. 148; parts: n_parts * 8 bytes per element of dk, at the head dim of the
+ * kernels): a piece (batch entries, K / V heads with their query heads) of a larger problem has the bits of the whole
+ * with the whole's kfa_bwd_parts_count. */
+int kfa_bwd_parts_n(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out,
+                    const KfaTensor4* dout, const float* lse, float* stats, float* parts, int n_parts, const KfaTensor4* dq,
+                    const KfaTensor4* dk, const KfaTensor4* dv, float scale, int block, int dtype, int* dev_status,
+                    void* stream);
+
 /* Zeros in the rows that kfa_fwd_varlen (n_tensors 1: t = {out}, with its statistics lse) or kfa_bwd_varlen (n_tensors 3:
  * t = {dq, dk, dv}; lse null) do not write for these sequences, for outputs that were not zero-filled beforehand. */
 int kfa_varlen_zero_rows(const KfaTensor4* t, int n_tensors, const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int n_seqs,

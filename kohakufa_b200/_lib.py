@@ -53,6 +53,7 @@ SYMBOLS = (
     "kfa_bwd_parts_bytes",
     "kfa_bwd_parts_count",
     "kfa_bwd_parts",
+    "kfa_bwd_parts_n",
     "kfa_varlen_zero_rows",
 )
 
@@ -134,6 +135,7 @@ def load() -> ctypes.CDLL:
         lib.kfa_fwd_narrow.argtypes = lib.kfa_fwd.argtypes
         lib.kfa_bwd_narrow.argtypes = lib.kfa_bwd_fused.argtypes
         lib.kfa_bwd_parts.argtypes = lib.kfa_bwd_fused.argtypes
+        lib.kfa_bwd_parts_n.argtypes = [T, T, T, T, T, fp, fp, fp, ctypes.c_int, T, T, T, ctypes.c_float, ctypes.c_int, ctypes.c_int, ip, vp]
         lib.kfa_varlen_zero_rows.argtypes = [T, ctypes.c_int, ip, ip, ctypes.c_int, ctypes.c_int, ctypes.c_int, fp, vp]
         lib.kfa_bwd_parts_bytes.restype = ctypes.c_int64
         lib.kfa_bwd_parts_bytes.argtypes = [T, T]

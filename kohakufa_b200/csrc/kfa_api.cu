@@ -768,13 +768,22 @@ int kfa_bwd_parts(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v,
                   const KfaTensor4* dout, const float* lse, float* stats, float* parts, const KfaTensor4* dq,
                   const KfaTensor4* dk, const KfaTensor4* dv, float scale, int block, int dtype, int* dev_status,
                   void* stream) {
+  return kfa_bwd_parts_n(q, k, v, out, dout, lse, stats, parts, kfa_bwd_parts_count(q, k, 0), dq, dk, dv, scale, block, dtype,
+                         dev_status, stream);
+}
+
+int kfa_bwd_parts_n(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out,
+                    const KfaTensor4* dout, const float* lse, float* stats, float* parts, int n_parts, const KfaTensor4* dq,
+                    const KfaTensor4* dk, const KfaTensor4* dv, float scale, int block, int dtype, int* dev_status,
+                    void* stream) {
   int rc;
   if ((rc = check_qkv(q, k, v, dtype, block, true)) || (rc = check_like(out, q, "out"))) return rc;
   Extra ex;
   ex.narrow = true;
-  ex.n_split = bwd_splits(q, k);
+  ex.n_split = n_parts;
   ex.parts = parts;
-  if (ex.n_split < 2) return fail(KFA_ERR_ARG, "kfa_bwd_parts: not a problem whose steps are shared out (kfa_bwd_parts_bytes is 0)");
+  if (n_parts < 2 || n_parts > 148 || k->shape[0] * k->shape[1] > 65535)
+    return fail(KFA_ERR_ARG, "kfa_bwd_parts: not a problem whose steps are shared out (kfa_bwd_parts_bytes is 0), or %d parts", n_parts);
   if (!parts || reinterpret_cast<uintptr_t>(parts) % 16) return fail(KFA_ERR_ARG, "parts: null or not 16-byte aligned");
   if ((rc = prepare_impl(out, dout, lse, stats, nullptr, dtype, stream, nullptr, true))) return rc;
   if ((rc = dkdv_impl(q, k, v, dout, stats, dk, dv, ex, scale, block, dtype, dev_status, stream))) return rc;

@@ -19,7 +19,7 @@ import ctypes
 import torch
 
 from kohakufa_b200 import _lib
-from kohakufa_b200.op import _check, use_fused_backward
+from kohakufa_b200.op import _check, backward_route
 
 
 def _is_bshd(t: torch.Tensor) -> bool:
@@ -75,7 +75,17 @@ class HostPipeline:
         self.lse = [torch.empty(nb, hq, 2, seq_q, dtype=torch.float32, device=self.device) for _ in range(2)]
         stats_floats = self.lib.kfa_bwd_stats_bytes(nb, hq, seq_q) // 4
         self.stats = [torch.empty(stats_floats, dtype=torch.float32, device=self.device) for _ in range(2)]
-        self.fused = use_fused_backward(dim, nb * hq)
+        # the op's route and, where it shares out a key tile's steps, its number of parts: a unit then has the op's bits
+        route = backward_route(dim, nb * hq)
+        shapes = _lib.KfaTensor4(), _lib.KfaTensor4()
+        for s, t in zip(shapes, (q, k)):
+            s.shape[:] = t.shape
+        self.n_parts = self.lib.kfa_bwd_parts_count(*map(ctypes.byref, shapes), int(route == 2)) if route in (0, 2) else 1
+        self.fused = route in (1, 2) and self.n_parts == 1
+        if self.n_parts > 1:
+            self.parts = [
+                torch.empty(2 * self.n_parts * nb * hk * seq_k * dim, dtype=torch.float32, device=self.device) for _ in range(2)
+            ]
         if self.fused:
             acc_floats = self.lib.kfa_bwd_dq_acc_bytes(nb, hq, seq_q, dim) // 4
             self.dq_acc = [torch.empty(acc_floats, dtype=torch.float32, device=self.device) for _ in range(2)]
@@ -92,7 +102,12 @@ class HostPipeline:
         with torch.cuda.device(self.device):
             _lib.check(self.lib.kfa_fwd(ref(q), ref(k), ref(v), ref(out), self.lse[buf].data_ptr(), scale, block, dtype,
                                         self.status.data_ptr(), stream))
-            if self.fused:
+            if self.n_parts > 1:
+                _lib.check(self.lib.kfa_bwd_parts_n(ref(q), ref(k), ref(v), ref(out), ref(dout), self.lse[buf].data_ptr(),
+                                                    self.stats[buf].data_ptr(), self.parts[buf].data_ptr(), self.n_parts,
+                                                    ref(dq), ref(dk), ref(dv), scale, block, dtype, self.status.data_ptr(),
+                                                    stream))
+            elif self.fused:
                 _lib.check(self.lib.kfa_bwd_fused(ref(q), ref(k), ref(v), ref(out), ref(dout), self.lse[buf].data_ptr(),
                                                   self.stats[buf].data_ptr(), self.dq_acc[buf].data_ptr(), ref(dq),
                                                   ref(dk), ref(dv), scale, block, dtype, self.status.data_ptr(), stream))

@@ -93,15 +93,19 @@ def use_fused_backward(dim: int, batch_heads: int) -> bool:
     return _backward_mode == "fused" or FUSED_IS_FASTER[dim]
 
 
-def _backward_route(q: Tensor) -> int:
+def backward_route(dim: int, batch_heads: int) -> int:
     """What the launch path is asked for: 3 the split kernels, one CTA per tile, 1 the fused ones, and in "auto" mode 0 the
     split ones, which share out their steps where few key tiles leave the GPU idle (``kfa_bwd_parts``), or 2 the fused ones
     unless that is faster."""
     if _backward_mode == "split":
         return 3
-    if not use_fused_backward(kernel_dim_for(q.shape[-1]), q.shape[0] * q.shape[1]):
+    if not use_fused_backward(kernel_dim_for(dim), batch_heads):
         return 0
     return 1 if _backward_mode == "fused" else 2
+
+
+def _backward_route(q: Tensor) -> int:
+    return backward_route(q.shape[-1], q.shape[0] * q.shape[1])
 
 
 def _strides_ok(t: Tensor) -> bool:

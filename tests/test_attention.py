@@ -397,3 +397,19 @@ def test_host_buffer_head_groups(storage):
     for g, w in zip(got, want):
         assert oracle.rel_l2(g, w.cpu()) < 1e-3
     assert torch.equal(got[0], want[0].cpu())
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+def test_host_buffer_short_key_sequence(dim):
+    """Where the op shares out a key tile's steps, units of one head pair have its bits all the same."""
+    from kohakufa_b200 import hostio
+
+    gen = torch.Generator().manual_seed(dim)
+    host = [torch.randn(2, s, h, dim, generator=gen).half().pin_memory().transpose(1, 2) for s, h in ((2100, 4), (77, 2), (77, 2), (2100, 4))]
+    pipe = hostio.HostPipeline(*host[:3], "cuda")
+    assert len(pipe.units) == 4 and pipe.n_parts > 1
+    got = hostio.attention_fwd_bwd_host(*host, pipeline=pipe)
+    torch.cuda.synchronize()
+    q, k, v = (t.cuda().requires_grad_() for t in host[:3])
+    for g, w in zip(got, run(q, k, v, host[3].cuda())):
+        assert torch.equal(g, w.cpu())
