@@ -498,7 +498,7 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   int Sq = p.Sq, Skv = p.Skv, q_base = 0, k_base = 0, bc = b;  // bc: batch coordinate in the tensors
   if (p.cu_q != nullptr) {
     q_base = p.cu_q[b];
-    Sq = p.cu_q[b + 1] - q_base;
+    Sq = min(p.cu_q[b + 1] - q_base, p.n_q128 * 128);  // (no statistics past the longest length that the plan states)
     k_base = p.cu_k[b];
     Skv = p.cu_k[b + 1] - k_base;
     bc = 0;

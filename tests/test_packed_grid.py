@@ -64,8 +64,8 @@ def check_halves(lengths, causal):
 
 @pytest.mark.parametrize("n_seqs", [3, 300])
 def test_rows_outside_the_sequences_are_zero(n_seqs):
-    """Freed memory full of NaN is what fresh outputs come from; rows before, after and between the computed ones
-    still read as zero, and so do the statistics."""
+    """Freed memory full of NaN is what fresh outputs come from; rows before and after the sequences still read as zero,
+    and so do the statistics."""
     lengths = [200, 300, 129] + [2] * (n_seqs - 3)
     q, k, v, dout, cu = packed(lengths, 2, 2, 64, extra=40)
     cu = cu + 7
@@ -99,3 +99,18 @@ def test_left_over_rows_of_any_width(heads, dim, first, tail):
     left[first : first + 70] = False
     assert not bool(out[left].any()) and not bool(lse[..., left].any())
     assert bool((out[~left] == 3).all()) and bool((lse[..., ~left] == 3).all()) and bool((wide[..., dim:] == 3).all())
+
+
+def test_plan_shorter_than_a_sequence():
+    """Rows past the longest length that a hand-made plan states (in whole tiles) are not computed: zeros in every output,
+    out of freed memory full of NaN, and the other sequence is as it is alone."""
+    q, k, v, dout, cu = packed([600, 100], 4, 2, 64)
+    junk = [torch.full((700, 4, 64), float("nan"), dtype=q.dtype, device="cuda") for _ in range(8)]
+    stats = torch.full((1 << 20,), float("nan"), device="cuda")
+    del junk, stats
+    got = run(q, k, v, dout, cu, (2, 120, 120))
+    sub = torch.tensor([0, 100], dtype=torch.int32, device="cuda")
+    alone = run(*(t[600:] for t in (q, k, v, dout)), sub, (1, 100, 100))
+    for t, one, covered in zip(got, alone, (256, 128, 128, 128)):  # query rows of a tile of the forward, of the backward, keys
+        assert bool(torch.isfinite(t).all()) and not bool(t[covered:600].any())
+        assert bool(t[:covered].any(-1).all()) and torch.equal(t[600:], one)

@@ -8,6 +8,7 @@ import torch
 
 from kohakufa_b200 import _lib, attention, op, set_backward
 from kohakufa_b200.mask import pack_mask_op
+from oracle import reference as oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -100,6 +101,22 @@ def test_shared_out_steps(dim, dtype, s_q, s_kv, heads, kv_heads, block):
         # the fp32 sums: at most the count of summed products (queries x heads of the group) times 2^-24 of the largest sum
         noise = s_q * (heads // kv_heads) * 2.0**-24 * float(b.abs().max())
         assert bool(((a - b).abs() <= ulp * b.abs() + noise + 2.0**-24).all())
+
+
+@pytest.mark.parametrize("dim", [40, 64, 128])
+def test_shared_out_steps_of_a_batch(dim):
+    """Several batch entries and grouped heads on the shared-out route, through the public call and against fp64 (tolerance of
+    the other fp16 parity tests: P, dS and the results are rounded to 11 bits)."""
+    gen = torch.Generator().manual_seed(dim)
+    q, k, v, dout = (torch.randn(3, s, h, dim, generator=gen).half().cuda().transpose(1, 2) for s, h in ((1100, 4), (77, 2), (77, 2), (1100, 4)))
+    ref = lambda t: ctypes.byref(_lib.tensor4(t))  # noqa: E731
+    assert _lib.load().kfa_bwd_parts_count(ref(q), ref(k), int(dim == 64)) == 4
+    qkv = [t.requires_grad_() for t in (q, k, v)]
+    out = attention(*qkv)
+    got = (out, *torch.autograd.grad(out, qkv, dout))
+    assert _lib.device_status() == 0
+    for g, w in zip(got, oracle.attention_fp64(q, k, v, dout, dim**-0.5, groups=2)):
+        assert oracle.metrics(g, w)["rel_err"] < 5e-3
 
 
 @pytest.mark.parametrize("dim", [64, 80])
