@@ -310,12 +310,8 @@ def plain_eager(*tensors: torch.Tensor) -> bool:
     mode, no ``torch.func`` transform, no forward-mode level, no tensor subclass and no tensor that only the
     dispatcher can resolve (batched gradients, negative views, zero tensors). Only then may it pass the dispatcher by;
     everything else sees the registered custom ops."""
-    if torch.compiler.is_compiling() or not (_host or host()).plain(*tensors):
-        return False
-    return not (
-        torch._C._len_torch_dispatch_stack()
-        or torch._C._len_torch_function_stack()
-        or torch._C._are_functorch_transforms_active()
-        or torch.autograd.forward_ad._current_level >= 0
-        or torch._C._get_tracing_state() is not None
+    return (
+        not torch.compiler.is_compiling()
+        and torch.autograd.forward_ad._current_level < 0
+        and (_host or host()).plain(*tensors)
     )

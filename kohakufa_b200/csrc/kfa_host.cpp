@@ -12,6 +12,9 @@
 #include <torch/csrc/Exceptions.h>
 
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -183,15 +186,21 @@ void need(Py_ssize_t got, Py_ssize_t want) {
 
 using Args = PyObject* const*;
 
-// plain(*tensors) -> bool: whether each is a torch.Tensor (no subclass) and what its address points to is its value. Batched
-// tensors (gradients of `is_grads_batched`), pending negations and zero tensors are torch.Tensor too, but only the
-// dispatcher resolves them.
+// plain(*tensors) -> bool: whether an operator on these tensors would go straight to its kernel. That is, no dispatch or
+// function mode, no torch.func transform and no tracer is active, and each is a torch.Tensor (no subclass) whose address
+// points to its value: batched tensors (gradients of `is_grads_batched`), pending negations and zero tensors are
+// torch.Tensor too, but only the dispatcher resolves them.
 PyObject* py_plain(Args a, Py_ssize_t n) {
   using c10::DispatchKey;
   static const uint64_t plain =
       c10::DispatchKeySet({DispatchKey::CPU, DispatchKey::CUDA, DispatchKey::ADInplaceOrView, DispatchKey::AutogradCPU,
                            DispatchKey::AutogradCUDA, DispatchKey::AutocastCPU, DispatchKey::AutocastCUDA})
           .raw_repr();
+  static const c10::DispatchKeySet interposed(
+      {DispatchKey::FuncTorchDynamicLayerFrontMode, DispatchKey::FuncTorchDynamicLayerBackMode, DispatchKey::Tracer});
+  if (c10::impl::tls_local_dispatch_key_set().included_.has_any(interposed) ||
+      c10::impl::TorchDispatchModeTLS::stack_len() > 0 || at::impl::PythonTorchFunctionTLS::stack_len() > 0)
+    Py_RETURN_FALSE;
   for (Py_ssize_t i = 0; i < n; ++i)
     if (Py_TYPE(a[i]) != reinterpret_cast<PyTypeObject*>(THPVariableClass) ||
         (THPVariable_Unpack(a[i]).key_set().raw_repr() & ~plain))
