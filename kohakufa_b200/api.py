@@ -107,7 +107,7 @@ def attention(
         k = _remove_key_mean(k, compute_dtype)
     q, k, v = (t.to(compute_dtype) for t in (q, k, v))
     softmax_scale = head_dim**-0.5 if scale is None else scale
-    if mask is None and _op.narrow(q, k, v):
+    if mask is None and _op.narrow(q, k, v, frame):
         out = _op.attention_narrow(q, k, v, softmax_scale, frame)
         return out.to(result_dtype) if out.dtype != result_dtype else out
     q, k, v = _fit_head_dim(q, k, v)

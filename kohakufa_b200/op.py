@@ -140,12 +140,37 @@ def _records(q: Tensor, k: Tensor, v: Tensor) -> bool:
     return torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
 
 
-def narrow(q: Tensor, k: Tensor, v: Tensor) -> bool:
+# Rows of an odd multiple of 16 bytes do not begin on 32-byte sectors, so a row of a tile's copy touches a sector more than
+# a widened one. Above 64 columns the backward's kernels wait for that, on every pair of tiles, while widening costs by the
+# row: from so many visible pairs per row copied on, it is the faster way there. (The forward is always faster narrow.)
+# Forward + backward, widened time over narrow time: dim 72: 2 x 16 heads x 6144 1.05, 8 x 12288 0.98; dim 88: 8 x 12288 1.03, 4 x
+# 16384 1.00; dim 104: 2 x 16 x 2048 1.17, 16 x 3072 1.00, 2 x 16 x 6144 0.94, 4 x 16384 0.83; dim 120: 2 x 16 x 6144 1.13, 16 x 8192
+# 1.00, 8 x 12288 0.98, 16 query and 4 K / V heads x 8192 0.93. Up to dim 56: 1.02 to 1.05 at 4 x 16384, more below.
+NARROW_REACH = {72: 4000, 88: 6000, 104: 1200, 120: 3000}
+
+
+def narrow_backward_pays(dim: int, heads: int, kv_heads: int, s_q: int, s_kv: int, block: int) -> bool:
+    """Whether forward + backward of these lengths take no longer with narrow rows than with widened copies."""
+    if dim not in NARROW_REACH:
+        return True
+    seen = s_q * s_kv
+    if block:
+        n = min(s_q, s_kv)
+        seen = min(seen, n * (n + block) // 2 + (s_q - n) * s_kv)
+    return seen * heads <= NARROW_REACH[dim] * (s_q * heads + 2 * s_kv * kv_heads)
+
+
+def narrow(q: Tensor, k: Tensor, v: Tensor, block_causal: int = 0) -> bool:
     """Whether ``attention_narrow`` takes these ``[B, H, S, D]`` inputs as they are: plain eager execution and a head
     dim that is an odd multiple of 8, whose columns up to the next multiple of 16 the kernels read as zeros
     (copying q, k, v, dout and the results to and from wider tensors costs more than a small problem's kernels:
-    forward + backward of 4 x 8 heads x 4096 queries x 77 keys at head dim 40 takes 128 us, 233 with the copies)."""
-    return q.shape[-1] % 16 == 8 and _lib.plain_eager(q, k, v) and _lib.host().narrow_ok(q, k, v)
+    forward + backward of 4 x 8 heads x 4096 queries x 77 keys at head dim 40 takes 128 us, 233 with the copies;
+    ``NARROW_REACH`` says where it no longer does)."""
+    if q.shape[-1] % 16 != 8 or not _lib.plain_eager(q, k, v) or not _lib.host().narrow_ok(q, k, v):
+        return False
+    return not _records(q, k, v) or narrow_backward_pays(
+        q.shape[-1], q.shape[1], k.shape[1], q.shape[2], k.shape[2], block_causal
+    )
 
 
 def attention_narrow(q: Tensor, k: Tensor, v: Tensor, scale: float, block_causal: int) -> Tensor:

@@ -97,6 +97,17 @@ def test_shared_out_steps_against_the_fused_kernel():
         assert count(heads, kv_heads, s_q, s_kv, 0) == 1
 
 
+def test_narrow_rows_where_they_pay():
+    """(dim, heads, K / V heads, queries, keys, frame): the two sides of the measurements beside the rule."""
+    for case in ((8, 4, 4, 16384, 16384, 0), (56, 16, 4, 65536, 65536, 0), (72, 16, 16, 6144, 6144, 0), (88, 8, 8, 12288, 12288, 0),
+                 (104, 16, 16, 2048, 2048, 0), (104, 16, 16, 4096, 4096, 1), (104, 8, 8, 8192, 128, 0), (120, 16, 4, 4096, 4096, 0),
+                 (120, 16, 16, 8192, 8192, 1)):  # fmt: skip
+        assert op.narrow_backward_pays(*case), case
+    for case in ((72, 8, 8, 12288, 12288, 0), (72, 16, 4, 8192, 8192, 0), (104, 16, 16, 4096, 4096, 0), (104, 16, 4, 4096, 4096, 1),
+                 (104, 8, 8, 12288, 12288, 1), (104, 8, 8, 4096, 8192, 0), (120, 16, 4, 6144, 6144, 0), (120, 4, 4, 16384, 16384, 0)):  # fmt: skip
+        assert not op.narrow_backward_pays(*case), case
+
+
 def test_causal_and_block_causal_are_exclusive():
     q, k, v = qkv()
     with pytest.raises(ValueError, match="causal is block_causal=1"):

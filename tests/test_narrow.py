@@ -79,3 +79,13 @@ def test_narrow_leaves_other_inputs_alone():
     for bad in (lambda: op.attention(q, k, v), lambda: attention(q, k[:, :3], v[:, :3])):
         with pytest.raises(ValueError):
             bad()
+
+
+def test_long_recorded_calls_are_widened():
+    """Where the backward's reads of narrow rows cost more than the copies: only calls that autograd records."""
+    q = torch.zeros(1, 20000, 1, 104, dtype=torch.float16, device="cuda").transpose(1, 2)
+    assert op.narrow(q, q, q)
+    leaf = q.detach().requires_grad_()
+    assert not op.narrow(leaf, q, q) and op.narrow(leaf[:, :, :1000], q[:, :, :1000], q[:, :, :1000])
+    with torch.no_grad():
+        assert op.narrow(leaf, q, q)
