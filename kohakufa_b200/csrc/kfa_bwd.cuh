@@ -564,7 +564,7 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // step s -> query tile and query head
   auto tile_of = [&](int s) { return use_list ? static_cast<int>(s_list[s] & 0xffffu) : first_i + (s_first + s) % n_per; };
   auto head_of = [&](int s) { return hk * p.group + (use_list ? static_cast<int>(s_list[s] >> 16) : (s_first + s) / n_per); };
-  const Ctl ctl{s_abort, p.status};
+  const Ctl ctl{s_abort};
   const bool dead = (*s_abort != 0);
 
   if (dead) {
@@ -832,6 +832,7 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_before();
   __syncthreads();
   if (*s_abort) {  // gave up (or an earlier kernel did): the rows of this CTA read as NaN
+    if (tid == 0) report_abort(s_abort, p.status);
     const int r1 = min(kv0 + 128, Skv);
     if (p.acc_mode == 0) {
       fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dk) + 2 * (bc * p.dk_sb + hk * p.dk_sh), p.dk_ss, k_base + kv0, k_base + r1, p.cols);
@@ -1055,7 +1056,7 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const uint32_t tmem = *s_tmem;
   if (use_list) n_steps = static_cast<int>(s_tmem[2]);
   auto tile_of = [&](int it) { return use_list ? static_cast<int>(s_list[it]) : it; };
-  const Ctl ctl{s_abort, p.status};
+  const Ctl ctl{s_abort};
   const bool dead = (*s_abort != 0);
 
   if (dead) {
@@ -1264,6 +1265,7 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   tc_fence_before();
   __syncthreads();
   if (*s_abort) {  // gave up (or an earlier kernel did): the rows of this CTA read as NaN
+    if (tid == 0) report_abort(s_abort, p.status);
     const int r1 = min(row0 + 128, Sq);
     if (p.acc_mode == 0)
       fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dq) + 2 * (bc * p.dq_sb + h * p.dq_sh), p.dq_ss, q_base + row0, q_base + r1, p.cols);

@@ -267,7 +267,7 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
-  const Ctl ctl{s_abort, p.status};
+  const Ctl ctl{s_abort};
   const bool dead = (*s_abort != 0);
 
   // Each role sets its own register budget first thing: the issue warpgroup (warps 12-15) gives registers
@@ -620,6 +620,7 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_before();
   __syncthreads();
   if (*s_abort) {  // gave up (or an earlier kernel did): dK, dV rows of this CTA read as NaN (dQ: see the convert kernel)
+    if (tid == 0) report_abort(s_abort, p.status);
     const int r1 = min(kv0 + 128, Skv);
     fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dk) + 2 * (b * p.dk_sb + hk * p.dk_sh), p.dk_ss, kv0, r1, p.cols);
     fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dv) + 2 * (b * p.dv_sb + hk * p.dv_sh), p.dv_ss, kv0, r1, p.cols);

@@ -340,7 +340,7 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     n_tiles[1] = n_tiles[1] > 0 ? n_max : 0;
   }
   auto tile_of = [&](int it) { return use_list ? static_cast<int>(s_list[it]) : it; };
-  const Ctl ctl{s_abort, p.status};
+  const Ctl ctl{s_abort};
   const bool dead = (*s_abort != 0);
 
   // Each role sets its register budget first (the kernel starts with 128 per thread).
@@ -740,6 +740,7 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   __syncthreads();
   if (warp == 8) TR(2, 1, 0, 5);
   if (*s_abort) {  // gave up (or an earlier kernel did): the rows of this CTA read as NaN
+    if (tid == 0) report_abort(s_abort, p.status);
     const int r1 = min(row0 + 256, Sq);
     const long long bhl = static_cast<long long>(b) * p.H + h;
     if (p.mode == 0) {

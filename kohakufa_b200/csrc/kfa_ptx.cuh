@@ -2,10 +2,9 @@
 // mbarriers with bounded waits, TMA tile loads, tensor-memory (TMEM) allocation,
 // tcgen05 MMAs with shared-memory / TMEM operands, TMEM loads and stores.
 //
-// Every wait in this file is bounded: a wait that runs out sets the CTA's abort flag and
-// a status word in global memory, and returns false; the caller leaves its loop and
-// falls through to the kernel's common teardown, which frees TMEM. No kernel here can
-// spin forever.
+// Every wait in this file is bounded: a wait that runs out leaves its code in the CTA's abort word and returns false;
+// the caller leaves its loop and falls through to the kernel's common teardown, which frees TMEM and reports the code
+// in a status word in global memory. No kernel here can spin forever.
 #pragma once
 
 #include <cuda.h>
@@ -66,7 +65,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 }
 
 // A limit this short only occurs in the test build whose waits are meant to run out: it then polls
-// without letting the hardware suspend the thread, and looks at the clock on every turn.
+// without letting the hardware suspend the thread.
 constexpr bool KFA_SHORT_WAITS = (KFA_WAIT_CYCLES < 1000000ll);
 
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
@@ -105,40 +104,35 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Per-CTA control block: abort flag in shared memory, status word in global memory.
+// Per-CTA control block: the abort word in shared memory. 0: fine; 1: an earlier kernel reported a failure; above: the code
+// of the wait of this CTA that gave up, which report_abort takes to the status word at the end of the kernel.
 struct Ctl {
   volatile int* s_abort;
-  int* g_status;
 };
 
-// Bounded wait for the phase with the given parity to complete. Returns false when the
-// CTA is aborting (this wait or another ran out of time, or another CTA reported a failure).
-// The first test stands apart from the polling loop: a wait whose phase has already completed (most of them,
-// in a pipeline that runs ahead) costs one try_wait and, for a warp, one vote.
-__device__ __forceinline__ bool mbar_wait_poll(uint32_t bar, uint32_t parity, volatile int* s_abort, int* g_status,
-                                            int site) {
+// Bounded wait for the phase with the given parity to complete. Returns false when the CTA is aborting (this wait or another
+// ran out of time). The first test stands apart from the polling loop: a wait whose phase has already completed (most of them,
+// in a pipeline that runs ahead) costs one try_wait and, for a warp, one vote. The loop is inlined at some thirty places of a
+// kernel and lies between their hot instructions, so it holds as little as it can: looking at the status word of other CTAs
+// as well, every so many turns, and reporting from here made the kernels 6 to 7 KB longer, and the fused backward at D = 64
+// wait that much longer for instructions (video: 64 heads x 4096, frames of 256: 459 -> 446 us, 32 x 12 x 201 dense: 54.8 ->
+// 53.4; forward there 29.5 -> 28.8).
+__device__ __forceinline__ bool mbar_wait_poll(uint32_t bar, uint32_t parity, volatile int* s_abort, int site) {
   const long long t0 = clock64();
-  uint32_t spins = 0;
-  for (;;) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (KFA_SHORT_WAITS || (++spins & 31u) == 0u) {
-      if (*s_abort) return false;
-      if ((spins & 1023u) == 0u && *reinterpret_cast<volatile int*>(g_status) != 0) {
-        *s_abort = 1;
-        return false;
-      }
-      if (clock64() - t0 > KFA_WAIT_CYCLES) {
-        *s_abort = 1;
-        atomicCAS(g_status, 0, KFA_DEV_TIMEOUT_BASE + site);
-        return false;
-      }
+#pragma unroll 1
+  while (!mbar_try_wait(bar, parity)) {
+    if (*s_abort != 0) return false;
+    if (clock64() - t0 > KFA_WAIT_CYCLES) {
+      *s_abort = KFA_DEV_TIMEOUT_BASE + site;
+      return false;
     }
   }
+  return true;
 }
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const Ctl& ctl, int site) {
-  if (mbar_try_wait(bar, parity)) return true;
-  return mbar_wait_poll(bar, parity, ctl.s_abort, ctl.g_status, site);
+  if (__builtin_expect(mbar_try_wait(bar, parity), 1)) return true;
+  return mbar_wait_poll(bar, parity, ctl.s_abort, site);
 }
 
 // For a thread that gives up while copies it has started may still be in flight: waits (bounded, without
@@ -154,8 +148,8 @@ __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
 // and every lane gets the same answer (false if any lane gave up).
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const Ctl& ctl, int site) {
   bool ok = mbar_try_wait(bar, parity);
-  if (__all_sync(0xffffffffu, ok)) return true;  // the phase had completed: about 25 clk
-  if (!ok) ok = mbar_wait_poll(bar, parity, ctl.s_abort, ctl.g_status, site);
+  if (__builtin_expect(__all_sync(0xffffffffu, ok), 1)) return true;  // the phase had completed: about 25 clk
+  if (!ok) ok = mbar_wait_poll(bar, parity, ctl.s_abort, site);
   return __all_sync(0xffffffffu, ok);
 }
 
@@ -165,7 +159,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, co
 // round trip is hidden, and the data was complete when the early test saw it.
 __device__ __forceinline__ bool mbar_wait_warp_probed(bool probed, uint32_t bar, uint32_t parity, const Ctl& ctl,
                                                       int site) {
-  if (__all_sync(0xffffffffu, probed)) return true;
+  if (__builtin_expect(__all_sync(0xffffffffu, probed), 1)) return true;
   return mbar_wait_warp(bar, parity, ctl, site);
 }
 
@@ -476,6 +470,10 @@ __device__ __forceinline__ void fill_rows_nan16(void* base, long long row_stride
     const long long r = r0 + i / chunks;
     *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(base) + 2 * (r * row_stride + (i % chunks) * 8)) = nan8;
   }
+}
+// One thread of a CTA whose abort word is set, after the CTA's last barrier: the first failure of all stays in the status word.
+__device__ __forceinline__ void report_abort(const volatile int* s_abort, int* status) {
+  if (*s_abort > 1) atomicCAS(status, 0, *s_abort);
 }
 __device__ __forceinline__ void fill_nan32(float* base, long long count) {
   for (long long i = threadIdx.x; i < count; i += blockDim.x) base[i] = __int_as_float(0x7fc00000);

@@ -48,7 +48,7 @@ kfa_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
-  const Ctl ctl{s_abort, p.status};
+  const Ctl ctl{s_abort};
   bool ok = (*s_abort == 0);
   if (ok && tid == 0) {
     mbar_expect_tx(bar0, 2 * CH * TILE_BYTES_64);
@@ -86,6 +86,7 @@ kfa_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) report_abort(s_abort, p.status);
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem, 128);

@@ -36,7 +36,7 @@ kfa_selftest_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
-  const Ctl ctl{s_abort, status};
+  const Ctl ctl{s_abort};
   const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
   bool ok = true;
 
@@ -94,6 +94,7 @@ kfa_selftest_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) report_abort(s_abort, status);
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem, 256);
