@@ -5,12 +5,12 @@ fallback. If it is missing, loading raises with the build command instead of deg
 """
 
 import ctypes
+import os
+import sys
 import threading
 from pathlib import Path
 
 import torch
-
-import os
 
 # The in-tree build; the environment variable KFA_LIBRARY points the package at another build of the same
 # sources (e.g. one compiled with different tuning macros) without touching the tree.
@@ -198,9 +198,17 @@ def host():
                 )
             from kohakufa_b200 import _kfa_host
 
-            _kfa_host.bind(KfaError, {n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in HOST_SYMBOLS})
+            entries = {n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in HOST_SYMBOLS}
+            _kfa_host.bind(KfaError, entries, _backward_route)
             _host = _kfa_host
     return _host
+
+
+def _backward_route(dim: int, batch_heads: int) -> int:
+    """What the C++ nodes ask when their backward runs: ``op.backward_route``, or -1 where the registered op has to run."""
+    if torch.compiler.is_compiling() or torch.autograd.forward_ad._current_level >= 0:
+        return -1
+    return sys.modules["kohakufa_b200.op"].backward_route(dim, batch_heads)
 
 
 def check(rc: int) -> None:

@@ -103,6 +103,11 @@ def attention(
     if compute_dtype not in COMPUTE_DTYPES:
         raise TypeError(f"compute_dtype {compute_dtype}: one of {COMPUTE_DTYPES}")
     result_dtype, head_dim = q.dtype, q.shape[-1]
+    if mask is None and not center_keys and q.dtype == k.dtype == v.dtype == compute_dtype:
+        # most calls: nothing to cast, widen or pack
+        out = _op.direct(q, k, v, head_dim**-0.5 if scale is None else scale, frame)
+        if out is not None:
+            return out
     if center_keys:
         k = _remove_key_mean(k, compute_dtype)
     q, k, v = (t.to(compute_dtype) for t in (q, k, v))

@@ -15,8 +15,8 @@ synchronisation, every buffer from the caching allocator, so ``torch.compile`` k
 CUDA graph capture works (after one eager call on the device, which creates the status word).
 
 ``attention`` and ``attention_varlen`` enter that launch path directly when nothing but plain eager execution
-is going on (``_lib.plain_eager``), through a ``torch.autograd.Function`` of their own where gradients are needed: the
-dispatch of a Python custom op costs more than a small problem's kernels. Under ``torch.compile``,
+is going on (``_lib.plain_eager``), through an autograd node in C++ where gradients are needed: the dispatch of a Python
+custom op, or a ``torch.autograd.Function``, costs more than a small problem's kernels. Under ``torch.compile``,
 dispatch or function modes, ``torch.func`` transforms, forward-mode differentiation, tracing or with tensor
 subclasses, and in a backward that is itself recorded, the custom ops run as they always have.
 
@@ -28,7 +28,6 @@ import os
 
 import torch
 from torch import Tensor
-from torch.autograd import Function
 
 from kohakufa_b200 import _lib
 
@@ -39,7 +38,9 @@ MAX_KERNEL_DIM = 128
 
 def kernel_dim_for(dim: int) -> int:
     """The smallest head dim a kernel is built for that holds ``dim``."""
-    return min(d for d in KERNEL_DIMS if d >= dim)
+    if dim > MAX_KERNEL_DIM:
+        raise ValueError(f"head dim {dim}: up to {MAX_KERNEL_DIM}")
+    return max(-(-dim // 16) * 16, 16)
 
 
 # Which backward runs. Two implementations exist:
@@ -175,9 +176,17 @@ def narrow(q: Tensor, k: Tensor, v: Tensor, block_causal: int = 0) -> bool:
 
 def attention_narrow(q: Tensor, k: Tensor, v: Tensor, scale: float, block_causal: int) -> Tensor:
     """``attention`` for inputs that ``narrow`` accepts."""
-    if _records(q, k, v):
-        return _Attention.apply(q, k, v, float(scale), int(block_causal))
-    return _lib.host().forward(q, k, v, float(scale), int(block_causal), _lib.status_word(q.device))[0]
+    host, args = _lib.host(), (q, k, v, float(scale), int(block_causal), _lib.status_word(q.device))
+    return host.attention(*args) if _records(q, k, v) else host.forward(*args)[0]
+
+
+def direct(q: Tensor, k: Tensor, v: Tensor, scale: float, block: int) -> Tensor | None:
+    """``attention`` without a mask, of plain eager inputs that the kernels take as they are; None for all others (and for the
+    first call on a device, whose status word does not exist yet)."""
+    if not _lib.plain_eager(q, k, v):
+        return None
+    word = _lib._status.get(q.get_device())
+    return None if word is None else _lib.host().call(q, k, v, scale, block, word)
 
 
 def _bshd_like(t: Tensor) -> Tensor:
@@ -231,29 +240,6 @@ def _backward(ctx, dout, dlse):
 attention_fwd_op.register_autograd(_backward, setup_context=_setup_context)
 
 
-class _Attention(Function):
-    """``attention_fwd_op`` with its gradient, for plain eager calls."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, scale, block):
-        out, lse = _lib.host().forward(q, k, v, scale, block, _lib.status_word(q.device))
-        ctx.save_for_backward(q, k, v, out, lse)
-        ctx.scale, ctx.block = scale, block
-        return out
-
-    @staticmethod
-    def backward(ctx, dout):
-        q, k, v, out, lse = ctx.saved_tensors
-        if not _strides_ok(dout):
-            dout = dout.contiguous()
-        if torch.is_grad_enabled() or not _lib.plain_eager(q, k, v, out, dout, lse):
-            grads = attention_bwd_op(q, k, v, out, dout, lse, ctx.scale, ctx.block)
-        else:
-            fused = _backward_route(q)
-            grads = _lib.host().backward(q, k, v, out, dout, lse, ctx.scale, ctx.block, _lib.status_word(q.device), fused)
-        return *grads, None, None
-
-
 # --------------------------------------------------------------------------------------
 # Boolean masks: ops of their own (the reference passes optional word tensors to its one op pair,
 # op.py:58-121); the packed words are saved for the backward.
@@ -305,30 +291,6 @@ def _masked_backward(ctx, dout, dlse):
 masked_fwd_op.register_autograd(_masked_backward, setup_context=_masked_setup)
 
 
-class _MaskedAttention(Function):
-    """``masked_fwd_op`` with its gradient, for plain eager calls."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, words, words_t, tiles, scale):
-        out, lse = _lib.host().forward_masked(q, k, v, words, tiles, scale, _lib.status_word(q.device))
-        ctx.save_for_backward(q, k, v, out, lse, words, words_t, tiles)
-        ctx.scale = scale
-        return out
-
-    @staticmethod
-    def backward(ctx, dout):
-        saved = ctx.saved_tensors
-        q, k, v, out, lse, words, words_t, tiles = saved
-        if not _strides_ok(dout):
-            dout = dout.contiguous()
-        args = (q, k, v, out, dout, lse, words, words_t, tiles, ctx.scale)
-        if torch.is_grad_enabled() or not _lib.plain_eager(dout, *saved):
-            grads = masked_bwd_op(*args)
-        else:
-            grads = _lib.host().backward_masked(*args, _lib.status_word(q.device))
-        return *grads, None, None, None, None
-
-
 def attention(
     q: Tensor,
     k: Tensor,
@@ -359,13 +321,12 @@ def attention(
         if not direct or not _lib.plain_eager(*words):
             return masked_fwd_op(q, k, v, *words, float(scale))[0]
         if _records(q, k, v):
-            return _MaskedAttention.apply(q, k, v, *words, float(scale))
+            return _lib.host().attention_masked(q, k, v, *words, float(scale), _lib.status_word(q.device))
         return _lib.host().forward_masked(q, k, v, packed.words, packed.tiles, float(scale), _lib.status_word(q.device))[0]
     if not direct:
         return attention_fwd_op(q, k, v, float(scale), int(block_causal))[0]
-    if _records(q, k, v):
-        return _Attention.apply(q, k, v, float(scale), int(block_causal))
-    return _lib.host().forward(q, k, v, float(scale), int(block_causal), _lib.status_word(q.device))[0]
+    host, args = _lib.host(), (q, k, v, float(scale), int(block_causal), _lib.status_word(q.device))
+    return host.attention(*args) if _records(q, k, v) else host.forward(*args)[0]
 
 
 # --------------------------------------------------------------------------------------
@@ -428,28 +389,6 @@ def _varlen_backward(ctx, dout, dlse):
 varlen_fwd_op.register_autograd(_varlen_backward, setup_context=_varlen_setup)
 
 
-class _VarlenAttention(Function):
-    """``varlen_fwd_op`` with its gradient, for plain eager calls."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, cu_q, cu_k, max_q, max_k, scale, block):
-        out, lse = _lib.host().forward_varlen(q, k, v, cu_q, cu_k, max_q, max_k, scale, block, _lib.status_word(q.device))
-        ctx.save_for_backward(q, k, v, out, lse, cu_q, cu_k)
-        ctx.plan = (max_q, max_k, scale, block)
-        return out
-
-    @staticmethod
-    def backward(ctx, dout):
-        saved = ctx.saved_tensors
-        q, k, v, out, lse, cu_q, cu_k = saved
-        args = (q, k, v, out, dout.contiguous(), lse, cu_q, cu_k, *ctx.plan)
-        if torch.is_grad_enabled() or not _lib.plain_eager(dout, *saved):
-            grads = varlen_bwd_op(*args)
-        else:
-            grads = _lib.host().backward_varlen(*args, _lib.status_word(q.device))
-        return *grads, None, None, None, None, None, None
-
-
 def varlen_plan(
     cu_seqlens_q: Tensor, cu_seqlens_k: Tensor, heads: int = 0, kv_heads: int = 0, block: int = 0
 ) -> tuple[int, int, int]:
@@ -499,5 +438,5 @@ def attention_varlen(
     if not direct:
         return varlen_fwd_op(*args)[0]
     if _records(q, k, v):
-        return _VarlenAttention.apply(*args)
+        return _lib.host().attention_varlen(*args, _lib.status_word(q.device))
     return _lib.host().forward_varlen(*args, _lib.status_word(q.device))[0]

@@ -5,6 +5,7 @@ import time
 
 import pytest
 import torch
+import torch.utils.checkpoint
 
 from kohakufa_b200 import _lib, attention, attention_varlen, pack_mask, set_backward, varlen_plan
 from kohakufa_b200 import op
@@ -144,6 +145,36 @@ def test_direct_path_and_autograd_features():
         q.mul_(1.0)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         out.backward(dout)
+
+
+@pytest.mark.gpu
+def test_recorded_calls_in_the_engine():
+    """The node's backward runs on a thread of the autograd engine: an error of the library there is the exception a direct
+    call raises, a checkpoint's recomputation (which leaves the forward by an exception of a saved-tensor hook) works, and
+    so does a backward that finds a dispatch mode (the registered op runs)."""
+    (q, k, v), dout = inputs()
+    out = attention(q, k, v)
+    flat = torch.empty(dout.numel() + 8, dtype=dout.dtype, device="cuda")[1 : dout.numel() + 1]
+    odd = flat.copy_(dout.transpose(1, 2).reshape(-1)).view(2, 200, 4, 128).transpose(1, 2)  # starts 2 bytes past a boundary
+    with pytest.raises(_lib.KfaError):
+        torch.autograd.grad(out, (q, k, v), odd, retain_graph=True)
+    want = torch.autograd.grad(out, (q, k, v), dout)
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(out, (q, k, v), dout)
+    out = torch.utils.checkpoint.checkpoint(attention, q, k, v, use_reentrant=False)
+    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(out, (q, k, v), dout), want))
+    seen = []
+
+    class Mode(torch.utils._python_dispatch.TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(func.name())
+            return func(*args, **(kwargs or {}))
+
+    out = attention(q, k, v)
+    with Mode():
+        got = torch.autograd.grad(out, (q, k, v), dout)
+    assert "kohakufa_b200::sm100_backward" in seen
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
 
 
 @pytest.mark.gpu
