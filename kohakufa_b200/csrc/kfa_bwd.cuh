@@ -35,6 +35,8 @@
 // One difference: dS = (dP - delta) * P uses the fp32 P, not the 16-bit rounded one (one rounding less).
 #pragma once
 
+#include <type_traits>
+
 #include "kfa_fwd.cuh"
 
 namespace kfa {
@@ -310,29 +312,6 @@ __device__ __forceinline__ void store_acc_row_f32(uint32_t taddr, int col0, int 
   }
 }
 
-// Writes a row of an fp32 accumulator (TMEM columns [col0, col0 + ncols), those below cols) times mul as 16-bit.
-template <bool BF16, int W = 32>
-__device__ __forceinline__ void store_acc_row(uint32_t taddr, int col0, int ncols, int cols, float mul, uint8_t* grow,
-                                              bool valid) {
-  for (int cc = col0; cc < col0 + ncols; cc += W) {
-    float o[W];
-    tmem_ldw<W>(taddr + cc, reinterpret_cast<uint32_t*>(o));
-    tmem_wait_ld();
-    if (valid) {
-#pragma unroll
-      for (int i = 0; i < W; i += 8) {
-        if (cc + i >= cols) break;
-        uint4 w;
-        w.x = pack16<BF16>(o[i] * mul, o[i + 1] * mul);
-        w.y = pack16<BF16>(o[i + 2] * mul, o[i + 3] * mul);
-        w.z = pack16<BF16>(o[i + 4] * mul, o[i + 5] * mul);
-        w.w = pack16<BF16>(o[i + 6] * mul, o[i + 7] * mul);
-        *reinterpret_cast<uint4*>(grow + 2 * (cc + i)) = w;
-      }
-    }
-  }
-}
-
 // P^T and dS^T in the dK / dV kernel. The per-query statistics (-m at st[0..], -log2 l at st[128..],
 // -delta at st[256..], in shared memory) belong to COLUMNS of the transposed tile, so every thread
 // needs them for every column it touches. With one TMEM lane (key) per thread that is all 64 columns
@@ -520,7 +499,22 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint32_t* s_list = reinterpret_cast<uint32_t*>(smem + Cfg::KV_SMEM_TILES + 256);
   const bool use_list = MASKW && p.mt != nullptr;
 
-  if (tid == 0) {
+  // (the thread that starts the copies also sets up the barriers: see the forward)
+  auto load_step = [&](int s, int i, int head) {  // Q_i, dO_i and the statistics into their slot
+    const int slot = s % NSL;
+    const uint32_t base = sSlot + slot * Cfg::KV_SLOT_BYTES;
+    mbar_expect_tx(bar(B_QREADY + slot), 2 * Cfg::TILE_BYTES + STATS_BYTES);
+    for (int ch = 0; ch < CH; ++ch) {
+      tma_load_4d(base + ch * Cfg::CHUNK_BYTES, &tmQ, bar(B_QREADY + slot), ch * Cfg::CHUNK_COLS, q_base + i * 128, head, bc);
+      tma_load_4d(base + Cfg::TILE_BYTES + ch * Cfg::CHUNK_BYTES, &tmDO, bar(B_QREADY + slot), ch * Cfg::CHUNK_COLS,
+                  q_base + i * 128, head, bc);
+    }
+    bulk_load(base + 2 * Cfg::TILE_BYTES, p.stats + (static_cast<long long>(b) * p.H + head) * p.stats_sh + i * 384ll, STATS_BYTES,
+              bar(B_QREADY + slot));
+  };
+  int issued = 0, earlier = 0;
+  if (warp == 9 && lane == 0) {
+    earlier = load_status(p.status);
     mbar_init(bar(B_KV), 1);
     for (int i = 0; i < NSL; ++i) {
       mbar_init(bar(B_QREADY + i), 1);
@@ -533,8 +527,19 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     mbar_init(bar(B_DS), 256);
     mbar_init(bar(B_ACC), 1);
     mbar_init(bar(B_DRAIN), 1);
-    *s_abort = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+    *s_abort = 0;
     fence_mbar_init();
+    fence_async_smem();
+    if (use_list || n_steps > 0) {
+      mbar_expect_tx(bar(B_KV), 2 * Cfg::TILE_BYTES);
+      for (int ch = 0; ch < CH; ++ch) {
+        tma_load_4d(sK + ch * Cfg::CHUNK_BYTES, &tmK, bar(B_KV), ch * Cfg::CHUNK_COLS, k_base + kv0, hk, bc);
+        tma_load_4d(sV + ch * Cfg::CHUNK_BYTES, &tmV, bar(B_KV), ch * Cfg::CHUNK_COLS, k_base + kv0, hk, bc);
+      }
+    }
+    if (!use_list)
+      for (; issued < min(n_steps, NSL); ++issued)
+        load_step(issued, first_i + (s_first + issued) % n_per, hk * p.group + (s_first + issued) / n_per);
   }
   if (warp == 0) {
     tmem_alloc(smem_u32(s_tmem), Cfg::TMEM_COLS);
@@ -565,45 +570,19 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   auto tile_of = [&](int s) { return use_list ? static_cast<int>(s_list[s] & 0xffffu) : first_i + (s_first + s) % n_per; };
   auto head_of = [&](int s) { return hk * p.group + (use_list ? static_cast<int>(s_list[s] >> 16) : (s_first + s) / n_per); };
   const Ctl ctl{s_abort};
-  const bool dead = (*s_abort != 0);
 
-  if (dead) {
-  } else if (warp == 9) {
+  if (warp == 9) {
     // =========================== TMA producer ===========================
-    if (lane == 0 && n_steps > 0) {
-      prefetch_tensormap(&tmQ);
-      prefetch_tensormap(&tmK);
-      prefetch_tensormap(&tmV);
-      prefetch_tensormap(&tmDO);
-      mbar_expect_tx(bar(B_KV), 2 * Cfg::TILE_BYTES);
-      for (int ch = 0; ch < CH; ++ch) {
-        tma_load_4d(sK + ch * Cfg::CHUNK_BYTES, &tmK, bar(B_KV), ch * Cfg::CHUNK_COLS, k_base + kv0, hk, bc);
-        tma_load_4d(sV + ch * Cfg::CHUNK_BYTES, &tmV, bar(B_KV), ch * Cfg::CHUNK_COLS, k_base + kv0, hk, bc);
-      }
-      bool ok = true;
-      int issued = 0;
-      for (int s = 0; s < n_steps; ++s) {
-        const int slot = s % NSL, use = s / NSL;
-        if (use > 0) ok = mbar_wait(bar(B_QFREE + slot), (use - 1) & 1, ctl, 11);
+    if (lane == 0) {
+      if (earlier != 0) *s_abort = 1;
+      bool ok = (earlier == 0);
+      for (int s = issued; s < n_steps && ok; ++s) {
+        if (s >= NSL) ok = mbar_wait(bar(B_QFREE + s % NSL), (s / NSL - 1) & 1, ctl, 11);
         if (!ok) break;
-        const int i = tile_of(s);
-        const int head = head_of(s);
-        const uint32_t base = sSlot + slot * Cfg::KV_SLOT_BYTES;
-        mbar_expect_tx(bar(B_QREADY + slot), 2 * Cfg::TILE_BYTES + STATS_BYTES);
-        for (int ch = 0; ch < CH; ++ch) {
-          tma_load_4d(base + ch * Cfg::CHUNK_BYTES, &tmQ, bar(B_QREADY + slot), ch * Cfg::CHUNK_COLS, q_base + i * 128, head, bc);
-          tma_load_4d(base + Cfg::TILE_BYTES + ch * Cfg::CHUNK_BYTES, &tmDO, bar(B_QREADY + slot), ch * Cfg::CHUNK_COLS,
-                      q_base + i * 128, head, bc);
-        }
-        bulk_load(base + 2 * Cfg::TILE_BYTES,
-                  p.stats + (static_cast<long long>(b) * p.H + head) * p.stats_sh + i * 384ll,
-                  STATS_BYTES, bar(B_QREADY + slot));
+        load_step(s, tile_of(s), head_of(s));
         issued = s + 1;
       }
-      if (!ok) {  // aborting: let the copies in flight land before the CTA gives up its shared memory
-        mbar_drain(bar(B_KV), 0);
-        for (int s = max(issued - NSL, 0); s < issued; ++s) mbar_drain(bar(B_QREADY + s % NSL), (s / NSL) & 1);
-      }
+      if (use_list && n_steps == 0) mbar_drain(bar(B_KV), 0);  // (nothing visible in a mask: nothing else waits for K and V)
     }
   } else if (warp == 8) {
     // =========================== MMA issue ===========================
@@ -821,9 +800,11 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (ok) {
         tc_fence_after();
         const uint32_t tacc = tmem + (hq ? Cfg::TM_ACC1 : Cfg::TM_ACC0) + lane_base;
-        if (p.acc_mode == 0)
-          store_acc_row<BF16, col_step(D)>(tacc, 0, D, p.cols, hq ? p.scale : 1.0f, grow, valid);
-        else
+        if (p.acc_mode == 0) {  // (K and V have been read for the last time)
+          const int w = 32 * (warp & 3);
+          store_rows16<BF16, D>(tacc, hq ? p.scale : 1.0f, (hq ? sV : sK) + 2 * D * w, min(Skv - kv0 - w, 32),
+                                grow - 2 * lane * (hq ? p.dk_ss : p.dv_ss), hq ? p.dk_ss : p.dv_ss, p.cols);
+        } else
           store_acc_row_f32<col_step(D)>(tacc, 0, D, hq ? p.scale : 1.0f, grow32, valid, p.acc_mode == 2);
       }
     }
@@ -833,6 +814,10 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   if (*s_abort) {  // gave up (or an earlier kernel did): the rows of this CTA read as NaN
     if (tid == 0) report_abort(s_abort, p.status);
+    if (warp == 9 && lane == 0) {  // the copies it has started land before the CTA leaves its shared memory
+      if (use_list || n_steps > 0) mbar_drain(bar(B_KV), 0);
+      for (int s = max(issued - NSL, 0); s < issued; ++s) mbar_drain(bar(B_QREADY + s % NSL), (s / NSL) & 1);
+    }
     const int r1 = min(kv0 + 128, Skv);
     if (p.acc_mode == 0) {
       fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dk) + 2 * (bc * p.dk_sb + hk * p.dk_sh), p.dk_ss, k_base + kv0, k_base + r1, p.cols);
@@ -1006,7 +991,24 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   uint16_t* s_list = reinterpret_cast<uint16_t*>(smem + Cfg::Q_SMEM_TILES + 256);
   const bool use_list = MASKW && p.mt != nullptr;
 
-  if (tid == 0) {
+  // (the thread that starts the copies also sets up the barriers: see the forward)
+  auto load_k = [&](int j, int tile) {
+    const int ks = j % NK;
+    mbar_expect_tx(bar(B_KREADY + ks), Cfg::TILE_BYTES);
+    for (int ch = 0; ch < CH; ++ch)
+      tma_load_4d(sKr + ks * Cfg::TILE_BYTES + ch * Cfg::CHUNK_BYTES, &tmK, bar(B_KREADY + ks), ch * Cfg::CHUNK_COLS,
+                  k_base + tile * 128, h / p.group, bc);
+  };
+  auto load_v = [&](int j, int tile) {
+    const int vs = j % NV;
+    mbar_expect_tx(bar(B_VREADY + vs), Cfg::TILE_BYTES);
+    for (int ch = 0; ch < CH; ++ch)
+      tma_load_4d(sVr + vs * Cfg::TILE_BYTES + ch * Cfg::CHUNK_BYTES, &tmV, bar(B_VREADY + vs), ch * Cfg::CHUNK_COLS,
+                  k_base + tile * 128, h / p.group, bc);
+  };
+  int issued_k = 0, issued_v = 0, earlier = 0;
+  if (warp == 9 && lane == 0) {
+    earlier = load_status(p.status);
     mbar_init(bar(B_Q), 1);
     for (int i = 0; i < NK; ++i) {
       mbar_init(bar(B_KREADY + i), 1);
@@ -1025,8 +1027,22 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     mbar_init(bar(B_DPREAD), 256);
     mbar_init(bar(B_DSFREE + 0), 1);
     mbar_init(bar(B_DSFREE + 1), 1);
-    *s_abort = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+    *s_abort = 0;
     fence_mbar_init();
+    fence_async_smem();
+    mbar_expect_tx(bar(B_Q), 2 * Cfg::TILE_BYTES);
+    for (int ch = 0; ch < CH; ++ch) {
+      tma_load_4d(sQ + ch * Cfg::CHUNK_BYTES, &tmQ, bar(B_Q), ch * Cfg::CHUNK_COLS, q_base + row0, h, bc);
+      tma_load_4d(sDO + ch * Cfg::CHUNK_BYTES, &tmDO, bar(B_Q), ch * Cfg::CHUNK_COLS, q_base + row0, h, bc);
+    }
+    if (!use_list)
+      for (int j = 0; j < min(n_steps, NK); ++j) {
+        load_k(j, j);
+        issued_k = j + 1;
+        if (j >= NV) continue;
+        load_v(j, j);
+        issued_v = j + 1;
+      }
   }
   if (warp == 0) {
     tmem_alloc(smem_u32(s_tmem), Cfg::TMEM_COLS);
@@ -1057,43 +1073,22 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   if (use_list) n_steps = static_cast<int>(s_tmem[2]);
   auto tile_of = [&](int it) { return use_list ? static_cast<int>(s_list[it]) : it; };
   const Ctl ctl{s_abort};
-  const bool dead = (*s_abort != 0);
 
-  if (dead) {
-  } else if (warp == 9) {
+  if (warp == 9) {
     if (lane == 0) {
-      prefetch_tensormap(&tmQ);
-      prefetch_tensormap(&tmK);
-      prefetch_tensormap(&tmV);
-      prefetch_tensormap(&tmDO);
-      mbar_expect_tx(bar(B_Q), 2 * Cfg::TILE_BYTES);
-      for (int ch = 0; ch < CH; ++ch) {
-        tma_load_4d(sQ + ch * Cfg::CHUNK_BYTES, &tmQ, bar(B_Q), ch * Cfg::CHUNK_COLS, q_base + row0, h, bc);
-        tma_load_4d(sDO + ch * Cfg::CHUNK_BYTES, &tmDO, bar(B_Q), ch * Cfg::CHUNK_COLS, q_base + row0, h, bc);
-      }
-      bool ok = true;
-      int issued_k = 0, issued_v = 0;
-      for (int j = 0; j < n_steps; ++j) {
-        const int ks = j % NK, vs = j % NV;
-        if (j >= NK) ok = mbar_wait(bar(B_KFREE + ks), (j / NK - 1) & 1, ctl, 51);
+      if (earlier != 0) *s_abort = 1;
+      bool ok = (earlier == 0);
+      for (int j = min(issued_k, issued_v); j < n_steps && ok; ++j) {
+        if (j >= issued_k) {
+          if (j >= NK) ok = mbar_wait(bar(B_KFREE + j % NK), (j / NK - 1) & 1, ctl, 51);
+          if (!ok) break;
+          load_k(j, tile_of(j));
+          issued_k = j + 1;
+        }
+        if (j >= NV) ok = mbar_wait(bar(B_VFREE + j % NV), (j / NV - 1) & 1, ctl, 52);
         if (!ok) break;
-        mbar_expect_tx(bar(B_KREADY + ks), Cfg::TILE_BYTES);
-        for (int ch = 0; ch < CH; ++ch)
-          tma_load_4d(sKr + ks * Cfg::TILE_BYTES + ch * Cfg::CHUNK_BYTES, &tmK, bar(B_KREADY + ks), ch * Cfg::CHUNK_COLS,
-                      k_base + tile_of(j) * 128, h / p.group, bc);
-        issued_k = j + 1;
-        if (j >= NV) ok = mbar_wait(bar(B_VFREE + vs), (j / NV - 1) & 1, ctl, 52);
-        if (!ok) break;
-        mbar_expect_tx(bar(B_VREADY + vs), Cfg::TILE_BYTES);
-        for (int ch = 0; ch < CH; ++ch)
-          tma_load_4d(sVr + vs * Cfg::TILE_BYTES + ch * Cfg::CHUNK_BYTES, &tmV, bar(B_VREADY + vs), ch * Cfg::CHUNK_COLS,
-                      k_base + tile_of(j) * 128, h / p.group, bc);
+        load_v(j, tile_of(j));
         issued_v = j + 1;
-      }
-      if (!ok) {  // aborting: let the copies in flight land before the CTA gives up its shared memory
-        mbar_drain(bar(B_Q), 0);
-        for (int j = max(issued_k - NK, 0); j < issued_k; ++j) mbar_drain(bar(B_KREADY + j % NK), (j / NK) & 1);
-        for (int j = max(issued_v - NV, 0); j < issued_v; ++j) mbar_drain(bar(B_VREADY + j % NV), (j / NV) & 1);
       }
     }
   } else if (warp == 8) {
@@ -1251,10 +1246,18 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       constexpr int SPLIT = ((D / 2 + 15) / 16) * 16;
       constexpr int W = (SPLIT % 32 == 0 && (D - SPLIT) % 32 == 0) ? 32 : 16;
       const int c0 = hk ? SPLIT : 0, nc = hk ? D - SPLIT : SPLIT;
-      if (p.acc_mode == 0) {
+      if (p.acc_mode == 0) {  // (Q and dO have been read for the last time)
+        const int w = 32 * (warp & 3);
         uint8_t* grow = reinterpret_cast<uint8_t*>(p.dq) +
-                        2 * (bc * p.dq_sb + h * p.dq_sh + static_cast<long long>(q_base + row) * p.dq_ss);
-        store_acc_row<BF16, W>(tmem + Cfg::TM_ACC0 + lane_base, c0, nc, p.cols, p.scale, grow, row < Sq);
+                        2 * (bc * p.dq_sb + h * p.dq_sh + static_cast<long long>(q_base + row0 + w) * p.dq_ss + c0);
+        auto store = [&](auto n) {
+          constexpr int NC = decltype(n)::value;
+          if constexpr (NC > 0)
+            store_rows16<BF16, NC>(tmem + Cfg::TM_ACC0 + lane_base + c0, p.scale, (hk ? sDO : sQ) + 2 * NC * w, min(Sq - row0 - w, 32),
+                                   grow, p.dq_ss, p.cols - c0);
+        };
+        if (hk == 0) store(std::integral_constant<int, SPLIT>());
+        else store(std::integral_constant<int, D - SPLIT>());
       } else {
         float* grow32 = p.dq32 + (static_cast<long long>(b) * p.H + h) * p.dq32_sh + static_cast<long long>(row) * D;
         store_acc_row_f32<W>(tmem + Cfg::TM_ACC0 + lane_base, c0, nc, p.scale, grow32, row < Sq, p.acc_mode == 2);
@@ -1266,6 +1269,11 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   __syncthreads();
   if (*s_abort) {  // gave up (or an earlier kernel did): the rows of this CTA read as NaN
     if (tid == 0) report_abort(s_abort, p.status);
+    if (warp == 9 && lane == 0) {  // the copies it has started land before the CTA leaves its shared memory
+      mbar_drain(bar(B_Q), 0);
+      for (int j = max(issued_k - NK, 0); j < issued_k; ++j) mbar_drain(bar(B_KREADY + j % NK), (j / NK) & 1);
+      for (int j = max(issued_v - NV, 0); j < issued_v; ++j) mbar_drain(bar(B_VREADY + j % NV), (j / NV) & 1);
+    }
     const int r1 = min(row0 + 128, Sq);
     if (p.acc_mode == 0)
       fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dq) + 2 * (bc * p.dq_sb + h * p.dq_sh), p.dq_ss, q_base + row0, q_base + r1, p.cols);

@@ -216,19 +216,26 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   // step s -> query head, query tile. Key tile kt starts its walk kt tiles in, so that the CTAs of a head
   // that run side by side add their dQ tiles to different places.
   const int rot = (n_per > 0) ? kt % n_per : 0;
-  auto tile_of = [&](int s) {
-    int r = s % n_per + rot;
-    if (r >= n_per) r -= n_per;
-    return first_i + r;
-  };
-  auto head_of = [&](int s) { return hk * p.group + s / n_per; };
-  auto tile_at = [&](const StepWalk& w) {  // the same without a division, for the loops that walk step by step
+  auto tile_at = [&](const StepWalk& w) {
     int r = w.rel + rot;
     if (r >= n_per) r -= n_per;
     return first_i + r;
   };
 
-  if (tid == 0) {
+  // (the thread that starts the copies also sets up the barriers: see the forward)
+  auto load_q = [&](int s, int i, int head) {
+    mbar_expect_tx(bar(B_QREADY + s % NQ), TB);
+    for (int ch = 0; ch < CH; ++ch)
+      tma_load_4d(sQ + s % NQ * TB + ch * TILE_BYTES_64, &tmQ, bar(B_QREADY + s % NQ), ch * 64, i * 128, head, b);
+  };
+  auto load_do = [&](int s, int i, int head) {
+    mbar_expect_tx(bar(B_DOREADY + s % NDO), TB);
+    for (int ch = 0; ch < CH; ++ch)
+      tma_load_4d(sDO + s % NDO * TB + ch * TILE_BYTES_64, &tmDO, bar(B_DOREADY + s % NDO), ch * 64, i * 128, head, b);
+  };
+  int earlier = 0, issued = 0, issued_dl = 0;  // (per producing thread: steps whose copies it has started)
+  if (warp == 13 && lane == 0) {
+    earlier = load_status(p.status);
     mbar_init(bar(B_KV), 1);
     for (int i = 0; i < NQ; ++i) {
       mbar_init(bar(B_QREADY + i), 1);
@@ -256,8 +263,19 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     mbar_init(bar(B_DLFREE), 256);
     mbar_init(bar(B_STGFREE), 1);
     mbar_init(bar(B_STGFULL), 128);
-    *s_abort = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+    *s_abort = 0;
     fence_mbar_init();
+    fence_async_smem();
+    if (n_steps > 0) {  // K, Q and V, dO of the first step
+      mbar_expect_tx(bar(B_KV), 2 * TB);
+      for (int ch = 0; ch < CH; ++ch) {
+        tma_load_4d(sK + ch * TILE_BYTES_64, &tmK, bar(B_KV), ch * 64, kv0, hk, b);
+        tma_load_4d(sV + ch * TILE_BYTES_64, &tmV, bar(B_KV), ch * 64, kv0, hk, b);
+      }
+      load_q(0, first_i + rot, hk * p.group);
+      load_do(0, first_i + rot, hk * p.group);
+      issued = 1;
+    }
   }
   if (warp == 0) {
     tmem_alloc(smem_u32(s_tmem), Cfg::TMEM_COLS);
@@ -268,84 +286,59 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
   const Ctl ctl{s_abort};
-  const bool dead = (*s_abort != 0);
 
   // Each role sets its own register budget first thing: the issue warpgroup (warps 12-15) gives registers
   // up, the others wait until theirs are available.
-  if (dead) {
-  } else if (warp == 15) {
+  if (warp == 15) {
     // =========================== copies of the per-query statistics ===========================
     reg_budget<FUSED_REGS_ISSUE>();
     if (lane == 0 && n_steps > 0) {
       bool ok = true;
-      int ml_issued = 0, dl_issued = 0;
-      for (int s = 0; s < n_steps; ++s) {
-        const float* src = p.stats + (static_cast<long long>(b) * p.H + head_of(s)) * p.stats_sh + tile_of(s) * 384ll;
+      StepWalk walk;
+      for (int s = 0; s < n_steps; ++s, walk.next(n_per)) {
+        const float* src = p.stats + (static_cast<long long>(b) * p.H + hk * p.group + walk.g) * p.stats_sh + tile_at(walk) * 384ll;
         const int slot = s & 1, use = s >> 1;
         if (use > 0) ok = mbar_wait(bar(B_MLFREE + slot), (use - 1) & 1, ctl, 48);
         if (!ok) break;
         mbar_expect_tx(bar(B_MLREADY + slot), Cfg::ML_BYTES);
         bulk_load(sML + slot * Cfg::ML_BYTES, src, Cfg::ML_BYTES, bar(B_MLREADY + slot));
-        ml_issued = s + 1;
+        issued = s + 1;
         if (s > 0) ok = mbar_wait(bar(B_DLFREE), (s - 1) & 1, ctl, 49);
         if (!ok) break;
         mbar_expect_tx(bar(B_DLREADY), Cfg::DELTA_BYTES);
         bulk_load(sDL, src + 256, Cfg::DELTA_BYTES, bar(B_DLREADY));
-        dl_issued = s + 1;
-      }
-      if (!ok) {
-        for (int s = max(ml_issued - 2, 0); s < ml_issued; ++s) mbar_drain(bar(B_MLREADY + (s & 1)), (s >> 1) & 1);
-        if (dl_issued > 0) mbar_drain(bar(B_DLREADY), (dl_issued - 1) & 1);
+        issued_dl = s + 1;
       }
     }
   } else if (warp == 13) {
     // =========================== TMA producer: K, V, then the Q ring ===========================
     reg_budget<FUSED_REGS_ISSUE>();
+    if (lane == 0 && earlier != 0) *s_abort = 1;
     if (lane == 0 && n_steps > 0) {
-      prefetch_tensormap(&tmQ);
-      prefetch_tensormap(&tmK);
-      prefetch_tensormap(&tmV);
-      mbar_expect_tx(bar(B_KV), 2 * TB);
-      for (int ch = 0; ch < CH; ++ch) {
-        tma_load_4d(sK + ch * TILE_BYTES_64, &tmK, bar(B_KV), ch * 64, kv0, hk, b);
-        tma_load_4d(sV + ch * TILE_BYTES_64, &tmV, bar(B_KV), ch * 64, kv0, hk, b);
-      }
-      bool ok = true;
-      int issued = 0;
-      for (int s = 0; s < n_steps; ++s) {
-        const int slot = s % NQ, use = s / NQ;
-        if (use > 0) ok = mbar_wait(bar(B_QFREE + slot), (use - 1) & 1, ctl, 31);
+      bool ok = (earlier == 0);
+      StepWalk walk;
+      walk.next(n_per);
+      for (int s = 1; s < n_steps && ok; ++s, walk.next(n_per)) {
+        if (s >= NQ) ok = mbar_wait(bar(B_QFREE + s % NQ), (s / NQ - 1) & 1, ctl, 31);
         if (!ok) break;
-        mbar_expect_tx(bar(B_QREADY + slot), TB);
-        for (int ch = 0; ch < CH; ++ch)
-          tma_load_4d(sQ + slot * TB + ch * TILE_BYTES_64, &tmQ, bar(B_QREADY + slot), ch * 64, tile_of(s) * 128,
-                      head_of(s), b);
+        load_q(s, tile_at(walk), hk * p.group + walk.g);
         issued = s + 1;
-      }
-      if (!ok) {  // aborting: let the copies in flight land before the CTA gives up its shared memory
-        mbar_drain(bar(B_KV), 0);
-        for (int s = max(issued - NQ, 0); s < issued; ++s) mbar_drain(bar(B_QREADY + s % NQ), (s / NQ) & 1);
       }
     }
   } else if (warp == 14) {
     // =========================== TMA producer: the dO ring ===========================
     reg_budget<FUSED_REGS_ISSUE>();
     if (lane == 0 && n_steps > 0) {
-      prefetch_tensormap(&tmDO);
       bool ok = true;
-      int issued = 0;
-      for (int s = 0; s < n_steps; ++s) {
-        const int slot = s % NDO, use = s / NDO;
-        if (use > 0) ok = mbar_wait(bar(B_DOFREE + slot), (use - 1) & 1, ctl, 32);
+      issued = 1;  // (the first was started with the barriers)
+      StepWalk walk;
+      walk.next(n_per);
+      for (int s = 1; s < n_steps; ++s, walk.next(n_per)) {
+        if (s >= NDO) ok = mbar_wait(bar(B_DOFREE + s % NDO), (s / NDO - 1) & 1, ctl, 32);
         if (!ok) break;
-        mbar_expect_tx(bar(B_DOREADY + slot), TB);
-        for (int ch = 0; ch < CH; ++ch)
-          tma_load_4d(sDO + slot * TB + ch * TILE_BYTES_64, &tmDO, bar(B_DOREADY + slot), ch * 64, tile_of(s) * 128,
-                      head_of(s), b);
+        load_do(s, tile_at(walk), hk * p.group + walk.g);
         issued = s + 1;
       }
-      if (!ok)
-        for (int s = max(issued - NDO, 0); s < issued; ++s) mbar_drain(bar(B_DOREADY + s % NDO), (s / NDO) & 1);
     }
   } else if (warp == 12) {
     // =========================== MMA issue ===========================
@@ -612,7 +605,10 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (ok) {
         tc_fence_after();
         const uint32_t tacc = tmem + (hq ? Cfg::TM_DK : Cfg::TM_DV) + lane_base;
-        store_acc_row<BF16>(tacc, 0, D, p.cols, hq ? p.scale : 1.0f, grow, valid);
+        // (K and V have been read for the last time)
+        const int w = 32 * (warp & 3);
+        store_rows16<BF16, D>(tacc, hq ? p.scale : 1.0f, (hq ? sV : sK) + 2 * D * w, min(Skv - kv0 - w, 32),
+                              grow - 2 * lane * (hq ? p.dk_ss : p.dv_ss), hq ? p.dk_ss : p.dv_ss, p.cols);
       }
     }
   }
@@ -621,6 +617,17 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __syncthreads();
   if (*s_abort) {  // gave up (or an earlier kernel did): dK, dV rows of this CTA read as NaN (dQ: see the convert kernel)
     if (tid == 0) report_abort(s_abort, p.status);
+    if (lane == 0 && n_steps > 0) {  // the copies that the producers have started land before the CTA leaves its shared memory
+      if (warp == 13) {
+        mbar_drain(bar(B_KV), 0);
+        for (int s = max(issued - NQ, 0); s < issued; ++s) mbar_drain(bar(B_QREADY + s % NQ), (s / NQ) & 1);
+      } else if (warp == 14) {
+        for (int s = max(issued - NDO, 0); s < issued; ++s) mbar_drain(bar(B_DOREADY + s % NDO), (s / NDO) & 1);
+      } else if (warp == 15) {
+        for (int s = max(issued - 2, 0); s < issued; ++s) mbar_drain(bar(B_MLREADY + (s & 1)), (s >> 1) & 1);
+        if (issued_dl > 0) mbar_drain(bar(B_DLREADY), (issued_dl - 1) & 1);
+      }
+    }
     const int r1 = min(kv0 + 128, Skv);
     fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dk) + 2 * (b * p.dk_sb + hk * p.dk_sh), p.dk_ss, kv0, r1, p.cols);
     fill_rows_nan16(reinterpret_cast<uint8_t*>(p.dv) + 2 * (b * p.dv_sb + hk * p.dv_sh), p.dv_ss, kv0, r1, p.cols);

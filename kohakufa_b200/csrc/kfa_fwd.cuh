@@ -283,7 +283,21 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   const bool use_list = MASKW && p.mt != nullptr;
 
   // ---- setup ----
-  if (tid == 0) {
+  // The thread that starts the copies sets up the barriers and starts the first ones at once: they fly while tensor memory
+  // is allocated and the roles find their places. It also looks at the status word, once those copies are on their way: an
+  // earlier failure aborts the CTA like one of its own waits. (Copies after the CTA's first barrier, behind the status word's
+  // round trip, and the epilogue a row per thread, against now: forward 32 x 12 x 201 rows, D = 64, 28.9 -> 25.4 us, 4 x 8 x
+  // 4096 x 77 keys, D = 48, 31.2 -> 26.2; 32 heads x 4096 causal, D = 128, 136 -> 133.)
+  auto load_kv = [&](int idx, int j) {  // K_j (even idx) or V_j into its stage of the ring
+    mbar_expect_tx(bar(B_KVREADY + idx % NS), Cfg::TILE_BYTES);
+    const CUtensorMap* map = (idx & 1) ? &tmV : &tmK;
+    for (int ch = 0; ch < CH; ++ch)
+      tma_load_4d(sKV + (idx % NS * CH + ch) * Cfg::CHUNK_BYTES, map, bar(B_KVREADY + idx % NS), ch * Cfg::CHUNK_COLS,
+                  k_base + j * 128, h / p.group, bc);
+  };
+  int kv_issued = 0, earlier = 0;
+  if (warp == 13 && lane == 0) {
+    earlier = load_status(p.status);
     mbar_init(bar(B_QREADY + 0), 1);
     mbar_init(bar(B_QREADY + 1), 1);
     for (int i = 0; i < NS; ++i) {
@@ -301,9 +315,18 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       mbar_init(bar(B_OFINAL + i), 1);
       mbar_init(bar(B_DRAIN + i), 1);
     }
-    // An earlier failure (status word already set): allocate, skip the work, free.
-    *s_abort = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+    *s_abort = 0;
     fence_mbar_init();
+    fence_async_smem();
+    for (int hf = 0; hf < 2; ++hf) {
+      if (n_tiles[hf] == 0) continue;
+      mbar_expect_tx(bar(B_QREADY + hf), Cfg::TILE_BYTES);
+      for (int ch = 0; ch < CH; ++ch)
+        tma_load_4d(sQ + (hf * CH + ch) * Cfg::CHUNK_BYTES, &tmQ, bar(B_QREADY + hf), ch * Cfg::CHUNK_COLS,
+                    q_base + row0 + 128 * hf, h, bc);
+    }
+    if (!use_list)
+      for (; kv_issued < min(2 * n_max, NS); ++kv_issued) load_kv(kv_issued, kv_issued >> 1);
   }
   if (warp == 0) {
     tmem_alloc(smem_u32(s_tmem), Cfg::TMEM_COLS);
@@ -341,49 +364,21 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   }
   auto tile_of = [&](int it) { return use_list ? static_cast<int>(s_list[it]) : it; };
   const Ctl ctl{s_abort};
-  const bool dead = (*s_abort != 0);
 
   // Each role sets its register budget first (the kernel starts with 128 per thread).
-  if (dead) {
-    // nothing to do
-  } else if (warp == 15) {
+  if (warp == 15) {
     reg_budget<FWD_REGS_ISSUE>();
   } else if (warp == 13) {
     // =========================== TMA producer ===========================
     reg_budget<FWD_REGS_ISSUE>();
     if (lane == 0) {
-      prefetch_tensormap(&tmQ);
-      prefetch_tensormap(&tmK);
-      prefetch_tensormap(&tmV);
-      for (int hf = 0; hf < 2; ++hf) {
-        if (n_tiles[hf] == 0) continue;
-        mbar_expect_tx(bar(B_QREADY + hf), Cfg::TILE_BYTES);
-        for (int ch = 0; ch < CH; ++ch)
-          tma_load_4d(sQ + (hf * CH + ch) * Cfg::CHUNK_BYTES, &tmQ, bar(B_QREADY + hf), ch * Cfg::CHUNK_COLS,
-                      q_base + row0 + 128 * hf, h, bc);
-      }
-      int armed[NS];  // last use index armed per stage (for the drain on abort)
-      for (int i = 0; i < NS; ++i) armed[i] = -1;
-      bool ok = true;
-      for (int idx = 0; idx < 2 * n_max && ok; ++idx) {
-        const int j = tile_of(idx >> 1);
-        const int stage = idx % NS;
-        const int use = idx / NS;
-        if (use > 0) ok = mbar_wait(bar(B_KVFREE + stage), (use - 1) & 1, ctl, 1);
+      if (earlier != 0) *s_abort = 1;
+      bool ok = (earlier == 0);
+      for (int idx = kv_issued; idx < 2 * n_max && ok; ++idx) {
+        if (idx >= NS) ok = mbar_wait(bar(B_KVFREE + idx % NS), (idx / NS - 1) & 1, ctl, 1);
         if (!ok) break;
-        mbar_expect_tx(bar(B_KVREADY + stage), Cfg::TILE_BYTES);
-        const CUtensorMap* map = (idx & 1) ? &tmV : &tmK;
-        for (int ch = 0; ch < CH; ++ch)
-          tma_load_4d(sKV + (stage * CH + ch) * Cfg::CHUNK_BYTES, map, bar(B_KVREADY + stage), ch * Cfg::CHUNK_COLS,
-                      k_base + j * 128, h / p.group, bc);
-        armed[stage] = use;
-      }
-      if (!ok) {
-        // Aborting: let the copies already in flight land before the CTA gives up its smem.
-        for (int hf = 0; hf < 2; ++hf)
-          if (n_tiles[hf] > 0) mbar_drain(bar(B_QREADY + hf), 0);
-        for (int i = 0; i < NS; ++i)
-          if (armed[i] >= 0) mbar_drain(bar(B_KVREADY + i), armed[i] & 1);
+        load_kv(idx, tile_of(idx >> 1));
+        kv_issued = idx + 1;
       }
     }
   } else if (warp == 12 || warp == 14) {
@@ -704,27 +699,10 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           log2_l = 0.f;
         }
         const bool valid = row < Sq;
-        uint8_t* orow = reinterpret_cast<uint8_t*>(p.o) +
-                        2 * (bc * p.o_sb + h * p.o_sh + static_cast<long long>(q_base + row) * p.o_ss);
-        constexpr int W = col_step(D);
-#pragma unroll
-        for (int cc = 0; cc < D; cc += W) {
-          float o[W];
-          tmem_ldw<W>(tO + cc, reinterpret_cast<uint32_t*>(o));
-          tmem_wait_ld();
-          if (valid) {
-#pragma unroll
-            for (int i = 0; i < W; i += 8) {
-              if (cc + i >= p.cols) break;
-              uint4 w;
-              w.x = pack16<BF16>(o[i] * inv, o[i + 1] * inv);
-              w.y = pack16<BF16>(o[i + 2] * inv, o[i + 3] * inv);
-              w.z = pack16<BF16>(o[i + 4] * inv, o[i + 5] * inv);
-              w.w = pack16<BF16>(o[i + 6] * inv, o[i + 7] * inv);
-              *reinterpret_cast<uint4*>(orow + 2 * (cc + i)) = w;
-            }
-          }
-        }
+        // (the half's Q tile has been read for the last time)
+        const int w0 = row0 + 128 * hf + 32 * (warp & 3);  // the warp's first row
+        uint8_t* orow = reinterpret_cast<uint8_t*>(p.o) + 2 * (bc * p.o_sb + h * p.o_sh + static_cast<long long>(q_base + w0) * p.o_ss);
+        store_rows16<BF16, D>(tO, inv, sQ + hf * Cfg::TILE_BYTES + 64 * D * (warp & 3), min(Sq - w0, 32), orow, p.o_ss, p.cols);
         if (valid) {
           float* lse = p.lse + (static_cast<long long>(bc) * p.H + h) * 2 * p.Sq + q_base;
           lse[row] = m;
@@ -741,6 +719,11 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   if (warp == 8) TR(2, 1, 0, 5);
   if (*s_abort) {  // gave up (or an earlier kernel did): the rows of this CTA read as NaN
     if (tid == 0) report_abort(s_abort, p.status);
+    if (warp == 13 && lane == 0) {  // the copies it has started land before the CTA leaves its shared memory
+      for (int hf = 0; hf < 2; ++hf)
+        if (n_tiles[hf] > 0) mbar_drain(bar(B_QREADY + hf), 0);
+      for (int idx = max(kv_issued - NS, 0); idx < kv_issued; ++idx) mbar_drain(bar(B_KVREADY + idx % NS), (idx / NS) & 1);
+    }
     const int r1 = min(row0 + 256, Sq);
     const long long bhl = static_cast<long long>(b) * p.H + h;
     if (p.mode == 0) {

@@ -183,10 +183,6 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
       : "memory");
 }
 
-__device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
-  asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
-}
-
 // ----------------------------------------------------------------------------------
 // Tensor memory
 // ----------------------------------------------------------------------------------
@@ -459,26 +455,6 @@ __device__ __forceinline__ void reg_budget() {
   }
 }
 
-// ----------------------------------------------------------------------------------
-// What a CTA that gives up leaves behind: NaN in every output row it owns, so that a timed-out wait
-// cannot pass for a result (0x7fff is a NaN in fp16 and in bf16). Called by all threads of the CTA.
-// ----------------------------------------------------------------------------------
-__device__ __forceinline__ void fill_rows_nan16(void* base, long long row_stride, int r0, int r1, int dim) {
-  const int chunks = dim / 8;
-  const uint4 nan8 = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
-  for (int i = threadIdx.x; i < (r1 - r0) * chunks; i += blockDim.x) {
-    const long long r = r0 + i / chunks;
-    *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(base) + 2 * (r * row_stride + (i % chunks) * 8)) = nan8;
-  }
-}
-// One thread of a CTA whose abort word is set, after the CTA's last barrier: the first failure of all stays in the status word.
-__device__ __forceinline__ void report_abort(const volatile int* s_abort, int* status) {
-  if (*s_abort > 1) atomicCAS(status, 0, *s_abort);
-}
-__device__ __forceinline__ void fill_nan32(float* base, long long count) {
-  for (long long i = threadIdx.x; i < count; i += blockDim.x) base[i] = __int_as_float(0x7fc00000);
-}
-
 template <int W>
 __device__ __forceinline__ void tmem_ldw(uint32_t taddr, uint32_t* r) {
   if constexpr (W == 32) tmem_ld32(taddr, r);
@@ -498,6 +474,9 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+
+// A load of the status word whose value is looked at later: its round trip to L2 (about 700 clk) stands in nobody's way.
+__device__ __forceinline__ int load_status(const int* status) { return *reinterpret_cast<const volatile int*>(status); }
 
 // Two fp32 -> one 32-bit word of two 16-bit values (lo in the low half), round to nearest even.
 template <bool BF16>
@@ -528,6 +507,66 @@ __device__ __forceinline__ float load16(const void* p) {
   } else {
     return __half2float(*reinterpret_cast<const __half*>(p));
   }
+}
+
+// ----------------------------------------------------------------------------------
+// Accumulator rows to global memory, as 16-bit
+// ----------------------------------------------------------------------------------
+// A warp's 32 rows (TMEM lanes) of NC columns times `mul` (of the thread's own row), through 32 * 2 NC bytes of shared memory
+// that nothing else uses any more: a thread holds a whole row, and a store of 16 bytes by each of 32 rows touches 32 lines
+// (2000 clk for the epilogue of a CTA at D = 64); from shared memory a store instruction writes whole rows one after the other.
+// The 16-byte pieces of row r are exchanged so that 8 rows' writes and a row's reads fall into different banks.
+// rows: how many of the 32 exist; g: the first row in global memory, `stride` elements from one to the next; pieces at columns
+// of `cols` (counted from the first) and above are not written.
+template <bool BF16, int NC>
+__device__ __forceinline__ void store_rows16(uint32_t taddr, float mul, uint32_t stage, int rows, void* g, long long stride, int cols) {
+  constexpr int P = NC / 8, W = NC % 32 == 0 ? 32 : 16;
+  constexpr int G = P % 8 == 0 ? 8 : (P % 4 == 0 ? 4 : 2);  // rows 8 / G apart would share banks
+  const int lane = threadIdx.x & 31;
+  const uint32_t own = stage + lane * (2 * NC), turn = (lane / (8 / G)) & (G - 1);
+#pragma unroll
+  for (int cc = 0; cc < NC; cc += W) {
+    float o[W];
+    tmem_ldw<W>(taddr + cc, reinterpret_cast<uint32_t*>(o));
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < W; i += 8)
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(own + ((((cc + i) / 8) ^ turn) << 4)),
+                   "r"(pack16<BF16>(o[i] * mul, o[i + 1] * mul)), "r"(pack16<BF16>(o[i + 2] * mul, o[i + 3] * mul)),
+                   "r"(pack16<BF16>(o[i + 4] * mul, o[i + 5] * mul)), "r"(pack16<BF16>(o[i + 6] * mul, o[i + 7] * mul))
+                   : "memory");
+  }
+  __syncwarp();
+#pragma unroll
+  for (int it = 0; it < P; ++it) {
+    const int n = it * 32 + lane, r = n / P, c = n - r * P;
+    uint4 w;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w)
+                 : "r"(stage + r * (2 * NC) + ((c ^ ((r / (8 / G)) & (G - 1))) << 4))
+                 : "memory");
+    if (r < rows && 8 * c < cols) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(g) + 2 * (r * stride + 8 * c)) = w;
+  }
+}
+
+// ----------------------------------------------------------------------------------
+// What a CTA that gives up leaves behind: NaN in every output row it owns, so that a timed-out wait
+// cannot pass for a result (0x7fff is a NaN in fp16 and in bf16). Called by all threads of the CTA.
+// ----------------------------------------------------------------------------------
+__device__ __forceinline__ void fill_rows_nan16(void* base, long long row_stride, int r0, int r1, int dim) {
+  const int chunks = dim / 8;
+  const uint4 nan8 = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
+  for (int i = threadIdx.x; i < (r1 - r0) * chunks; i += blockDim.x) {
+    const long long r = r0 + i / chunks;
+    *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(base) + 2 * (r * row_stride + (i % chunks) * 8)) = nan8;
+  }
+}
+// One thread of a CTA whose abort word is set, after the CTA's last barrier: the first failure of all stays in the status word.
+__device__ __forceinline__ void report_abort(const volatile int* s_abort, int* status) {
+  if (*s_abort > 1) atomicCAS(status, 0, *s_abort);
+}
+__device__ __forceinline__ void fill_nan32(float* base, long long count) {
+  for (long long i = threadIdx.x; i < count; i += blockDim.x) base[i] = __int_as_float(0x7fc00000);
 }
 
 }  // namespace kfa
