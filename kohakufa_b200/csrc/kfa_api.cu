@@ -155,14 +155,16 @@ bool number_compactly(int n_seqs, int n_max, int rows, int tile, int scans) {
 }
 
 template <int D, bool BF16, bool MASKW, bool COMPACT>
-int launch_fwd_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const kfa::FwdParams& p,
-                 cudaStream_t s) {
+int launch_fwd_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, kfa::FwdParams p, cudaStream_t s) {
   auto kern = kfa::kfa_fwd_kernel<D, BF16, MASKW, COMPACT>;
   constexpr int smem = MASKW ? kfa::FwdCfg<D>::SMEM_BYTES_LIST : kfa::FwdCfg<D>::SMEM_BYTES;
   int rc = set_smem(kern, smem);
   if (rc) return rc;
   const long long grid = COMPACT ? packed_tiles(p.B, p.n_q_tiles, p.Sq, 256) * p.H : static_cast<long long>(p.B) * p.H * p.n_q_tiles;
   if (grid > 0x7fffffffll) return fail(KFA_ERR_ARG, "too many tiles");
+  p.order = kfa::TileOrder::of(p.B * p.H, p.n_q_tiles, p.H);
+  p.by_frame = kfa::FastDiv::by(p.P > 0 ? p.P : 1);
+  p.by_group = kfa::FastDiv::by(p.group);
   kern<<<static_cast<unsigned>(grid), kfa::FWD_THREADS, smem, s>>>(mq, mk, mv, p);
   KFA_CUDA(cudaGetLastError());
   return KFA_OK;
@@ -184,9 +186,16 @@ int launch_prepare(const kfa::PrepParams& p, cudaStream_t s) {
   return KFA_OK;
 }
 
+void set_divisors(kfa::BwdParams& p, int heads, int n_tiles) {
+  p.order = kfa::TileOrder::of(p.B * heads, n_tiles, heads);
+  p.by_frame = kfa::FastDiv::by(p.P > 0 ? p.P : 1);
+  p.by_group = kfa::FastDiv::by(p.group);
+  p.by_split = kfa::FastDiv::by(p.n_split > 1 ? p.n_split : 1);
+}
+
 template <int D, bool BF16, bool MASKW>
 int launch_dkdv_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
-                  const kfa::BwdParams& p, cudaStream_t s) {
+                  kfa::BwdParams p, cudaStream_t s) {
   auto kern = kfa::kfa_bwd_dkdv_kernel<D, BF16, MASKW>;
   constexpr int smem = MASKW ? kfa::BwdCfg<D>::KV_SMEM_BYTES_LIST : kfa::BwdCfg<D>::KV_SMEM_BYTES;
   int rc = set_smem(kern, smem);
@@ -194,6 +203,7 @@ int launch_dkdv_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMa
   const long long grid = p.compact ? packed_tiles(p.B, p.n_k128, p.Skv, 128) * p.Hkv
                                    : static_cast<long long>(p.B) * p.Hkv * p.n_k128 * (p.n_split > 1 ? p.n_split : 1);
   if (grid > 0x7fffffffll) return fail(KFA_ERR_ARG, "too many tiles");
+  set_divisors(p, p.Hkv, p.n_k128);
   kern<<<static_cast<unsigned>(grid), kfa::BWD_THREADS, smem, s>>>(mq, mk, mv, mdo, p);
   KFA_CUDA(cudaGetLastError());
   return KFA_OK;
@@ -207,13 +217,14 @@ int launch_dkdv(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap&
 
 template <int D, bool BF16, bool MASKW>
 int launch_dq_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
-                const kfa::BwdParams& p, cudaStream_t s) {
+                kfa::BwdParams p, cudaStream_t s) {
   auto kern = kfa::kfa_bwd_dq_kernel<D, BF16, MASKW>;
   constexpr int smem = MASKW ? kfa::BwdCfg<D>::Q_SMEM_BYTES_LIST : kfa::BwdCfg<D>::Q_SMEM_BYTES;
   int rc = set_smem(kern, smem);
   if (rc) return rc;
   const long long grid = p.compact ? packed_tiles(p.B, p.n_q128, p.Sq, 128) * p.H : static_cast<long long>(p.B) * p.H * p.n_q128;
   if (grid > 0x7fffffffll) return fail(KFA_ERR_ARG, "too many tiles");
+  set_divisors(p, p.H, p.n_q128);
   kern<<<static_cast<unsigned>(grid), kfa::BWD_THREADS, smem, s>>>(mq, mk, mv, mdo, p);
   KFA_CUDA(cudaGetLastError());
   return KFA_OK;
@@ -575,13 +586,14 @@ int dq_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const
 
 template <int D, bool BF16>
 int launch_fused(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
-                 const kfa::BwdParams& p, float* dq_acc, cudaStream_t s) {
+                 kfa::BwdParams p, float* dq_acc, cudaStream_t s) {
   auto kern = kfa::kfa_bwd_fused_kernel<D, BF16>;
   constexpr int smem = kfa::FusedCfg<D>::SMEM_BYTES;
   int rc = set_smem(kern, smem);
   if (rc) return rc;
   const long long grid = static_cast<long long>(p.B) * p.Hkv * p.n_k128;
   if (grid > 0x7fffffffll) return fail(KFA_ERR_ARG, "too many tiles");
+  set_divisors(p, p.Hkv, p.n_k128);
   kern<<<static_cast<unsigned>(grid), kfa::FUSED_THREADS, smem, s>>>(mq, mk, mv, mdo, p, dq_acc);
   KFA_CUDA(cudaGetLastError());
   return KFA_OK;

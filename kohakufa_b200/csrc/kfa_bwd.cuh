@@ -42,6 +42,8 @@
 namespace kfa {
 
 struct BwdParams {
+  TileOrder order;                       // (filled where the kernel is launched, as are the next three)
+  FastDiv by_frame, by_group, by_split;  // divisions by P (1 if dense), group, n_split
   void* dq;  // [B, H, Sq, D] view
   long long dq_sb, dq_sh, dq_ss;
   void* dk;  // [B, H, Skv, D] view
@@ -448,7 +450,7 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   constexpr int B_DRAIN = 6 + 2 * NSL;
   constexpr int B_PLO = 7 + 2 * NSL;      // the first 32 queries of P^T(i) stored by both warpgroups
   constexpr int N_BARS = 8 + 2 * NSL;
-  static_assert(N_BARS * 8 + 16 <= 256, "barrier block too small");
+  static_assert(N_BARS * 8 + 16 <= 256 && N_BARS <= 32, "barrier block too small; a lane each sets them up");
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + N_BARS);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
   const uint32_t bar0 = smem_u32(bars);
@@ -461,15 +463,13 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   // tile decode (groups of heads, tile-major inside); when causal the first key tiles see the most queries and come first
   int b, hk, kt;
-  const int split = (!MASKW && p.n_split > 1) ? blockIdx.x % p.n_split : 0;
+  const int cell = (!MASKW && p.n_split > 1) ? static_cast<int>(p.by_split.div(blockIdx.x)) : blockIdx.x;
+  const int split = (!MASKW && p.n_split > 1) ? blockIdx.x - cell * p.n_split : 0;
   if (!MASKW && p.compact) {
     int n_tiles;
     if (!decode_packed<128>(blockIdx.x, p.cu_k, p.B, p.Hkv, p.n_k128, b, hk, kt, n_tiles)) return;
   } else {
-    int bh;  // over batch x K / V heads
-    decode_tile((!MASKW && p.n_split > 1) ? blockIdx.x / p.n_split : blockIdx.x, p.B * p.Hkv, p.n_k128, bh, kt);
-    b = bh / p.Hkv;
-    hk = bh % p.Hkv;
+    p.order.decode(cell, b, hk, kt);  // over batch x K / V heads
   }
   float* dk32 = p.dk32 + split * p.split_stride;
   float* dv32 = p.dv32 + split * p.split_stride;
@@ -483,7 +483,7 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     bc = 0;
     if (kv0 >= Skv) return;  // the whole CTA, before anything is set up
   }
-  const int first_i = (p.P > 0) ? static_cast<int>((static_cast<long long>(kv0 / p.P) * p.P) / 128) : 0;
+  const int first_i = (p.P > 0) ? static_cast<int>(p.by_frame.div(kv0) * p.P) / 128 : 0;
   // steps: for every query head of this K / V head's group, the query tiles that see these keys
   const int n_per = max((Sq + 127) / 128 - first_i, 0);
   int n_steps = n_per * p.group;
@@ -494,7 +494,7 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     n_steps = min(per, n_steps - s_first);
   }
   const bool ragged_keys = kv0 + 128 > Skv;
-  const int i_full = (p.P > 0 && !ragged_keys) ? first_full_tile(kv0, p.P) : 0;  // query tiles before it are masked steps
+  const int i_full = (p.P > 0 && !ragged_keys) ? first_full_tile(kv0, p.P, p.by_frame) : 0;  // query tiles before it are masked steps
   // boolean masks with a tile table: the (query head, query tile) steps this CTA runs, in shared memory
   uint32_t* s_list = reinterpret_cast<uint32_t*>(smem + Cfg::KV_SMEM_TILES + 256);
   const bool use_list = MASKW && p.mt != nullptr;
@@ -513,23 +513,20 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               bar(B_QREADY + slot));
   };
   int issued = 0, earlier = 0;
-  if (warp == 9 && lane == 0) {
-    earlier = load_status(p.status);
-    mbar_init(bar(B_KV), 1);
-    for (int i = 0; i < NSL; ++i) {
-      mbar_init(bar(B_QREADY + i), 1);
-      mbar_init(bar(B_QFREE + i), 1);
-    }
-    mbar_init(bar(B_S), 1);
-    mbar_init(bar(B_DP), 1);
-    mbar_init(bar(B_P), 256);
-    mbar_init(bar(B_PLO), 256);
-    mbar_init(bar(B_DS), 256);
-    mbar_init(bar(B_ACC), 1);
-    mbar_init(bar(B_DRAIN), 1);
-    *s_abort = 0;
+  StepWalk walk;  // (s_first is not 0 only where a key tile's steps are shared out)
+  if (!MASKW && s_first > 0 && n_steps > 0) {
+    walk.rel = s_first % n_per;
+    walk.g = s_first / n_per;
+  }
+  if (warp == 9) {
+    if (lane < N_BARS) mbar_init(bar(lane), (lane == B_P || lane == B_PLO || lane == B_DS) ? 256 : 1);
+    if (lane == 0) *s_abort = 0;
     fence_mbar_init();
     fence_async_smem();
+    __syncwarp();
+  }
+  if (warp == 9 && lane == 0) {
+    earlier = load_status(p.status);
     if (use_list || n_steps > 0) {
       mbar_expect_tx(bar(B_KV), 2 * Cfg::TILE_BYTES);
       for (int ch = 0; ch < CH; ++ch) {
@@ -537,9 +534,10 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tma_load_4d(sV + ch * Cfg::CHUNK_BYTES, &tmV, bar(B_KV), ch * Cfg::CHUNK_COLS, k_base + kv0, hk, bc);
       }
     }
-    if (!use_list)
-      for (; issued < min(n_steps, NSL); ++issued)
-        load_step(issued, first_i + (s_first + issued) % n_per, hk * p.group + (s_first + issued) / n_per);
+    if (!use_list && n_steps > 0) {
+      load_step(0, first_i + walk.rel, hk * p.group + walk.g);
+      issued = 1;
+    }
   }
   if (warp == 0) {
     tmem_alloc(smem_u32(s_tmem), Cfg::TMEM_COLS);
@@ -566,22 +564,25 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
   if (use_list) n_steps = static_cast<int>(s_tmem[2]);
-  // step s -> query tile and query head
-  auto tile_of = [&](int s) { return use_list ? static_cast<int>(s_list[s] & 0xffffu) : first_i + (s_first + s) % n_per; };
-  auto head_of = [&](int s) { return hk * p.group + (use_list ? static_cast<int>(s_list[s] >> 16) : (s_first + s) / n_per); };
+  // listed step s -> query tile and query head (the other steps are walked through)
+  auto tile_of = [&](int s) { return static_cast<int>(s_list[s] & 0xffffu); };
+  auto head_of = [&](int s) { return hk * p.group + static_cast<int>(s_list[s] >> 16); };
   const Ctl ctl{s_abort};
 
   if (warp == 9) {
     // =========================== TMA producer ===========================
     if (lane == 0) {
-      if (earlier != 0) *s_abort = 1;
-      bool ok = (earlier == 0);
-      for (int s = issued; s < n_steps && ok; ++s) {
+      if (!use_list) walk.next(n_per);
+      bool ok = true;
+      for (int s = issued; s < n_steps && ok; ++s, walk.next(n_per)) {
         if (s >= NSL) ok = mbar_wait(bar(B_QFREE + s % NSL), (s / NSL - 1) & 1, ctl, 11);
         if (!ok) break;
-        load_step(s, tile_of(s), head_of(s));
+        if (use_list) load_step(s, tile_of(s), head_of(s));
+        else load_step(s, first_i + walk.rel, hk * p.group + walk.g);
         issued = s + 1;
+        if (s == 2 && earlier != 0) ok = false;
       }
+      if (earlier != 0) *s_abort = 1;
       if (use_list && n_steps == 0) mbar_drain(bar(B_KV), 0);  // (nothing visible in a mask: nothing else waits for K and V)
     }
   } else if (warp == 8) {
@@ -666,7 +667,7 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const int kr = kv0 + (warp & 3) * 32 + 16 * (e >> 1) + (lane >> 2) + 8 * (e & 1);
       qmin[e] = 0;
       if (kr >= Skv) qmin[e] = 0x7fffffff;
-      else if (p.P > 0) qmin[e] = (kr / p.P) * p.P;
+      else if (p.P > 0) qmin[e] = static_cast<int>(p.by_frame.div(kr)) * p.P;
     }
     const float2 c2 = make_float2(p.c, p.c);
     bool ok = true;
@@ -675,8 +676,8 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int* mkey[4] = {nullptr, nullptr, nullptr, nullptr};
     uint2 wnext[4];
     auto mask_fetch = [&](int s) {
-      const int i = tile_of(s);
-      const int head = head_of(s);
+      const int i = use_list ? tile_of(s) : first_i + s % n_per;
+      const int head = use_list ? head_of(s) : hk * p.group + s / n_per;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         wnext[e] = make_uint2(0u, 0u);
@@ -690,11 +691,6 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (kr < Skv) mkey[e] = p.mwt + bc * p.mwt_sb + static_cast<long long>(kr) * p.mwt_row;
       }
       if (n_steps > 0) mask_fetch(0);
-    }
-    StepWalk walk;
-    if (!MASKW && n_steps > 0) {
-      walk.rel = s_first % n_per;
-      walk.g = s_first / n_per;
     }
     for (int s = 0; s < n_steps; ++s, walk.next(n_per)) {
       uint2 wcur[4];
@@ -955,7 +951,7 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   constexpr int B_DPREAD = B_S + 6;            // both warpgroups hold dP(j) in registers (256 arrivals)
   constexpr int B_DSFREE = B_S + 7;            // 2: dQ(j), which read dS buffer j % 2, has retired
   constexpr int N_BARS = B_S + 9;
-  static_assert(N_BARS * 8 + 16 <= 256, "barrier block too small");
+  static_assert(N_BARS * 8 + 16 <= 256 && N_BARS <= 32, "barrier block too small; a lane each sets them up");
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + N_BARS);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
   const uint32_t bar0 = smem_u32(bars);
@@ -967,10 +963,7 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   if (!MASKW && p.compact) {
     if (!decode_packed<128>(blockIdx.x, p.cu_q, p.B, p.H, p.n_q128, b, h, t, n_q128)) return;
   } else {
-    int bh;
-    decode_tile(blockIdx.x, p.B * p.H, p.n_q128, bh, t);
-    b = bh / p.H;
-    h = bh % p.H;
+    p.order.decode(blockIdx.x, b, h, t);
   }
   const int bh = b * p.H + h;
   const int qt = (p.P > 0) ? (n_q128 - 1 - t) : t;
@@ -985,64 +978,48 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     if (row0 >= Sq || Skv <= 0) return;  // the whole CTA, before anything is set up
   }
   const int last = min(row0 + 127, Sq - 1);
-  int n_steps = (key_limit(last, p.P, Skv) + 127) / 128;
-  const int n_unmasked = key_limit(row0, p.P, Skv) / 128;
+  int n_steps = (key_limit(last, p.P, p.by_frame, Skv) + 127) / 128;
+  const int n_unmasked = key_limit(row0, p.P, p.by_frame, Skv) / 128;
   // boolean masks with a tile table: the key tiles this CTA visits, in shared memory
   uint16_t* s_list = reinterpret_cast<uint16_t*>(smem + Cfg::Q_SMEM_TILES + 256);
   const bool use_list = MASKW && p.mt != nullptr;
 
   // (the thread that starts the copies also sets up the barriers: see the forward)
+  const int h_kv = static_cast<int>(p.by_group.div(h));
   auto load_k = [&](int j, int tile) {
     const int ks = j % NK;
     mbar_expect_tx(bar(B_KREADY + ks), Cfg::TILE_BYTES);
     for (int ch = 0; ch < CH; ++ch)
       tma_load_4d(sKr + ks * Cfg::TILE_BYTES + ch * Cfg::CHUNK_BYTES, &tmK, bar(B_KREADY + ks), ch * Cfg::CHUNK_COLS,
-                  k_base + tile * 128, h / p.group, bc);
+                  k_base + tile * 128, h_kv, bc);
   };
   auto load_v = [&](int j, int tile) {
     const int vs = j % NV;
     mbar_expect_tx(bar(B_VREADY + vs), Cfg::TILE_BYTES);
     for (int ch = 0; ch < CH; ++ch)
       tma_load_4d(sVr + vs * Cfg::TILE_BYTES + ch * Cfg::CHUNK_BYTES, &tmV, bar(B_VREADY + vs), ch * Cfg::CHUNK_COLS,
-                  k_base + tile * 128, h / p.group, bc);
+                  k_base + tile * 128, h_kv, bc);
   };
   int issued_k = 0, issued_v = 0, earlier = 0;
-  if (warp == 9 && lane == 0) {
-    earlier = load_status(p.status);
-    mbar_init(bar(B_Q), 1);
-    for (int i = 0; i < NK; ++i) {
-      mbar_init(bar(B_KREADY + i), 1);
-      mbar_init(bar(B_KFREE + i), 1);
-    }
-    for (int i = 0; i < NV; ++i) {
-      mbar_init(bar(B_VREADY + i), 1);
-      mbar_init(bar(B_VFREE + i), 1);
-    }
-    mbar_init(bar(B_S), 1);
-    mbar_init(bar(B_DP), 1);
-    mbar_init(bar(B_SREAD), 256);
-    mbar_init(bar(B_DS), 256);
-    mbar_init(bar(B_ACC), 1);
-    mbar_init(bar(B_DRAIN), 1);
-    mbar_init(bar(B_DPREAD), 256);
-    mbar_init(bar(B_DSFREE + 0), 1);
-    mbar_init(bar(B_DSFREE + 1), 1);
-    *s_abort = 0;
+  if (warp == 9) {
+    if (lane < N_BARS) mbar_init(bar(lane), (lane == B_SREAD || lane == B_DS || lane == B_DPREAD) ? 256 : 1);
+    if (lane == 0) *s_abort = 0;
     fence_mbar_init();
     fence_async_smem();
+    __syncwarp();
+  }
+  if (warp == 9 && lane == 0) {
+    earlier = load_status(p.status);
     mbar_expect_tx(bar(B_Q), 2 * Cfg::TILE_BYTES);
     for (int ch = 0; ch < CH; ++ch) {
       tma_load_4d(sQ + ch * Cfg::CHUNK_BYTES, &tmQ, bar(B_Q), ch * Cfg::CHUNK_COLS, q_base + row0, h, bc);
       tma_load_4d(sDO + ch * Cfg::CHUNK_BYTES, &tmDO, bar(B_Q), ch * Cfg::CHUNK_COLS, q_base + row0, h, bc);
     }
-    if (!use_list)
-      for (int j = 0; j < min(n_steps, NK); ++j) {
-        load_k(j, j);
-        issued_k = j + 1;
-        if (j >= NV) continue;
-        load_v(j, j);
-        issued_v = j + 1;
-      }
+    if (!use_list) {
+      load_k(0, 0);
+      load_v(0, 0);
+      issued_k = issued_v = 1;
+    }
   }
   if (warp == 0) {
     tmem_alloc(smem_u32(s_tmem), Cfg::TMEM_COLS);
@@ -1076,20 +1053,19 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
   if (warp == 9) {
     if (lane == 0) {
-      if (earlier != 0) *s_abort = 1;
-      bool ok = (earlier == 0);
-      for (int j = min(issued_k, issued_v); j < n_steps && ok; ++j) {
-        if (j >= issued_k) {
-          if (j >= NK) ok = mbar_wait(bar(B_KFREE + j % NK), (j / NK - 1) & 1, ctl, 51);
-          if (!ok) break;
-          load_k(j, tile_of(j));
-          issued_k = j + 1;
-        }
+      bool ok = true;
+      for (int j = issued_k; j < n_steps && ok; ++j) {
+        if (j >= NK) ok = mbar_wait(bar(B_KFREE + j % NK), (j / NK - 1) & 1, ctl, 51);
+        if (!ok) break;
+        load_k(j, tile_of(j));
+        issued_k = j + 1;
         if (j >= NV) ok = mbar_wait(bar(B_VFREE + j % NV), (j / NV - 1) & 1, ctl, 52);
         if (!ok) break;
         load_v(j, tile_of(j));
         issued_v = j + 1;
+        if (j == 2 && earlier != 0) ok = false;
       }
+      if (earlier != 0) *s_abort = 1;
     }
   } else if (warp == 8) {
     // MMA issue: the whole warp converged, one elected lane issues.
@@ -1169,7 +1145,7 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     const float2 nm = make_float2(st[r_in], st[r_in]);                // -m
     const float2 nl = make_float2(st[128 + r_in], st[128 + r_in]);    // -log2 l
     const float2 nd = make_float2(st[256 + r_in], st[256 + r_in]);    // -delta
-    const int my_limit = key_limit(min(row, Sq - 1), p.P, Skv);
+    const int my_limit = key_limit(min(row, Sq - 1), p.P, p.by_frame, Skv);
     const float2 c2 = make_float2(p.c, p.c);
     bool ok = true;
     // boolean mask: the two words of this row for the warpgroup's 64 keys of a tile, fetched a tile ahead

@@ -203,19 +203,18 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
 
   // tile decode (groups of heads, tile-major inside); under a causal mask the first key tiles see the most queries and come first
-  int bh, kt;  // bh over batch x K / V heads
-  decode_tile(blockIdx.x, p.B * p.Hkv, p.n_k128, bh, kt);
-  const int b = bh / p.Hkv, hk = bh % p.Hkv;
+  int b, hk, kt;
+  p.order.decode(blockIdx.x, b, hk, kt);
   const int kv0 = kt * 128;
   const int Sq = p.Sq, Skv = p.Skv;
-  const int first_i = (p.P > 0) ? static_cast<int>((static_cast<long long>(kv0 / p.P) * p.P) / 128) : 0;
+  const int first_i = (p.P > 0) ? static_cast<int>(p.by_frame.div(kv0) * p.P) / 128 : 0;
   const int n_per = max((Sq + 127) / 128 - first_i, 0);  // query tiles that see these keys
   const int n_steps = n_per * p.group;                   // ... for every query head of the group
   const bool ragged_keys = kv0 + 128 > Skv;
-  const int i_full = (p.P > 0 && !ragged_keys) ? first_full_tile(kv0, p.P) : 0;  // query tiles before it are masked steps
+  const int i_full = (p.P > 0 && !ragged_keys) ? first_full_tile(kv0, p.P, p.by_frame) : 0;  // query tiles before it are masked steps
   // step s -> query head, query tile. Key tile kt starts its walk kt tiles in, so that the CTAs of a head
   // that run side by side add their dQ tiles to different places.
-  const int rot = (n_per > 0) ? kt % n_per : 0;
+  const int rot = (kt < n_per) ? kt : (n_per > 0 ? kt % n_per : 0);
   auto tile_at = [&](const StepWalk& w) {
     int r = w.rel + rot;
     if (r >= n_per) r -= n_per;
@@ -234,38 +233,18 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       tma_load_4d(sDO + s % NDO * TB + ch * TILE_BYTES_64, &tmDO, bar(B_DOREADY + s % NDO), ch * 64, i * 128, head, b);
   };
   int earlier = 0, issued = 0, issued_dl = 0;  // (per producing thread: steps whose copies it has started)
-  if (warp == 13 && lane == 0) {
-    earlier = load_status(p.status);
-    mbar_init(bar(B_KV), 1);
-    for (int i = 0; i < NQ; ++i) {
-      mbar_init(bar(B_QREADY + i), 1);
-      mbar_init(bar(B_QFREE + i), 1);
+  if (warp == 13) {
+    for (int i = lane; i < N_BARS; i += 32) {  // arrivals: see the list of the barriers
+      const bool both = i == B_PLO || i == B_P || i == B_DS || i == B_DLFREE || (i >= B_MLFREE && i < B_MLFREE + 2);
+      mbar_init(bar(i), both ? 256 : (i == B_DQFREE || i == B_STGFULL ? 128 : 1));
     }
-    for (int i = 0; i < NDO; ++i) {
-      mbar_init(bar(B_DOREADY + i), 1);
-      mbar_init(bar(B_DOFREE + i), 1);
-    }
-    mbar_init(bar(B_S), 1);
-    mbar_init(bar(B_DP), 1);
-    mbar_init(bar(B_PLO), 256);
-    mbar_init(bar(B_P), 256);
-    mbar_init(bar(B_DS), 256);
-    mbar_init(bar(B_DSFREE), 1);
-    mbar_init(bar(B_DQ), 1);
-    mbar_init(bar(B_DQFREE), 128);
-    mbar_init(bar(B_ACC), 1);
-    mbar_init(bar(B_DRAIN), 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(B_MLREADY + i), 1);
-      mbar_init(bar(B_MLFREE + i), 256);
-    }
-    mbar_init(bar(B_DLREADY), 1);
-    mbar_init(bar(B_DLFREE), 256);
-    mbar_init(bar(B_STGFREE), 1);
-    mbar_init(bar(B_STGFULL), 128);
-    *s_abort = 0;
+    if (lane == 0) *s_abort = 0;
     fence_mbar_init();
     fence_async_smem();
+    __syncwarp();
+  }
+  if (warp == 13 && lane == 0) {
+    earlier = load_status(p.status);
     if (n_steps > 0) {  // K, Q and V, dO of the first step
       mbar_expect_tx(bar(B_KV), 2 * TB);
       for (int ch = 0; ch < CH; ++ch) {
@@ -313,9 +292,8 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   } else if (warp == 13) {
     // =========================== TMA producer: K, V, then the Q ring ===========================
     reg_budget<FUSED_REGS_ISSUE>();
-    if (lane == 0 && earlier != 0) *s_abort = 1;
     if (lane == 0 && n_steps > 0) {
-      bool ok = (earlier == 0);
+      bool ok = true;
       StepWalk walk;
       walk.next(n_per);
       for (int s = 1; s < n_steps && ok; ++s, walk.next(n_per)) {
@@ -323,8 +301,10 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         if (!ok) break;
         load_q(s, tile_at(walk), hk * p.group + walk.g);
         issued = s + 1;
+        if (s == 2 && earlier != 0) ok = false;
       }
     }
+    if (lane == 0 && earlier != 0) *s_abort = 1;
   } else if (warp == 14) {
     // =========================== TMA producer: the dO ring ===========================
     reg_budget<FUSED_REGS_ISSUE>();
@@ -509,7 +489,7 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const int kr = kv0 + (warp & 3) * 32 + 16 * (e >> 1) + (lane >> 2) + 8 * (e & 1);
       qmin[e] = 0;
       if (kr >= Skv) qmin[e] = 0x7fffffff;
-      else if (p.P > 0) qmin[e] = (kr / p.P) * p.P;
+      else if (p.P > 0) qmin[e] = static_cast<int>(p.by_frame.div(kr)) * p.P;
     }
     // dS^T box of this warpgroup, first row this thread writes
     const uint32_t s_row0 = sDS + hq * TILE_BYTES_64 + static_cast<uint32_t>((warp & 3) * 32 + (lane >> 2)) * 128u;

@@ -35,7 +35,39 @@
 
 namespace kfa {
 
+// Launch order of the main kernels: the (batch, head) pairs in groups of 8; inside a group tile-major. Under a
+// causal mask every head's tiles run from the heaviest to the lightest, so a group's heavy tiles all start
+// before its light ones and the launch ends on light tiles (head after head, the last wave would hold
+// heavy tiles of the last heads: 4 % of the forward's time at 128 heads, 30 % at 16), while the CTAs that
+// run side by side still share the K / V (or Q / dO) of a few heads in L2.
+// Divisors from the host: with divisions by run-time values the first copy of a CTA started 1100 to 1500 clk after the CTA, of
+// 13000 for a forward of two key tiles. That, barriers set up by a lane each, the other copies behind the CTA's barrier and
+// no mask code for parts that a warp sees whole: forward 32 x 12 x 201 rows, D = 64, 25.3 -> 23.1 us, 4 x 8 x 4096 x 77 keys, D =
+// 48, 26.1 -> 22.9, 2 x 16 x 2048 causal, D = 96, 58.4 -> 53.6; fused backward of the first 46.8 -> 44.0.
+struct TileOrder {
+  FastDiv per_group, last, heads;  // tiles of 8 pairs; pairs of the last group; heads of a batch entry
+  uint32_t full;                   // groups of 8 pairs
+  static TileOrder of(int n_bh, int n_tiles, int heads) {
+    return {FastDiv::by(8u * static_cast<uint32_t>(n_tiles)), FastDiv::by(n_bh % 8 ? n_bh % 8 : 8), FastDiv::by(heads),
+            static_cast<uint32_t>(n_bh / 8)};
+  }
+  __device__ __forceinline__ void decode(uint32_t idx, int& b, int& h, int& t) const {
+    const uint32_t g = per_group.div(idx), r = idx - g * per_group.d;
+    uint32_t tile = r >> 3, in = r & 7u;
+    if (g == full) {
+      tile = last.div(r);
+      in = r - tile * last.d;
+    }
+    const uint32_t bh = 8 * g + in, bb = heads.div(bh);
+    t = static_cast<int>(tile);
+    b = static_cast<int>(bb);
+    h = static_cast<int>(bh - bb * heads.d);
+  }
+};
+
 struct FwdParams {
+  TileOrder order;          // (filled where the kernel is launched, as are the next two)
+  FastDiv by_frame, by_group;  // divisions by P (1 if dense) and by group
   void* o;  // [B, H, Sq, D] view; element strides; last dim contiguous
   long long o_sb, o_sh, o_ss;
   float* lse;  // [B, H, 2, Sq]: plane 0 = m, plane 1 = log2(l)
@@ -117,10 +149,10 @@ struct FwdCfg {
 };
 
 // Keys visible to query row r: [0, key_limit).
-__device__ __forceinline__ int key_limit(int r, int P, int Skv) {
+__device__ __forceinline__ int key_limit(int r, int P, const FastDiv& by_frame, int Skv) {
   if (P <= 0) return Skv;
-  long long lim = (static_cast<long long>(r / P) + 1) * P;
-  return lim < Skv ? static_cast<int>(lim) : Skv;
+  const uint32_t lim = (by_frame.div(r) + 1) * static_cast<uint32_t>(P);  // at most r + P
+  return static_cast<int>(min(lim, static_cast<uint32_t>(Skv)));
 }
 
 // Debug build only (-DKFA_TRACE): CTA 0 of the forward and of the dK / dV kernel records clock64() at its
@@ -135,24 +167,9 @@ __device__ long long kfa_trace[6][64][2][8];
 // First 128-row query tile all of whose rows see every key of the 128-key tile at kv0 (block-causal frame
 // P > 0, the key tile complete): tile i is fully visible iff key_limit(128 i) >= kv0 + 128, which is monotone
 // in i. Computed once per CTA, so that the key-major loops do no division per step.
-__device__ __forceinline__ int first_full_tile(int kv0, int P) {
-  const long long t = (static_cast<long long>(kv0) + 128 + P - 1) / P - 1;
-  return static_cast<int>((t * P + 127) / 128);
-}
-
-// Launch order of the main kernels: the (batch, head) pairs in groups of 8; inside a group tile-major. Under a
-// causal mask every head's tiles run from the heaviest to the lightest, so a group's heavy tiles all start
-// before its light ones and the launch ends on light tiles (head after head, the last wave would hold
-// heavy tiles of the last heads: 4 % of the forward's time at 128 heads, 30 % at 16), while the CTAs that
-// run side by side still share the K / V (or Q / dO) of a few heads in L2.
-__device__ __forceinline__ void decode_tile(int idx, int n_bh, int n_tiles, int& bh, int& t) {
-  constexpr int G = 8;
-  const int per_group = G * n_tiles;
-  const int g = idx / per_group;
-  const int r = idx - g * per_group;
-  const int gs = min(G, n_bh - g * G);
-  t = r / gs;
-  bh = g * G + (r - t * gs);
+__device__ __forceinline__ int first_full_tile(int kv0, int P, const FastDiv& by_frame) {
+  const uint32_t t = by_frame.div(static_cast<uint32_t>(kv0) + 127u + static_cast<uint32_t>(P)) - 1;
+  return static_cast<int>((t * static_cast<uint32_t>(P) + 127u) / 128u);
 }
 
 // The same for a packed batch numbered without the tiles that shorter sequences do not have (rule: number_compactly in
@@ -178,7 +195,9 @@ __device__ __forceinline__ bool decode_packed(int idx, const int* cu, int n_seqs
       n_tiles = __shfl_sync(0xffffffffu, n, f);
       const int first = before + __shfl_sync(0xffffffffu, end, f) - n_tiles * H;
       b = b0 + f;
-      decode_tile(idx - first, H, n_tiles, h, t);
+      const int per_group = 8 * n_tiles, g = (idx - first) / per_group, r = idx - first - g * per_group, gs = min(8, H - 8 * g);
+      t = r / gs;
+      h = 8 * g + (r - t * gs);
       return true;
     }
     before += __shfl_sync(0xffffffffu, end, 31);
@@ -247,10 +266,7 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   if constexpr (COMPACT) {
     if (!decode_packed<256>(blockIdx.x, p.cu_q, p.B, p.H, p.n_q_tiles, b, h, t, n_q_tiles)) return;
   } else {
-    int bh;
-    decode_tile(blockIdx.x, p.B * p.H, p.n_q_tiles, bh, t);
-    b = bh / p.H;
-    h = bh % p.H;
+    p.order.decode(blockIdx.x, b, h, t);
   }
   const int q_tile = (p.P > 0) ? (n_q_tiles - 1 - t) : t;
   const int row0 = q_tile * 256;  // relative to the sequence's first row
@@ -270,8 +286,8 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     const int first = row0 + 128 * hf;
     if (first < Sq) {
       const int last = min(first + 127, Sq - 1);
-      n_tiles[hf] = (key_limit(last, p.P, Skv) + 127) / 128;
-      n_unmasked[hf] = key_limit(first, p.P, Skv) / 128;
+      n_tiles[hf] = (key_limit(last, p.P, p.by_frame, Skv) + 127) / 128;
+      n_unmasked[hf] = key_limit(first, p.P, p.by_frame, Skv) / 128;
     } else {
       n_tiles[hf] = 0;
       n_unmasked[hf] = 0;
@@ -288,36 +304,28 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   // earlier failure aborts the CTA like one of its own waits. (Copies after the CTA's first barrier, behind the status word's
   // round trip, and the epilogue a row per thread, against now: forward 32 x 12 x 201 rows, D = 64, 28.9 -> 25.4 us, 4 x 8 x
   // 4096 x 77 keys, D = 48, 31.2 -> 26.2; 32 heads x 4096 causal, D = 128, 136 -> 133.)
+  const int h_kv = static_cast<int>(p.by_group.div(h));
   auto load_kv = [&](int idx, int j) {  // K_j (even idx) or V_j into its stage of the ring
     mbar_expect_tx(bar(B_KVREADY + idx % NS), Cfg::TILE_BYTES);
     const CUtensorMap* map = (idx & 1) ? &tmV : &tmK;
     for (int ch = 0; ch < CH; ++ch)
       tma_load_4d(sKV + (idx % NS * CH + ch) * Cfg::CHUNK_BYTES, map, bar(B_KVREADY + idx % NS), ch * Cfg::CHUNK_COLS,
-                  k_base + j * 128, h / p.group, bc);
+                  k_base + j * 128, h_kv, bc);
   };
   int kv_issued = 0, earlier = 0;
-  if (warp == 13 && lane == 0) {
-    earlier = load_status(p.status);
-    mbar_init(bar(B_QREADY + 0), 1);
-    mbar_init(bar(B_QREADY + 1), 1);
-    for (int i = 0; i < NS; ++i) {
-      mbar_init(bar(B_KVREADY + i), 1);
-      mbar_init(bar(B_KVFREE + i), 2);  // one arrival per MMA warp
+  if (warp == 13) {
+    for (int i = lane; i < N_BARS; i += 32) {  // arrivals: see the list of the barriers
+      const bool rows = (i >= B_PREADY && i < B_OFINAL) || i >= B_ALPHA;
+      mbar_init(bar(i), rows ? 128 : (i >= B_KVFREE && i < B_SREADY ? 2 : 1));
     }
-    for (int i = 0; i < 4; ++i) {
-      mbar_init(bar(B_SREADY + i), 1);
-      mbar_init(bar(B_PREADY + i), 128);
-      mbar_init(bar(B_PVDONE + i), 1);
-      mbar_init(bar(B_ALPHA + i), 128);
-      mbar_init(bar(B_OREADY + i), 128);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(B_OFINAL + i), 1);
-      mbar_init(bar(B_DRAIN + i), 1);
-    }
-    *s_abort = 0;
+    if (lane == 0) *s_abort = 0;
     fence_mbar_init();
     fence_async_smem();
+    __syncwarp();
+  }
+  if (warp == 13 && lane == 0) {  // what the first scores need; the other copies once the CTA is past its barrier
+    earlier = load_status(p.status);
+    if (!use_list) load_kv(kv_issued++, 0);
     for (int hf = 0; hf < 2; ++hf) {
       if (n_tiles[hf] == 0) continue;
       mbar_expect_tx(bar(B_QREADY + hf), Cfg::TILE_BYTES);
@@ -325,8 +333,6 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         tma_load_4d(sQ + (hf * CH + ch) * Cfg::CHUNK_BYTES, &tmQ, bar(B_QREADY + hf), ch * Cfg::CHUNK_COLS,
                     q_base + row0 + 128 * hf, h, bc);
     }
-    if (!use_list)
-      for (; kv_issued < min(2 * n_max, NS); ++kv_issued) load_kv(kv_issued, kv_issued >> 1);
   }
   if (warp == 0) {
     tmem_alloc(smem_u32(s_tmem), Cfg::TMEM_COLS);
@@ -372,14 +378,15 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     // =========================== TMA producer ===========================
     reg_budget<FWD_REGS_ISSUE>();
     if (lane == 0) {
-      if (earlier != 0) *s_abort = 1;
-      bool ok = (earlier == 0);
+      bool ok = true;
       for (int idx = kv_issued; idx < 2 * n_max && ok; ++idx) {
+        if (idx == 3 && earlier != 0) break;
         if (idx >= NS) ok = mbar_wait(bar(B_KVFREE + idx % NS), (idx / NS - 1) & 1, ctl, 1);
         if (!ok) break;
         load_kv(idx, tile_of(idx >> 1));
         kv_issued = idx + 1;
       }
+      if (earlier != 0) *s_abort = 1;
     }
   } else if (warp == 12 || warp == 14) {
     // =========================== MMA issue ===========================
@@ -535,7 +542,7 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     const uint32_t tS = tmem + (hf ? Cfg::TM_S1 : Cfg::TM_S0) + lane_base;
     const int nt = n_tiles[hf];
     const int nu = n_unmasked[hf];
-    const int my_limit = key_limit(min(row, Sq - 1), p.P, Skv);
+    const int my_limit = key_limit(min(row, Sq - 1), p.P, p.by_frame, Skv);
     const float c = p.c;
 
     float m = -INFINITY;
@@ -581,7 +588,7 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             for (int i = 0; i < PK; ++i)
               if (!((mbits[(PK / 32) * part + (i >> 5)] >> (i & 31)) & 1u)) s[i] = -INFINITY;
           }
-        } else if (masked) {
+        } else if (masked && __any_sync(0xffffffffu, lim < PK)) {
 #pragma unroll
           for (int i = 0; i < PK; ++i)
             if (i >= lim) s[i] = -INFINITY;

@@ -35,6 +35,27 @@ enum : int {
 // never shortened, also not in the test build that sets a tiny KFA_WAIT_CYCLES.
 #define KFA_DRAIN_CYCLES 4000000000ll
 
+// Division by a number the host knows (Granlund and Montgomery, "Division by invariant integers using multiplication", 1994,
+// figure 4.1): four instructions for any 32-bit dividend. A division by a run-time value takes some 150 clk, and a CTA's first
+// copy waited for half a dozen of them one after the other.
+struct FastDiv {
+  uint32_t d, mul, sh1, sh2;
+  static FastDiv by(uint32_t d) {
+    uint32_t l = 0;
+    while (l < 32 && (1ull << l) < d) ++l;  // ceil(log2 d)
+    const uint64_t mul = ((((1ull << l) - d) << 32) / d) + 1;
+    return {d, static_cast<uint32_t>(mul), l < 1 ? l : 1u, l > 1 ? l - 1 : 0u};
+  }
+  __host__ __device__ __forceinline__ uint32_t div(uint32_t n) const {
+#ifdef __CUDA_ARCH__
+    const uint32_t t = __umulhi(mul, n);
+#else
+    const uint32_t t = static_cast<uint32_t>((static_cast<uint64_t>(mul) * n) >> 32);
+#endif
+    return (t + ((n - t) >> sh1)) >> sh2;
+  }
+};
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -537,15 +558,20 @@ __device__ __forceinline__ void store_rows16(uint32_t taddr, float mul, uint32_t
                    : "memory");
   }
   __syncwarp();
+  uint8_t* at = reinterpret_cast<uint8_t*>(g) + 2 * ((lane / P) * stride + 8 * (lane % P));
 #pragma unroll
   for (int it = 0; it < P; ++it) {
     const int n = it * 32 + lane, r = n / P, c = n - r * P;
+    if (it > 0) {
+      if constexpr (32 % P == 0) at += 2 * (32 / P) * stride;
+      else at = reinterpret_cast<uint8_t*>(g) + 2 * (r * stride + 8 * c);
+    }
     uint4 w;
     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w)
                  : "r"(stage + r * (2 * NC) + ((c ^ ((r / (8 / G)) & (G - 1))) << 4))
                  : "memory");
-    if (r < rows && 8 * c < cols) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(g) + 2 * (r * stride + 8 * c)) = w;
+    if (r < rows && 8 * c < cols) *reinterpret_cast<uint4*>(at) = w;
   }
 }
 
