@@ -395,7 +395,7 @@ def main():
     # matmuls of the algorithmic count (2 forward + 5 backward) each kernel delivers; the split dQ kernel's
     # S and dP are recomputation and count for nothing
     units = {"fwd": 2, "fused": 5, "dkdv": 4, "dq": 1}
-    names = {"fwd": "kfa_fwd_kernel", "fused": "kfa_bwd_fused_kernel", "dkdv": "kfa_bwd_dkdv_kernel", "dq": "kfa_bwd_dq_kernel"}
+    names = {"fwd": "kfa_fwd_kernel", "fused": "kfa_bwd_fused_kernel", "dkdv": "kfa_bwd_split_kernel (dK / dV alone)", "dq": "kfa_bwd_split_kernel (dQ alone)"}
     dominant = max((n for n in units if n in kernel_ms), key=lambda n: kernel_ms[n])
     # the kernels were timed on this rank's local tensors (the whole problem unless ring mode)
     local_rows = cfg.seq // world if ring_mode else cfg.seq
@@ -442,7 +442,7 @@ def main():
             "clock-normalised = 4096 MAC x 2 x 148 SMs x the median SM clock sampled during the timed region; "
             "traffic = DRAM bytes of one launch from an ncu capture of a small case of the same shape, scaled by the (batch, head) pairs",
         },
-        "gpu_launches": (3 * world + 5 if ring_mode else 4) * args.steps,  # fwd + 3 backward launches either way
+        "gpu_launches": (3 * world + 5 if ring_mode else 4 if "fused" in kernel_ms else 3) * args.steps,  # fwd; prepare, fused, convert or prepare, split
         "clocks": clocks,
         "e2e": e2e,
     }

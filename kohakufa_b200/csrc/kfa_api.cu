@@ -193,47 +193,37 @@ void set_divisors(kfa::BwdParams& p, int heads, int n_tiles) {
   p.by_split = kfa::FastDiv::by(p.n_split > 1 ? p.n_split : 1);
 }
 
+// One launch of the dK/dV CTAs of pk and the dQ CTAs of pq; either may be null.
 template <int D, bool BF16, bool MASKW>
-int launch_dkdv_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
-                  kfa::BwdParams p, cudaStream_t s) {
-  auto kern = kfa::kfa_bwd_dkdv_kernel<D, BF16, MASKW>;
-  constexpr int smem = MASKW ? kfa::BwdCfg<D>::KV_SMEM_BYTES_LIST : kfa::BwdCfg<D>::KV_SMEM_BYTES;
+int launch_split_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
+                   const kfa::BwdParams* pk, const kfa::BwdParams* pq, cudaStream_t s) {
+  auto kern = kfa::kfa_bwd_split_kernel<D, BF16, MASKW>;
+  using Cfg = kfa::BwdCfg<D>;
+  constexpr int smem = MASKW ? std::max(Cfg::KV_SMEM_BYTES_LIST, Cfg::Q_SMEM_BYTES_LIST) : std::max(Cfg::KV_SMEM_BYTES, Cfg::Q_SMEM_BYTES);
   int rc = set_smem(kern, smem);
   if (rc) return rc;
-  const long long grid = p.compact ? packed_tiles(p.B, p.n_k128, p.Skv, 128) * p.Hkv
-                                   : static_cast<long long>(p.B) * p.Hkv * p.n_k128 * (p.n_split > 1 ? p.n_split : 1);
-  if (grid > 0x7fffffffll) return fail(KFA_ERR_ARG, "too many tiles");
-  set_divisors(p, p.Hkv, p.n_k128);
-  kern<<<static_cast<unsigned>(grid), kfa::BWD_THREADS, smem, s>>>(mq, mk, mv, mdo, p);
+  long long n_dkdv = 0, n_dq = 0;
+  kfa::BwdParams a = pk ? *pk : *pq, b = pq ? *pq : *pk;
+  if (pk) {
+    n_dkdv = a.compact ? packed_tiles(a.B, a.n_k128, a.Skv, 128) * a.Hkv
+                       : static_cast<long long>(a.B) * a.Hkv * a.n_k128 * (a.n_split > 1 ? a.n_split : 1);
+    set_divisors(a, a.Hkv, a.n_k128);
+  }
+  if (pq) {
+    n_dq = b.compact ? packed_tiles(b.B, b.n_q128, b.Sq, 128) * b.H : static_cast<long long>(b.B) * b.H * b.n_q128;
+    set_divisors(b, b.H, b.n_q128);
+  }
+  if (n_dkdv + n_dq > 0x7fffffffll) return fail(KFA_ERR_ARG, "too many tiles");
+  kern<<<static_cast<unsigned>(n_dkdv + n_dq), kfa::BWD_THREADS, smem, s>>>(mq, mk, mv, mdo, a, b, static_cast<unsigned>(n_dkdv));
   KFA_CUDA(cudaGetLastError());
   return KFA_OK;
 }
 
 template <int D, bool BF16>
-int launch_dkdv(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
-                const kfa::BwdParams& p, cudaStream_t s) {
-  return p.mwt ? launch_dkdv_t<D, BF16, true>(mq, mk, mv, mdo, p, s) : launch_dkdv_t<D, BF16, false>(mq, mk, mv, mdo, p, s);
-}
-
-template <int D, bool BF16, bool MASKW>
-int launch_dq_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
-                kfa::BwdParams p, cudaStream_t s) {
-  auto kern = kfa::kfa_bwd_dq_kernel<D, BF16, MASKW>;
-  constexpr int smem = MASKW ? kfa::BwdCfg<D>::Q_SMEM_BYTES_LIST : kfa::BwdCfg<D>::Q_SMEM_BYTES;
-  int rc = set_smem(kern, smem);
-  if (rc) return rc;
-  const long long grid = p.compact ? packed_tiles(p.B, p.n_q128, p.Sq, 128) * p.H : static_cast<long long>(p.B) * p.H * p.n_q128;
-  if (grid > 0x7fffffffll) return fail(KFA_ERR_ARG, "too many tiles");
-  set_divisors(p, p.H, p.n_q128);
-  kern<<<static_cast<unsigned>(grid), kfa::BWD_THREADS, smem, s>>>(mq, mk, mv, mdo, p);
-  KFA_CUDA(cudaGetLastError());
-  return KFA_OK;
-}
-
-template <int D, bool BF16>
-int launch_dq(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
-              const kfa::BwdParams& p, cudaStream_t s) {
-  return p.mw ? launch_dq_t<D, BF16, true>(mq, mk, mv, mdo, p, s) : launch_dq_t<D, BF16, false>(mq, mk, mv, mdo, p, s);
+int launch_split(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
+                 const kfa::BwdParams* pk, const kfa::BwdParams* pq, cudaStream_t s) {
+  return (pk ? pk->mwt != nullptr : pq->mw != nullptr) ? launch_split_t<D, BF16, true>(mq, mk, mv, mdo, pk, pq, s)
+                                                       : launch_split_t<D, BF16, false>(mq, mk, mv, mdo, pk, pq, s);
 }
 
 // Runs `call` with KD = the head dim and KB = (dtype is bf16) as compile-time constants.
@@ -463,9 +453,9 @@ int prepare_impl(const KfaTensor4* out, const KfaTensor4* dout, const float* lse
   KFA_DISPATCH(D, dtype, (launch_prepare<KD, KB>(p, s)));
 }
 
-int dkdv_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* dout,
-              const float* stats, const KfaTensor4* dk, const KfaTensor4* dv, const Extra& ex, float scale, int block,
-              int dtype, int* dev_status, void* stream) {
+int dkdv_params(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* dout,
+                const float* stats, const KfaTensor4* dk, const KfaTensor4* dv, const Extra& ex, float scale, int block,
+                int dtype, int* dev_status, kfa::BwdParams& p) {
   int rc;
   if ((rc = check_qkv(q, k, v, dtype, block, ex.narrow)) || (rc = check_like(dout, q, "dout")) ||
       (rc = check_like(dk, k, "dk")) || (rc = check_like(dv, v, "dv")) || (rc = check_varlen(ex.vl, q, k)) ||
@@ -473,11 +463,6 @@ int dkdv_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, con
     return rc;
   if (ex.mwt && (block != 0 || ex.vl)) return fail(KFA_ERR_ARG, "a boolean mask excludes block-causal and packed batches");
   if (!stats || !dev_status) return fail(KFA_ERR_ARG, "stats / dev_status: null pointer");
-  CUtensorMap mq, mk, mv, mdo;
-  if ((rc = make_map(q, dtype, &mq, "q")) || (rc = make_map(k, dtype, &mk, "k")) ||
-      (rc = make_map(v, dtype, &mv, "v")) || (rc = make_map(dout, dtype, &mdo, "dout")))
-    return rc;
-  kfa::BwdParams p;
   fill_bwd_params(p, q, k, stats, scale, block, dev_status);
   apply_extra(p, ex);
   p.compact = ex.vl && number_compactly(p.B, p.n_k128, p.Skv, 128, 6);
@@ -489,7 +474,6 @@ int dkdv_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, con
   p.dv_sb = dv->stride[0];
   p.dv_sh = dv->stride[1];
   p.dv_ss = dv->stride[2];
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (ex.n_split > 1) {
     const long long floats = k->shape[0] * k->shape[1] * k->shape[2] * kernel_dim(k->shape[3]);
     p.n_split = ex.n_split;
@@ -499,7 +483,7 @@ int dkdv_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, con
     p.dv32 = ex.parts + floats;
     p.dk32_sh = p.dv32_sh = k->shape[2] * kernel_dim(k->shape[3]);
   }
-  KFA_DISPATCH(kernel_dim(q->shape[3]), dtype, (launch_dkdv<KD, KB>(mq, mk, mv, mdo, p, s)));
+  return KFA_OK;
 }
 
 template <int D, bool BF16>
@@ -558,8 +542,8 @@ int sum_splits_impl(const KfaTensor4* dk, const KfaTensor4* dv, const Extra& ex,
   KFA_DISPATCH(kernel_dim(dk->shape[3]), dtype, (launch_sum_splits<KD, KB>(p, static_cast<int>(bh), s)));
 }
 
-int dq_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* dout, const float* stats,
-            const KfaTensor4* dq, const Extra& ex, float scale, int block, int dtype, int* dev_status, void* stream) {
+int dq_params(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* dout, const float* stats,
+              const KfaTensor4* dq, const Extra& ex, float scale, int block, int dtype, int* dev_status, kfa::BwdParams& p) {
   int rc;
   if ((rc = check_qkv(q, k, v, dtype, block, ex.narrow)) || (rc = check_like(dout, q, "dout")) ||
       (rc = check_like(dq, q, "dq")) || (rc = check_varlen(ex.vl, q, k)) ||
@@ -567,11 +551,6 @@ int dq_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const
     return rc;
   if (ex.mw && (block != 0 || ex.vl)) return fail(KFA_ERR_ARG, "a boolean mask excludes block-causal and packed batches");
   if (!stats || !dev_status) return fail(KFA_ERR_ARG, "stats / dev_status: null pointer");
-  CUtensorMap mq, mk, mv, mdo;
-  if ((rc = make_map(q, dtype, &mq, "q")) || (rc = make_map(k, dtype, &mk, "k")) ||
-      (rc = make_map(v, dtype, &mv, "v")) || (rc = make_map(dout, dtype, &mdo, "dout")))
-    return rc;
-  kfa::BwdParams p;
   fill_bwd_params(p, q, k, stats, scale, block, dev_status);
   apply_extra(p, ex);
   p.compact = ex.vl && number_compactly(p.B, p.n_q128, p.Sq, 128, 6);
@@ -579,8 +558,23 @@ int dq_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const
   p.dq_sb = dq->stride[0];
   p.dq_sh = dq->stride[1];
   p.dq_ss = dq->stride[2];
+  return KFA_OK;
+}
+
+// dK and dV (where dk is given), dQ (where dq is) by the split kernel.
+int split_impl(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* dout, const float* stats,
+               const KfaTensor4* dq, const KfaTensor4* dk, const KfaTensor4* dv, const Extra& ex_kv, const Extra& ex_q,
+               float scale, int block, int dtype, int* dev_status, void* stream, bool kv, bool qs) {
+  int rc;
+  kfa::BwdParams pk, pq;
+  if (kv && (rc = dkdv_params(q, k, v, dout, stats, dk, dv, ex_kv, scale, block, dtype, dev_status, pk))) return rc;
+  if (qs && (rc = dq_params(q, k, v, dout, stats, dq, ex_q, scale, block, dtype, dev_status, pq))) return rc;
+  CUtensorMap mq, mk, mv, mdo;
+  if ((rc = make_map(q, dtype, &mq, "q")) || (rc = make_map(k, dtype, &mk, "k")) ||
+      (rc = make_map(v, dtype, &mv, "v")) || (rc = make_map(dout, dtype, &mdo, "dout")))
+    return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  KFA_DISPATCH(kernel_dim(q->shape[3]), dtype, (launch_dq<KD, KB>(mq, mk, mv, mdo, p, s)));
+  KFA_DISPATCH(kernel_dim(q->shape[3]), dtype, (launch_split<KD, KB>(mq, mk, mv, mdo, kv ? &pk : nullptr, qs ? &pq : nullptr, s)));
 }
 
 
@@ -674,13 +668,13 @@ int kfa_bwd_prepare(const KfaTensor4* out, const KfaTensor4* dout, const float* 
 int kfa_bwd_dkdv(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* dout,
                  const float* stats, const KfaTensor4* dk, const KfaTensor4* dv, float scale, int block, int dtype,
                  int* dev_status, void* stream) {
-  return dkdv_impl(q, k, v, dout, stats, dk, dv, Extra{}, scale, block, dtype, dev_status, stream);
+  return split_impl(q, k, v, dout, stats, nullptr, dk, dv, Extra{}, Extra{}, scale, block, dtype, dev_status, stream, true, false);
 }
 
 int kfa_bwd_dq(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* dout,
                const float* stats, const KfaTensor4* dq, float scale, int block, int dtype, int* dev_status,
                void* stream) {
-  return dq_impl(q, k, v, dout, stats, dq, Extra{}, scale, block, dtype, dev_status, stream);
+  return split_impl(q, k, v, dout, stats, dq, nullptr, nullptr, Extra{}, Extra{}, scale, block, dtype, dev_status, stream, false, true);
 }
 
 int kfa_fwd_varlen(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out, float* lse,
@@ -714,8 +708,7 @@ int kfa_bwd_masked(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v
   int rc;
   if ((rc = check_like(out, q, "out")) || (rc = check_tiles(tiles))) return rc;
   if ((rc = prepare_impl(out, dout, lse, stats, nullptr, dtype, stream))) return rc;
-  if ((rc = dkdv_impl(q, k, v, dout, stats, dk, dv, ex_kv, scale, 0, dtype, dev_status, stream))) return rc;
-  return dq_impl(q, k, v, dout, stats, dq, ex_q, scale, 0, dtype, dev_status, stream);
+  return split_impl(q, k, v, dout, stats, dq, dk, dv, ex_kv, ex_q, scale, 0, dtype, dev_status, stream, true, true);
 }
 
 int kfa_bwd_varlen(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out,
@@ -728,8 +721,7 @@ int kfa_bwd_varlen(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v
   if ((rc = prepare_impl(out, dout, lse, stats, &vl, dtype, stream))) return rc;
   Extra ex;
   ex.vl = &vl;
-  if ((rc = dkdv_impl(q, k, v, dout, stats, dk, dv, ex, scale, block, dtype, dev_status, stream))) return rc;
-  return dq_impl(q, k, v, dout, stats, dq, ex, scale, block, dtype, dev_status, stream);
+  return split_impl(q, k, v, dout, stats, dq, dk, dv, ex, ex, scale, block, dtype, dev_status, stream, true, true);
 }
 
 int kfa_bwd(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out,
@@ -738,8 +730,7 @@ int kfa_bwd(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const
   int rc;
   if ((rc = check_like(out, q, "out"))) return rc;
   if ((rc = kfa_bwd_prepare(out, dout, lse, stats, dtype, stream))) return rc;
-  if ((rc = kfa_bwd_dkdv(q, k, v, dout, stats, dk, dv, scale, block, dtype, dev_status, stream))) return rc;
-  return kfa_bwd_dq(q, k, v, dout, stats, dq, scale, block, dtype, dev_status, stream);
+  return split_impl(q, k, v, dout, stats, dq, dk, dv, Extra{}, Extra{}, scale, block, dtype, dev_status, stream, true, true);
 }
 
 int kfa_fwd_narrow(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* out, float* lse,
@@ -762,8 +753,7 @@ int kfa_bwd_narrow(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v
     if ((rc = fused_impl(q, k, v, dout, stats, dq_acc, dk, dv, scale, block, dtype, dev_status, stream, true))) return rc;
     return convert_impl(dq_acc, dq, scale, dtype, dev_status, stream, true);
   }
-  if ((rc = dkdv_impl(q, k, v, dout, stats, dk, dv, ex, scale, block, dtype, dev_status, stream))) return rc;
-  return dq_impl(q, k, v, dout, stats, dq, ex, scale, block, dtype, dev_status, stream);
+  return split_impl(q, k, v, dout, stats, dq, dk, dv, ex, ex, scale, block, dtype, dev_status, stream, true, true);
 }
 
 int kfa_bwd_parts_count(const KfaTensor4* q, const KfaTensor4* k, int against_fused) {
@@ -798,9 +788,8 @@ int kfa_bwd_parts_n(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* 
     return fail(KFA_ERR_ARG, "kfa_bwd_parts: not a problem whose steps are shared out (kfa_bwd_parts_bytes is 0), or %d parts", n_parts);
   if (!parts || reinterpret_cast<uintptr_t>(parts) % 16) return fail(KFA_ERR_ARG, "parts: null or not 16-byte aligned");
   if ((rc = prepare_impl(out, dout, lse, stats, nullptr, dtype, stream, nullptr, true))) return rc;
-  if ((rc = dkdv_impl(q, k, v, dout, stats, dk, dv, ex, scale, block, dtype, dev_status, stream))) return rc;
-  if ((rc = sum_splits_impl(dk, dv, ex, dtype, stream))) return rc;
-  return dq_impl(q, k, v, dout, stats, dq, ex, scale, block, dtype, dev_status, stream);
+  if ((rc = split_impl(q, k, v, dout, stats, dq, dk, dv, ex, ex, scale, block, dtype, dev_status, stream, true, true))) return rc;
+  return sum_splits_impl(dk, dv, ex, dtype, stream);
 }
 
 int kfa_varlen_zero_rows(const KfaTensor4* t, int n_tensors, const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int n_seqs,

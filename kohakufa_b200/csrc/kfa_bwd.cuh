@@ -1,21 +1,22 @@
-// Attention backward for sm_100a, as three kernels:
+// Attention backward for sm_100a, as two kernels:
 //
 //   kfa_bwd_prepare_kernel   delta = rowsum(fp32(dO) * fp32(O)); packs (-m, -log2 l, -delta) per
 //                            128-row query tile, padded rows get -m = -inf so their P is 0
 //                            (reference: src/kohakufa/sm100/bwd.py:1358-1388)
-//   kfa_bwd_dkdv_kernel      one CTA per (batch, head, 128-key tile), looping over the query
+//   kfa_bwd_split_kernel, in one launch:
+//     bwd_dkdv               one CTA per (batch, head, 128-key tile), looping over the query
 //                            tiles that see it, everything transposed (keys on TMEM lanes):
 //                              S^T = K Q_i^T, dP^T = V dO_i^T, dV += P^T dO_i, dK += dS^T Q_i
 //                            (reference: bwd.py:565-694 MMAs, 967-1127 P / dS partitions)
-//   kfa_bwd_dq_kernel        one CTA per (batch, head, 128-query tile), looping over key tiles:
+//     bwd_dq                 one CTA per (batch, head, 128-query tile), looping over key tiles:
 //                              S = Q K_j^T, dP = dO V_j^T, dQ += dS K_j
 //
 // The reference fuses dQ into the key-major kernel and accumulates it with fp32 reduce-adds into
-// a scratch buffer (bwd.py:1135-1232, 1391-1410). Here dQ has its own query-major kernel: two more
+// a scratch buffer (bwd.py:1135-1232, 1391-1410). Here dQ has query-major CTAs of its own: two more
 // MMAs per tile pair, but no atomics, no fp32 accumulator round trip through HBM, and dQ is
 // bit-reproducible run to run.
 //
-// Roles in both main kernels (320 threads):
+// Roles in both kinds of CTA ("the dK/dV kernel", "the dQ kernel" below; 320 threads):
 //   warps 0-3  columns 0-63 of every 128x128 score tile     warp 8  MMA issue (converged, one lane issues)
 //   warps 4-7  columns 64-127                               warp 9  TMA producer
 // Thread t of a warpgroup owns TMEM lane t (a key row in the dK/dV kernel, a query row in the dQ
@@ -424,10 +425,8 @@ __device__ __forceinline__ void ds_cols_by_key(const float2* dp, const float2* p
 // 18.5, and 4.5 for the sum.
 // ---------------------------------------------------------------------------------------
 template <int D, bool BF16, bool MASKW>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
-kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                    const BwdParams p) {
+__device__ __forceinline__ void bwd_dkdv(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
+                                         const CUtensorMap& tmDO, const BwdParams& p, unsigned block) {
   using Cfg = BwdCfg<D>;
   constexpr int CH = Cfg::CHUNKS;
   constexpr int NSL = Cfg::KV_SLOTS;
@@ -458,16 +457,16 @@ kfa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
 #ifdef KFA_TRACE
-  const bool trace_on = (blockIdx.x == 0) && (lane == 0);
+  const bool trace_on = (block == 0) && (lane == 0);
 #endif
 
   // tile decode (groups of heads, tile-major inside); when causal the first key tiles see the most queries and come first
   int b, hk, kt;
-  const int cell = (!MASKW && p.n_split > 1) ? static_cast<int>(p.by_split.div(blockIdx.x)) : blockIdx.x;
-  const int split = (!MASKW && p.n_split > 1) ? blockIdx.x - cell * p.n_split : 0;
+  const int cell = (!MASKW && p.n_split > 1) ? static_cast<int>(p.by_split.div(block)) : static_cast<int>(block);
+  const int split = (!MASKW && p.n_split > 1) ? static_cast<int>(block) - cell * p.n_split : 0;
   if (!MASKW && p.compact) {
     int n_tiles;
-    if (!decode_packed<128>(blockIdx.x, p.cu_k, p.B, p.Hkv, p.n_k128, b, hk, kt, n_tiles)) return;
+    if (!decode_packed<128>(static_cast<int>(block), p.cu_k, p.B, p.Hkv, p.n_k128, b, hk, kt, n_tiles)) return;
   } else {
     p.order.decode(cell, b, hk, kt);  // over batch x K / V heads
   }
@@ -921,10 +920,8 @@ __global__ void __launch_bounds__(256) kfa_zero_rows_kernel(const ZeroRowsParams
 // dQ
 // ---------------------------------------------------------------------------------------
 template <int D, bool BF16, bool MASKW>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
-kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                  const BwdParams p) {
+__device__ __forceinline__ void bwd_dq(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
+                                       const CUtensorMap& tmDO, const BwdParams& p, unsigned block) {
   using Cfg = BwdCfg<D>;
   constexpr int CH = Cfg::CHUNKS;
   constexpr int NK = Cfg::NK, NV = Cfg::NV;
@@ -961,9 +958,9 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
   int b, h, t, n_q128 = p.n_q128;
   if (!MASKW && p.compact) {
-    if (!decode_packed<128>(blockIdx.x, p.cu_q, p.B, p.H, p.n_q128, b, h, t, n_q128)) return;
+    if (!decode_packed<128>(static_cast<int>(block), p.cu_q, p.B, p.H, p.n_q128, b, h, t, n_q128)) return;
   } else {
-    p.order.decode(blockIdx.x, b, h, t);
+    p.order.decode(static_cast<int>(block), b, h, t);
   }
   const int bh = b * p.H + h;
   const int qt = (p.P > 0) ? (n_q128 - 1 - t) : t;
@@ -1261,6 +1258,20 @@ kfa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     tc_fence_after();
     tmem_dealloc(tmem, Cfg::TMEM_COLS);
   }
+}
+
+// Both in one launch: CTAs 0 .. n_dkdv - 1 run the first, the others the second. Neither needs the other's results, and as
+// launches of their own each ended in a wave of its own that filled the GPU in part (3.46 waves of 148 CTAs ran as 4, twice).
+// Forward + backward with two launches -> one, us: 16 heads x 4096, D = 128, 614 -> 575; 16 packed sequences of up to 2048, 16 query
+// and 4 K / V heads, D = 128, 490 -> 458; 2 x 16 x 2048 causal, D = 96, 177 -> 173; a mask of 2048 x 2048, D = 64, 120 -> 112; 2 x 32 x
+// 8192 causal, D = 128, 4428 -> 4344.
+template <int D, bool BF16, bool MASKW>
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+kfa_bwd_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
+                     const __grid_constant__ BwdParams p_dkdv, const __grid_constant__ BwdParams p_dq, unsigned n_dkdv) {
+  if (blockIdx.x < n_dkdv) bwd_dkdv<D, BF16, MASKW>(tmQ, tmK, tmV, tmDO, p_dkdv, blockIdx.x);
+  else bwd_dq<D, BF16, MASKW>(tmQ, tmK, tmV, tmDO, p_dq, blockIdx.x - n_dkdv);
 }
 
 }  // namespace kfa

@@ -146,7 +146,7 @@ int kfa_cp_bwd_dkdv_step(const KfaTensor4* q, const KfaTensor4* k, const KfaTens
   p.dv32 = dv_acc->ptr;
   p.dv32_sh = dv_acc->head_stride;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  KFA_DISPATCH(q->shape[3], dtype, (launch_dkdv<KD, KB>(mq, mk, mv, mdo, p, s)));
+  KFA_DISPATCH(q->shape[3], dtype, (launch_split<KD, KB>(mq, mk, mv, mdo, &p, nullptr, s)));
 }
 
 int kfa_cp_bwd_dq_step(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v, const KfaTensor4* dout,
@@ -167,7 +167,7 @@ int kfa_cp_bwd_dq_step(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor
   p.dq32 = dq_acc->ptr;
   p.dq32_sh = dq_acc->head_stride;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  KFA_DISPATCH(q->shape[3], dtype, (launch_dq<KD, KB>(mq, mk, mv, mdo, p, s)));
+  KFA_DISPATCH(q->shape[3], dtype, (launch_split<KD, KB>(mq, mk, mv, mdo, nullptr, &p, s)));
 }
 
 }  // extern "C"
