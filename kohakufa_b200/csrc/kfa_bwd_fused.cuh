@@ -618,43 +618,47 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
 }
 
-// dq = 16-bit(scale * accumulator), or NaN if the status word says that a kernel gave up: one CTA per (128-query tile, batch x head); the accumulator tile is
-// [D / 4][128 rows][4] floats (see above), so a warp reads 512 contiguous bytes per load.
+// dq = 16-bit(scale * accumulator), or NaN if the status word says that a kernel gave up: one CTA per (128-query tile, batch x
+// head); the accumulator tile is [D / 4][128 rows][4] floats (see above), so a warp reads 512 contiguous bytes per load. A warp
+// has 32 rows of half the columns: all its loads go ahead, the status word's among them, and the rows leave through shared
+// memory (as in store_rows16). Bound by memory where it is large, by the two round trips where it is small. Rows stored by
+// threads, behind the status word's round trip, -> now, us: 384 heads x 201, D = 64, 8.8 -> 6.1; 64 x 4096 15.7 -> 13.8 (101 MB: 7.3
+// TB/s, partly from L2); 128 x 8192 70.5 -> 61.6; 16 x 4100 5.7 -> 4.5; 32 x 8192, D = 128, 65.0 -> 38.6.
 template <int D, bool BF16>
 __global__ void __launch_bounds__(256) kfa_bwd_dq_convert_kernel(const float* __restrict__ dq_acc, void* dq,
                                                                  long long dq_sb, long long dq_sh, long long dq_ss,
                                                                  int H, int Sq, int cols, float scale, const int* status) {
+  constexpr int P = D / 16;                             // 16-byte pieces of a row's half
+  constexpr int G = P % 8 == 0 ? 8 : 4;                 // (P = 4 or 8)
+  __shared__ uint4 stage[8][32 * P];
   const int tile = blockIdx.x, bh = blockIdx.y;
   const int b = bh / H, h = bh % H;
-  const int r_in = threadIdx.x & 127, half = threadIdx.x >> 7;
-  const int row = tile * 128 + r_in;
-  if (row >= Sq) return;
-  const float* src = dq_acc + static_cast<long long>(bh) * dq_acc_head_floats(Sq, D) +
-                     static_cast<long long>(tile) * (128 * D) + r_in * 4;
-  uint8_t* drow = reinterpret_cast<uint8_t*>(dq) + 2 * (b * dq_sb + h * dq_sh + static_cast<long long>(row) * dq_ss);
-  if (*status != 0) {  // a kernel before this one gave up: the accumulator is incomplete
-    for (int c8 = half * (D / 16); c8 < min((half + 1) * (D / 16), cols / 8); ++c8)
-      *reinterpret_cast<uint4*>(drow + 16 * c8) = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
-    return;
-  }
-  auto piece = [&](int c8) {
-    const float4 a = *reinterpret_cast<const float4*>(src + (2 * c8) * 512);
-    const float4 c = *reinterpret_cast<const float4*>(src + (2 * c8 + 1) * 512);
-    uint4 w;
-    w.x = pack16<BF16>(a.x * scale, a.y * scale);
-    w.y = pack16<BF16>(a.z * scale, a.w * scale);
-    w.z = pack16<BF16>(c.x * scale, c.y * scale);
-    w.w = pack16<BF16>(c.z * scale, c.w * scale);
-    *reinterpret_cast<uint4*>(drow + 16 * c8) = w;
-  };
-  // Two loops, so that all loads of a full row's half go ahead of its stores: with the end at `cols` in the first every piece
-  // waited for its loads, and large accumulators took 1.8 times as long (128 x 4096 rows, D = 64, 201 MB: 38 -> 66 us, now 37;
-  // 74 x 8192, D = 64: 49, 89, 47).
-  if (cols == D) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half = warp >> 2;
+  const int row0 = tile * 128 + 32 * (warp & 3);
+  if (row0 >= Sq) return;  // (rows past Sq in the last warp: zeros of the accumulator's whole tile)
+  const float4* src = reinterpret_cast<const float4*>(dq_acc + static_cast<long long>(bh) * dq_acc_head_floats(Sq, D) +
+                                                      static_cast<long long>(tile) * (128 * D)) +
+                      half * (2 * P * 128) + 32 * (warp & 3) + lane;
+  const int gave_up = load_status(status);
+  float4 v[2 * P];
 #pragma unroll
-    for (int c8 = half * (D / 16); c8 < (half + 1) * (D / 16); ++c8) piece(c8);
-  } else {
-    for (int c8 = half * (D / 16); c8 < min((half + 1) * (D / 16), cols / 8); ++c8) piece(c8);
+  for (int i = 0; i < 2 * P; ++i) v[i] = src[i * 128];
+  uint4* mine = stage[warp];
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    const float4 a = v[2 * i], c = v[2 * i + 1];
+    uint4 w = make_uint4(pack16<BF16>(a.x * scale, a.y * scale), pack16<BF16>(a.z * scale, a.w * scale),
+                         pack16<BF16>(c.x * scale, c.y * scale), pack16<BF16>(c.z * scale, c.w * scale));
+    if (gave_up != 0) w = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);  // the accumulator is incomplete
+    mine[lane * P + (i ^ ((lane / (8 / G)) & (G - 1)))] = w;
+  }
+  __syncwarp();
+  uint8_t* drow = reinterpret_cast<uint8_t*>(dq) + 2 * (b * dq_sb + h * dq_sh + static_cast<long long>(row0) * dq_ss);
+#pragma unroll
+  for (int it = 0; it < P; ++it) {
+    const int n = it * 32 + lane, r = n / P, c = n % P, c8 = half * P + c;
+    const uint4 w = mine[r * P + (c ^ ((r / (8 / G)) & (G - 1)))];
+    if (row0 + r < Sq && 8 * c8 < cols) *reinterpret_cast<uint4*>(drow + 2 * r * dq_ss + 16 * c8) = w;
   }
 }
 
