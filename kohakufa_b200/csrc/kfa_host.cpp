@@ -501,9 +501,15 @@ Three registered(const char* name, const T&... args) {
   return c10::Dispatcher::singleton().findSchemaOrThrow(name, "").template typed<Three(T...)>().call(args...);
 }
 
-at::Tensor usable(const at::Tensor& g) { return strides_ok(g) ? g : g.contiguous(); }  // e.g. an expanded gradient
+// e.g. an expanded gradient; while a compiler traces with symbolic sizes there are no strides to look at
+at::Tensor usable(const at::Tensor& g) {
+  return !g.unsafeGetTensorImpl()->has_symbolic_sizes_strides() && strides_ok(g) ? g : g.contiguous();
+}
 
+// The nodes are traceable (is_traceable): compiled autograd then puts the registered op, which is what a backward takes under
+// its dispatch modes, into its graph, where it would otherwise break the graph at the node (an error with fullgraph=True).
 struct Attention : torch::autograd::Function<Attention> {
+  static constexpr bool is_traceable = true;
   static at::Tensor forward(AutogradContext* ctx, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const Call& c) {
     auto [out, lse] = released([&] { return run_forward(q, k, v, static_cast<float>(c.scale), static_cast<int>(c.block), c.status); });
     keep(ctx, c, {q, k, v, out, lse});
@@ -526,6 +532,7 @@ struct Attention : torch::autograd::Function<Attention> {
 };
 
 struct MaskedAttention : torch::autograd::Function<MaskedAttention> {
+  static constexpr bool is_traceable = true;
   static at::Tensor forward(AutogradContext* ctx, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
                             const std::array<at::Tensor, 3>& mask, const Call& c) {
     auto [out, lse] = released([&] { return run_forward_masked(q, k, v, mask[0], mask[2], static_cast<float>(c.scale), c.status); });
@@ -548,6 +555,7 @@ struct MaskedAttention : torch::autograd::Function<MaskedAttention> {
 };
 
 struct VarlenAttention : torch::autograd::Function<VarlenAttention> {
+  static constexpr bool is_traceable = true;
   static at::Tensor forward(AutogradContext* ctx, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
                             const std::array<at::Tensor, 2>& cu, const Call& c) {
     auto [out, lse] = released([&] {
