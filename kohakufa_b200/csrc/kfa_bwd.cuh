@@ -430,6 +430,7 @@ __device__ __forceinline__ void bwd_dkdv(const CUtensorMap& tmQ, const CUtensorM
   using Cfg = BwdCfg<D>;
   constexpr int CH = Cfg::CHUNKS;
   constexpr int NSL = Cfg::KV_SLOTS;
+  static_assert(NSL >= 2, "the producer looks at an earlier failure ahead of its first wait");
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -574,12 +575,12 @@ __device__ __forceinline__ void bwd_dkdv(const CUtensorMap& tmQ, const CUtensorM
       if (!use_list) walk.next(n_per);
       bool ok = true;
       for (int s = issued; s < n_steps && ok; ++s, walk.next(n_per)) {
+        if (s == 2 && earlier != 0) break;  // before the first wait: see the forward
         if (s >= NSL) ok = mbar_wait(bar(B_QFREE + s % NSL), (s / NSL - 1) & 1, ctl, 11);
         if (!ok) break;
         if (use_list) load_step(s, tile_of(s), head_of(s));
         else load_step(s, first_i + walk.rel, hk * p.group + walk.g);
         issued = s + 1;
-        if (s == 2 && earlier != 0) ok = false;
       }
       if (earlier != 0) *s_abort = 1;
       if (use_list && n_steps == 0) mbar_drain(bar(B_KV), 0);  // (nothing visible in a mask: nothing else waits for K and V)
@@ -925,6 +926,7 @@ __device__ __forceinline__ void bwd_dq(const CUtensorMap& tmQ, const CUtensorMap
   using Cfg = BwdCfg<D>;
   constexpr int CH = Cfg::CHUNKS;
   constexpr int NK = Cfg::NK, NV = Cfg::NV;
+  static_assert(NK >= 2 && NV >= 2, "the producer looks at an earlier failure ahead of its first wait");
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -1052,6 +1054,7 @@ __device__ __forceinline__ void bwd_dq(const CUtensorMap& tmQ, const CUtensorMap
     if (lane == 0) {
       bool ok = true;
       for (int j = issued_k; j < n_steps && ok; ++j) {
+        if (j == 2 && earlier != 0) break;  // before the first wait: see the forward
         if (j >= NK) ok = mbar_wait(bar(B_KFREE + j % NK), (j / NK - 1) & 1, ctl, 51);
         if (!ok) break;
         load_k(j, tile_of(j));
@@ -1060,7 +1063,6 @@ __device__ __forceinline__ void bwd_dq(const CUtensorMap& tmQ, const CUtensorMap
         if (!ok) break;
         load_v(j, tile_of(j));
         issued_v = j + 1;
-        if (j == 2 && earlier != 0) ok = false;
       }
       if (earlier != 0) *s_abort = 1;
     }

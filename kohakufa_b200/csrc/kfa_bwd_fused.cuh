@@ -152,6 +152,7 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   using Cfg = FusedCfg<D>;
   constexpr int CH = Cfg::CHUNKS;
   constexpr int NQ = Cfg::NQ, NDO = Cfg::NDO;
+  static_assert(NQ >= 2, "the producer looks at an earlier failure ahead of its first wait");
   constexpr int TB = Cfg::TILE_BYTES;
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -297,11 +298,11 @@ kfa_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       StepWalk walk;
       walk.next(n_per);
       for (int s = 1; s < n_steps && ok; ++s, walk.next(n_per)) {
+        if (s == 2 && earlier != 0) break;  // before the first wait: see the forward
         if (s >= NQ) ok = mbar_wait(bar(B_QFREE + s % NQ), (s / NQ - 1) & 1, ctl, 31);
         if (!ok) break;
         load_q(s, tile_at(walk), hk * p.group + walk.g);
         issued = s + 1;
-        if (s == 2 && earlier != 0) ok = false;
       }
     }
     if (lane == 0 && earlier != 0) *s_abort = 1;

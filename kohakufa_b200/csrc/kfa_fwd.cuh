@@ -226,6 +226,7 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   using Cfg = FwdCfg<D>;
   constexpr int CH = Cfg::CHUNKS;
   constexpr int NS = Cfg::STAGES;
+  static_assert(NS >= 3, "the producer looks at an earlier failure ahead of its first wait");
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -300,8 +301,9 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 
   // ---- setup ----
   // The thread that starts the copies sets up the barriers and starts the first ones at once: they fly while tensor memory
-  // is allocated and the roles find their places. It also looks at the status word, once those copies are on their way: an
-  // earlier failure aborts the CTA like one of its own waits. (Copies after the CTA's first barrier, behind the status word's
+  // is allocated and the roles find their places. It also looks at the status word, once those copies are on their way and
+  // before it waits for anything: an earlier failure aborts the CTA like one of its own waits, without the time that such a wait
+  // may take (a grid whose waits run out holds the GPU for one limit, not for one limit a wave). (Copies after the CTA's first barrier, behind the status word's
   // round trip, and the epilogue a row per thread, against now: forward 32 x 12 x 201 rows, D = 64, 28.9 -> 25.4 us, 4 x 8 x
   // 4096 x 77 keys, D = 48, 31.2 -> 26.2; 32 heads x 4096 causal, D = 128, 136 -> 133.)
   const int h_kv = static_cast<int>(p.by_group.div(h));
