@@ -103,8 +103,8 @@ def attention(
     if compute_dtype not in COMPUTE_DTYPES:
         raise TypeError(f"compute_dtype {compute_dtype}: one of {COMPUTE_DTYPES}")
     result_dtype, head_dim = q.dtype, q.shape[-1]
-    if mask is None and not center_keys and q.dtype == k.dtype == v.dtype == compute_dtype:
-        # most calls: nothing to cast, widen or pack
+    if mask is None and not center_keys and not head_dim % 16 and q.dtype == k.dtype == v.dtype == compute_dtype:
+        # most calls: nothing to cast, widen or pack (other head dims are refused there, and looked at twice for nothing)
         out = _op.direct(q, k, v, head_dim**-0.5 if scale is None else scale, frame)
         if out is not None:
             return out

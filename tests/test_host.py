@@ -108,6 +108,16 @@ def test_narrow_rows_where_they_pay():
         assert not op.narrow_backward_pays(*case), case
 
 
+@pytest.mark.parametrize("dim,asked", [(8, 0), (40, 0), (20, 0), (16, 1), (64, 1), (128, 1)])
+def test_only_head_dims_of_the_kernels_ask_for_the_direct_call(monkeypatch, dim, asked):
+    calls = []
+    monkeypatch.setattr(op, "direct", lambda *args: calls.append(args))
+    q, k, v = (torch.zeros(1, 2, 8, dim, dtype=torch.float16) for _ in range(3))
+    with pytest.raises(ValueError, match="CUDA tensors only"):
+        api.attention(q, k, v)
+    assert len(calls) == asked
+
+
 def test_causal_and_block_causal_are_exclusive():
     q, k, v = qkv()
     with pytest.raises(ValueError, match="causal is block_causal=1"):
