@@ -186,7 +186,7 @@ def direct(q: Tensor, k: Tensor, v: Tensor, scale: float, block: int) -> Tensor 
     if not _lib.plain_eager(q, k, v):
         return None
     word = _lib._status.get(q.get_device())
-    return None if word is None else _lib.host().call(q, k, v, scale, block, word)
+    return None if word is None else _lib.host().call(q, k, v, float(scale), block, word)
 
 
 def _bshd_like(t: Tensor) -> Tensor:

@@ -118,6 +118,22 @@ def test_only_head_dims_of_the_kernels_ask_for_the_direct_call(monkeypatch, dim,
     assert len(calls) == asked
 
 
+def test_the_direct_call_takes_a_scale_as_float_does(monkeypatch):
+    """As the other ways through ``attention`` do: whatever ``float()`` makes a number of."""
+    scales = []
+
+    class Host:
+        def call(self, q, k, v, scale, block, word):
+            scales.append(scale)
+
+    monkeypatch.setattr(_lib, "plain_eager", lambda *tensors: True)
+    monkeypatch.setattr(_lib, "host", Host)
+    monkeypatch.setattr(_lib, "_status", {-1: torch.zeros(1, dtype=torch.int32)})
+    for scale in (0.25, 1, "0.25", torch.tensor(0.25)):
+        op.direct(*qkv(), scale, 0)
+    assert scales == [0.25, 1.0, 0.25, 0.25] and all(type(s) is float for s in scales)
+
+
 def test_causal_and_block_causal_are_exclusive():
     q, k, v = qkv()
     with pytest.raises(ValueError, match="causal is block_causal=1"):
