@@ -36,7 +36,7 @@ enum : int {
 #define KFA_DRAIN_CYCLES 4000000000ll
 
 // Division by a number the host knows (Granlund and Montgomery, "Division by invariant integers using multiplication", 1994,
-// figure 4.1): four instructions for any 32-bit dividend. A division by a run-time value takes some 150 clk, and a CTA's first
+// figure 4.1): five operations for any 32-bit dividend. A division by a run-time value takes some 150 clk, and a CTA's first
 // copy waited for half a dozen of them one after the other.
 struct FastDiv {
   uint32_t d, mul, sh1, sh2;
