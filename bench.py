@@ -352,7 +352,7 @@ def main():
         stop.record()
         barrier()
         # per-kernel device times, same workload, still inside the sampled region
-        kernel_ms = time_kernels(cfg, q, k, v, dout, args.steps, not fused)
+        kernel_ms = time_kernels(cfg, q, k, v, dout, args.steps, not fused, ring_mode)
         # a short timed region can end before nvidia-smi's next sample: keep the same load running
         # (untimed) until three samples under load exist, for at most 1.5 s
         t_extra = time.perf_counter()
@@ -392,10 +392,11 @@ def main():
         return
 
     peaks, peak_kind = measured_peaks()
-    # matmuls of the algorithmic count (2 forward + 5 backward) each kernel delivers; the split dQ kernel's
-    # S and dP are recomputation and count for nothing
-    units = {"fwd": 2, "fused": 5, "dkdv": 4, "dq": 1}
-    names = {"fwd": "kfa_fwd_kernel", "fused": "kfa_bwd_fused_kernel", "dkdv": "kfa_bwd_split_kernel (dK / dV alone)", "dq": "kfa_bwd_split_kernel (dQ alone)"}
+    # matmuls of the algorithmic count (2 forward + 5 backward) each kernel delivers; the S and dP of the split
+    # kernel's dQ CTAs are recomputation and count for nothing. (Steps of the ring launch its two kinds of CTA apart.)
+    units = {"fwd": 2, "fused": 5, "split": 5, "dkdv": 4, "dq": 1}
+    names = {"fwd": "kfa_fwd_kernel", "fused": "kfa_bwd_fused_kernel", "split": "kfa_bwd_split_kernel",
+             "dkdv": "kfa_bwd_split_kernel (dK / dV alone)", "dq": "kfa_bwd_split_kernel (dQ alone)"}  # fmt: skip
     dominant = max((n for n in units if n in kernel_ms), key=lambda n: kernel_ms[n])
     # the kernels were timed on this rank's local tensors (the whole problem unless ring mode)
     local_rows = cfg.seq // world if ring_mode else cfg.seq
@@ -459,12 +460,11 @@ def main():
 # small case of the configuration's shape: (kernel, S, D, block) -> (bytes, (batch, head) pairs of the
 # captured launch). A launch's traffic grows in proportion to the pairs, so a full launch is scaled by them.
 NCU_DRAM_BYTES = {
-    ("dkdv", 8192, 128, 1): (173.8e6, 16),
-    ("dq", 8192, 128, 1): (157.1e6, 16),
-    ("fwd", 8192, 128, 1): (114.8e6, 16),
-    ("fused", 8192, 128, 1): (299.9e6, 16),
-    ("fused", 4096, 64, 256): (294.7e6, 64),
-    ("fwd", 4096, 64, 256): (118.5e6, 64),
+    ("split", 8192, 128, 1): (354.2e6, 16),
+    ("fwd", 8192, 128, 1): (116.4e6, 16),
+    ("fused", 8192, 128, 1): (309.9e6, 16),
+    ("fused", 4096, 64, 256): (294.8e6, 64),
+    ("fwd", 4096, 64, 256): (118.1e6, 64),
 }
 
 
@@ -494,8 +494,9 @@ def bind_to_gpu_cpus(index):
         return {"bound_to": None, "note": f"affinity not set: {type(exc).__name__}"}
 
 
-def time_kernels(cfg, q, k, v, dout, reps, deterministic=False):
-    """Average device time of each kernel of one step, CUDA events on the launching stream."""
+def time_kernels(cfg, q, k, v, dout, reps, deterministic=False, apart=False):
+    """Average device time of each kernel of one step, CUDA events on the launching stream. ``split`` is the split backward
+    less its statistics kernel; ``apart``: its two kinds of CTA in launches of their own instead, as the ring has them."""
     import ctypes
 
     from kohakufa_b200 import _lib
@@ -516,9 +517,16 @@ def time_kernels(cfg, q, k, v, dout, reps, deterministic=False):
     if deterministic:
         calls |= {
             "prepare": lambda: lib.kfa_bwd_prepare(T["out"], T["dout"], lse.data_ptr(), stats.data_ptr(), code, stream),
-            "dkdv": lambda: lib.kfa_bwd_dkdv(T["q"], T["k"], T["v"], T["dout"], stats.data_ptr(), T["dk"], T["dv"], scale, block, code, word, stream),
-            "dq": lambda: lib.kfa_bwd_dq(T["q"], T["k"], T["v"], T["dout"], stats.data_ptr(), T["dq"], scale, block, code, word, stream),
         }
+        if apart:
+            calls |= {
+                "dkdv": lambda: lib.kfa_bwd_dkdv(T["q"], T["k"], T["v"], T["dout"], stats.data_ptr(), T["dk"], T["dv"], scale, block, code, word, stream),
+                "dq": lambda: lib.kfa_bwd_dq(T["q"], T["k"], T["v"], T["dout"], stats.data_ptr(), T["dq"], scale, block, code, word, stream),
+            }
+        else:
+            calls["split"] = lambda: lib.kfa_bwd(
+                T["q"], T["k"], T["v"], T["out"], T["dout"], lse.data_ptr(), stats.data_ptr(), T["dq"], T["dk"], T["dv"], scale, block, code, word, stream
+            )
     else:
         acc = q.new_empty(lib.kfa_bwd_dq_acc_bytes(*q.shape) // 4, dtype=torch.float32)
         calls |= {
@@ -536,7 +544,10 @@ def time_kernels(cfg, q, k, v, dout, reps, deterministic=False):
             b.record()
             events[name].append((a, b))
     torch.cuda.synchronize()
-    return {n: sum(a.elapsed_time(b) for a, b in ev) / len(ev) for n, ev in events.items()}
+    ms = {n: sum(a.elapsed_time(b) for a, b in ev) / len(ev) for n, ev in events.items()}
+    if "split" in ms:
+        ms["split"] -= ms["prepare"]
+    return ms
 
 
 def ring_record(rank, world, dev, barrier, steps=2):
