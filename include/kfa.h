@@ -19,8 +19,9 @@
  *     message (thread-local).
  *   - `dev_status` points to one int32 in device memory, zero before the first call. A kernel
  *     whose internal wait ran out of time writes a nonzero code there and finishes early
- *     instead of hanging; later launches that see a nonzero word do nothing. The host reads
- *     it whenever it wants to (tests do after every call).
+ *     instead of hanging, and fills the output rows it owns with NaN. Later launches that see a
+ *     nonzero word do part or all of their work, writes to accumulators and carries included, and
+ *     leave NaN in their outputs. The host reads the word whenever it wants to (tests do after every call).
  */
 #ifndef KFA_H_
 #define KFA_H_
@@ -218,7 +219,7 @@ int kfa_bwd_masked(const KfaTensor4* q, const KfaTensor4* k, const KfaTensor4* v
  * tensors it was given, a serving loop that may not touch cudaMalloc because it synchronises the
  * device, a process whose memory is fully pre-carved. For them the library keeps ONE statistics
  * buffer of KFA_STATIC_SCRATCH_BYTES inside its own device image (every GPU that loads libkfa.so
- * holds these bytes until the process exits) and this entry point runs the same three kernels on it.
+ * holds these bytes until the process exits) and this entry point runs kfa_bwd's two kernels on it.
  * It calls no cudaMalloc, cudaFree or other allocating routine.
  *
  *   - Limit: kfa_bwd_stats_bytes(B, H, Sq) <= KFA_STATIC_SCRATCH_BYTES, i.e. B * H * ceil(Sq / 128) <=

@@ -265,7 +265,7 @@ def check_status(device=None) -> None:
 
     The kernels never hang: a wait that exceeds its (seconds-long) limit makes the CTA fill the output
     rows it owns with NaN, record ``100 + wait id`` in a per-device status word and leave; every later
-    launch on that device then skips its work and leaves its outputs as NaN as well. Nothing on the
+    launch on that device may still do part or all of its work, but leaves its outputs as NaN as well. Nothing on the
     launch path reads the word back (that would synchronise), so call this where the program
     synchronises anyway, e.g. after ``loss.item()`` or the optimizer step: NaN gradients plus a nonzero
     status mean "a kernel timed out", not "the model diverged". Reads one int from the device."""

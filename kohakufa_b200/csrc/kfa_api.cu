@@ -143,11 +143,13 @@ long long packed_tiles(int n_seqs, int n_max, int rows, int tile) {
 // Whether the grid of a packed batch numbers the tiles that exist (decode_packed) or, as a rectangle, every sequence's up
 // to the tiles of the longest. A CTA of the rectangle that finds its sequence too short costs about 1 us of an SM, because
 // it needs all of its shared memory to start; a CTA of the other numbering first scans the lengths, 32 at a time, one
-// load's latency each. `scans`: how many of those an empty CTA costs as much as (measured: 8 in the forward, 6 in the
-// backward); how many tiles exist is estimated, the last tile of a sequence as half there. Rectangle -> numbering of the
-// tiles that exist, D = 64, 8 heads, causal, forward + backward, lengths spread evenly up to the longest, in us: 32 x 512 106
-// -> 98, 64 x 512 195 -> 183, 96 x 512 296 -> 282, 128 x 512 401 -> 398, 192 x 512 621 -> 649, 128 x 2048 1899 -> 1854, 128 x
-// 128 129 -> 139; 64 of 512 each 320 -> 326. One of 4096 rows among n of up to 64: n = 256 1689 -> 622, 1000 6234 -> 2626.
+// load's latency each. `scans`: how many of those an empty CTA costs as much as (8 in the forward, 6 in the backward, measured
+// when a CTA's start took longer and dK / dV and dQ were launches of their own); how many tiles exist is estimated, the last tile
+// of a sequence as half there. Rectangle, numbering of the tiles that exist and this rule (forward and backward choose apart),
+// D = 64, 8 heads, causal, forward + backward, lengths spread evenly up to the longest, in us: 32 x 512 117, 115, 117; 64 x 512
+// 186, 192, 192; 96 x 512 261, 275, 270; 128 x 512 341, 367, 341; 192 x 512 498, 560, 498; 128 x 2048 1840, 1860, 1856; 128 x 128
+// 121, 133, 121; 64 of 512 each 278, 295, 278. One of 4096 rows among n of up to 64: n = 256 1446, 604, 602; 1000 5264, 2529, 2527.
+// (The rule is up to 4 % on the slower side where the two are close.)
 bool number_compactly(int n_seqs, int n_max, int rows, int tile, int scans) {
   const long long all = static_cast<long long>(n_seqs) * n_max;
   const long long exist = std::min(all, static_cast<long long>(rows) / tile + (n_seqs + 1) / 2);
@@ -499,13 +501,19 @@ int launch_sum_splits(const kfa::SumParams& p, int bh, cudaStream_t s) {
 // less than half of the GPU: as many as it has SMs for, with at least 4 steps (of about 1.4 us) each, which pay for the
 // CTA's set-up and the sum of the parts. The order of the sums depends on this number, and so on batch and heads, which
 // is why self attention, whose dK and dV do not depend on what else is in the batch, is left alone.
-// against_fused: 1 also where the fused kernel takes no longer. It does five products for seven, so the dQ kernel's CTAs
-// (set-up and epilogue about two steps, spread over the GPU; nearly for nothing if they are one wave) have to take less than
-// the steps that a CTA is spared. Whole backward at D = 64, fused and shared out, in us (queries x keys, heads): 1024 x 77:
-// 8 heads 25 and 23, 20 heads 27 and 29, 74 heads 33 and 41; 2048 x 77: 37 heads 45 and 41, 49 heads 51 and 55; 4096 x 77:
-// 8 heads 64 and 29, 40 heads 86 and 81, 49 heads 96 and 99, 74 heads 114 and 141; 16384 x 77: 40 heads 321 and 290, 50 heads
-// 348 and 366; 4096 x 512: 16 heads 68 and 70, 64 query and 16 K / V heads 245 and 229; 8192 x 1024, 8 heads: 113 and 107.
-// (The line is on the faster side of all 100 shapes measured.)
+// against_fused: 1 also where the fused kernel took no longer. It does five products for seven, so the dQ kernel's CTAs
+// (set-up and epilogue about two steps, spread over the GPU; nearly for nothing if they are one wave) had to take less than
+// the steps that a CTA is spared.
+// Both lines were drawn when dK / dV and dQ were launches of their own. In one launch the dQ CTAs fill the SMs that few dK / dV
+// CTAs leave idle. Sharing out still gains where a key tile's CTA outlasts the dQ work of an SM; beyond that it costs up to 18 %,
+// and with one part the split kernels are faster than the fused one more often than the second line says.
+// Whole backward now, D = 64, in us, with one part, the rule's number of parts (n) and fused; queries x keys, heads:
+//   1024 x 77:   8 heads 17.4, 15.8 (2), 22.5;   20 heads 18.1, 16.1 (2), 23.6;    74 heads 28.9, 35.3 (2), 28.7
+//   2048 x 77:   20 heads 29.4, 22.1 (4), 37.6;  37 heads 30.1, 34.5 (4), 40.6;    49 heads 36.2, 43.4 (3), 44.4
+//   4096 x 77:   8 heads 49.4, 20.7 (8), 61.1;   32 heads 54.3, 52.9 (4), 72.9;    40 heads 57.9, 63.7 (3), 79.3;    74 heads 110, 119 (2), 102
+//   16384 x 77:  24 heads 198, 149 (6), 265;     40 heads 227, 238 (3), 306;       74 heads 417, 430 (2), 394
+//   4096 x 512:  8 heads 50.9, 37.2 (4), 59.3;   16 heads 52.3, 56.8 (2), 62.8;    64 query and 16 K / V heads 195, 200 (2), 236
+//   8192 x 1024: 8 heads 96.4, 90.9 (2), 111;    32 query and 8 K / V heads 379, 336 (2), 437
 // (148 SMs: what this library is built for.)
 int bwd_splits(const KfaTensor4* q, const KfaTensor4* k, bool against_fused = false) {
   for (int i = 0; i < 4; ++i)

@@ -41,9 +41,7 @@ namespace kfa {
 // heavy tiles of the last heads: 4 % of the forward's time at 128 heads, 30 % at 16), while the CTAs that
 // run side by side still share the K / V (or Q / dO) of a few heads in L2.
 // Divisors from the host: with divisions by run-time values the first copy of a CTA started 1100 to 1500 clk after the CTA, of
-// 13000 for a forward of two key tiles. That, barriers set up by a lane each, the other copies behind the CTA's barrier and
-// no mask code for parts that a warp sees whole: forward 32 x 12 x 201 rows, D = 64, 25.3 -> 23.1 us, 4 x 8 x 4096 x 77 keys, D =
-// 48, 26.1 -> 22.9, 2 x 16 x 2048 causal, D = 96, 58.4 -> 53.6; fused backward of the first 46.8 -> 44.0.
+// 13000 for a forward of two key tiles. What that gave, with all else at a CTA's start, stands in the kernel.
 struct TileOrder {
   FastDiv per_group, last, heads;  // tiles of 8 pairs; pairs of the last group; heads of a batch entry
   uint32_t full;                   // groups of 8 pairs
@@ -303,9 +301,10 @@ kfa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   // The thread that starts the copies sets up the barriers and starts the first ones at once: they fly while tensor memory
   // is allocated and the roles find their places. It also looks at the status word, once those copies are on their way and
   // before it waits for anything: an earlier failure aborts the CTA like one of its own waits, without the time that such a wait
-  // may take (a grid whose waits run out holds the GPU for one limit, not for one limit a wave). (Copies after the CTA's first barrier, behind the status word's
-  // round trip, and the epilogue a row per thread, against now: forward 32 x 12 x 201 rows, D = 64, 28.9 -> 25.4 us, 4 x 8 x
-  // 4096 x 77 keys, D = 48, 31.2 -> 26.2; 32 heads x 4096 causal, D = 128, 136 -> 133.)
+  // may take (a grid whose waits run out holds the GPU for one limit, not for one limit a wave). Against copies after the CTA's first
+  // barrier, behind the status word's round trip, with divisions by run-time values on the way and an epilogue of a row per thread:
+  // forward 32 x 12 x 201 rows, D = 64, 28.9 -> 23.1 us, 4 x 8 x 4096 x 77 keys, D = 48, 31.2 -> 22.9, 2 x 16 x 2048 causal, D = 96,
+  // 59.9 -> 53.6, 32 heads x 4096 causal, D = 128, 136 -> 133; fused backward of the first 54.8 -> 44.0.
   const int h_kv = static_cast<int>(p.by_group.div(h));
   auto load_kv = [&](int idx, int j) {  // K_j (even idx) or V_j into its stage of the ring
     mbar_expect_tx(bar(B_KVREADY + idx % NS), Cfg::TILE_BYTES);

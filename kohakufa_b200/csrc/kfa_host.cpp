@@ -1,8 +1,8 @@
 // The launch path of a call, in C++: argument checks, output and scratch allocation, tensor descriptors and the
 // libkfa call itself, for the torch ops of op.py and mask.py. In Python (a dozen ctypes structures, half a dozen
 // allocations, the dispatch of a Python custom op) a small problem's call took several times its kernels: a forward
-// of 1 x 8 heads x 64 rows 67 us, now 10.5; forward + backward of 2 x 4 heads x 512 rows 286 us, now 93, of which about 45
-// are the autograd engine's own (a step through one view takes 35); with a boolean mask of 2048 x 2048 395 us, now 121.
+// of 1 x 8 heads x 64 rows 67 us, now 10; forward + backward of 2 x 4 heads x 512 rows 286 us, now 90, of which about 45
+// are the autograd engine's own (a step through one view takes 35); with a boolean mask of 2048 x 2048 395 us, now 110.
 //
 // A plain CPython extension module (`_kfa_host`), for the torch and the Python it was built with only: the build leaves
 // their names in it, and _lib.host() does not load it under others. It holds no state but the addresses of the libkfa
@@ -423,7 +423,7 @@ PyObject* py_backward_varlen(Args a, Py_ssize_t n) {
 
 // ---------------------------------------------------------------------------------------------------------------------
 // Calls that autograd records. The nodes are C++ ones: a torch.autograd.Function in Python took another 30 to 40 us a
-// step, on a thread of the engine that has to wait for the GIL (forward + backward of 2 x 4 x 512 rows: 122 -> 93 us with call() below).
+// step, on a thread of the engine that has to wait for the GIL (forward + backward of 2 x 4 x 512 rows: 118 -> 90 us with call() below).
 // Saved tensors go through torch's own SavedVariable (hooks, version checks, release).
 // ---------------------------------------------------------------------------------------------------------------------
 using torch::autograd::AutogradContext;

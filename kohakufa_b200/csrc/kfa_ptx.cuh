@@ -134,10 +134,11 @@ struct Ctl {
 // Bounded wait for the phase with the given parity to complete. Returns false when the CTA is aborting (this wait or another
 // ran out of time). The first test stands apart from the polling loop: a wait whose phase has already completed (most of them,
 // in a pipeline that runs ahead) costs one try_wait and, for a warp, one vote. The loop is inlined at some thirty places of a
-// kernel and lies between their hot instructions, so it holds as little as it can: looking at the status word of other CTAs
-// as well, every so many turns, and reporting from here made the kernels 6 to 7 KB longer, and the fused backward at D = 64
-// wait that much longer for instructions (video: 64 heads x 4096, frames of 256: 459 -> 446 us, 32 x 12 x 201 dense: 54.8 ->
-// 53.4; forward there 29.5 -> 28.8).
+// kernel and lies between their hot instructions, so it holds as little as it can. It does not look at the failures of other CTAs:
+// a CTA that is already waiting goes on to its own limit, a CTA that starts later sees the failure before its first wait (see the
+// forward), so that a failing grid ends within about one limit of its first failure. (A look at the status word every so many turns, and reporting from
+// here, made the kernels 6 to 7 KB longer and the fused backward at D = 64 wait that much longer for instructions: 64 heads x 4096,
+// frames of 256, 446 -> 459 us, 32 x 12 x 201 dense 53.4 -> 54.8.)
 __device__ __forceinline__ bool mbar_wait_poll(uint32_t bar, uint32_t parity, volatile int* s_abort, int site) {
   const long long t0 = clock64();
 #pragma unroll 1

@@ -144,9 +144,9 @@ def _records(q: Tensor, k: Tensor, v: Tensor) -> bool:
 # Rows of an odd multiple of 16 bytes do not begin on 32-byte sectors, so a row of a tile's copy touches a sector more than
 # a widened one. Above 64 columns the backward's kernels wait for that, on every pair of tiles, while widening costs by the
 # row: from so many visible pairs per row copied on, it is the faster way there. (The forward is always faster narrow.)
-# Forward + backward, widened time over narrow time: dim 72: 2 x 16 heads x 6144 1.05, 8 x 12288 0.98; dim 88: 8 x 12288 1.03, 4 x
-# 16384 1.00; dim 104: 2 x 16 x 2048 1.17, 16 x 3072 1.00, 2 x 16 x 6144 0.94, 4 x 16384 0.83; dim 120: 2 x 16 x 6144 1.13, 16 x 8192
-# 1.00, 8 x 12288 0.98, 16 query and 4 K / V heads x 8192 0.93. Up to dim 56: 1.02 to 1.05 at 4 x 16384, more below.
+# Forward + backward, widened time over narrow time: dim 72: 2 x 16 heads x 6144 1.06, 8 x 12288 0.99, 4 x 16384 0.95; dim 88: 2 x 16 x
+# 6144 1.10, 8 x 12288 1.04, 4 x 16384 1.00; dim 104: 2 x 16 x 2048 1.21, 16 x 3072 1.07, 2 x 16 x 6144 0.94, 4 x 16384 0.83; dim 120: 2 x
+# 16 x 6144 1.11, 16 x 8192 1.04, 8 x 12288 1.00, 16 query and 4 K / V heads x 8192 0.96. Up to dim 56: 1.01 to 1.07 at 4 x 16384.
 NARROW_REACH = {72: 4000, 88: 6000, 104: 1200, 120: 3000}
 
 
